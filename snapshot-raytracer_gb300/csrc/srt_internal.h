@@ -78,6 +78,10 @@ cudaError_t launch_pair_build(const float* src, float2* dst, const int64_t pn[3]
 cudaError_t launch_trace(int mode, const TraceArgs& a, cudaStream_t s, int64_t* kernels);
 // FP64 re-trace of the rays listed by a MIXED trace (count read on the device).
 cudaError_t launch_refine(const TraceArgs& a, cudaStream_t s, int64_t* kernels);
+// The FP64 form of a small range, one warp per ray (srt_retrace.cu): launch_trace
+// takes it up to kWideFp64Rays rays.
+constexpr int64_t kWideFp64Rays = 14000;
+cudaError_t launch_wide_fp64(const TraceArgs& a, cudaStream_t s, int64_t* kernels);
 
 // Progressive reads of an HDF5 field (srt_io.cpp), for srt_fields_load_h5.
 // h5_field_open reads the header and checks the dataset as

@@ -297,6 +297,7 @@ SRT_HD void tricubic_pair(const Rows& rows, const CRW<float>& X, const CRW<float
 // ------------------------------------------------------------ cell lookup
 
 SRT_HD int wrap64(int64_t c, int n) {
+  if ((uint64_t)c < (uint64_t)n) return (int)c;  // inside the box: no 64-bit division
   int64_t r = c % n;
   if (r < 0) r += n;
   return (int)r;
@@ -324,44 +325,260 @@ SRT_HD int64_t cell_base_pair(const Geom& G, int cx, int cy, int cz) {
   return (int64_t)cx + G.px * (int64_t)cy + G.pxy2 * (int64_t)cz;
 }
 
-// FP64 / REF16 interpolation of one field at a double-precision position.
-// IT is the arithmetic type (double for FP64, float for REF16); in REF16 the
-// cell offset is float(x) - float(floor(x)) (snapshot-raytracer.cu:223-230).
-template <typename IT, typename TapT>
-SRT_HD void interp_std(const TapT* f, const Geom& G, double x, double y, double z, Tri<IT>& r) {
-  const double fx = floor(x), fy = floor(y), fz = floor(z);
-  const int64_t ix = (int64_t)fx, iy = (int64_t)fy, iz = (int64_t)fz;
-  IT tx, ty, tz;
-  if (sizeof(IT) == sizeof(float)) {
-    tx = (IT)((float)x - (float)ix);
-    ty = (IT)((float)y - (float)iy);
-    tz = (IT)((float)z - (float)iz);
-  } else {
-    tx = (IT)(x - fx);
-    ty = (IT)(y - fy);
-    tz = (IT)(z - fz);
-  }
-  CRW<IT> X, Y, Z;
-  cr_weights(tx, X);
-  cr_weights(ty, Y);
-  cr_weights(tz, Z);
+// REF16 interpolation of one field at a double-precision position: FP32, the
+// cell offset taken as float(x) - float(floor(x)) (snapshot-raytracer.cu:223-230).
+template <typename TapT>
+SRT_HD void interp_ref16(const TapT* f, const Geom& G, double x, double y, double z, Tri<float>& r) {
+  const int64_t ix = (int64_t)floor(x), iy = (int64_t)floor(y), iz = (int64_t)floor(z);
+  CRW<float> X, Y, Z;
+  cr_weights((float)x - (float)ix, X);
+  cr_weights((float)y - (float)iy, Y);
+  cr_weights((float)z - (float)iz, Z);
   const int64_t base = cell_base(G, wrap64(ix, G.n[0]), wrap64(iy, G.n[1]), wrap64(iz, G.n[2]));
-  tricubic<IT, TapT>(f, base, G.px, G.pxy, X, Y, Z, r);
+  tricubic<float, TapT>(f, base, G.px, G.pxy, X, Y, Z, r);
 }
 
-// --------------------------------------------- right-hand side, FP64 / REF16
+// --------------------------------------------------- fused chains (FP64, dd)
 
-// Square root of the state type R (double, or the double-float dd).
+// A running sum of products in the state type R of the FP64 form and of the
+// re-trace: double, one fused multiply-add per product; dd, the compensated
+// dot product of Ogita, Rump and Oishi ("Accurate sum and dot product", 2005).
+// The FP64 form writes its sums as chains rather than expressions so that the
+// one-lane and the warp-per-ray kernels round alike whatever the compiler
+// would contract.
+template <typename R>
+struct Chain;
+
+template <>
+struct Chain<double> {
+  double s;
+  SRT_HD Chain(double x = 0.0) : s(x) {}
+  SRT_HD void add(double w, double x) { s = fma(w, x, s); }
+  SRT_HD void add(double w, float x) { s = fma(w, (double)x, s); }
+  SRT_HD double value() const { return s; }
+};
+
+template <>
+struct Chain<dd> {
+  float s, c;
+  SRT_HD Chain() : s(0.f), c(0.f) {}
+  SRT_HD Chain(const dd& x) : s(x.hi), c(x.lo) {}
+  SRT_HD void add(const dd& w, float x) {  // += w * x
+    const float p = w.hi * x;
+    const float e = fmaf(w.hi, x, -p);
+    float t, q;
+    dd_two_sum(s, p, t, q);
+    s = t;
+    c += fmaf(w.lo, x, e + q);
+  }
+  SRT_HD void add(const dd& w, const dd& x) {  // += w * x
+    const float p = w.hi * x.hi;
+    const float e = fmaf(w.hi, x.hi, -p);
+    float t, q;
+    dd_two_sum(s, p, t, q);
+    s = t;
+    c += fmaf(w.hi, x.lo, fmaf(w.lo, x.hi, e + q));
+  }
+  SRT_HD dd value() const {
+    float h, l;
+    dd_fast_two_sum(s, c, h, l);
+    return dd(h, l);
+  }
+};
+
+// a b + c as one chain
+template <typename R>
+SRT_HD R fma_r(const R& a, const R& b, const R& c) {
+  Chain<R> s(c);
+  s.add(a, b);
+  return s.value();
+}
+
 SRT_HD double sqrt_r(double x) { return sqrt(x); }
 SRT_HD dd sqrt_r(const dd& x) { return dd_sqrt(x); }
 
+// ------------------------------------------------- right-hand side, FP64
+
+// cr_weights in Horner form, one fused operation per power.
+SRT_HD void cr_weights_fp64(double t, CRW<double>& c) {
+  const double a2 = fma(-1.5, t, 2.0);
+  c.w[0] = fma(fma(-0.5, t, 1.0), t, -0.5) * t;
+  c.w[1] = fma(fma(1.5, t, -2.5) * t, t, 1.0);
+  c.w[2] = fma(a2, t, 0.5) * t;
+  c.w[3] = fma(0.5, t, -0.5) * t * t;
+  c.g[0] = fma(a2, t, -0.5);
+  c.g[1] = fma(4.5, t, -5.0) * t;
+  c.g[2] = fma(fma(-4.5, t, 4.0), t, 0.5);
+  c.g[3] = fma(1.5, t, -1.0) * t;
+  c.h[0] = fma(-3.0, t, 2.0);
+  c.h[1] = fma(9.0, t, -5.0);
+  c.h[2] = fma(-9.0, t, 4.0);
+  c.h[3] = fma(3.0, t, -1.0);
+}
+
+// FP64 interpolation of one field: `tricubic` as fused chains.
+SRT_HD void interp_fp64(const float* __restrict__ f, const Geom& G, double x, double y, double z, Tri<double>& r) {
+  const double fx = floor(x), fy = floor(y), fz = floor(z);
+  CRW<double> X, Y, Z;
+  cr_weights_fp64(x - fx, X);
+  cr_weights_fp64(y - fy, Y);
+  cr_weights_fp64(z - fz, Z);
+  const int64_t base =
+      cell_base(G, wrap64((int64_t)fx, G.n[0]), wrap64((int64_t)fy, G.n[1]), wrap64((int64_t)fz, G.n[2]));
+  double v = 0, g0 = 0, g1 = 0, g2 = 0, h00 = 0, h01 = 0, h02 = 0, h11 = 0, h12 = 0, h22 = 0;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    double a = 0, ay = 0, ayy = 0, ax = 0, axy = 0, axx = 0;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const float* row = f + base + c * G.pxy + b * G.px;
+      Chain<double> rv, rx, rxx;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const double p = (double)ldg(row + i);
+        rv.add(X.w[i], p);
+        rx.add(X.g[i], p);
+        rxx.add(X.h[i], p);
+      }
+      a = fma(Y.w[b], rv.s, a);
+      ay = fma(Y.g[b], rv.s, ay);
+      ayy = fma(Y.h[b], rv.s, ayy);
+      ax = fma(Y.w[b], rx.s, ax);
+      axy = fma(Y.g[b], rx.s, axy);
+      axx = fma(Y.w[b], rxx.s, axx);
+    }
+    v = fma(Z.w[c], a, v);
+    g0 = fma(Z.w[c], ax, g0);
+    g1 = fma(Z.w[c], ay, g1);
+    g2 = fma(Z.g[c], a, g2);
+    h00 = fma(Z.w[c], axx, h00);
+    h01 = fma(Z.w[c], axy, h01);
+    h02 = fma(Z.g[c], ax, h02);
+    h11 = fma(Z.w[c], ayy, h11);
+    h12 = fma(Z.g[c], ay, h12);
+    h22 = fma(Z.h[c], a, h22);
+  }
+  r.v = v;
+  r.g[0] = g0;
+  r.g[1] = g1;
+  r.g[2] = g2;
+  r.h[0] = h00;
+  r.h[1] = h01;
+  r.h[2] = h02;
+  r.h[3] = h11;
+  r.h[4] = h12;
+  r.h[5] = h22;
+}
+
+SRT_HD double dot3(const double* a, double b0, double b1, double b2) {
+  Chain<double> c;
+  c.add(a[0], b0);
+  c.add(a[1], b1);
+  c.add(a[2], b2);
+  return c.s;
+}
+
+// What the B components contribute (snapshot-raytracer.cu:377-460), G the
+// matrix of B's gradients (row C = grad B_C) and H_C its Hessians: the values,
+// ngB = G^T n, Gn = G n, nlap = n . Laplacian B, S = sum_C n_C H_C and the
+// symmetrised K_ij = (H_i n)_j + (H_j n)_i, which give the tidal matrix
+// T = S - K / 2 and the e.n.grad B scalars e.(Gn + ngB) / 2.
+struct BSums64 {
+  double val[3], ngB[3], Gn[3], nlap, S[6], K[6];
+};
+
+template <int C>
+SRT_HD void add_b_fp64(const FieldPtrs& F, const Geom& G, const double* x, const double* n, BSums64& B) {
+  Tri<double> r;
+  interp_fp64(F.b[C], G, C == 0 ? x[0] - 0.5 : x[0], C == 1 ? x[1] - 0.5 : x[1], C == 2 ? x[2] - 0.5 : x[2], r);
+  B.val[C] = r.v;
+  for (int i = 0; i < 3; ++i) B.ngB[i] = fma(r.g[i], n[C], C == 0 ? 0.0 : B.ngB[i]);
+  B.Gn[C] = dot3(r.g, n[0], n[1], n[2]);
+  B.nlap = fma(n[C], r.h[0] + r.h[3] + r.h[5], C == 0 ? 0.0 : B.nlap);
+  for (int u = 0; u < 6; ++u) B.S[u] = fma(r.h[u], n[C], C == 0 ? 0.0 : B.S[u]);
+  const int kIdx[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+  for (int i = 0; i < 3; ++i) {  // row C, column i of the three H_C n
+    const double row[3] = {r.h[kIdx[i][0]], r.h[kIdx[i][1]], r.h[kIdx[i][2]]};
+    const double Hn = dot3(row, n[0], n[1], n[2]);
+    double& k = B.K[kIdx[C][i]];  // met at component min(i, C) first, max(i, C) second
+    k = i == C ? Hn + Hn : (i > C ? Hn : k + Hn);
+  }
+}
+
+// 19-component right-hand side of the FP64 form. State: 0-2 x, 3-5 n, 6-8 e1,
+// 9-11 e2, 12 dA, 13 dA', 14-15 sigma1/2, 16-17 ellipticity1/2, 18 rotation
+// (snapshot-raytracer.cu:317-335, :338-509). The warp-per-ray kernels
+// (srt_wide.cuh) form the same values by the same operations.
+SRT_HD void rhs_fp64(const double* y, double* dy, const FieldPtrs& F, const Geom& G) {
+  double u[3][3];  // n, e1, e2
+  for (int v = 0; v < 3; ++v) {
+    const double* c = y + 3 + 3 * v;
+    const double r = sqrt(dot3(c, c[0], c[1], c[2]));
+    for (int i = 0; i < 3; ++i) u[v][i] = c[i] / r;
+  }
+  const double *n = u[0], *a = u[1], *b = u[2];
+  BSums64 B;
+  add_b_fp64<0>(F, G, y, n, B);
+  add_b_fp64<1>(F, G, y, n, B);
+  add_b_fp64<2>(F, G, y, n, B);
+  Tri<double> p;
+  interp_fp64(F.phi, G, y[0], y[1], y[2], p);
+  const double dA = y[12], dAp = y[13], s1 = y[14], s2 = y[15], el1 = y[16], el2 = y[17];
+  const double phi1 = fma(2.0, p.v, 1.0);
+  double v[3], w[3];
+  for (int i = 0; i < 3; ++i) {
+    dy[i] = fma(n[i], -phi1, -B.val[i]);
+    v[i] = fma(2.0, p.g[i], B.ngB[i]);
+    // 2 e.grad phi + e.n.grad B = e.w
+    w[i] = fma(0.5, B.Gn[i] + B.ngB[i], 2.0 * p.g[i]);
+  }
+  const double nv = dot3(n, v[0], v[1], v[2]), aw = dot3(a, w[0], w[1], w[2]), bw = dot3(b, w[0], w[1], w[2]);
+  for (int i = 0; i < 3; ++i) {
+    dy[3 + i] = fma(n[i], -nv, v[i]);  // v - n (n.v)
+    dy[6 + i] = n[i] * -aw;
+    dy[9 + i] = n[i] * -bw;
+  }
+  // 4 L, L = n.grad phi + n.(n.grad B) / 4
+  const double L4 = fma(4.0, dot3(p.g, n[0], n[1], n[2]), dot3(n, B.ngB[0], B.ngB[1], B.ngB[2]));
+  double Hn[3], He[3][3], Ha[3], Hb[3];
+  const int kIdx[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+  for (int i = 0; i < 3; ++i) {
+    const double row[3] = {p.h[kIdx[i][0]], p.h[kIdx[i][1]], p.h[kIdx[i][2]]};
+    Hn[i] = dot3(row, n[0], n[1], n[2]);
+    // effective tidal matrix Hess phi + T / 2
+    for (int j = 0; j < 3; ++j) He[i][j] = fma(-0.25, B.K[kIdx[i][j]], fma(0.5, B.S[kIdx[i][j]], row[j]));
+  }
+  for (int i = 0; i < 3; ++i) {
+    Ha[i] = dot3(He[i], a[0], a[1], a[2]);
+    Hb[i] = dot3(He[i], b[0], b[1], b[2]);
+  }
+  // -P_perp:Hess phi + n.Laplacian B / 2, P_perp:H = n^T H n - tr H
+  const double PHq = fma(0.5, B.nlap, (p.h[0] + p.h[3] + p.h[5]) - dot3(n, Hn[0], Hn[1], Hn[2]));
+  const double S1 = dot3(a, Ha[0], Ha[1], Ha[2]) - dot3(b, Hb[0], Hb[1], Hb[2]);
+  const double S2 = 2.0 * dot3(a, Hb[0], Hb[1], Hb[2]);
+  const double dA2 = dA * dA;
+  // the dA > 1/2 branch's terms, formed either way and selected (where dA = 0
+  // they are not finite and not selected)
+  const bool on = dA > 0.5;
+  const double q = sqrt(fma(el2, el2, fma(el1, el1, 4.0)));
+  const double quo0 = fma(s2, s2, s1 * s1) / (dA2 * dA), quo1 = s1 * q / dA2, quo2 = s2 * q / dA2;
+  const double quo3 = fma(s2, el1, s1 * -el2) / (dA2 * (q + 2.0));
+  dy[12] = -dAp;
+  dy[13] = fma(dA, PHq, fma(L4, -dAp, on ? quo0 : 0.0));
+  dy[14] = fma(S1, dA2, L4 * s1);
+  dy[15] = fma(S2, dA2, L4 * s2);
+  dy[16] = on ? -2.0 * quo1 : 0.0;
+  dy[17] = on ? -2.0 * quo2 : 0.0;
+  dy[18] = on ? quo3 : 0.0;
+}
+
+// ------------------------------------------------- right-hand side, REF16
+
 // Unit vectors n, e1, e2 of the full state y (snapshot-raytracer.cu:338-349).
-// R: the state's real type (double; dd in the re-trace of flagged rays).
-template <typename R>
-SRT_HD void rhs_frame(const R* y, R* n, R* a, R* b) {
-  const R rn = sqrt_r(y[3] * y[3] + y[4] * y[4] + y[5] * y[5]);
-  const R ra = sqrt_r(y[6] * y[6] + y[7] * y[7] + y[8] * y[8]);
-  const R rb = sqrt_r(y[9] * y[9] + y[10] * y[10] + y[11] * y[11]);
+SRT_HD void rhs_frame(const double* y, double* n, double* a, double* b) {
+  const double rn = sqrt(y[3] * y[3] + y[4] * y[4] + y[5] * y[5]);
+  const double ra = sqrt(y[6] * y[6] + y[7] * y[7] + y[8] * y[8]);
+  const double rb = sqrt(y[9] * y[9] + y[10] * y[10] + y[11] * y[11]);
   for (int i = 0; i < 3; ++i) {
     n[i] = y[3 + i] / rn;
     a[i] = y[6 + i] / ra;
@@ -373,7 +590,7 @@ SRT_HD void rhs_frame(const R* y, R* n, R* a, R* b) {
 // n.grad B, the e.n.grad B scalars, the tidal matrix and n . Laplacian B.
 // The e_i.grad B vectors the reference also forms there are never used and
 // are not computed.
-template <typename IT, typename R = double>
+template <typename IT>
 struct BSums {
   IT val[3], ngB[3], e1ngB, e2ngB, nlap;
   IT T[6];  // xx, xy, xz, yy, yz, zz
@@ -383,24 +600,24 @@ struct BSums {
     for (int i = 0; i < 6; ++i) T[i] = 0;
   }
   // Adds component c's value, gradient and Hessian r.
-  SRT_HD void add(int c, const Tri<IT>& r, const R* n, const R* a, const R* b) {
+  SRT_HD void add(int c, const Tri<IT>& r, const double* n, const double* a, const double* b) {
     val[c] = r.v;
     for (int i = 0; i < 3; ++i) ngB[i] = (IT)(ngB[i] + r.g[i] * n[c]);
-    const R gn = r.g[0] * n[0] + r.g[1] * n[1] + r.g[2] * n[2];
-    const R ga = r.g[0] * a[0] + r.g[1] * a[1] + r.g[2] * a[2];
-    const R gb = r.g[0] * b[0] + r.g[1] * b[1] + r.g[2] * b[2];
+    const double gn = r.g[0] * n[0] + r.g[1] * n[1] + r.g[2] * n[2];
+    const double ga = r.g[0] * a[0] + r.g[1] * a[1] + r.g[2] * a[2];
+    const double gb = r.g[0] * b[0] + r.g[1] * b[1] + r.g[2] * b[2];
     e1ngB = (IT)(e1ngB + 0.5 * a[c] * gn + 0.5 * n[c] * ga);
     e2ngB = (IT)(e2ngB + 0.5 * b[c] * gn + 0.5 * n[c] * gb);
     // H n for this component's Hessian (rows of the symmetric matrix)
-    const R Hn0 = r.h[0] * n[0] + r.h[1] * n[1] + r.h[2] * n[2];
-    const R Hn1 = r.h[1] * n[0] + r.h[3] * n[1] + r.h[4] * n[2];
-    const R Hn2 = r.h[2] * n[0] + r.h[4] * n[1] + r.h[5] * n[2];
-    const R Hn[3] = {Hn0, Hn1, Hn2};
+    const double Hn0 = r.h[0] * n[0] + r.h[1] * n[1] + r.h[2] * n[2];
+    const double Hn1 = r.h[1] * n[0] + r.h[3] * n[1] + r.h[4] * n[2];
+    const double Hn2 = r.h[2] * n[0] + r.h[4] * n[1] + r.h[5] * n[2];
+    const double Hn[3] = {Hn0, Hn1, Hn2};
     // T_ij += n_c H_ij - 1/2 (delta_ci (H n)_j + delta_cj (H n)_i)
     const int kIdx[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
     for (int i = 0; i < 3; ++i)
       for (int j = i; j < 3; ++j) {
-        R d = r.h[kIdx[i][j]] * n[c];
+        double d = r.h[kIdx[i][j]] * n[c];
         if (i == c) d -= 0.5 * Hn[j];
         if (j == c) d -= 0.5 * Hn[i];
         T[kIdx[i][j]] = (IT)(T[kIdx[i][j]] + d);
@@ -409,51 +626,42 @@ struct BSums {
   }
 };
 
-// The four quotients of the dA > 1/2 branch, each divided where it is formed
-// (the re-trace's lane groups share them out instead: GroupDiv).
-struct LocalDiv {
-  template <typename R>
-  SRT_HD void operator()(const R* num, const R* den, R* quo) const {
-    for (int j = 0; j < 4; ++j) quo[j] = num[j] / den[j];
-  }
-};
-
 // The right-hand side from the frame, the B sums and phi's interpolation p
 // (snapshot-raytracer.cu:462-509).
-template <typename IT, typename R = double, typename Div = LocalDiv>
-SRT_HD void rhs_finish(const R* y, const R* n, const R* a, const R* b, const BSums<IT, R>& B, const Tri<IT>& p,
-                       R* dy, const Div& div = Div()) {
-  const R dA = y[12], dAp = y[13], s1 = y[14], s2 = y[15], el1 = y[16], el2 = y[17];
-  const R phi1 = 1.0 + 2.0 * p.v;
+template <typename IT>
+SRT_HD void rhs_finish(const double* y, const double* n, const double* a, const double* b, const BSums<IT>& B, const Tri<IT>& p,
+                       double* dy) {
+  const double dA = y[12], dAp = y[13], s1 = y[14], s2 = y[15], el1 = y[16], el2 = y[17];
+  const double phi1 = 1.0 + 2.0 * p.v;
   for (int i = 0; i < 3; ++i) dy[i] = -n[i] * phi1 - B.val[i];
   // -P_perp v with P_perp = n n^T - I  ->  v - n (n.v)
-  const R v0 = 2.0 * p.g[0] + B.ngB[0], v1 = 2.0 * p.g[1] + B.ngB[1], v2 = 2.0 * p.g[2] + B.ngB[2];
-  const R nv = n[0] * v0 + n[1] * v1 + n[2] * v2;
+  const double v0 = 2.0 * p.g[0] + B.ngB[0], v1 = 2.0 * p.g[1] + B.ngB[1], v2 = 2.0 * p.g[2] + B.ngB[2];
+  const double nv = n[0] * v0 + n[1] * v1 + n[2] * v2;
   dy[3] = v0 - n[0] * nv;
   dy[4] = v1 - n[1] * nv;
   dy[5] = v2 - n[2] * nv;
-  const R ag = a[0] * p.g[0] + a[1] * p.g[1] + a[2] * p.g[2];
-  const R bg = b[0] * p.g[0] + b[1] * p.g[1] + b[2] * p.g[2];
+  const double ag = a[0] * p.g[0] + a[1] * p.g[1] + a[2] * p.g[2];
+  const double bg = b[0] * p.g[0] + b[1] * p.g[1] + b[2] * p.g[2];
   for (int i = 0; i < 3; ++i) {
     dy[6 + i] = -2.0 * n[i] * ag - n[i] * B.e1ngB;
     dy[9 + i] = -2.0 * n[i] * bg - n[i] * B.e2ngB;
   }
-  const R L = n[0] * p.g[0] + n[1] * p.g[1] + n[2] * p.g[2] +
+  const double L = n[0] * p.g[0] + n[1] * p.g[1] + n[2] * p.g[2] +
                    0.25 * (n[0] * B.ngB[0] + n[1] * B.ngB[1] + n[2] * B.ngB[2]);
   // P_perp : H = n^T H n - tr H
-  const R nHn = n[0] * n[0] * p.h[0] + n[1] * n[1] * p.h[3] + n[2] * n[2] * p.h[5] +
+  const double nHn = n[0] * n[0] * p.h[0] + n[1] * n[1] * p.h[3] + n[2] * n[2] * p.h[5] +
                      2.0 * (n[0] * n[1] * p.h[1] + n[0] * n[2] * p.h[2] + n[1] * n[2] * p.h[4]);
-  const R PH = nHn - (p.h[0] + p.h[3] + p.h[5]);
+  const double PH = nHn - (p.h[0] + p.h[3] + p.h[5]);
   dy[12] = -dAp;
   dy[13] = -4.0 * dAp * L - PH * dA + 0.5 * B.nlap * dA;
   // effective tidal matrix H + T/2 projected on the shear basis
   IT He[6];
   for (int i = 0; i < 6; ++i) He[i] = (IT)(p.h[i] + 0.5 * B.T[i]);
-  const R S1 = (a[0] * a[0] - b[0] * b[0]) * He[0] + (a[1] * a[1] - b[1] * b[1]) * He[3] +
+  const double S1 = (a[0] * a[0] - b[0] * b[0]) * He[0] + (a[1] * a[1] - b[1] * b[1]) * He[3] +
                     (a[2] * a[2] - b[2] * b[2]) * He[5] +
                     2.0 * ((a[0] * a[1] - b[0] * b[1]) * He[1] + (a[0] * a[2] - b[0] * b[2]) * He[2] +
                            (a[1] * a[2] - b[1] * b[2]) * He[4]);
-  const R S2 = 2.0 * (a[0] * b[0] * He[0] + a[1] * b[1] * He[3] + a[2] * b[2] * He[5]) +
+  const double S2 = 2.0 * (a[0] * b[0] * He[0] + a[1] * b[1] * He[3] + a[2] * b[2] * He[5]) +
                     2.0 * ((a[0] * b[1] + a[1] * b[0]) * He[1] + (a[0] * b[2] + a[2] * b[0]) * He[2] +
                            (a[1] * b[2] + a[2] * b[1]) * He[4]);
   dy[14] = 4.0 * s1 * L + S1 * dA * dA;
@@ -462,45 +670,44 @@ SRT_HD void rhs_finish(const R* y, const R* n, const R* a, const R* b, const BSu
   // operations when it is taken; where dA = 0 they are not finite and not
   // selected)
   const bool on = dA > 0.5;
-  const R dA2 = dA * dA;
-  const R q = sqrt_r(4.0 + el1 * el1 + el2 * el2);
-  const R num[4] = {s1 * s1 + s2 * s2, -2.0 * s1 * q, -2.0 * s2 * q, -(s1 * el2 - s2 * el1)};
-  const R den[4] = {dA2 * dA, dA2, dA2, dA2 * (2.0 + q)};
-  R quo[4];
-  div(num, den, quo);
-  const R zero(0.0);
-  const R t13 = dy[13] + quo[0];
+  const double dA2 = dA * dA;
+  const double q = sqrt(4.0 + el1 * el1 + el2 * el2);
+  const double num[4] = {s1 * s1 + s2 * s2, -2.0 * s1 * q, -2.0 * s2 * q, -(s1 * el2 - s2 * el1)};
+  const double den[4] = {dA2 * dA, dA2, dA2, dA2 * (2.0 + q)};
+  double quo[4];
+  for (int j = 0; j < 4; ++j) quo[j] = num[j] / den[j];
+  const double zero = 0.0;
+  const double t13 = dy[13] + quo[0];
   dy[13] = on ? t13 : dy[13];
   dy[16] = on ? quo[1] : zero;
   dy[17] = on ? quo[2] : zero;
   dy[18] = on ? quo[3] : zero;
 }
 
-// 19-component right-hand side on the full state y (FP64 or REF16 arithmetic).
-// State: 0-2 x, 3-5 n, 6-8 e1, 9-11 e2, 12 dA, 13 dA', 14-15 sigma1/2,
-// 16-17 ellipticity1/2, 18 rotation (snapshot-raytracer.cu:317-335).
+// 19-component right-hand side on the full state y in the reference's own
+// arithmetic (FP16 B taps, FP32 interpolation and sums, FP64 state), or
+// rhs_fp64.
 template <int MODE>
 SRT_HD void rhs_std(const double* y, double* dy, const FieldPtrs& F, const Geom& G) {
-  typedef typename std::conditional<MODE == kREF16, float, double>::type IT;
-  double n[3], a[3], b[3];
-  rhs_frame(y, n, a, b);
-  BSums<IT> B;
-  B.clear();
+  if constexpr (MODE == kFP64) {
+    rhs_fp64(y, dy, F, G);
+  } else {
+    double n[3], a[3], b[3];
+    rhs_frame(y, n, a, b);
+    BSums<float> B;
+    B.clear();
 #pragma unroll 1
-  for (int c = 0; c < 3; ++c) {
-    const double off[3] = {c == 0 ? 0.5 : 0.0, c == 1 ? 0.5 : 0.0, c == 2 ? 0.5 : 0.0};
-    Tri<IT> r;
-    if (MODE == kREF16) {
-      interp_std<IT, __half>(F.bh[c], G, y[0] - off[0], y[1] - off[1], y[2] - off[2], r);
-      tri_scale(r, (IT)(1.0 / 134217728.0));  // taps hold B * 2^27
-    } else {
-      interp_std<IT, float>(F.b[c], G, y[0] - off[0], y[1] - off[1], y[2] - off[2], r);
+    for (int c = 0; c < 3; ++c) {
+      const double off[3] = {c == 0 ? 0.5 : 0.0, c == 1 ? 0.5 : 0.0, c == 2 ? 0.5 : 0.0};
+      Tri<float> r;
+      interp_ref16<__half>(F.bh[c], G, y[0] - off[0], y[1] - off[1], y[2] - off[2], r);
+      tri_scale(r, (float)(1.0 / 134217728.0));  // taps hold B * 2^27
+      B.add(c, r, n, a, b);
     }
-    B.add(c, r, n, a, b);
+    Tri<float> p;
+    interp_ref16<float>(F.phi, G, y[0], y[1], y[2], p);
+    rhs_finish<float>(y, n, a, b, B, p, dy);
   }
-  Tri<IT> p;
-  interp_std<IT, float>(F.phi, G, y[0], y[1], y[2], p);
-  rhs_finish<IT>(y, n, a, b, B, p, dy);
 }
 
 // ------------------------------------------------------------ ray geometry
@@ -561,13 +768,16 @@ SRT_HD void step_std(const FieldPtrs& F, const Geom& G, double* y, double* ks) {
 #pragma unroll 1
   for (int st = 0; st < 4; ++st) {
     const double c = (st == 3) ? 1.0 : 0.5;
-    for (int j = 0; j < 19; ++j) ys[j] = (st == 0) ? y[j] : y[j] + c * k[j];
+    for (int j = 0; j < 19; ++j) ys[j] = (st == 0) ? y[j] : fma(c, k[j], y[j]);
     rhs_std<MODE>(ys, k, F, G);
     if (ks && st < 3)
       for (int j = 0; j < 19; ++j) ks[19 * st + j] = k[j];
-    for (int j = 0; j < 19; ++j) acc[j] = (st == 0) ? k[j] : ((st < 3) ? acc[j] + 2.0 * k[j] : acc[j]);
+    for (int j = 0; j < 19; ++j) acc[j] = (st == 0) ? k[j] : ((st < 3) ? fma(2.0, k[j], acc[j]) : acc[j]);
   }
-  for (int j = 0; j < 19; ++j) y[j] += (acc[j] + k[j]) / 6.0;
+  // FP64 multiplies by 1/6 (one fused operation); REF16 divides, as the
+  // reference does
+  for (int j = 0; j < 19; ++j)
+    y[j] = MODE == kFP64 ? fma(acc[j] + k[j], 1.0 / 6.0, y[j]) : y[j] + (acc[j] + k[j]) / 6.0;
 }
 
 // The six maps from the final state (snapshot-raytracer.cu:566-582).
@@ -587,137 +797,6 @@ SRT_HD void trace_ray_std(const FieldPtrs& F, const Geom& G, const RayDir& d, in
 #pragma unroll 1
   for (int step = 0; step < n_steps; ++step) step_std<MODE>(F, G, y, nullptr);
   extract_std(d, G, y, out);
-}
-
-// ------------------------------------------- double-float (dd) ray driver
-//
-// The FP64 scheme above in double-float arithmetic (srt_dd.cuh), for the
-// re-trace of the MIXED form's flagged rays: the same state, stages and
-// right-hand side (rhs_frame, BSums, rhs_finish instantiated with dd), the
-// interpolation's dot products accumulated in the compensated form of Ogita,
-// Rump and Oishi ("Accurate sum and dot product", 2005). The trajectory stays
-// ~1e-14 from the FP64 one, far inside the guard's margin.
-
-// Compensated accumulator: s + c, products added with their rounding errors.
-struct DdAcc {
-  float s = 0.f, c = 0.f;
-  SRT_HD void add(const dd& w, float x) {  // += w * x
-    const float p = w.hi * x;
-    const float e = fmaf(w.hi, x, -p);
-    float t, q;
-    dd_two_sum(s, p, t, q);
-    s = t;
-    c += fmaf(w.lo, x, e + q);
-  }
-  SRT_HD void add(const dd& w, const dd& x) {  // += w * x
-    const float p = w.hi * x.hi;
-    const float e = fmaf(w.hi, x.hi, -p);
-    float t, q;
-    dd_two_sum(s, p, t, q);
-    s = t;
-    c += fmaf(w.hi, x.lo, fmaf(w.lo, x.hi, e + q));
-  }
-  SRT_HD dd value() const {
-    float h, l;
-    dd_fast_two_sum(s, c, h, l);
-    return dd(h, l);
-  }
-};
-
-// tricubic<dd, float>: the same passes with compensated accumulation.
-SRT_HD void tricubic_dd(const float* __restrict__ f, int64_t base, int64_t px, int64_t pxy, const CRW<dd>& X,
-                        const CRW<dd>& Y, const CRW<dd>& Z, Tri<dd>& r) {
-  DdAcc v, g0, g1, g2, h00, h01, h02, h11, h12, h22;
-#pragma unroll 1
-  for (int c = 0; c < 4; ++c) {
-    DdAcc a, ay, ayy, ax, axy, axx;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const float* row = f + base + c * pxy + b * px;
-      const float p[4] = {ldg(row), ldg(row + 1), ldg(row + 2), ldg(row + 3)};
-      DdAcc rv, rx, rxx;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        rv.add(X.w[i], p[i]);
-        rx.add(X.g[i], p[i]);
-        rxx.add(X.h[i], p[i]);
-      }
-      const dd RV = rv.value(), RX = rx.value(), RXX = rxx.value();
-      a.add(Y.w[b], RV);
-      ay.add(Y.g[b], RV);
-      ayy.add(Y.h[b], RV);
-      ax.add(Y.w[b], RX);
-      axy.add(Y.g[b], RX);
-      axx.add(Y.w[b], RXX);
-    }
-    const dd A = a.value(), AY = ay.value(), AYY = ayy.value(), AX = ax.value(), AXY = axy.value(),
-             AXX = axx.value();
-    v.add(Z.w[c], A);
-    g0.add(Z.w[c], AX);
-    g1.add(Z.w[c], AY);
-    g2.add(Z.g[c], A);
-    h00.add(Z.w[c], AXX);
-    h01.add(Z.w[c], AXY);
-    h02.add(Z.g[c], AX);
-    h11.add(Z.w[c], AYY);
-    h12.add(Z.g[c], AY);
-    h22.add(Z.h[c], A);
-  }
-  r.v = v.value();
-  r.g[0] = g0.value();
-  r.g[1] = g1.value();
-  r.g[2] = g2.value();
-  r.h[0] = h00.value();
-  r.h[1] = h01.value();
-  r.h[2] = h02.value();
-  r.h[3] = h11.value();
-  r.h[4] = h12.value();
-  r.h[5] = h22.value();
-}
-
-// interp_std<double, float> in dd: cell from the dd position, dd offsets.
-SRT_HD void interp_dd(const float* f, const Geom& G, const dd& x, const dd& y, const dd& z, Tri<dd>& r) {
-  const dd fx = dd_floor(x), fy = dd_floor(y), fz = dd_floor(z);
-  const int64_t ix = (int64_t)fx.hi + (int64_t)fx.lo, iy = (int64_t)fy.hi + (int64_t)fy.lo,
-                iz = (int64_t)fz.hi + (int64_t)fz.lo;
-  CRW<dd> X, Y, Z;
-  cr_weights(x - fx, X);
-  cr_weights(y - fy, Y);
-  cr_weights(z - fz, Z);
-  const int64_t base = cell_base(G, wrap64(ix, G.n[0]), wrap64(iy, G.n[1]), wrap64(iz, G.n[2]));
-  tricubic_dd(f, base, G.px, G.pxy, X, Y, Z, r);
-}
-
-// rhs_std<kFP64> in dd.
-SRT_HD void rhs_dd(const dd* y, dd* dy, const FieldPtrs& F, const Geom& G) {
-  dd n[3], a[3], b[3];
-  rhs_frame<dd>(y, n, a, b);
-  BSums<dd, dd> B;
-  B.clear();
-  const dd half(0.5f);
-#pragma unroll 1
-  for (int c = 0; c < 3; ++c) {
-    Tri<dd> r;
-    interp_dd(F.b[c], G, c == 0 ? y[0] - half : y[0], c == 1 ? y[1] - half : y[1], c == 2 ? y[2] - half : y[2], r);
-    B.add(c, r, n, a, b);
-  }
-  Tri<dd> p;
-  interp_dd(F.phi, G, y[0], y[1], y[2], p);
-  rhs_finish<dd, dd>(y, n, a, b, B, p, dy);
-}
-
-// init_std / extract_std in dd (the step is step_dd_group in srt_kernels.cu).
-SRT_HD void init_dd(const RayDir& d, const Geom& G, dd* y) {
-  double y64[19];
-  init_std(d, G, y64);
-  for (int j = 0; j < 19; ++j) y[j] = dd(y64[j]);
-}
-
-
-SRT_HD void extract_dd(const RayDir& d, const Geom& G, const dd* y, float out[6]) {
-  double y64[19];
-  for (int j = 0; j < 19; ++j) y64[j] = (double)y[j];
-  extract_std(d, G, y64, out);
 }
 
 // -------------------------------------------------------------- MIXED mode
