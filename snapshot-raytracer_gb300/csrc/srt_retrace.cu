@@ -102,7 +102,7 @@ cudaError_t sm_count(int* sms) {
 // ones in double-float arithmetic on the FP32 pipes (maps within one float
 // ulp). The environment variable SRT_REFINE_DD_MIN overrides dd_min (tests use
 // it to reach both on small skies).
-constexpr int64_t kRefineWarpsPerSubpartition = 2;
+constexpr int64_t kRefineWarpsPerSubpartition = 1;
 
 cudaError_t launch_refine(const TraceArgs& a, cudaStream_t s, int64_t* kernels) {
   int sms = 0;
