@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 #include "srt_adjoint.cuh"
 #include "srt_internal.h"
@@ -73,7 +74,9 @@ struct AdjArgs {
   FieldPtrs F;
   Geom G;
   int64_t nside, pix_begin, count;
-  const int64_t* rays;
+  int64_t* rays;  // RING pixels, Morton order; kNearBit: near a cell face
+  int64_t* near;  // [0] the number of marked rays, [1 ...] their slots
+  float* bases;   // [12][count]: n0, e1, e2 and eta of the rays' MixedRay
   int n_steps, C, nseg;
   const float* w[6];  // map weights, indexed by ring - pix_begin
   void* ckpt;         // [nseg + 1][state][count]
@@ -101,41 +104,109 @@ __device__ __forceinline__ void load_vec(const T* base, int64_t count, int64_t s
 // Floats of one step of the MIXED tape: the four stage inputs.
 constexpr int kTapeStep = 4 * 19;
 
-// PAIR: the forward steps read the row-pair field arrays (srt_fields.pr).
-// Forward trace storing the state every C steps (and the final state). MAPS
-// (srt_forward_tape): also the maps, with the cell-face guard of the trace
-// kernel and its list of rays to re-trace; the arithmetic is the trace
-// kernel's, so the maps are srt_forward's.
-template <bool PAIR, bool MAPS>
-__global__ void __launch_bounds__(128, MAPS ? 2 : 1) ckpt_kernel_mixed(const AdjArgs A) {
-  const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (slot >= A.count) return;
-  const int64_t ring = A.rays[slot];
-  const RayDir d = ray_dir_pix(A.nside, ring);
-  MixedRay R;
-  float y[kMixedState], x0[3];
+// The rays' straight-ray bases, stored by the checkpointing forward: forming
+// them takes ~150 FP64 instructions a ray, which every segment's two launches
+// would repeat (3 % of a 512^3 / nside 256 / 256 steps gradient).
+__device__ __forceinline__ void store_bases(const AdjArgs& A, int64_t slot, const MixedRay& R) {
+  store_vec(A.bases, A.count, slot, R.n0, 3);
+  store_vec(A.bases + 3 * A.count, A.count, slot, R.a0, 3);
+  store_vec(A.bases + 6 * A.count, A.count, slot, R.b0, 3);
+  store_vec(A.bases + 9 * A.count, A.count, slot, R.eta, 3);
+}
+__device__ __forceinline__ void load_bases(const AdjArgs& A, int64_t slot, MixedRay& R) {
+  load_vec(A.bases, A.count, slot, R.n0, 3);
+  load_vec(A.bases + 3 * A.count, A.count, slot, R.a0, 3);
+  load_vec(A.bases + 6 * A.count, A.count, slot, R.b0, 3);
+  load_vec(A.bases + 9 * A.count, A.count, slot, R.eta, 3);
+}
+
+// Rays whose trajectory comes within the cell-face guard (a few in 10,000) keep
+// the four-tap passes' trajectory in the adjoint. Which side of a face FP32
+// rounding puts such a ray on decides its Hessian weights there, and with them
+// single voxels of the gradient (by up to 4e-3 of its rms at 512^3 / nside 256 /
+// 256 steps), so the second-difference passes' rounding is not let decide it:
+// ckpt_kernel_mixed marks and lists these rays, near_ckpt_kernel traces their
+// checkpoints again, and the segment kernel's first blocks take them apart.
+constexpr int64_t kNearBit = int64_t(1) << 62;
+
+__device__ __forceinline__ int64_t ring_of(const AdjArgs& A, int64_t slot) { return A.rays[slot] & ~kNearBit; }
+__device__ __forceinline__ bool is_near(const AdjArgs& A, int64_t slot) { return (A.rays[slot] & kNearBit) != 0; }
+
+// f(slot) for each marked ray of `warps` warps' list, all 32 lanes of a warp
+// together.
+template <typename Fn>
+__device__ __forceinline__ void for_near_rays(const AdjArgs& A, int64_t warps, const Fn& f) {
+  const int64_t n = A.near[0];
+  for (int64_t i = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5); i < n; i += warps) f(A.near[1 + i]);
+}
+
+// Touches the footprints of the step after `step` along the straight ray, two
+// rows of one field per lane, so that the ray's own loads find them in L1: a
+// marked ray is traced by a warp whose lanes all hold it, with no neighbours
+// to share taps with (38 -> 11 us a step).
+__device__ __forceinline__ void prefetch_step(const AdjArgs& A, const MixedRay& R, const float* x0, const float* y,
+                                              int step) {
+  const int lane = threadIdx.x & 31, f = lane >> 3, sub = lane & 7;
+  int cell[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const float p = x0[i] - (float)(step + 1) * R.n0[i] + y[i] - (f == i ? 0.5f : 0.f);
+    cell[i] = wrap32((int)floorf(p), A.G.n[i], A.G.invn[i]);
+  }
+  const float* v = (f == 3 ? A.F.phi : (f == 0 ? A.F.b[0] : (f == 1 ? A.F.b[1] : A.F.b[2]))) +
+                   (cell_base(A.G, cell[0], cell[1], cell[2]) + (sub >> 1) * A.G.pxy + 2 * (sub & 1) * A.G.px) * A.G.ts;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float t;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(t) : "l"(v + ((e >> 1) * A.G.px + 3 * (e & 1)) * A.G.ts));
+    (void)t;
+  }
+}
+
+// Forward trace of one ray storing the state every C steps (and the final
+// state); y holds the final state.
+template <int LAYOUT>
+__device__ __forceinline__ void ckpt_ray(const AdjArgs& A, int64_t slot, const RayDir& d, MixedRay& R, float* y,
+                                         Guard& gd) {
+  float x0[3];
   mixed_observer(A.G, x0);
   init_mixed(d, R, y);
+  if (LAYOUT != kFourTaps) store_bases(A, slot, R);
   float* ck = (float*)A.ckpt;
   store_vec(ck, A.count, slot, y, kMixedState);
-  // MAPS: the guard of the trace kernel; else disabled (cell-face proximity
-  // matters for the maps, not for the gradient)
-  __shared__ float guard_m[MAPS ? 128 : 1][2];
-  Guard gd;
-  if (MAPS) {
-    gd.m = guard_m[threadIdx.x];
-    gd.m[0] = 0.f;
-  }
 #pragma unroll 1
   for (int st = 0; st < A.n_steps; ++st) {
-    if (MAPS) gd.begin_step(y);
-    step_mixed<PAIR>(R, A.F, A.G, x0, st, y, nullptr, 0, gd);
-    if (MAPS) gd.end_step(st);
+    if (LAYOUT == kFourTaps) prefetch_step(A, R, x0, y, st);
+    if (gd.m) gd.begin_step(y);
+    step_mixed<LAYOUT>(R, A.F, A.G, x0, st, y, nullptr, 0, gd);
+    if (gd.m) gd.end_step(st);
     const int done = st + 1;
     if (done % A.C == 0 || done == A.n_steps) {
       const int k = (done + A.C - 1) / A.C;
       store_vec(ck + (int64_t)k * kMixedState * A.count, A.count, slot, y, kMixedState);
     }
+  }
+}
+
+// The checkpoints of every ray, with the cell-face guard of the trace kernel;
+// marks the rays it catches. MAPS (srt_forward_tape): also the maps and the
+// list of rays to re-trace; the arithmetic is the trace kernel's, so the maps
+// are srt_forward's.
+template <int LAYOUT, bool MAPS>
+__global__ void __launch_bounds__(128, 2) ckpt_kernel_mixed(const AdjArgs A) {
+  const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (slot >= A.count) return;
+  const int64_t ring = ring_of(A, slot);
+  MixedRay R;
+  float y[kMixedState];
+  __shared__ float guard_m[128][2];
+  Guard gd;
+  gd.m = guard_m[threadIdx.x];
+  gd.m[0] = 0.f;
+  ckpt_ray<LAYOUT>(A, slot, ray_dir_pix(A.nside, ring), R, y, gd);
+  if (gd.near) {
+    A.rays[slot] = ring | kNearBit;
+    A.near[1 + atomicAdd((unsigned long long*)A.near, 1ull)] = slot;
   }
   if (MAPS) {
     const int64_t o = ring - A.pix_begin;
@@ -150,12 +221,23 @@ __global__ void __launch_bounds__(128, MAPS ? 2 : 1) ckpt_kernel_mixed(const Adj
   }
 }
 
+// The marked rays' checkpoints by the four-tap passes, one warp per ray. Few
+// rays: the launch is about one ray's latency.
+__global__ void __launch_bounds__(128, 2) near_ckpt_kernel(const AdjArgs A) {
+  for_near_rays(A, (int64_t)gridDim.x * 4, [&](int64_t slot) {
+    MixedRay R;
+    float y[kMixedState];
+    Guard gd;  // disabled
+    ckpt_ray<kFourTaps>(A, slot, ray_dir_pix(A.nside, ring_of(A, slot)), R, y, gd);
+  });
+}
+
 // Cotangent of the final state from the map weights (the transpose of
 // extract_mixed) -> lam [19][count].
 __global__ void __launch_bounds__(128) final_cotangent_kernel_mixed(const AdjArgs A, float* lam) {
   const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (slot >= A.count) return;
-  const int64_t ring = A.rays[slot];
+  const int64_t ring = ring_of(A, slot);
   const int64_t o = ring - A.pix_begin;
   const RayDir d = ray_dir_pix(A.nside, ring);
   MixedRay R;
@@ -187,25 +269,38 @@ __global__ void __launch_bounds__(128) final_cotangent_kernel_mixed(const AdjArg
   store_vec(lam, A.count, slot, l, 19);
 }
 
-// Recompute segment sgi from its checkpoint, storing the four stage inputs
-// of every step: tape [C][4 x 19][count].
-template <bool PAIR>
-__global__ void __launch_bounds__(128, 2) segment_kernel_mixed(const AdjArgs A, int sgi) {
-  const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (slot >= A.count) return;
-  const RayDir d = ray_dir_pix(A.nside, A.rays[slot]);
+// Recompute segment sgi of one ray from its checkpoint, storing the four stage
+// inputs of every step: tape [C][4 x 19][count].
+template <int LAYOUT>
+__device__ __forceinline__ void segment_ray(const AdjArgs& A, int sgi, int64_t slot) {
   MixedRay R;
   float y[kMixedState], x0[3];
   mixed_observer(A.G, x0);
-  init_mixed(d, R, y);
+  load_bases(A, slot, R);
   const int s0 = sgi * A.C, s1 = min(s0 + A.C, A.n_steps);
   load_vec((const float*)A.ckpt + (int64_t)sgi * kMixedState * A.count, A.count, slot, y, kMixedState);
   float* tape = (float*)A.seg;
 #pragma unroll 1
   for (int st = s0; st < s1; ++st) {
     Guard gd;  // disabled
-    step_mixed<PAIR>(R, A.F, A.G, x0, st, y, tape + (int64_t)(st - s0) * kTapeStep * A.count + slot, A.count, gd);
+    if (LAYOUT == kFourTaps) prefetch_step(A, R, x0, y, st);
+    step_mixed<LAYOUT>(R, A.F, A.G, x0, st, y, tape + (int64_t)(st - s0) * kTapeStep * A.count + slot, A.count, gd);
   }
+}
+
+// The first kNearBlocks blocks take the marked rays by the four-tap passes
+// (first, so that their latency hides behind the other rays').
+constexpr int kNearBlocks = 38;
+constexpr int kNearCkptBlocks = 304;
+
+template <int LAYOUT>
+__global__ void __launch_bounds__(128, 2) segment_kernel_mixed(const AdjArgs A, int sgi) {
+  if (blockIdx.x < kNearBlocks) {
+    for_near_rays(A, kNearBlocks * 4, [&](int64_t slot) { segment_ray<kFourTaps>(A, sgi, slot); });
+    return;
+  }
+  const int64_t slot = (int64_t)(blockIdx.x - kNearBlocks) * 128 + threadIdx.x;
+  if (slot < A.count && !is_near(A, slot)) segment_ray<LAYOUT>(A, sgi, slot);
 }
 
 // Backward sweep over segment sgi: per step, backwards, the RK4 adjoint
@@ -215,7 +310,7 @@ __global__ void __launch_bounds__(128, 2) segment_kernel_mixed(const AdjArgs A, 
 // while the current stage runs); l carried in lam between segments. l and the
 // running sum of the a's live in shared memory (one column per thread) to keep
 // registers for the field passes.
-template <typename AccB, typename AccP, bool PAIR>
+template <typename AccB, typename AccP, int LAYOUT>
 __device__ __forceinline__ void sweep_segment(const AdjArgs& A, int sgi, int64_t slot, const MixedRay& R,
                                               const float* x0, float* lam, const AccB* accb, const AccP& accp,
                                               float (*s_lam)[128], float (*s_tot)[128]) {
@@ -244,7 +339,7 @@ __device__ __forceinline__ void sweep_segment(const AdjArgs& A, int sgi, int64_t
       for (int j = 0; j < 19; ++j) u[j] = ld_stream(tape + ((int64_t)(qn >> 2) * kTapeStep + 19 * (qn & 3) + j) * A.count);
     }
     for (int j = 0; j < 19; ++j) an[j] = 0.f;
-    rhs_vjp<float, AccB, AccP, PAIR>(V, A.F, A.G, fb, an, accb, accp);
+    rhs_vjp<float, AccB, AccP, LAYOUT>(V, A.F, A.G, fb, an, accb, accp);
     // the step's running sum of the a's restarts at its last stage
     for (int j = 0; j < 19; ++j) s_tot[j][t] = (stage == 3 ? 0.f : s_tot[j][t]) + an[j];
     if (stage == 0)
@@ -261,13 +356,18 @@ __device__ __forceinline__ void sweep_segment(const AdjArgs& A, int sgi, int64_t
 
 // BGRAD: the B gradient is wanted (else the B passes are compiled without a
 // scatter).
-template <typename Acc, bool PAIR, bool BGRAD>
-__global__ void __launch_bounds__(128, SRT_SWEEP_MIN_BLOCKS) sweep_kernel_mixed(const AdjArgs A, int sgi, float* lam, const Acc a0,
-                                                           const Acc a1, const Acc a2, const Acc a3) {
+template <typename Acc, int LAYOUT, bool BGRAD>
+__global__ void __launch_bounds__(128, SRT_SWEEP_MIN_BLOCKS)
+    sweep_kernel_mixed(const AdjArgs A, int sgi, float* lam, Acc a0, Acc a1, Acc a2, Acc a3) {
   __shared__ float s_lam[19][128];
   __shared__ float s_tot[19][128];
   const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (slot >= A.count) return;
+  if constexpr (TakesCells<Acc>::value) {  // this warp's copy of the region around the observer
+    const int64_t copy = ((slot >> 5) % kHotCopies) * (kHotSide * kHotSide * kHotSide);
+    for (Acc* a : {&a0, &a1, &a2, &a3})
+      if (a->hot) a->hot += copy;
+  }
   typedef typename std::conditional<BGRAD, Acc, AccNone>::type AccB;
   AccB accb[3];
   if constexpr (BGRAD) {
@@ -275,28 +375,34 @@ __global__ void __launch_bounds__(128, SRT_SWEEP_MIN_BLOCKS) sweep_kernel_mixed(
     accb[1] = a1;
     accb[2] = a2;
   }
-  const RayDir d = ray_dir_pix(A.nside, A.rays[slot]);
   MixedRay R;
   float x0[3];
-  {
-    float y[kMixedState];
-    init_mixed(d, R, y);
-  }
+  load_bases(A, slot, R);
   mixed_observer(A.G, x0);
-  sweep_segment<AccB, Acc, PAIR>(A, sgi, slot, R, x0, lam, accb, a3, s_lam, s_tot);
+  sweep_segment<AccB, Acc, LAYOUT>(A, sgi, slot, R, x0, lam, accb, a3, s_lam, s_tot);
+}
+
+// f(std::integral_constant<int, LAYOUT>()) for a handle's layout.
+template <typename Fn>
+void with_layout(int layout, const Fn& f) {
+  if (layout == kCells)
+    f(std::integral_constant<int, kCells>());
+  else if (layout == kPairs)
+    f(std::integral_constant<int, kPairs>());
+  else
+    f(std::integral_constant<int, kPlanes>());
 }
 
 template <typename Acc>
-void launch_sweep(const AdjArgs& A, int sgi, float* lam, const Acc* a, bool pair, bool bgrad, unsigned blocks,
+void launch_sweep(const AdjArgs& A, int sgi, float* lam, const Acc* a, int layout, bool bgrad, unsigned blocks,
                   cudaStream_t s) {
-  if (pair && bgrad)
-    sweep_kernel_mixed<Acc, true, true><<<blocks, 128, 0, s>>>(A, sgi, lam, a[0], a[1], a[2], a[3]);
-  else if (pair)
-    sweep_kernel_mixed<Acc, true, false><<<blocks, 128, 0, s>>>(A, sgi, lam, a[0], a[1], a[2], a[3]);
-  else if (bgrad)
-    sweep_kernel_mixed<Acc, false, true><<<blocks, 128, 0, s>>>(A, sgi, lam, a[0], a[1], a[2], a[3]);
-  else
-    sweep_kernel_mixed<Acc, false, false><<<blocks, 128, 0, s>>>(A, sgi, lam, a[0], a[1], a[2], a[3]);
+  with_layout(layout, [&](auto l) {
+    constexpr int L = decltype(l)::value;
+    if (bgrad)
+      sweep_kernel_mixed<Acc, L, true><<<blocks, 128, 0, s>>>(A, sgi, lam, a[0], a[1], a[2], a[3]);
+    else
+      sweep_kernel_mixed<Acc, L, false><<<blocks, 128, 0, s>>>(A, sgi, lam, a[0], a[1], a[2], a[3]);
+  });
 }
 
 // ------------------------------------------------------------- FP64 mode
@@ -304,7 +410,7 @@ void launch_sweep(const AdjArgs& A, int sgi, float* lam, const Acc* a, bool pair
 __global__ void __launch_bounds__(128) ckpt_kernel_fp64(const AdjArgs A) {
   const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (slot >= A.count) return;
-  const RayDir d = ray_dir_pix(A.nside, A.rays[slot]);
+  const RayDir d = ray_dir_pix(A.nside, ring_of(A, slot));
   double y[19];
   init_std(d, A.G, y);
   double* ck = (double*)A.ckpt;
@@ -326,7 +432,7 @@ __global__ void __launch_bounds__(128) reverse_kernel_fp64(const AdjArgs A, cons
   const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (slot >= A.count) return;
   const Acc acc[4] = {a0, a1, a2, a3};
-  const int64_t ring = A.rays[slot];
+  const int64_t ring = ring_of(A, slot);
   const int64_t o = ring - A.pix_begin;
   const RayDir d = ray_dir_pix(A.nside, ring);
   const double* ck = (const double*)A.ckpt;
@@ -416,54 +522,87 @@ struct PadRead<unsigned long long> {  // fixed point: exact integer sums
   __device__ T operator()(int64_t q) const { return g[q]; }
   __device__ static double value(T s) { return (double)(long long)s / kFixedScale; }
 };
+
+// Value of padded position (i, j, k) of an accumulator grid; for cells, the
+// transpose of cell_of: the second differences gather their neighbours'
+// cotangents (symmetric stencils; only positions 1 .. n + 1 hold any).
+template <typename G>
+__device__ __forceinline__ typename PadRead<G>::T pad_value(const PadRead<G>& rd, int64_t i, int64_t j, int64_t k,
+                                                            int64_t p0, int64_t p1) {
+  return rd(i + p0 * (j + p1 * k));
+}
 template <>
-struct PadRead<float4> {  // row-expanded FP32: taps of the rows starting at q, q-1, q-2, q-3
+struct PadRead<float4> {
   typedef float T;
   const float4* g;
-  __device__ T operator()(int64_t q) const {
-    float s = g[q].x;
-    if (q >= 1) s += g[q - 1].y;
-    if (q >= 2) s += g[q - 2].z;
-    if (q >= 3) s += g[q - 3].w;
-    return s;
-  }
   __device__ static double value(T s) { return (double)s; }
 };
+__device__ __forceinline__ float pad_value(const PadRead<float4>& rd, int64_t i, int64_t j, int64_t k, int64_t p0,
+                                           int64_t p1) {
+  float s = 0.f;
+#pragma unroll
+  for (int b = -1; b <= 1; ++b)
+#pragma unroll
+    for (int a = -1; a <= 1; ++a) {
+      if (i + a < 0 || i + a >= p0 || j + b < 0 || j + b >= p1) continue;
+      const float4 c = __ldg(rd.g + (i + a) + p0 * ((j + b) + p1 * k));
+      const float wx = a == 0 ? -2.f : 1.f, wy = b == 0 ? -2.f : 1.f;
+      float v = wx * wy * c.w;
+      if (a == 0) v += wy * c.y;
+      if (b == 0) v += wx * c.z;
+      if (a == 0 && b == 0) v += c.x;
+      s += v;
+    }
+  return s;
+}
+
+// Adds the copies of the region around the observer (behind the grid's pvox
+// entries) into the grid.
+__global__ void __launch_bounds__(256) merge_hot_kernel(float4* g, int64_t pvox, const Geom G) {
+  constexpr int kRegion = kHotSide * kHotSide * kHotSide;
+  const int q = blockIdx.x * 256 + threadIdx.x;
+  const int x = q % kHotSide + G.n[0] / 2 - kHotSide / 2, y = q / kHotSide % kHotSide + G.n[1] / 2 - kHotSide / 2,
+            z = q / (kHotSide * kHotSide) + G.n[2] / 2 - kHotSide / 2;
+  float4* dst = g + x + G.px * y + G.pxy * z;
+  float4 s = *dst;
+  for (int c = 0; c < kHotCopies; ++c) {
+    const float4 v = g[pvox + (int64_t)c * kRegion + q];
+    s.x += v.x;
+    s.y += v.y;
+    s.z += v.z;
+    s.w += v.w;
+  }
+  *dst = s;
+}
 
 // For voxel (i, j, k): sum of the padded copies (the interior one and the
-// halo copies) -> out[v * stride + comp] (+= when accumulate).
+// halo copies) -> out[v * stride + comp] (+= when accumulate). Blocks of 32 x 8
+// voxels of a plane (the cells' stencils share their neighbours in L1), looping
+// where an axis is longer than the grid.
 template <typename G>
-__global__ void fold_kernel(const G* __restrict__ padded, int64_t n0, int64_t n1, int64_t n2, float* out, int stride,
-                            int comp, int accumulate, unsigned* ovf) {
-  const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n0 * n1 * n2) return;
+__global__ void __launch_bounds__(256) fold_kernel(const G* __restrict__ padded, int64_t n0, int64_t n1, int64_t n2,
+                                                   float* out, int stride, int comp, int accumulate, unsigned* ovf) {
+  const int64_t i = (int64_t)blockIdx.x * 32 + threadIdx.x;
+  if (i >= n0) return;
   const PadRead<G> rd{padded};
-  const int64_t i = v % n0, j = (v / n0) % n1, k = v / (n0 * n1);
   const int64_t p0 = n0 + 3, p1 = n1 + 3;
   int64_t pi[4], pj[4], pk[4];
-  int ni = 0, nj = 0, nk = 0;
-  // padded coordinate q maps to voxel (q - 1) mod n for q in [0, n + 3)
-  pi[ni++] = i + 1;
-  if (i == n0 - 1) pi[ni++] = 0;
-  if (i == 0) pi[ni++] = n0 + 1;
-  if (i == 1 % n0) pi[ni++] = n0 + 2;
-  pj[nj++] = j + 1;
-  if (j == n1 - 1) pj[nj++] = 0;
-  if (j == 0) pj[nj++] = n1 + 1;
-  if (j == 1 % n1) pj[nj++] = n1 + 2;
-  pk[nk++] = k + 1;
-  if (k == n2 - 1) pk[nk++] = 0;
-  if (k == 0) pk[nk++] = n2 + 1;
-  if (k == 1 % n2) pk[nk++] = n2 + 2;
-  typename PadRead<G>::T sum = 0;
-  for (int a = 0; a < nk; ++a)
-    for (int b = 0; b < nj; ++b)
-      for (int c = 0; c < ni; ++c) sum += rd(pi[c] + p0 * (pj[b] + p1 * pk[a]));
-  const double dval = PadRead<G>::value(sum);
-  if (ovf && !(fabs(dval) < kFixedLimit)) atomicOr(ovf, 1u);  // fixed point near or past its range
-  const float val = (float)dval;
-  float* dst = out + v * stride + comp;
-  *dst = accumulate ? *dst + val : val;
+  const int ni = padded_coords(i, n0, pi);
+  for (int64_t k = blockIdx.z; k < n2; k += gridDim.z) {
+    const int nk = padded_coords(k, n2, pk);
+    for (int64_t j = (int64_t)blockIdx.y * 8 + threadIdx.y; j < n1; j += (int64_t)gridDim.y * 8) {
+      const int nj = padded_coords(j, n1, pj);
+      typename PadRead<G>::T sum = 0;
+      for (int a = 0; a < nk; ++a)
+        for (int b = 0; b < nj; ++b)
+          for (int c = 0; c < ni; ++c) sum += pad_value(rd, pi[c], pj[b], pk[a], p0, p1);
+      const double dval = PadRead<G>::value(sum);
+      if (ovf && !(fabs(dval) < kFixedLimit)) atomicOr(ovf, 1u);  // fixed point near or past its range
+      const float val = (float)dval;
+      float* dst = out + (i + n0 * (j + n1 * k)) * stride + comp;
+      *dst = accumulate ? *dst + val : val;
+    }
+  }
 }
 
 }  // namespace srt
@@ -548,7 +687,9 @@ struct srt_tape {
   int device = 0;
   int64_t nside = 0, pix_begin = 0, pix_count = 0;
   int n_steps = 0, C = 0, nseg = 0;
-  int64_t* rays = nullptr;  // Morton-ordered RING pixels (device)
+  int64_t* rays = nullptr;  // Morton-ordered RING pixels (device), marked near a cell face
+  int64_t* near = nullptr;  // their number and slots (device)
+  float* bases = nullptr;   // [12][pix_count] (device)
   float* ckpt = nullptr;    // [nseg + 1][kMixedState][pix_count] (device)
   int64_t bytes = 0;
 };
@@ -601,7 +742,7 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
   int prev = 0;
   cudaGetDevice(&prev);
   if (prev != f->device) cudaSetDevice(f->device);
-  DevBuf counts, offsets, rays, wdev, ckpt, seg, lam, gacc[4], gout_phi, gout_b, ovf;
+  DevBuf counts, offsets, rays, near, bases, wdev, ckpt, seg, lam, gacc[4], gout_phi, gout_b, ovf;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   int64_t kernels = 0, h2d = 0, d2h = 0;
   {
@@ -628,11 +769,11 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
     float* out_b = dev_io ? db_xyz : (float*)gout_b.p;
     if (pix_count > 0 && (dphi || db_xyz)) {
       // ---- ray list (a tape brings its own)
-      const int64_t* ray_list = tape ? tape->rays : nullptr;
+      int64_t* ray_list = tape ? tape->rays : nullptr;
       if (!tape) {
         rc = build_ray_list(nside, pix_begin, pix_count, s, counts, offsets, rays, &kernels, "srt_vjp");
         if (rc != SRT_OK) goto done;
-        ray_list = (const int64_t*)rays.p;
+        ray_list = (int64_t*)rays.p;
       }
 
       // ---- weights on the device
@@ -654,14 +795,23 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
       const int state = fp64 ? 19 : kMixedState;
       const size_t esz = fp64 ? sizeof(double) : sizeof(float);
       if (!tape) VJP_TRY(ckpt.alloc((size_t)(nseg + 1) * state * pix_count * esz), "cudaMalloc(checkpoints)");
+      if (!tape && !fp64) {
+        VJP_TRY(near.alloc((pix_count + 1) * sizeof(int64_t)), "cudaMalloc(near rays)");
+        VJP_TRY(cudaMemsetAsync(near.p, 0, sizeof(int64_t), s), "clear near rays");
+        VJP_TRY(bases.alloc((size_t)12 * pix_count * sizeof(float)), "cudaMalloc(ray bases)");
+      }
+      // copies of the region around the observer (FP32 accumulation), where the
+      // grid holds the region
+      const bool hot = !fp64 && !determ && std::min(f->n[0], std::min(f->n[1], f->n[2])) >= kHotSide;
+      const int64_t acc_entries = pvox + (hot ? (int64_t)kHotCopies * kHotSide * kHotSide * kHotSide : 0);
       // per-step records of one segment: FP64 y, k1, k2, k3; MIXED the four stage inputs
       VJP_TRY(seg.alloc((size_t)C * (fp64 ? state + 57 : kTapeStep) * pix_count * esz), "cudaMalloc(segment records)");
       if (!fp64) VJP_TRY(lam.alloc((size_t)19 * pix_count * sizeof(float)), "cudaMalloc(state cotangents)");
       for (int fld = 0; fld < 4; ++fld) {
         const bool want = (fld == 3) ? (dphi != nullptr) : (db_xyz != nullptr);
         if (!want) continue;
-        VJP_TRY(gacc[fld].alloc(pvox * accsz), "cudaMalloc(gradient accumulators)");
-        VJP_TRY(cudaMemsetAsync(gacc[fld].p, 0, pvox * accsz, s), "clear accumulators");
+        VJP_TRY(gacc[fld].alloc(acc_entries * accsz), "cudaMalloc(gradient accumulators)");
+        VJP_TRY(cudaMemsetAsync(gacc[fld].p, 0, acc_entries * accsz, s), "clear accumulators");
       }
       if (determ) {  // fixed-point range flag
         VJP_TRY(ovf.alloc(sizeof(unsigned)), "cudaMalloc(overflow flag)");
@@ -675,6 +825,8 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
       A.pix_begin = pix_begin;
       A.count = pix_count;
       A.rays = ray_list;
+      A.near = tape ? tape->near : (int64_t*)near.p;
+      A.bases = tape ? tape->bases : (float*)bases.p;
       A.n_steps = n_steps;
       A.C = C;
       A.nseg = nseg;
@@ -705,52 +857,54 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
       } else {
         // forward with checkpoints; then per segment, backwards: recompute
         // the segment's tape, sweep it
-        const bool pair = f->pr[0] != nullptr;
-        if (tape) {
-          // the checkpoints come from srt_forward_tape
-        } else if (pair) {
-          ckpt_kernel_mixed<true, false><<<blocks, 128, 0, s>>>(A);
-        } else {
-          ckpt_kernel_mixed<false, false><<<blocks, 128, 0, s>>>(A);
+        const int layout = f->layout();
+        if (!tape) {  // else the checkpoints come from srt_forward_tape
+          with_layout(layout, [&](auto l) { ckpt_kernel_mixed<decltype(l)::value, false><<<blocks, 128, 0, s>>>(A); });
+          near_ckpt_kernel<<<std::min<unsigned>(blocks * 32, kNearCkptBlocks), 128, 0, s>>>(A);
         }
         final_cotangent_kernel_mixed<<<blocks, 128, 0, s>>>(A, (float*)lam.p);
-        kernels += tape ? 1 : 2;
+        kernels += tape ? 1 : 3;
         AccF32 af[4];
         AccFixed ax[4];
         make_acc<AccF32, float4>(af, A.acc);
+        for (int fld = 0; fld < 4; ++fld) af[fld].hot = hot ? pvox : 0;
         make_acc<AccFixed, unsigned long long>(ax, A.acc);
         for (int fld = 0; fld < 4; ++fld) ax[fld].ovf = (unsigned*)ovf.p;
         const bool bgrad = db_xyz != nullptr;
         for (int sgi = nseg - 1; sgi >= 0; --sgi) {
-          if (pair)
-            segment_kernel_mixed<true><<<blocks, 128, 0, s>>>(A, sgi);
-          else
-            segment_kernel_mixed<false><<<blocks, 128, 0, s>>>(A, sgi);
+          with_layout(layout, [&](auto l) { segment_kernel_mixed<decltype(l)::value><<<blocks + kNearBlocks, 128, 0, s>>>(A, sgi); });
           if (determ)
-            launch_sweep<AccFixed>(A, sgi, (float*)lam.p, ax, pair, bgrad, blocks, s);
+            launch_sweep<AccFixed>(A, sgi, (float*)lam.p, ax, layout, bgrad, blocks, s);
           else
-            launch_sweep<AccF32>(A, sgi, (float*)lam.p, af, pair, bgrad, blocks, s);
+            launch_sweep<AccF32>(A, sgi, (float*)lam.p, af, layout, bgrad, blocks, s);
           kernels += 2;
         }
       }
       if (fp64) kernels += 2;
+      for (int fld = 0; fld < 4 && hot; ++fld) {
+        if (!gacc[fld].p) continue;
+        merge_hot_kernel<<<kHotSide * kHotSide * kHotSide / 256, 256, 0, s>>>((float4*)gacc[fld].p, pvox, A.G);
+        ++kernels;
+      }
       VJP_TRY(cudaGetLastError(), "adjoint kernels");
       // ---- fold onto the periodic grid
-      const unsigned fblocks = (unsigned)((vox + 255) / 256);
+      const dim3 fgrid((unsigned)((f->n[0] + 31) / 32), (unsigned)std::min<int64_t>((f->n[1] + 7) / 8, 65535),
+                       (unsigned)std::min<int64_t>(f->n[2], 65535));
+      const dim3 fblock(32, 8);
       for (int fld = 0; fld < 4; ++fld) {
         if (!gacc[fld].p) continue;
         float* dst = (fld == 3) ? out_phi : out_b;
         const int stride = (fld == 3) ? 1 : 3, comp = (fld == 3) ? 0 : fld;
         const int accum = accumulate ? 1 : 0;
         if (determ)
-          fold_kernel<unsigned long long><<<fblocks, 256, 0, s>>>((const unsigned long long*)gacc[fld].p, f->n[0],
+          fold_kernel<unsigned long long><<<fgrid, fblock, 0, s>>>((const unsigned long long*)gacc[fld].p, f->n[0],
                                                                  f->n[1], f->n[2], dst, stride, comp, accum,
                                                                  (unsigned*)ovf.p);
         else if (fp64)
-          fold_kernel<double><<<fblocks, 256, 0, s>>>((const double*)gacc[fld].p, f->n[0], f->n[1], f->n[2], dst,
+          fold_kernel<double><<<fgrid, fblock, 0, s>>>((const double*)gacc[fld].p, f->n[0], f->n[1], f->n[2], dst,
                                                      stride, comp, accum, nullptr);
         else
-          fold_kernel<float4><<<fblocks, 256, 0, s>>>((const float4*)gacc[fld].p, f->n[0], f->n[1], f->n[2], dst,
+          fold_kernel<float4><<<fgrid, fblock, 0, s>>>((const float4*)gacc[fld].p, f->n[0], f->n[1], f->n[2], dst,
                                                      stride, comp, accum, nullptr);
         ++kernels;
       }
@@ -834,7 +988,7 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
   cudaGetDevice(&prev);
   if (prev != f->device) cudaSetDevice(f->device);
   srt_tape* t = new (std::nothrow) srt_tape();
-  DevBuf counts, offsets, rays, ckpt, dmaps, rlist, rcount;
+  DevBuf counts, offsets, rays, near, bases, ckpt, dmaps, rlist, rcount;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   int64_t kernels = 0;
   if (!t) {
@@ -845,6 +999,9 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
     rc = build_ray_list(nside, pix_begin, pix_count, s, counts, offsets, rays, &kernels, "srt_forward_tape");
     if (rc != SRT_OK) goto done;
     VJP_TRY(ckpt.alloc((size_t)(nseg + 1) * kMixedState * pix_count * sizeof(float)), "cudaMalloc(checkpoints)");
+    VJP_TRY(near.alloc((pix_count + 1) * sizeof(int64_t)), "cudaMalloc(near rays)");
+    VJP_TRY(cudaMemsetAsync(near.p, 0, sizeof(int64_t), s), "clear near rays");
+    VJP_TRY(bases.alloc((size_t)12 * pix_count * sizeof(float)), "cudaMalloc(ray bases)");
     VJP_TRY(rlist.alloc(pix_count * sizeof(int64_t)), "cudaMalloc(refine list)");
     VJP_TRY(rcount.alloc(sizeof(unsigned long long)), "cudaMalloc(refine count)");
     VJP_TRY(cudaMemsetAsync(rcount.p, 0, sizeof(unsigned long long), s), "clear refine count");
@@ -862,7 +1019,9 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
     A.nside = nside;
     A.pix_begin = pix_begin;
     A.count = pix_count;
-    A.rays = (const int64_t*)rays.p;
+    A.rays = (int64_t*)rays.p;
+    A.near = (int64_t*)near.p;
+    A.bases = (float*)bases.p;
     A.n_steps = n_steps;
     A.C = C;
     A.nseg = nseg;
@@ -874,11 +1033,9 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
     VJP_TRY(cudaEventCreate(&e1), "cudaEventCreate");
     VJP_TRY(cudaEventRecord(e0, s), "cudaEventRecord");
     const unsigned blocks = (unsigned)((pix_count + 127) / 128);
-    if (f->pr[0])
-      ckpt_kernel_mixed<true, true><<<blocks, 128, 0, s>>>(A);
-    else
-      ckpt_kernel_mixed<false, true><<<blocks, 128, 0, s>>>(A);
-    ++kernels;
+    with_layout(f->layout(), [&](auto l) { ckpt_kernel_mixed<decltype(l)::value, true><<<blocks, 128, 0, s>>>(A); });
+    near_ckpt_kernel<<<std::min<unsigned>(blocks * 32, kNearCkptBlocks), 128, 0, s>>>(A);
+    kernels += 2;
     VJP_TRY(cudaGetLastError(), "checkpointing forward");
     TraceArgs ta;
     ta.F = A.F;
@@ -918,9 +1075,13 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
     t->C = C;
     t->nseg = nseg;
     t->rays = (int64_t*)rays.p;
+    t->near = (int64_t*)near.p;
+    t->bases = (float*)bases.p;
     t->ckpt = (float*)ckpt.p;
-    t->bytes = pix_count * (int64_t)sizeof(int64_t) + (int64_t)(nseg + 1) * kMixedState * pix_count * 4;
+    t->bytes = (2 * pix_count + 1) * (int64_t)sizeof(int64_t) + 48 * pix_count + (int64_t)(nseg + 1) * kMixedState * pix_count * 4;
     rays.p = nullptr;  // owned by the tape from here on
+    near.p = nullptr;
+    bases.p = nullptr;
     ckpt.p = nullptr;
     *out = t;
     t = nullptr;
@@ -951,6 +1112,8 @@ extern "C" int srt_tape_destroy(srt_tape* tape) {
   cudaGetDevice(&prev);
   if (prev != tape->device) cudaSetDevice(tape->device);
   if (tape->rays) cudaFree(tape->rays);
+  if (tape->near) cudaFree(tape->near);
+  if (tape->bases) cudaFree(tape->bases);
   if (tape->ckpt) cudaFree(tape->ckpt);
   if (prev != tape->device) cudaSetDevice(prev);
   delete tape;

@@ -29,14 +29,10 @@ struct CRW4 {  // Catmull-Rom weights for value and d/dt .. d3/dt3
   T w[4], g[4], h[4], k[4];
 };
 
-// FP32 (the MIXED form) takes the forward's Horner-form weights.
 template <typename T>
 SRT_HD void cr_weights4(T t, CRW4<T>& c) {
   CRW<T> b;
-  if constexpr (sizeof(T) == sizeof(float))
-    cr_weights_mixed(t, b);
-  else
-    cr_weights(t, b);
+  cr_weights(t, b);
   for (int i = 0; i < 4; ++i) {
     c.w[i] = b.w[i];
     c.g[i] = b.g[i];
@@ -50,32 +46,65 @@ SRT_HD void cr_weights4(T t, CRW4<T>& c) {
 
 // ---------------------------------------------------------- accumulators
 
-// Where the tap cotangents go: one call per 4-tap x-row of a tricubic
-// footprint (padded index `row` of its first tap). Three flavours:
-//   AccF32    FP32 atomics into a row-expanded grid: entry r (a float4) holds
-//             the four tap contributions of rows starting at padded index r,
-//             so one 16-byte vector atomic carries a whole row; the fold
-//             kernel adds entry q.x + (q-1).y + (q-2).z + (q-3).w per voxel;
-//   AccF64    FP64 atomics into a halo-padded grid (one per tap);
+// Where the tap cotangents go. Three flavours:
+//   AccF32    FP32 vector atomics into a grid of cells (float4 per padded
+//             voxel): the cotangents of a voxel's value and of its second
+//             differences along y, x and both, which fold_kernel gathers onto
+//             the voxels; one 16-byte atomic carries a tap's four;
+//   AccF64    FP64 atomics into a halo-padded grid (one per tap), one call per
+//             4-tap x-row of a tricubic footprint (padded index `row` of its
+//             first tap);
 //   AccFixed  64-bit fixed point into a halo-padded grid (order-independent,
-//             so repeated runs give identical bits).
+//             so repeated runs give identical bits), by rows too.
 // A null grid (gradient not requested) ignores the contributions, and the
 // passes skip forming them (active() is false).
+// base: accumulator index of voxel (cx-1, cy-1, cz-1); px, pxy: its strides.
+struct Scatter {
+  int64_t base, px, pxy;
+};
+
+// Near the observer every ray adds to the same few voxels, and atomics on one
+// address run one after another: there each warp adds to one of kHotCopies
+// copies of a kHotSide^3 region around the observer (behind the grid, merged
+// into it afterwards), spreading them over as many addresses. 256^3 / nside 128:
+// the first 12 of 128 steps took 9.0 ms against ~3.1 for the others.
+constexpr int kHotSide = 32, kHotCopies = 16;
+
+// Index in a copy of the footprint that starts at cell (cx, cy, cz), or -1 where
+// it leaves the region (padded positions n / 2 - kHotSide / 2 on).
+SRT_HD int hot_base(const Geom& G, const int* c) {
+  const unsigned x = (unsigned)(c[0] - G.n[0] / 2 + kHotSide / 2), y = (unsigned)(c[1] - G.n[1] / 2 + kHotSide / 2),
+                 z = (unsigned)(c[2] - G.n[2] / 2 + kHotSide / 2);
+  const bool in = x <= kHotSide - 4 && y <= kHotSide - 4 && z <= kHotSide - 4;
+  return in ? (int)(x + kHotSide * (y + kHotSide * z)) : -1;
+}
+
 struct AccF32 {
   float4* g;
+  int64_t hot = 0;  // index of this warp's copy; 0: no copies
   SRT_HD bool active() const { return g != nullptr; }
-  SRT_HD void add_row(int64_t row, float c0, float c1, float c2, float c3) const {
-    if (!g) return;
+  // where the footprint at padded base index `base` goes
+  SRT_HD Scatter place(int64_t base, int hbase, const Geom& G) const {
+    if (hot && hbase >= 0) return Scatter{hot + hbase, kHotSide, kHotSide * kHotSide};
+    return Scatter{base, G.px, G.pxy};
+  }
+  SRT_HD void add_cell(int64_t q, float4 v) const {
 #if defined(__CUDA_ARCH__)
-    atomicAdd(g + row, make_float4(c0, c1, c2, c3));
+    atomicAdd(g + q, v);
 #else
-    g[row].x += c0;
-    g[row].y += c1;
-    g[row].z += c2;
-    g[row].w += c3;
+    g[q].x += v.x;
+    g[q].y += v.y;
+    g[q].z += v.z;
+    g[q].w += v.w;
 #endif
   }
 };
+
+// Accumulators that take a tap's cell (add_cell) rather than rows of taps.
+template <typename Acc>
+struct TakesCells : std::false_type {};
+template <>
+struct TakesCells<AccF32> : std::true_type {};
 
 struct AccF64 {
   double* g;
@@ -153,7 +182,7 @@ struct AccNone {
 // Hessian entries are the unique components (off-diagonal cotangents already
 // hold both symmetric halves).
 template <typename T, typename Acc>
-SRT_HD void tricubic_vjp(const float* __restrict__ f, int64_t base, int64_t px, int64_t pxy, T tx, T ty, T tz,
+SRT_HD void tricubic_vjp(const float* __restrict__ f, int64_t base, int64_t px, int64_t pxy, int ts, T tx, T ty, T tz,
                          const T* qb, Tri<T>& Q, T* xb, const Acc& acc) {
   CRW4<T> X, Y, Z;
   cr_weights4(tx, X);
@@ -181,8 +210,8 @@ SRT_HD void tricubic_vjp(const float* __restrict__ f, int64_t base, int64_t px, 
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int64_t row = base + c * pxy + b * px;
-      const float* rp = f + row;
-      const T p0 = (T)ldg(rp), p1 = (T)ldg(rp + 1), p2 = (T)ldg(rp + 2), p3 = (T)ldg(rp + 3);
+      const float* rp = f + row * ts;
+      const T p0 = (T)ldg(rp), p1 = (T)ldg(rp + ts), p2 = (T)ldg(rp + 2 * ts), p3 = (T)ldg(rp + 3 * ts);
       const T r0 = X.w[0] * p0 + X.w[1] * p1 + X.w[2] * p2 + X.w[3] * p3;
       const T r1 = X.g[0] * p0 + X.g[1] * p1 + X.g[2] * p2 + X.g[3] * p3;
       const T r2 = X.h[0] * p0 + X.h[1] * p1 + X.h[2] * p2 + X.h[3] * p3;
@@ -236,182 +265,138 @@ SRT_HD void tricubic_vjp(const float* __restrict__ f, int64_t base, int64_t px, 
            qb[6] * o102 + qb[7] * o021 + qb[8] * o012 + qb[9] * o003;
 }
 
-// The same pass in FP32 with every product on packed pairs (two FP32 FMAs
-// per instruction), as in tricubic_pair: rows y and y+1 of a slice come as one
-// float2 per x tap from `rows` (PairRows: the row-pair array; SingleRows: the
-// single layout, two loads per tap pair). base: the single-layout index of
-// voxel (cx-1, cy-1, cz-1), where the tap cotangents go.
-template <typename Acc, typename Rows>
-SRT_HD void tricubic_vjp_pair(const Rows& rows, int64_t base, int64_t px, int64_t pxy, float tx, float ty, float tz,
-                              const float* qb, Tri<float>& Q, float* xb, const Acc& acc) {
-  CRW4<float> X, Y, Z;
-  cr_weights4(tx, X);
-  cr_weights4(ty, Y);
-  cr_weights4(tz, Z);
-  float2 xw[4], xg[4], xh[4];
-  for (int i = 0; i < 4; ++i) {
-    xw[i] = dup2(X.w[i]);
-    xg[i] = dup2(X.g[i]);
-    xh[i] = dup2(X.h[i]);
-  }
+// The same pass for the MIXED form, in FP32 on the second-difference form of
+// the cubic (CWD): the x pass on packed pairs as in tricubic_mixed, with its
+// third derivative (one packed subtraction a row), the y pass on scalars, the
+// z pass on pairs of outputs, and the next slice's data loaded while the
+// current one is processed.
+// The tap cotangents are formed in the basis the passes read: per slice, for
+// the four inner taps, the cotangents of the value and of the second
+// differences along y, x and both (60 operations a slice against 72 plus the
+// row factors on sixteen taps). AccF32 adds them as they are, one 16-byte
+// vector atomic per inner tap, and fold_kernel applies the (symmetric) second
+// differences once per voxel; the other accumulators get them expanded to taps.
+// 332 lane operations without the scatter against 536 on four taps.
+template <typename Acc, typename Src>
+SRT_HD void tricubic_vjp_mixed(const Src& src, const Scatter& sc, float tx, float ty, float tz, const float* qb,
+                               Tri<float>& Q, float* xb, const Acc& acc) {
+  CWD X, Y;
+  CRW<float> Z;
+  cr_weights_diff(tx, X);
+  cr_weights_diff(ty, Y);
+  cr_weights_mixed(tz, Z);
+  const XDup xd(X);
   const bool scatter = acc.active();  // this field's gradient was requested
-  // y weights and per-row scatter factors of rows (0, 1) and (2, 3)
-  float2 yw[2], yg[2], yh[2], yk[2], Aw[2], Bw[2], Dw[2], Ag[2], Bg[2], Ah[2];
-  for (int pr = 0; pr < 2; ++pr) {
-    const int b0 = 2 * pr, b1 = 2 * pr + 1;
-    yw[pr] = make_float2(Y.w[b0], Y.w[b1]);
-    yg[pr] = make_float2(Y.g[b0], Y.g[b1]);
-    yh[pr] = make_float2(Y.h[b0], Y.h[b1]);
-    yk[pr] = make_float2(Y.k[b0], Y.k[b1]);
-    Aw[pr] = ffma2(dup2(qb[0]), yw[pr], ffma2(dup2(qb[2]), yg[pr], fmul2(dup2(qb[7]), yh[pr])));
-    Bw[pr] = ffma2(dup2(qb[3]), yw[pr], fmul2(dup2(qb[8]), yg[pr]));
-    Dw[pr] = fmul2(dup2(qb[9]), yw[pr]);
-    Ag[pr] = ffma2(dup2(qb[1]), yw[pr], fmul2(dup2(qb[5]), yg[pr]));
-    Bg[pr] = fmul2(dup2(qb[6]), yw[pr]);
-    Ah[pr] = fmul2(dup2(qb[4]), yw[pr]);
-  }
-  // z pass (and an unconditional prefetch): packed for the passes without a
-  // scatter (they have the registers to spare), on the operand pairs the y
-  // sums form: value weight (o000, o100)
-  // (o010, o110) (o020, o120) (o200, o210) (o030, o300), derivative weight
-  // (o001, o101) (o011, o111) (o021, -) (o201, -), second derivative
-  // (o002, o102) (o012, -), third (o003, -); scalar where the scatter's
-  // working set is live. Every output is the same FMA chain over the slices.
-  constexpr bool kPackedZ = std::is_same<Acc, AccNone>::value;
-  float o000 = 0, o001 = 0, o002 = 0, o003 = 0, o010 = 0, o011 = 0, o012 = 0, o020 = 0, o021 = 0, o030 = 0;
-  float o100 = 0, o101 = 0, o102 = 0, o110 = 0, o111 = 0, o120 = 0, o200 = 0, o201 = 0, o210 = 0, o300 = 0;
+  // outputs oXYZ by derivative order, as pairs (two orders of the same z weight);
+  // x and y third derivatives are summed as thirds
   const float2 z0 = make_float2(0.f, 0.f);
-  float2 W0 = z0, W1 = z0, W2 = z0, W3 = z0, W4 = z0, G0 = z0, G1 = z0, G2 = z0, G3 = z0, H0 = z0, H1 = z0, K0 = z0;
-  // taps of the next slice, loaded while the current one is processed
-  float2 nt[8];
-  for (int pr = 0; pr < 2; ++pr)
-    for (int i = 0; i < 4; ++i) nt[4 * pr + i] = rows(0, pr, i);
-#pragma unroll 1
+  float2 W0 = z0, W1 = z0, W2 = z0, W3 = z0, W4 = z0, G0 = z0, G1 = z0, G2 = z0, H0 = z0;
+  float o102 = 0.f, o003 = 0.f;
+  SliceData nt = src.load(0);
+  // whole where no scatter follows each slice (the phi-only sweep at 512^3 /
+  // nside 256 / 256 steps: 217 -> 200 ms), by two with it (fully unrolled it
+  // costs more in instruction fetch than it saves: 58.7 against 60.6 ms for a
+  // 256^3 / nside 128 / 128 steps vjp, 59.3 in a loop)
+  constexpr int kUnroll = std::is_same<Acc, AccNone>::value ? 4 : 2;
+#pragma unroll kUnroll
   for (int c = 0; c < 4; ++c) {
-    float2 s00 = z0, s01 = z0, s02 = z0, s03 = z0, s10 = z0, s11 = z0, s12 = z0, s20 = z0, s21 = z0, s30 = z0;
     // this slice's z weights by selection (an indexed read of Z would put
     // it in local memory)
-    const float zwc = c == 0 ? Z.w[0] : (c == 1 ? Z.w[1] : (c == 2 ? Z.w[2] : Z.w[3]));
-    const float zgc = c == 0 ? Z.g[0] : (c == 1 ? Z.g[1] : (c == 2 ? Z.g[2] : Z.g[3]));
-    const float zhc = c == 0 ? Z.h[0] : (c == 1 ? Z.h[1] : (c == 2 ? Z.h[2] : Z.h[3]));
-    const float zkc = c == 0 ? Z.k[0] : (c == 1 ? Z.k[1] : (c == 2 ? Z.k[2] : Z.k[3]));
-    const float2 zw = dup2(zwc), zg = dup2(zgc), zh = dup2(zhc);
-    float2 ct[8];
-    for (int i = 0; i < 8; ++i) ct[i] = nt[i];
-    if constexpr (kPackedZ) {  // the last slice reloads itself: no branch in the loop
-      const int cn = c < 3 ? c + 1 : 3;
-      for (int pr = 0; pr < 2; ++pr)
-        for (int i = 0; i < 4; ++i) nt[4 * pr + i] = rows(cn, pr, i);
-    } else if (c < 3) {  // (fewer registers where the scatter's working set is live)
-      for (int pr = 0; pr < 2; ++pr)
-        for (int i = 0; i < 4; ++i) nt[4 * pr + i] = rows(c + 1, pr, i);
+    const float zw = c == 0 ? Z.w[0] : (c == 1 ? Z.w[1] : (c == 2 ? Z.w[2] : Z.w[3]));
+    const float zg = c == 0 ? Z.g[0] : (c == 1 ? Z.g[1] : (c == 2 ? Z.g[2] : Z.g[3]));
+    const float zh = c == 0 ? Z.h[0] : (c == 1 ? Z.h[1] : (c == 2 ? Z.h[2] : Z.h[3]));
+    const float zk = c == 0 ? -3.f : (c == 1 ? 9.f : (c == 2 ? -9.f : 3.f));
+    XRow x[2];
+    {
+      const SliceData ct = nt;
+      nt = src.load(c < 3 ? c + 1 : 3);  // the last slice reloads itself: no branch in the loop
+      Src::template x_pass<true>(ct, xd, x);
     }
+    const YIn v = Src::at(x[0].v, x[1].v), g = Src::at(x[0].g, x[1].g), h = Src::at(x[0].h, x[1].h),
+              k = Src::at(x[0].k, x[1].k);
+    const float mv = v.v2 - v.v1, mg = g.v2 - g.v1, mh = h.v2 - h.v1, mk = k.v2 - k.v1;
+    const float s00 = y_value(Y, v, mv), s01 = y_first(Y, v, mv), s02 = y_second(Y, v), s03 = v.e2 - v.e1;
+    const float s10 = y_value(Y, g, mg), s11 = y_first(Y, g, mg), s12 = y_second(Y, g);
+    const float s20 = y_value(Y, h, mh), s21 = y_first(Y, h, mh), s30 = y_value(Y, k, mk);
+    const float2 P0 = make_float2(s00, s01), P1 = make_float2(s10, s11), P2 = make_float2(s02, s20);
+    W0 = ffma2(dup2(zw), P0, W0);
+    W1 = ffma2(dup2(zw), P1, W1);
+    W2 = ffma2(dup2(zw), P2, W2);
+    W3 = ffma2(dup2(zw), make_float2(s12, s21), W3);
+    W4 = ffma2(dup2(zw), make_float2(s03, s30), W4);
+    G0 = ffma2(dup2(zg), P0, G0);
+    G1 = ffma2(dup2(zg), P1, G1);
+    G2 = ffma2(dup2(zg), P2, G2);
+    H0 = ffma2(dup2(zh), P0, H0);
+    o102 = fmaf(zh, s10, o102);
+    o003 = fmaf(zk, s00, o003);
+    if (scatter) {
+      // per order in x, the cotangents of the row's value and second difference
+      // along y at rows 1 and 2: (value, difference) pairs per row
+      const float a0 = fmaf(qb[0], zw, fmaf(qb[3], zg, qb[9] * zh)), a1 = fmaf(qb[2], zw, qb[8] * zg), a2 = qb[7] * zw;
+      const float b0 = fmaf(qb[1], zw, qb[6] * zg), b1 = qb[5] * zw, c0 = qb[4] * zw;
+      const float w2 = fmaf(Y.t, a0, a1), g2 = fmaf(Y.t, b0, b1), h2 = Y.t * c0;
+      const float2 Cw[2] = {make_float2(a0 - w2, fmaf(Y.w0, a0, fmaf(Y.g0, a1, Y.h0 * a2))),
+                            make_float2(w2, fmaf(Y.w3, a0, fmaf(Y.g3, a1, Y.h3 * a2)))};
+      const float2 Cg[2] = {make_float2(b0 - g2, fmaf(Y.w0, b0, Y.g0 * b1)),
+                            make_float2(g2, fmaf(Y.w3, b0, Y.g3 * b1))};
+      const float2 Ch[2] = {make_float2(c0 - h2, Y.w0 * c0), make_float2(h2, Y.w3 * c0)};
+      const int64_t row = sc.base + c * sc.pxy, px = sc.px;
+      float2 p1[2], p2[2], e1[2], e2[2];
 #pragma unroll
-    for (int pr = 0; pr < 2; ++pr) {
-      const float2 t0 = ct[4 * pr], t1 = ct[4 * pr + 1], t2 = ct[4 * pr + 2], t3 = ct[4 * pr + 3];
-      float2 r0 = fmul2(xw[0], t0), r1 = fmul2(xg[0], t0), r2 = fmul2(xh[0], t0), r3 = fmul2(dup2(X.k[0]), t0);
-      r0 = ffma2(xw[1], t1, r0);
-      r1 = ffma2(xg[1], t1, r1);
-      r2 = ffma2(xh[1], t1, r2);
-      r3 = ffma2(dup2(X.k[1]), t1, r3);
-      r0 = ffma2(xw[2], t2, r0);
-      r1 = ffma2(xg[2], t2, r1);
-      r2 = ffma2(xh[2], t2, r2);
-      r3 = ffma2(dup2(X.k[2]), t2, r3);
-      r0 = ffma2(xw[3], t3, r0);
-      r1 = ffma2(xg[3], t3, r1);
-      r2 = ffma2(xh[3], t3, r2);
-      r3 = ffma2(dup2(X.k[3]), t3, r3);
-      s00 = ffma2(yw[pr], r0, s00);
-      s01 = ffma2(yg[pr], r0, s01);
-      s02 = ffma2(yh[pr], r0, s02);
-      s03 = ffma2(yk[pr], r0, s03);
-      s10 = ffma2(yw[pr], r1, s10);
-      s11 = ffma2(yg[pr], r1, s11);
-      s12 = ffma2(yh[pr], r1, s12);
-      s20 = ffma2(yw[pr], r2, s20);
-      s21 = ffma2(yg[pr], r2, s21);
-      s30 = ffma2(yw[pr], r3, s30);
-      if (scatter) {  // tap cotangents of the two rows
-        const float2 Cw = ffma2(zw, Aw[pr], ffma2(zg, Bw[pr], fmul2(zh, Dw[pr])));
-        const float2 Cg = ffma2(zw, Ag[pr], fmul2(zg, Bg[pr]));
-        const float2 Ch = fmul2(zw, Ah[pr]);
-        float2 v[4];
-        for (int i = 0; i < 4; ++i) v[i] = ffma2(xw[i], Cw, ffma2(xg[i], Cg, fmul2(xh[i], Ch)));
-        const int64_t row = base + c * pxy + 2 * pr * px;
-        acc.add_row(row, v[0].x, v[1].x, v[2].x, v[3].x);
-        acc.add_row(row + px, v[0].y, v[1].y, v[2].y, v[3].y);
+      for (int j = 0; j < 2; ++j) {
+        p2[j] = ffma2(xd.t, Cw[j], Cg[j]);
+        p1[j] = fsub2(Cw[j], p2[j]);
+        e1[j] = ffma2(xd.w0, Cw[j], ffma2(xd.g0, Cg[j], fmul2(xd.h0, Ch[j])));
+        e2[j] = ffma2(xd.w3, Cw[j], ffma2(xd.g3, Cg[j], fmul2(xd.h3, Ch[j])));
+        if constexpr (TakesCells<Acc>::value) {
+          acc.add_cell(row + (j + 1) * px + 1, make_float4(p1[j].x, p1[j].y, e1[j].x, e1[j].y));
+          acc.add_cell(row + (j + 1) * px + 2, make_float4(p2[j].x, p2[j].y, e2[j].x, e2[j].y));
+        }
+      }
+      if constexpr (!TakesCells<Acc>::value) {
+        const float2 n2 = dup2(-2.f);
+        float2 t[2][4];  // taps along x of (value, difference along y) at rows 1 and 2
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          t[j][0] = e1[j];
+          t[j][1] = fadd2(ffma2(n2, e1[j], p1[j]), e2[j]);
+          t[j][2] = fadd2(ffma2(n2, e2[j], p2[j]), e1[j]);
+          t[j][3] = e2[j];
+        }
+        float r1[4], r2[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          r1[i] = fmaf(-2.f, t[0][i].y, t[0][i].x) + t[1][i].y;
+          r2[i] = fmaf(-2.f, t[1][i].y, t[1][i].x) + t[0][i].y;
+        }
+        acc.add_row(row, t[0][0].y, t[0][1].y, t[0][2].y, t[0][3].y);
+        acc.add_row(row + px, r1[0], r1[1], r1[2], r1[3]);
+        acc.add_row(row + 2 * px, r2[0], r2[1], r2[2], r2[3]);
+        acc.add_row(row + 3 * px, t[1][0].y, t[1][1].y, t[1][2].y, t[1][3].y);
       }
     }
-    if constexpr (kPackedZ) {
-      const float2 P0 = make_float2(s00.x + s00.y, s10.x + s10.y), P1 = make_float2(s01.x + s01.y, s11.x + s11.y);
-      const float2 P2 = make_float2(s02.x + s02.y, s12.x + s12.y), P3 = make_float2(s20.x + s20.y, s21.x + s21.y);
-      const float2 P4 = make_float2(s03.x + s03.y, s30.x + s30.y);
-      W0 = ffma2(zw, P0, W0);
-      W1 = ffma2(zw, P1, W1);
-      W2 = ffma2(zw, P2, W2);
-      W3 = ffma2(zw, P3, W3);
-      W4 = ffma2(zw, P4, W4);
-      G0 = ffma2(zg, P0, G0);
-      G1 = ffma2(zg, P1, G1);
-      G2 = ffma2(zg, P2, G2);
-      G3 = ffma2(zg, P3, G3);
-      H0 = ffma2(zh, P0, H0);
-      H1 = ffma2(zh, P1, H1);
-      K0 = ffma2(dup2(zkc), P0, K0);
-    } else {
-      const float S00 = s00.x + s00.y, S01 = s01.x + s01.y, S02 = s02.x + s02.y, S03 = s03.x + s03.y;
-      const float S10 = s10.x + s10.y, S11 = s11.x + s11.y, S12 = s12.x + s12.y;
-      const float S20 = s20.x + s20.y, S21 = s21.x + s21.y, S30 = s30.x + s30.y;
-      o000 += zwc * S00; o001 += zgc * S00; o002 += zhc * S00; o003 += zkc * S00;
-      o010 += zwc * S01; o011 += zgc * S01; o012 += zhc * S01;
-      o020 += zwc * S02; o021 += zgc * S02;
-      o030 += zwc * S03;
-      o100 += zwc * S10; o101 += zgc * S10; o102 += zhc * S10;
-      o110 += zwc * S11; o111 += zgc * S11;
-      o120 += zwc * S12;
-      o200 += zwc * S20; o201 += zgc * S20;
-      o210 += zwc * S21;
-      o300 += zwc * S30;
-    }
   }
-  if constexpr (kPackedZ) {
-    o000 = W0.x, o100 = W0.y, o010 = W1.x, o110 = W1.y, o020 = W2.x, o120 = W2.y;
-    o200 = W3.x, o210 = W3.y, o030 = W4.x, o300 = W4.y;
-    o001 = G0.x, o101 = G0.y, o011 = G1.x, o111 = G1.y, o021 = G2.x, o201 = G3.x;
-    o002 = H0.x, o102 = H0.y, o012 = H1.x, o003 = K0.x;
-  }
-  Q.v = o000;
-  Q.g[0] = o100;
-  Q.g[1] = o010;
-  Q.g[2] = o001;
-  Q.h[0] = o200;
-  Q.h[1] = o110;
-  Q.h[2] = o101;
-  Q.h[3] = o020;
-  Q.h[4] = o011;
-  Q.h[5] = o002;
-  xb[0] += qb[0] * o100 + qb[1] * o200 + qb[2] * o110 + qb[3] * o101 + qb[4] * o300 + qb[5] * o210 +
-           qb[6] * o201 + qb[7] * o120 + qb[8] * o111 + qb[9] * o102;
-  xb[1] += qb[0] * o010 + qb[1] * o110 + qb[2] * o020 + qb[3] * o011 + qb[4] * o210 + qb[5] * o120 +
-           qb[6] * o111 + qb[7] * o030 + qb[8] * o021 + qb[9] * o012;
-  xb[2] += qb[0] * o001 + qb[1] * o101 + qb[2] * o011 + qb[3] * o002 + qb[4] * o201 + qb[5] * o111 +
-           qb[6] * o102 + qb[7] * o021 + qb[8] * o012 + qb[9] * o003;
-}
-
-// One field's pass: FP32 (MIXED) in the packed form, reading the row-pair
-// array (PAIR) or the single layout; FP64 in the plain form.
-template <bool PAIR, typename T, typename Acc>
-SRT_HD void field_pass(const float* f, const float2* fp, int64_t base, int64_t basep, const Geom& G, const T* t,
-                       const T* qb, Tri<T>& Q, T* xb, const Acc& acc) {
-  if constexpr (sizeof(T) == sizeof(float)) {
-    if constexpr (PAIR)
-      tricubic_vjp_pair<Acc>(PairRows{fp, basep, G.px, G.pxy2}, base, G.px, G.pxy, t[0], t[1], t[2], qb, Q, xb, acc);
-    else
-      tricubic_vjp_pair<Acc>(SingleRows{f, base, G.px, G.pxy}, base, G.px, G.pxy, t[0], t[1], t[2], qb, Q, xb, acc);
-  } else {
-    tricubic_vjp<T, Acc>(f, base, G.px, G.pxy, t[0], t[1], t[2], qb, Q, xb, acc);
-  }
+  const float o030 = 3.f * W4.x, o300 = 3.f * W4.y;
+  Q.v = W0.x;
+  Q.g[0] = W1.x;
+  Q.g[1] = W0.y;
+  Q.g[2] = G0.x;
+  Q.h[0] = W2.y;
+  Q.h[1] = W1.y;
+  Q.h[2] = G1.x;
+  Q.h[3] = W2.x;
+  Q.h[4] = G0.y;
+  Q.h[5] = H0.x;
+  // o000 W0.x, o010 W0.y, o100 W1.x, o110 W1.y, o020 W2.x, o200 W2.y, o120 W3.x,
+  // o210 W3.y, o001 G0.x, o011 G0.y, o101 G1.x, o111 G1.y, o021 G2.x, o201 G2.y,
+  // o002 H0.x, o012 H0.y: xb_j += qb . dQ/dx_j
+  xb[0] += qb[0] * W1.x + qb[1] * W2.y + qb[2] * W1.y + qb[3] * G1.x + qb[4] * o300 + qb[5] * W3.y + qb[6] * G2.y +
+           qb[7] * W3.x + qb[8] * G1.y + qb[9] * o102;
+  xb[1] += qb[0] * W0.y + qb[1] * W1.y + qb[2] * W2.x + qb[3] * G0.y + qb[4] * W3.y + qb[5] * W3.x + qb[6] * G1.y +
+           qb[7] * o030 + qb[8] * G2.x + qb[9] * H0.y;
+  xb[2] += qb[0] * G0.x + qb[1] * G1.x + qb[2] * G0.y + qb[3] * H0.x + qb[4] * G2.y + qb[5] * G1.y + qb[6] * o102 +
+           qb[7] * G2.x + qb[8] * H0.y + qb[9] * o003;
 }
 
 // -------------------------------------------------------- stage and core
@@ -425,7 +410,8 @@ struct StageView {
   T A, Ap, s1, s2, e1, e2;
   bool branch;         // dA > 1/2
   int64_t base[4];     // padded base index per field: B_x, B_y, B_z, phi
-  int64_t basep[4];    // the same cells in the row-pair layout
+  int64_t basep[4];    // the same cells in the row-pair layout (kPairs)
+  int hbase[4];        // the same cells near the observer (hot_base; MIXED)
   T t[4][3];           // cell offsets per field and axis
 };
 
@@ -434,210 +420,198 @@ SRT_HD int sym_idx(int i, int j) {
   return (i == j) ? (i == 0 ? 0 : (i == 1 ? 3 : 5)) : ((i + j == 1) ? 1 : ((i + j == 2) ? 2 : 4));
 }
 
+// One field's pass: FP32 (MIXED) from the handle's layout; FP64 in the plain form.
+template <int LAYOUT, typename T, typename Acc>
+SRT_HD void field_pass(const FieldPtrs& F, int f, const StageView<T>& V, const Geom& G, const T* qb, Tri<T>& Q, T* xb,
+                       const Acc& acc) {
+  const int64_t base = V.base[f], basep = V.basep[f];
+  const T* t = V.t[f];
+  if constexpr (sizeof(T) == sizeof(float)) {
+    Scatter sc{base, G.px, G.pxy};
+    if constexpr (TakesCells<Acc>::value) sc = acc.place(base, V.hbase[f], G);
+    tricubic_vjp_mixed<Acc>(cell_source<LAYOUT>(F, G, f, base, basep), sc, t[0], t[1], t[2], qb, Q, xb, acc);
+  } else
+    tricubic_vjp<T, Acc>(f == 3 ? F.phi : F.b[f], base, G.px, G.pxy, G.ts, t[0], t[1], t[2], qb, Q, xb, acc);
+}
+
+SRT_HD float fm(float a, float b, float c) { return fmaf(a, b, c); }
+SRT_HD double fm(double a, double b, double c) { return fma(a, b, c); }
 template <typename T>
-SRT_HD T symv(const T* h, int i, int j) { return h[sym_idx(i, j)]; }
+SRT_HD T vdot(const T* a, const T* b) { return fm(a[2], b[2], fm(a[1], b[1], a[0] * b[0])); }
+// Row i of a symmetric matrix (xx xy xz yy yz zz) times v.
+template <typename T>
+SRT_HD T sym_row(const T* h, int i, const T* v) {
+  return fm(h[sym_idx(i, 2)], v[2], fm(h[sym_idx(i, 1)], v[1], h[sym_idx(i, 0)] * v[0]));
+}
+
+// What the B components' passes share. Cotangents, known before any field is
+// read: u = (n.grad B)bar + e1bar e1 / 2 + e2bar e2 / 2, h1 = e1bar / 2,
+// h2 = e2bar / 2, Tb that of the tidal matrix and D its diagonal plus that of
+// n . Laplacian B. Sums over the components as BSums64's (Gn = G n,
+// ngB = G^T n, S = sum_C n_C H_C, K_ij = (H_i n)_j + (H_j n)_i).
+template <typename T>
+struct BVjp {
+  T u[3], h1, h2, Tb[6], D[3];
+  T Gn[3], ngB[3], S[6], K[6], nlap;
+};
 
 // One B component's share of rhs_vjp: its cotangents (value, gradient,
-// Hessian) from the state-only intermediate cotangents, the fused pass, the
-// forward aggregates and its terms of the state cotangents.
-template <int C, bool PAIR, typename T, typename Acc>
-SRT_HD void vjp_b_component(const StageView<T>& V, const FieldPtrs& F, const Geom& G, const T* fb, const T* ngBb, T e1b,
-                            T e2b, T nlapb, const T* Tb, const Acc& acc, T* xb, T* nb, T* ab, T* bb, T* ngB, T& e1ngB,
-                            T& e2ngB, T& nlap, T* Tm) {
+// Hessian), the fused pass, the forward sums and its terms of nb, the cotangent
+// of n (those of e1 and e2 follow from the sums).
+template <int C, int LAYOUT, typename T, typename Acc>
+SRT_HD void vjp_b_component(const StageView<T>& V, const FieldPtrs& F, const Geom& G, const T* fb, BVjp<T>& B,
+                            const Acc& acc, T* xb, T* nb) {
   const T* n = V.n;
-  const T* a = V.a;
-  const T* b = V.b;
-  const T nc = n[C], ac = a[C], bc = b[C];
+  const T nc = n[C], n2 = T(2) * nc, kap = fm(B.h1, V.a[C], B.h2 * V.b[C]);
+  const T Tc[3] = {B.Tb[sym_idx(C, 0)], B.Tb[sym_idx(C, 1)], B.Tb[sym_idx(C, 2)]};
   T qb[10];
   qb[0] = -fb[C];
-  for (int i = 0; i < 3; ++i)
-    qb[1 + i] = nc * ngBb[i] + T(0.5) * e1b * (ac * n[i] + nc * a[i]) + T(0.5) * e2b * (bc * n[i] + nc * b[i]);
-  // Hessian cotangent: n_c Tb + n_c nlapb I - sym(e_c Tb_c. (x) n)
-  for (int i = 0; i < 3; ++i)
-    for (int j = i; j < 3; ++j) {
-      T m = nc * symv(Tb, i, j) + ((i == j) ? nc * nlapb : T(0));
-      m -= T(0.5) * (symv(Tb, C, i) * n[j] + symv(Tb, C, j) * n[i]);
-      // unique components: off-diagonals hold both halves
-      qb[4 + sym_idx(i, j)] = (i == j) ? m : T(2) * m;
-    }
-  Tri<T> Q;
-  field_pass<PAIR, T, Acc>(F.b[C], F.pr[C], V.base[C], V.basep[C], G, V.t[C], qb, Q, xb, acc);
-  // forward aggregates
-  for (int i = 0; i < 3; ++i) ngB[i] += Q.g[i] * nc;
-  const T gn = Q.g[0] * n[0] + Q.g[1] * n[1] + Q.g[2] * n[2];
-  const T ga = Q.g[0] * a[0] + Q.g[1] * a[1] + Q.g[2] * a[2];
-  const T gbb = Q.g[0] * b[0] + Q.g[1] * b[1] + Q.g[2] * b[2];
-  e1ngB += T(0.5) * (ac * gn + nc * ga);
-  e2ngB += T(0.5) * (bc * gn + nc * gbb);
-  T Hn[3];
-  for (int i = 0; i < 3; ++i) Hn[i] = symv(Q.h, i, 0) * n[0] + symv(Q.h, i, 1) * n[1] + symv(Q.h, i, 2) * n[2];
-  for (int i = 0; i < 3; ++i)
-    for (int j = i; j < 3; ++j) {
-      T d = Q.h[sym_idx(i, j)] * nc;
-      if (i == C) d -= T(0.5) * Hn[j];
-      if (j == C) d -= T(0.5) * Hn[i];
-      Tm[sym_idx(i, j)] += d;
-    }
-  const T trH = Q.h[0] + Q.h[3] + Q.h[5];
-  nlap += trH * nc;
-  // this component's share of the state cotangents
-  T HT = 0;  // H_c : Tb (full contraction)
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) HT += symv(Q.h, i, j) * symv(Tb, i, j);
-  nb[C] += Q.g[0] * ngBb[0] + Q.g[1] * ngBb[1] + Q.g[2] * ngBb[2] + trH * nlapb + HT + T(0.5) * e1b * ga +
-           T(0.5) * e2b * gbb;
-  for (int k = 0; k < 3; ++k) {
-    T tk = 0;
-    for (int j = 0; j < 3; ++j) tk += symv(Tb, C, j) * symv(Q.h, j, k);
-    nb[k] += T(0.5) * e1b * ac * Q.g[k] + T(0.5) * e2b * bc * Q.g[k] - tk;
-    ab[k] += T(0.5) * e1b * nc * Q.g[k];
-    bb[k] += T(0.5) * e2b * nc * Q.g[k];
+  for (int i = 0; i < 3; ++i) qb[1 + i] = fm(nc, B.u[i], kap * n[i]);
+  // Hessian cotangent n_c (Tb + nlapb I) - sym(Tb_c. (x) n), off-diagonals
+  // holding both halves
+  for (int i = 0; i < 3; ++i) {
+    qb[4 + sym_idx(i, i)] = fm(nc, B.D[i], -(Tc[i] * n[i]));
+    for (int j = i + 1; j < 3; ++j)
+      qb[4 + sym_idx(i, j)] = fm(n2, B.Tb[sym_idx(i, j)], -fm(Tc[i], n[j], Tc[j] * n[i]));
   }
-  ab[C] += T(0.5) * e1b * gn;
-  bb[C] += T(0.5) * e2b * gn;
+  Tri<T> Q;
+  field_pass<LAYOUT, T, Acc>(F, C, V, G, qb, Q, xb, acc);
+  for (int i = 0; i < 3; ++i) B.ngB[i] = fm(Q.g[i], nc, C == 0 ? T(0) : B.ngB[i]);
+  B.Gn[C] = vdot(Q.g, n);
+  B.nlap = fm(nc, Q.h[0] + Q.h[3] + Q.h[5], C == 0 ? T(0) : B.nlap);
+  for (int k = 0; k < 6; ++k) B.S[k] = fm(nc, Q.h[k], C == 0 ? T(0) : B.S[k]);
+  for (int i = 0; i < 3; ++i) {
+    const T Hn = sym_row(Q.h, i, n);
+    T& k = B.K[sym_idx(C, i)];  // met at component min(i, C) first, max(i, C) second
+    k = i == C ? Hn + Hn : (i > C ? Hn : k + Hn);
+  }
+  // H_c : (Tb + nlapb I)
+  const T HT = fm(Q.h[0], B.D[0], fm(Q.h[3], B.D[1], Q.h[5] * B.D[2])) +
+               T(2) * fm(Q.h[1], B.Tb[1], fm(Q.h[2], B.Tb[2], Q.h[4] * B.Tb[4]));
+  nb[C] += vdot(Q.g, B.u) + HT;
+  for (int k = 0; k < 3; ++k) nb[k] += fm(kap, Q.g[k], -sym_row(Q.h, k, Tc));
 }
 
 // yb += J(u)^T fb for the stage described by V; tap cotangents go to accb[0..2]
 // (B_x, B_y, B_z) and accp (phi).
-template <typename T, typename AccB, typename AccP, bool PAIR = false>
+template <typename T, typename AccB, typename AccP, int LAYOUT = kPlanes>
 SRT_HD void rhs_vjp(const StageView<T>& V, const FieldPtrs& F, const Geom& G, const T* fb, T* yb, const AccB* accb,
                     const AccP& accp) {
   const T* n = V.n;
   const T* a = V.a;
   const T* b = V.b;
   // ---- intermediate cotangents (state only)
-  const T nfx = n[0] * fb[0] + n[1] * fb[1] + n[2] * fb[2];
-  const T nfn = n[0] * fb[3] + n[1] * fb[4] + n[2] * fb[5];
-  const T sab = -(n[0] * fb[6] + n[1] * fb[7] + n[2] * fb[8]);
-  const T sbb = -(n[0] * fb[9] + n[1] * fb[10] + n[2] * fb[11]);
-  const T phib = T(-2) * nfx;
+  const T nfx = vdot(n, fb), nfn = vdot(n, fb + 3);
+  const T e1b = -vdot(n, fb + 6), e2b = -vdot(n, fb + 9);
   T vb[3];
-  for (int i = 0; i < 3; ++i) vb[i] = fb[3 + i] - n[i] * nfn;
-  const T agb = T(2) * sab, bgb = T(2) * sbb, e1b = sab, e2b = sbb;
+  for (int i = 0; i < 3; ++i) vb[i] = fm(-n[i], nfn, fb[3 + i]);
   T Apb = -fb[12];
-  const T Lb = T(-4) * V.Ap * fb[13] + T(4) * V.s1 * fb[14] + T(4) * V.s2 * fb[15];
-  const T PHb = -V.A * fb[13];
-  const T nlapb = T(0.5) * V.A * fb[13];
-  const T S1b = V.A * V.A * fb[14], S2b = V.A * V.A * fb[15];
+  const T Lb = T(4) * fm(V.s1, fb[14], fm(V.s2, fb[15], -(V.Ap * fb[13])));
+  const T PHb = -V.A * fb[13], nlapb = T(0.5) * V.A * fb[13];
+  const T A2 = V.A * V.A;
+  const T S1b = A2 * fb[14], S2b = A2 * fb[15];
   // the dA > 1/2 branch's terms, formed either way and selected (no branch;
   // where dA = 0 they are not finite and not selected)
   T Ab = 0, s1b = 0, s2b = 0, el1b = 0, el2b = 0;
   {
-    const T A2 = V.A * V.A, A3 = A2 * V.A;
-    const T q = sqrt(T(4) + V.e1 * V.e1 + V.e2 * V.e2);
-    T bs1 = T(2) * V.s1 / A3 * fb[13];
-    T bs2 = T(2) * V.s2 / A3 * fb[13];
-    T bA = T(-3) * (V.s1 * V.s1 + V.s2 * V.s2) / (A3 * V.A) * fb[13];
-    bs1 += T(-2) * q / A2 * fb[16];
-    T qb = T(-2) * V.s1 / A2 * fb[16];
-    bA += T(4) * V.s1 * q / A3 * fb[16];
-    bs2 += T(-2) * q / A2 * fb[17];
-    qb += T(-2) * V.s2 / A2 * fb[17];
-    bA += T(4) * V.s2 * q / A3 * fb[17];
-    const T D = A2 * (T(2) + q), N = V.s1 * V.e2 - V.s2 * V.e1;
-    const T Nb = -fb[18] / D, Db = N * fb[18] / (D * D);
-    bs1 += V.e2 * Nb;
-    T be2 = V.s1 * Nb;
-    bs2 += -V.e1 * Nb;
-    T be1 = -V.s2 * Nb;
-    bA += T(2) * V.A * (T(2) + q) * Db;
-    qb += A2 * Db;
-    be1 += V.e1 / q * qb;
-    be2 += V.e2 / q * qb;
+    const T iA = T(1) / V.A, iA2 = iA * iA, iA3 = iA2 * iA;
+    const T q = sqrt(fm(V.e2, V.e2, fm(V.e1, V.e1, T(4))));
+    const T iD = T(1) / (A2 * (T(2) + q));  // of the rotation's quotient N / D
+    const T N = fm(V.s1, V.e2, -(V.s2 * V.e1)), Nb = -fb[18] * iD, NN = N * Nb;  // D times D's cotangent is -NN
+    const T sf = fm(V.s1, fb[16], V.s2 * fb[17]), c13 = T(2) * iA3 * fb[13], cq = T(-2) * q * iA2;
+    const T bs1 = fm(V.s1, c13, fm(cq, fb[16], V.e2 * Nb)), bs2 = fm(V.s2, c13, fm(cq, fb[17], -(V.e1 * Nb)));
+    const T bA = iA * (T(-1.5) * fm(V.s1, V.s1, V.s2 * V.s2) * c13 + T(-2) * fm(cq, sf, NN));
+    const T qq = fm(T(-2) * iA2, sf, -(A2 * iD) * NN) / q;  // q's cotangent over q
     s1b = V.branch ? bs1 : T(0);
     s2b = V.branch ? bs2 : T(0);
     Ab = V.branch ? bA : T(0);
-    el1b = V.branch ? be1 : T(0);
-    el2b = V.branch ? be2 : T(0);
+    el1b = V.branch ? fm(V.e1, qq, -(V.s2 * Nb)) : T(0);
+    el2b = V.branch ? fm(V.e2, qq, V.s1 * Nb) : T(0);
   }
-  // cotangent of the effective tidal matrix He = H + T/2 (full symmetric)
-  T Heb[6];
-  for (int i = 0; i < 3; ++i)
-    for (int j = i; j < 3; ++j)
-      Heb[sym_idx(i, j)] = (a[i] * a[j] - b[i] * b[j]) * S1b + (a[i] * b[j] + b[i] * a[j]) * S2b;
-  T Tb[6];
-  for (int u = 0; u < 6; ++u) Tb[u] = T(0.5) * Heb[u];
-  T gb[3], ngBb[3];
+  // cotangent of the effective tidal matrix He = H + T/2:
+  // (a a - b b) S1b + (a b + b a) S2b = a p + b r, symmetric
+  T p[3], r[3], Heb[6];
   for (int i = 0; i < 3; ++i) {
-    gb[i] = T(2) * vb[i] + agb * a[i] + bgb * b[i] + n[i] * Lb;
-    ngBb[i] = vb[i] + T(0.25) * n[i] * Lb;
+    p[i] = fm(S1b, a[i], S2b * b[i]);
+    r[i] = fm(S2b, a[i], -(S1b * b[i]));
   }
-  T nb[3] = {0, 0, 0}, ab[3] = {0, 0, 0}, bb[3] = {0, 0, 0}, xb[3] = {0, 0, 0};
-  // aggregates of the forward
-  T ngB[3] = {0, 0, 0}, e1ngB = 0, e2ngB = 0, nlap = 0, Tm[6] = {0, 0, 0, 0, 0, 0};
+  for (int i = 0; i < 3; ++i)
+    for (int j = i; j < 3; ++j) Heb[sym_idx(i, j)] = fm(a[i], p[j], b[i] * r[j]);
+  BVjp<T> B;
+  B.h1 = T(0.5) * e1b;
+  B.h2 = T(0.5) * e2b;
+  for (int k = 0; k < 6; ++k) B.Tb[k] = T(0.5) * Heb[k];
+  for (int i = 0; i < 3; ++i) {
+    B.D[i] = B.Tb[sym_idx(i, i)] + nlapb;
+    const T ngBb = fm(T(0.25) * n[i], Lb, vb[i]);
+    B.u[i] = fm(B.h1, a[i], fm(B.h2, b[i], ngBb));
+  }
+  T nb[3] = {0, 0, 0}, xb[3] = {0, 0, 0};
 
   // ---- B components (compile-time component index: no local-memory arrays)
-  vjp_b_component<0, PAIR, T, AccB>(V, F, G, fb, ngBb, e1b, e2b, nlapb, Tb, accb[0], xb, nb, ab, bb, ngB, e1ngB, e2ngB,
-                                    nlap, Tm);
-  vjp_b_component<1, PAIR, T, AccB>(V, F, G, fb, ngBb, e1b, e2b, nlapb, Tb, accb[1], xb, nb, ab, bb, ngB, e1ngB, e2ngB,
-                                    nlap, Tm);
-  vjp_b_component<2, PAIR, T, AccB>(V, F, G, fb, ngBb, e1b, e2b, nlapb, Tb, accb[2], xb, nb, ab, bb, ngB, e1ngB, e2ngB,
-                                    nlap, Tm);
+  vjp_b_component<0, LAYOUT, T, AccB>(V, F, G, fb, B, accb[0], xb, nb);
+  vjp_b_component<1, LAYOUT, T, AccB>(V, F, G, fb, B, accb[1], xb, nb);
+  vjp_b_component<2, LAYOUT, T, AccB>(V, F, G, fb, B, accb[2], xb, nb);
 
   // ---- phi
   Tri<T> P;
   {
     T qb[10];
-    qb[0] = phib;
-    for (int i = 0; i < 3; ++i) qb[1 + i] = gb[i];
+    qb[0] = T(-2) * nfx;
     for (int i = 0; i < 3; ++i)
-      for (int j = i; j < 3; ++j) {
-        const T m = Heb[sym_idx(i, j)] + (n[i] * n[j] - ((i == j) ? T(1) : T(0))) * PHb;
-        qb[4 + sym_idx(i, j)] = (i == j) ? m : T(2) * m;
-      }
-    field_pass<PAIR, T, AccP>(F.phi, F.pr[3], V.base[3], V.basep[3], G, V.t[3], qb, P, xb, accp);
+      qb[1 + i] = fm(T(2), fm(e1b, a[i], fm(e2b, b[i], vb[i])), n[i] * Lb);
+    for (int i = 0; i < 3; ++i) {
+      const T t = n[i] * PHb;
+      qb[4 + sym_idx(i, i)] = fm(n[i], t, Heb[sym_idx(i, i)] - PHb);
+      for (int j = i + 1; j < 3; ++j) qb[4 + sym_idx(i, j)] = T(2) * fm(t, n[j], Heb[sym_idx(i, j)]);
+    }
+    field_pass<LAYOUT, T, AccP>(F, 3, V, G, qb, P, xb, accp);
   }
   const T* g = P.g;
+  // ---- the rest of n's cotangent, and those of e1, e2 and the scalars
+  T v[3], w[3], Hn[3];
   for (int i = 0; i < 3; ++i) {
-    nb[i] += -(T(1) + T(2) * P.v) * fb[i];
-    ab[i] += agb * g[i];
-    bb[i] += bgb * g[i];
-    nb[i] += T(2) * PHb * (symv(P.h, i, 0) * n[0] + symv(P.h, i, 1) * n[1] + symv(P.h, i, 2) * n[2]);
+    v[i] = fm(T(2), g[i], B.ngB[i]);
+    w[i] = fm(T(0.5), B.Gn[i] + B.ngB[i], T(2) * g[i]);  // e.w = 2 e.grad phi + e.n.grad B
+    Hn[i] = sym_row(P.h, i, n);
   }
-
-  // ---- terms of the field aggregates
-  T v[3];
-  for (int i = 0; i < 3; ++i) v[i] = T(2) * g[i] + ngB[i];
-  const T nv = n[0] * v[0] + n[1] * v[1] + n[2] * v[2];
-  const T sa = T(2) * (a[0] * g[0] + a[1] * g[1] + a[2] * g[2]) + e1ngB;
-  const T sb = T(2) * (b[0] * g[0] + b[1] * g[1] + b[2] * g[2]) + e2ngB;
-  const T L = n[0] * g[0] + n[1] * g[1] + n[2] * g[2] + T(0.25) * (n[0] * ngB[0] + n[1] * ngB[1] + n[2] * ngB[2]);
+  const T nv = vdot(n, v), sa = vdot(a, w), sb = vdot(b, w);
+  const T L4 = fm(T(4), vdot(n, g), vdot(n, B.ngB)), phi1 = fm(T(2), P.v, T(1)), PH2 = T(2) * PHb;
   for (int i = 0; i < 3; ++i) {
-    nb[i] += -nv * fb[3 + i] - v[i] * nfn;
-    nb[i] += -sa * fb[6 + i] - sb * fb[9 + i];
-    nb[i] += (g[i] + T(0.25) * ngB[i]) * Lb;
+    T t = fm(T(0.25), B.ngB[i], g[i]) * Lb;
+    t = fm(PH2, Hn[i], t);
+    t = fm(-phi1, fb[i], t);
+    t = fm(-nv, fb[3 + i], t);
+    t = fm(-v[i], nfn, t);
+    t = fm(-sa, fb[6 + i], t);
+    nb[i] += fm(-sb, fb[9 + i], t);
   }
-  Apb += T(-4) * L * fb[13];
-  s1b += T(4) * L * fb[14];
-  s2b += T(4) * L * fb[15];
-  const T nHn = n[0] * n[0] * P.h[0] + n[1] * n[1] * P.h[3] + n[2] * n[2] * P.h[5] +
-                T(2) * (n[0] * n[1] * P.h[1] + n[0] * n[2] * P.h[2] + n[1] * n[2] * P.h[4]);
-  const T PH = nHn - (P.h[0] + P.h[3] + P.h[5]);
-  Ab += (-PH + T(0.5) * nlap) * fb[13];
-  T He[6];
-  for (int u = 0; u < 6; ++u) He[u] = P.h[u] + T(0.5) * Tm[u];
-  T Hea[3], Heb3[3];
+  Apb = fm(-L4, fb[13], Apb);
+  s1b = fm(L4, fb[14], s1b);
+  s2b = fm(L4, fb[15], s2b);
+  // -P_perp:H + n.Laplacian B / 2
+  Ab = fm(fm(T(0.5), B.nlap, (P.h[0] + P.h[3] + P.h[5]) - vdot(n, Hn)), fb[13], Ab);
+  T He[6], ab[3], bb[3], Hea[3], Heb3[3];
+  for (int k = 0; k < 6; ++k) He[k] = fm(T(-0.25), B.K[k], fm(T(0.5), B.S[k], P.h[k]));
   for (int i = 0; i < 3; ++i) {
-    Hea[i] = symv(He, i, 0) * a[0] + symv(He, i, 1) * a[1] + symv(He, i, 2) * a[2];
-    Heb3[i] = symv(He, i, 0) * b[0] + symv(He, i, 1) * b[1] + symv(He, i, 2) * b[2];
+    Hea[i] = sym_row(He, i, a);
+    Heb3[i] = sym_row(He, i, b);
   }
-  const T S1 = (a[0] * Hea[0] + a[1] * Hea[1] + a[2] * Hea[2]) - (b[0] * Heb3[0] + b[1] * Heb3[1] + b[2] * Heb3[2]);
-  const T S2 = T(2) * (a[0] * Heb3[0] + a[1] * Heb3[1] + a[2] * Heb3[2]);
-  Ab += T(2) * V.A * (S1 * fb[14] + S2 * fb[15]);
+  const T S1 = vdot(a, Hea) - vdot(b, Heb3), S2 = T(2) * vdot(a, Heb3);
+  Ab = fm(T(2) * V.A, fm(S1, fb[14], S2 * fb[15]), Ab);
+  const T S1d = T(2) * S1b, S2d = T(2) * S2b;
   for (int i = 0; i < 3; ++i) {
-    ab[i] += T(2) * Hea[i] * S1b + T(2) * Heb3[i] * S2b;
-    bb[i] += T(-2) * Heb3[i] * S1b + T(2) * Hea[i] * S2b;
+    ab[i] = fm(e1b, w[i], fm(S1d, Hea[i], S2d * Heb3[i]));
+    bb[i] = fm(e2b, w[i], fm(S2d, Hea[i], -(S1d * Heb3[i])));
   }
 
   // ---- through the normalisations, into the state cotangent
-  const T nnb = n[0] * nb[0] + n[1] * nb[1] + n[2] * nb[2];
-  const T aab = a[0] * ab[0] + a[1] * ab[1] + a[2] * ab[2];
-  const T bbb = b[0] * bb[0] + b[1] * bb[1] + b[2] * bb[2];
+  const T nnb = vdot(n, nb), aab = vdot(a, ab), bbb = vdot(b, bb);
   for (int i = 0; i < 3; ++i) {
     yb[i] += xb[i];
-    yb[3 + i] += V.rn * (nb[i] - n[i] * nnb);
-    yb[6 + i] += V.ra * (ab[i] - a[i] * aab);
-    yb[9 + i] += V.rb * (bb[i] - b[i] * bbb);
+    yb[3 + i] = fm(V.rn, fm(-n[i], nnb, nb[i]), yb[3 + i]);
+    yb[6 + i] = fm(V.ra, fm(-a[i], aab, ab[i]), yb[6 + i]);
+    yb[9 + i] = fm(V.rb, fm(-b[i], bbb, bb[i]), yb[9 + i]);
   }
   yb[12] += Ab;
   yb[13] += Apb;
@@ -724,6 +698,7 @@ SRT_HD void stage_view_mixed(const float* d, float s, const MixedRay& R, const G
     }
     V.base[f] = cell_base(G, cell[0], cell[1], cell[2]);
     V.basep[f] = cell_base_pair(G, cell[0], cell[1], cell[2]);
+    V.hbase[f] = hot_base(G, cell);
   }
 }
 

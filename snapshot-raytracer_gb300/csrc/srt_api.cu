@@ -118,6 +118,8 @@ struct HostTimer {
 
 // Largest slab of a host field staged on the device at a time.
 constexpr int64_t kSlabBytes = 512ll << 20;
+// The same where a kernel reads mapped host memory into the slab: half of L2.
+constexpr int64_t kMappedSlabBytes = 64ll << 20;
 
 
 // Device address of host memory the GPU can read directly (pinned and mapped:
@@ -169,17 +171,21 @@ Geom make_geom(const srt_fields* f) {
   g.px = f->pn[0];
   g.pxy = f->pn[0] * f->pn[1];
   g.pxy2 = f->pn[0] * (f->pn[1] - 1);
+  g.ts = f->cell[0] ? 4 : 1;
   return g;
 }
 
 FieldPtrs make_ptrs(const srt_fields* f) {
   FieldPtrs p;
-  p.phi = f->phi;
+  p.phi = f->values(3);
   for (int c = 0; c < 3; ++c) {
-    p.b[c] = f->b[c];
+    p.b[c] = f->values(c);
     p.bh[c] = f->bh[c];
   }
-  for (int c = 0; c < 4; ++c) p.pr[c] = f->pr[c];
+  for (int c = 0; c < 4; ++c) {
+    p.pr[c] = f->pr[c];
+    p.cell[c] = f->cell[c];
+  }
   return p;
 }
 
@@ -221,15 +227,60 @@ int srt_device_count(void) {
 
 namespace {
 
-// Row-pair arrays for the packed MIXED path, when they fit with room to spare
-// (unless SRT_FIELDS_NO_PAIRS).
-int build_row_pairs(srt_fields* f, unsigned flags, cudaStream_t s) {
-  if (flags & SRT_FIELDS_NO_PAIRS) return SRT_OK;
-  const int64_t pair_bytes = 4 * f->pn[0] * (f->pn[1] - 1) * f->pn[2] * (int64_t)sizeof(float2);
+// Bytes of device memory an allocation of the fields may take: what is free and
+// what the pool holds unused, less room to spare.
+int64_t field_budget(const srt_fields* f) {
   size_t free_b = 0, total_b = 0;
-  const bool have = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess;
-  const int64_t avail = (int64_t)free_b + pool_reusable_bytes(f->device);
-  if (!have || pair_bytes + (int64_t(4) << 30) >= avail) return SRT_OK;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
+  return (int64_t)free_b + pool_reusable_bytes(f->device) - (int64_t(4) << 30);
+}
+
+// Device arrays of the laid-out fields of an n0 x n1 x n2 grid (no contents):
+// cells where they fit (64 bytes per padded voxel for the four fields) unless
+// SRT_FIELDS_NO_PAIRS, else planes (16 bytes), which finish_fields may add row
+// pairs to (another 32).
+int alloc_fields(srt_fields* f, int64_t n0, int64_t n1, int64_t n2, unsigned flags, cudaStream_t s) {
+  cudaGetDevice(&f->device);
+  for (int i = 0; i < 3; ++i) {
+    f->n[i] = (i == 0 ? n0 : (i == 1 ? n1 : n2));
+    f->pn[i] = f->n[i] + 3;
+  }
+  const int64_t pvox = f->pn[0] * f->pn[1] * f->pn[2];
+  if (!(flags & SRT_FIELDS_NO_PAIRS) && 64 * pvox < field_budget(f)) {
+    for (int c = 3; c >= 0; --c) {
+      cudaError_t e = pool_alloc((void**)&f->cell[c], pvox * sizeof(float4), s);
+      if (e != cudaSuccess) return cuda_error(e, c == 3 ? "allocate phi" : "allocate B");
+    }
+    f->bytes = 64 * pvox;
+    return SRT_OK;
+  }
+  cudaError_t e = pool_alloc((void**)&f->phi, pvox * sizeof(float), s);
+  if (e != cudaSuccess) return cuda_error(e, "allocate phi");
+  for (int c = 0; c < 3; ++c) {
+    e = pool_alloc((void**)&f->b[c], pvox * sizeof(float), s);
+    if (e != cudaSuccess) return cuda_error(e, "allocate B");
+  }
+  f->bytes = 16 * pvox;
+  return SRT_OK;
+}
+
+// Lays out planes k0 .. k1-1 of phi (comps 1) or of the interleaved B (3) from
+// device memory (or, into planes, from mapped pinned host memory).
+cudaError_t lay_out(srt_fields* f, const float* src, int comps, int64_t k0, int64_t k1, cudaStream_t s) {
+  if (f->cell[0]) {
+    float4* const dst[3] = {comps == 1 ? f->cell[3] : f->cell[0], f->cell[1], f->cell[2]};
+    return launch_cells(src, comps, dst, f->n, k0, k1, s);
+  }
+  float* const dst[3] = {comps == 1 ? f->phi : f->b[0], f->b[1], f->b[2]};
+  return launch_pad_fields(src, comps, dst, f->n, f->pn, k0, k1, s);
+}
+
+// The last step of a layout: row-pair copies of planes, when they fit
+// (unless SRT_FIELDS_NO_PAIRS).
+int finish_fields(srt_fields* f, unsigned flags, cudaStream_t s) {
+  if ((flags & SRT_FIELDS_NO_PAIRS) || f->cell[0]) return SRT_OK;
+  const int64_t pair_bytes = 4 * f->pn[0] * (f->pn[1] - 1) * f->pn[2] * (int64_t)sizeof(float2);
+  if (pair_bytes >= field_budget(f)) return SRT_OK;
   const float* srcs[4] = {f->b[0], f->b[1], f->b[2], f->phi};
   cudaError_t e = cudaSuccess;
   for (int c = 0; c < 4 && e == cudaSuccess; ++c) {
@@ -239,28 +290,6 @@ int build_row_pairs(srt_fields* f, unsigned flags, cudaStream_t s) {
   }
   if (e != cudaSuccess) return cuda_error(e, "row pairs");
   f->bytes += pair_bytes;
-  if (!(flags & SRT_ASYNC)) {
-    e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return cuda_error(e, "row pairs");
-  }
-  return SRT_OK;
-}
-
-// Device arrays of the laid-out fields of an n0 x n1 x n2 grid (no contents).
-int alloc_fields(srt_fields* f, int64_t n0, int64_t n1, int64_t n2, cudaStream_t s) {
-  cudaGetDevice(&f->device);
-  for (int i = 0; i < 3; ++i) {
-    f->n[i] = (i == 0 ? n0 : (i == 1 ? n1 : n2));
-    f->pn[i] = f->n[i] + 3;
-  }
-  const int64_t pvox = f->pn[0] * f->pn[1] * f->pn[2];
-  cudaError_t e = pool_alloc((void**)&f->phi, pvox * sizeof(float), s);
-  if (e != cudaSuccess) return cuda_error(e, "allocate phi");
-  for (int c = 0; c < 3; ++c) {
-    e = pool_alloc((void**)&f->b[c], pvox * sizeof(float), s);
-    if (e != cudaSuccess) return cuda_error(e, "allocate B");
-  }
-  f->bytes = 4 * pvox * (int64_t)sizeof(float);
   return SRT_OK;
 }
 
@@ -285,38 +314,30 @@ int srt_fields_create(const float* phi, const float* b_xyz, int64_t n0, int64_t 
   srt_fields* f = new (std::nothrow) srt_fields();
   if (!f) return set_error(SRT_ERR_OUT_OF_MEMORY, "srt_fields_create: host allocation failed");
   {
-    cudaGetDevice(&f->device);
-    for (int i = 0; i < 3; ++i) {
-      f->n[i] = (i == 0 ? n0 : (i == 1 ? n1 : n2));
-      f->pn[i] = f->n[i] + 3;
-    }
-    const int64_t pvox = f->pn[0] * f->pn[1] * f->pn[2];
+    rc = alloc_fields(f, n0, n1, n2, flags, s);
+    if (rc != SRT_OK) goto fail;
     const int64_t plane = n0 * n1;
     const int64_t vox = plane * n2;
-    SRT_CUDA_TRY(pool_alloc((void**)&f->phi, pvox * sizeof(float), s), "allocate phi");
-    for (int c = 0; c < 3; ++c) SRT_CUDA_TRY(pool_alloc((void**)&f->b[c], pvox * sizeof(float), s), "allocate B");
-    f->bytes = 4 * pvox * (int64_t)sizeof(float);
-    float* const phi_dst[3] = {f->phi, nullptr, nullptr};
     // host inputs in mapped pinned memory (cudaHostAlloc / cudaHostRegister)
-    // are read by the layout kernel itself over the host link, with no
-    // staging copy; other host memory streams through a device slab
+    // are read by a kernel over the host link, with no staging copy by the copy
+    // engines; other host memory streams through a device slab
     const float* phi_src = phi;
     const float* b_src = b_xyz;
-    bool direct = dev_in;
+    bool mapped = false;
     if (!dev_in && !(flags & SRT_FIELDS_STAGED)) {
       const float* dp = mapped_device_pointer(phi);
       const float* db = mapped_device_pointer(b_xyz);
       if (dp && db) {
         phi_src = dp;
         b_src = db;
-        direct = true;
+        mapped = true;
       }
     }
-    if (direct) {
+    if (dev_in || (mapped && !f->cell[0])) {
       NvtxRange upload(dev_in ? "layout" : "layout from mapped host memory");
-      SRT_CUDA_TRY(launch_pad_fields(phi_src, 1, phi_dst, f->n, f->pn, 0, n2, s), "pad phi");
-      SRT_CUDA_TRY(launch_pad_fields(b_src, 3, f->b, f->n, f->pn, 0, n2, s), "pad B");
-    } else if ((flags & SRT_ASYNC) && pool_alloc((void**)&slab, 4 * vox * sizeof(float), s) == cudaSuccess) {
+      SRT_CUDA_TRY(lay_out(f, phi_src, 1, 0, n2, s), "lay out phi");
+      SRT_CUDA_TRY(lay_out(f, b_src, 3, 0, n2, s), "lay out B");
+    } else if (!mapped && (flags & SRT_ASYNC) && pool_alloc((void**)&slab, 4 * vox * sizeof(float), s) == cudaSuccess) {
       // asynchronous: the whole input through one staging buffer, so the
       // copy engines move it without waiting for a layout kernel between
       // slabs (those would wait for SM slots while other work runs), then
@@ -324,38 +345,44 @@ int srt_fields_create(const float* phi, const float* b_xyz, int64_t n0, int64_t 
       NvtxRange upload("upload (one staging buffer) and layout");
       SRT_CUDA_TRY(cudaMemcpyAsync(slab, phi, vox * sizeof(float), cudaMemcpyHostToDevice, s), "copy phi");
       SRT_CUDA_TRY(cudaMemcpyAsync(slab + vox, b_xyz, 3 * vox * sizeof(float), cudaMemcpyHostToDevice, s), "copy B");
-      SRT_CUDA_TRY(launch_pad_fields(slab, 1, phi_dst, f->n, f->pn, 0, n2, s), "pad phi");
-      SRT_CUDA_TRY(launch_pad_fields(slab + vox, 3, f->b, f->n, f->pn, 0, n2, s), "pad B");
+      SRT_CUDA_TRY(lay_out(f, slab, 1, 0, n2, s), "lay out phi");
+      SRT_CUDA_TRY(lay_out(f, slab + vox, 3, 0, n2, s), "lay out B");
     } else {
       cudaGetLastError();  // a failed whole-input staging allocation falls back to slabs
-      // Stream host planes through one device slab on s: H2D copy, then the
-      // pad kernel. (A second slab with the copies on their own stream was
+      // Stream host planes through one device slab on s: H2D copy (or the
+      // mapped read, in slabs that stay in L2 for the layout kernel), then the
+      // layout kernel. (A second slab with the copies on their own stream was
       // measured slower in steady use: 250-310 ms against 190-210 ms for the
       // 17 GB of a 1024^3 handle from pinned memory.)
-      int64_t kslab = kSlabBytes / (plane * 3 * (int64_t)sizeof(float));
-      if (kslab < 1) kslab = 1;
-      if (kslab > n2) kslab = n2;
-      SRT_CUDA_TRY(pool_alloc((void**)&slab, kslab * plane * 3 * sizeof(float), s), "allocate slab");
       // pass 0: phi (one component per voxel); pass 1: B (three, interleaved)
       NvtxRange upload("upload and layout");
       for (int pass = 0; pass < 2; ++pass) {
         const int comps = pass == 0 ? 1 : 3;
-        const float* src = pass == 0 ? phi : b_xyz;
+        const float* src = pass == 0 ? phi_src : b_src;
+        int64_t kslab = (mapped ? kMappedSlabBytes : kSlabBytes) / (plane * comps * (int64_t)sizeof(float));
+        if (kslab < 1) kslab = 1;
+        if (kslab > n2) kslab = n2;
+        SRT_CUDA_TRY(pool_alloc((void**)&slab, kslab * plane * comps * sizeof(float), s), "allocate slab");
         for (int64_t k0 = 0; k0 < n2; k0 += kslab) {
           const int64_t k1 = k0 + kslab < n2 ? k0 + kslab : n2;
-          SRT_CUDA_TRY(cudaMemcpyAsync(slab, src + comps * k0 * plane, comps * (k1 - k0) * plane * sizeof(float),
-                                       cudaMemcpyHostToDevice, s),
-                       "copy field slab");
-          SRT_CUDA_TRY(launch_pad_fields(slab, comps, pass == 0 ? phi_dst : f->b, f->n, f->pn, k0, k1, s),
-                       pass == 0 ? "pad phi" : "pad B");
+          const float* from = src + comps * k0 * plane;
+          const int64_t count = comps * (k1 - k0) * plane;
+          if (mapped)
+            SRT_CUDA_TRY(launch_fetch(from, slab, count, s), "fetch field slab");
+          else
+            SRT_CUDA_TRY(cudaMemcpyAsync(slab, from, count * sizeof(float), cudaMemcpyHostToDevice, s),
+                         "copy field slab");
+          SRT_CUDA_TRY(lay_out(f, slab, comps, k0, k1, s), pass == 0 ? "lay out phi" : "lay out B");
         }
+        pool_free(slab, s);  // stream-ordered: after the field's last layout kernel on s
+        slab = nullptr;
       }
     }
-    if (!(flags & SRT_ASYNC)) SRT_CUDA_TRY(cudaStreamSynchronize(s), "field layout");
-    pool_free(slab, s);  // stream-ordered: after the last pad kernel on s
+    pool_free(slab, s);
     slab = nullptr;
-    rc = build_row_pairs(f, flags, s);
+    rc = finish_fields(f, flags, s);
     if (rc != SRT_OK) goto fail;
+    if (!(flags & SRT_ASYNC)) SRT_CUDA_TRY(cudaStreamSynchronize(s), "field layout");
   }
   *out = f;
   return SRT_OK;
@@ -379,7 +406,10 @@ int srt_fields_destroy(srt_fields* f) {
     pool_free(f->b[c], 0);
     pool_free(f->bh[c], 0);
   }
-  for (int c = 0; c < 4; ++c) pool_free(f->pr[c], 0);
+  for (int c = 0; c < 4; ++c) {
+    pool_free(f->pr[c], 0);
+    pool_free(f->cell[c], 0);
+  }
   cudaDeviceSynchronize();
   if (prev != f->device) cudaSetDevice(prev);
   delete f;
@@ -455,7 +485,7 @@ int srt_forward(const srt_fields* fields, int64_t nside, int64_t pix_begin, int6
       cudaError_t e = cudaSuccess;
       for (int c = 0; c < 3 && e == cudaSuccess; ++c) e = pool_alloc((void**)&h[c], pvox * sizeof(__half), s);
       for (int c = 0; c < 3 && e == cudaSuccess; ++c) {
-        e = launch_quantize_half(f->b[c], h[c], pvox, s);
+        e = launch_quantize_half(f->values(c), f->cell[c] ? 4 : 1, h[c], pvox, s);
         ++kernels;
       }
       if (e != cudaSuccess) {
@@ -503,7 +533,7 @@ int srt_forward(const srt_fields* fields, int64_t nside, int64_t pix_begin, int6
       SRT_CUDA_TRY(cudaEventCreate(&em), "cudaEventCreate");
       SRT_CUDA_TRY(cudaEventRecord(e0, s), "cudaEventRecord");
     }
-    const int kmode = (precision == SRT_PRECISION_MIXED && f->pr[0]) ? kMIXED_PAIR : precision;
+    const int kmode = precision == SRT_PRECISION_MIXED ? f->mixed_mode() : precision;
     SRT_CUDA_TRY(launch_trace(kmode, a, s, &kernels), "trace kernel launch");
     if (timed) SRT_CUDA_TRY(cudaEventRecord(em, s), "cudaEventRecord");  // trace kernel done
     if (refine) SRT_CUDA_TRY(launch_refine(a, s, &kernels), "refine kernel launch");
@@ -676,7 +706,7 @@ int srt_fields_load_h5(const char* phi_path, const char* b_path, const char* dse
   double layout_ms = 0.0, tail_ms = 0.0;
   bool announced_b = false, announced_bdims = false, announced_upload = false;
   rc = f ? SRT_OK : set_error(SRT_ERR_OUT_OF_MEMORY, "srt_fields_load_h5: host allocation failed");
-  if (rc == SRT_OK && have_device) rc = alloc_fields(f, n0, n1, n2, s);
+  if (rc == SRT_OK && have_device) rc = alloc_fields(f, n0, n1, n2, flags, s);
   int64_t kslab = kSlabBytes / (plane * 3 * (int64_t)sizeof(float));
   if (kslab < 1) kslab = 1;
   if (kslab > n2) kslab = n2;
@@ -691,7 +721,6 @@ int srt_fields_load_h5(const char* phi_path, const char* b_path, const char* dse
   for (int field = 0; field < 2 && rc == SRT_OK; ++field) {
     const int comps = field == 0 ? 1 : 3;
     const float* host = field == 0 ? hphi_data : hb_data;
-    float* const phi_dst[3] = {f->phi, nullptr, nullptr};
     for (int64_t k0 = 0; k0 < n2 && rc == SRT_OK; k0 += kslab) {
       const int64_t k1 = k0 + kslab < n2 ? k0 + kslab : n2;
       const int64_t need = k1 * plane * comps;
@@ -742,7 +771,7 @@ int srt_fields_load_h5(const char* phi_path, const char* b_path, const char* dse
       const auto tl = std::chrono::steady_clock::now();
       cudaError_t e = cudaMemcpyAsync(slab, host + k0 * plane * comps, (k1 - k0) * plane * comps * sizeof(float),
                                       cudaMemcpyHostToDevice, s);
-      if (e == cudaSuccess) e = launch_pad_fields(slab, comps, field == 0 ? phi_dst : f->b, f->n, f->pn, k0, k1, s);
+      if (e == cudaSuccess) e = lay_out(f, slab, comps, k0, k1, s);
       if (e == cudaSuccess) e = cudaStreamSynchronize(s);
       if (e != cudaSuccess) rc = cuda_error(e, "srt_fields_load_h5: layout");
       layout_ms += ms_since(tl);
@@ -765,7 +794,7 @@ int srt_fields_load_h5(const char* phi_path, const char* b_path, const char* dse
   if (slab) pool_free(slab, s);
   if (rc == SRT_OK) {
     const auto tt = std::chrono::steady_clock::now();
-    rc = build_row_pairs(f, flags & SRT_FIELDS_NO_PAIRS, s);
+    rc = finish_fields(f, flags, s);
     if (rc == SRT_OK) {
       cudaError_t e = cudaStreamSynchronize(s);
       if (e != cudaSuccess) rc = cuda_error(e, "srt_fields_load_h5");

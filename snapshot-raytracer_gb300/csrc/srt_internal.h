@@ -14,11 +14,19 @@ struct srt_fields {
   int device = 0;
   int64_t n[3] = {0, 0, 0};
   int64_t pn[3] = {0, 0, 0};  // padded extents n + 3
-  float* phi = nullptr;       // padded FP32 planes
+  // either cells (B_x, B_y, B_z, phi; 16 bytes per padded voxel), or padded FP32
+  // planes and, where they fit, row-pair copies in the same order
+  float4* cell[4] = {nullptr, nullptr, nullptr, nullptr};
+  float* phi = nullptr;
   float* b[3] = {nullptr, nullptr, nullptr};
+  float2* pr[4] = {nullptr, nullptr, nullptr, nullptr};
   __half* bh[3] = {nullptr, nullptr, nullptr};  // padded half(B * 2^27), made on first REF16 use
-  float2* pr[4] = {nullptr, nullptr, nullptr, nullptr};  // row-pair arrays B_x, B_y, B_z, phi (MIXED fast path)
   int64_t bytes = 0;
+  int layout() const { return cell[0] ? srt::kCells : (pr[0] ? srt::kPairs : srt::kPlanes); }
+  // the MIXED trace kernel of this layout
+  int mixed_mode() const { return cell[0] ? srt::kMIXED_CELL : (pr[0] ? srt::kMIXED_PAIR : srt::kMIXED); }
+  // the values of B component c (0-2) or phi (3), make_geom's ts floats apart
+  const float* values(int c) const { return cell[c] ? &cell[c]->x : (c == 3 ? phi : b[c]); }
 };
 
 namespace srt {
@@ -71,10 +79,15 @@ FieldPtrs make_ptrs(const srt_fields* f);
 // (comps 3, dst[0..2]); device memory or mapped pinned host memory.
 cudaError_t launch_pad_fields(const float* src, int comps, float* const dst[3], const int64_t n[3],
                               const int64_t pn[3], int64_t k0, int64_t k1, cudaStream_t s);
-cudaError_t launch_quantize_half(const float* src, __half* dst, int64_t count, cudaStream_t s);
+// src: device memory.
+cudaError_t launch_cells(const float* src, int comps, float4* const dst[3], const int64_t n[3], int64_t k0, int64_t k1,
+                         cudaStream_t s);
+// count floats from mapped pinned host memory to device memory.
+cudaError_t launch_fetch(const float* src, float* dst, int64_t count, cudaStream_t s);
+cudaError_t launch_quantize_half(const float* src, int ts, __half* dst, int64_t count, cudaStream_t s);
 cudaError_t launch_pair_build(const float* src, float2* dst, const int64_t pn[3], cudaStream_t s);
 
-// Trace kernel launch (mode = kFP64 / kMIXED / kREF16).
+// Trace kernel launch (mode = kFP64 / kREF16 / a handle's mixed_mode()).
 cudaError_t launch_trace(int mode, const TraceArgs& a, cudaStream_t s, int64_t* kernels);
 // FP64 re-trace of the rays listed by a MIXED trace (count read on the device).
 cudaError_t launch_refine(const TraceArgs& a, cudaStream_t s, int64_t* kernels);

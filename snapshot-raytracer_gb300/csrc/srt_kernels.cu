@@ -3,6 +3,7 @@
 //                          of the interleaved B field (every source voxel read once)
 //                          (replaces vector3_to_half, snapshot-raytracer.cu:585-597,
 //                          and the staged uploads of :774-844)
+//   * cells_kernel         the same into cells (value and second differences)
 //   * quantize_half_kernel half(B * 2^27) planes for the REF16 mode
 //   * trace_kernel<MODE>   one thread per ray: HEALPix pixel centre -> initial
 //                          state -> n_steps RK4 steps -> six maps
@@ -17,19 +18,6 @@
 namespace srt {
 
 // ------------------------------------------------------------- field layout
-
-// Padded coordinates of source coordinate c on an axis of extent n: padded
-// coordinate q holds voxel (q - 1) mod n for q in [0, n + 3), so c appears at
-// c + 1 and, near the ends, in the halo (n - 1 -> 0, 0 -> n + 1, 1 -> n + 2).
-// Returns how many of out[0..3] it filled.
-__device__ __forceinline__ int padded_coords(int64_t c, int64_t n, int64_t out[4]) {
-  int m = 0;
-  out[m++] = c + 1;
-  if (c == n - 1) out[m++] = 0;
-  if (c == 0) out[m++] = n + 1;
-  if (c == 1 % n) out[m++] = n + 2;
-  return m;
-}
 
 // One thread per source voxel of planes k0 .. k1-1 (x fastest, `comps` floats
 // per voxel: 1 for phi, 3 for the interleaved B), each source byte read once
@@ -93,14 +81,101 @@ cudaError_t launch_pad_fields(const float* src, int comps, float* const dst[3], 
   return cudaGetLastError();
 }
 
-__global__ void quantize_half_kernel(const float* __restrict__ src, __half* __restrict__ dst, int64_t count) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < count) dst[i] = __float2half_rn(src[i] * 134217728.0f);
+// Cells (cell_of) of planes kb .. of a source field (x fastest, COMPS floats
+// per voxel), written at every padded position, halo copies included: block of
+// 32 x 8 padded positions of a plane, their voxels and a ring of neighbours
+// (periodic) staged in shared memory, each cell one 16-byte store. Bound by
+// those stores: 16 bytes written per voxel and field for 4 read. grid: x, y over the padded
+// plane (y looping where it is longer than the grid), z over planes.
+constexpr int kCellX = 32, kCellY = 8;
+
+template <int COMPS>
+__global__ void __launch_bounds__(kCellX* kCellY) cells_kernel(const float* __restrict__ src, float4* __restrict__ d0,
+                                                               float4* __restrict__ d1, float4* __restrict__ d2, int n0,
+                                                               int n1, int64_t n2, int64_t k0) {
+  __shared__ float tile[COMPS][kCellY + 2][kCellX + 2];
+  const int px = n0 + 3, py = n1 + 3;
+  const int64_t k = k0 + blockIdx.z;
+  const float* plane = src + (int64_t)blockIdx.z * n0 * n1 * COMPS;
+  const int t = threadIdx.y * kCellX + threadIdx.x;
+  const int i = blockIdx.x * kCellX + threadIdx.x;
+  for (int jb = blockIdx.y * kCellY; jb < py; jb += gridDim.y * kCellY) {
+    __syncthreads();
+    for (int e = t; e < (kCellY + 2) * (kCellX + 2); e += kCellX * kCellY) {
+      const int ty = e / (kCellX + 2), tx = e % (kCellX + 2);
+      // padded position -> voxel: (position - 1) mod n, one ring wider
+      const int qi = (int)blockIdx.x * kCellX + tx - 1, qj = jb + ty - 1;
+      if (qi > px || qj > py) continue;
+      int vi = (qi - 1) % n0, vj = (qj - 1) % n1;
+      vi += vi < 0 ? n0 : 0;
+      vj += vj < 0 ? n1 : 0;
+      const float* p = plane + ((int64_t)vj * n0 + vi) * COMPS;
+#pragma unroll
+      for (int c = 0; c < COMPS; ++c) tile[c][ty][tx] = p[c];
+    }
+    __syncthreads();
+    const int j = jb + threadIdx.y;
+    if (i >= px || j >= py) continue;
+    int64_t pk[4];
+    const int nk = padded_coords(k, n2, pk);
+    float4* const dst[3] = {d0, d1, d2};
+#pragma unroll
+    for (int c = 0; c < COMPS; ++c) {
+      float v[3][3];
+#pragma unroll
+      for (int b = 0; b < 3; ++b)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) v[b][a] = tile[c][threadIdx.y + b][threadIdx.x + a];
+      const float4 cell = cell_of(v);
+      for (int a = 0; a < nk; ++a) __stcs(dst[c] + i + (int64_t)px * (j + (int64_t)py * pk[a]), cell);
+    }
+  }
 }
 
-cudaError_t launch_quantize_half(const float* src, __half* dst, int64_t count, cudaStream_t s) {
+cudaError_t launch_cells(const float* src, int comps, float4* const dst[3], const int64_t n[3], int64_t k0, int64_t k1,
+                         cudaStream_t s) {
+  const int64_t plane = n[0] * n[1];
+  for (int64_t kb = k0; kb < k1; kb += 65535) {
+    const int64_t ke = kb + 65535 < k1 ? kb + 65535 : k1;
+    const dim3 grid((unsigned)((n[0] + 3 + kCellX - 1) / kCellX),
+                    (unsigned)std::min<int64_t>((n[1] + 3 + kCellY - 1) / kCellY, 65535), (unsigned)(ke - kb));
+    const dim3 block(kCellX, kCellY);
+    const float* p = src + (kb - k0) * plane * comps;
+    if (comps == 3)
+      cells_kernel<3><<<grid, block, 0, s>>>(p, dst[0], dst[1], dst[2], (int)n[0], (int)n[1], n[2], kb);
+    else
+      cells_kernel<1><<<grid, block, 0, s>>>(p, dst[0], nullptr, nullptr, (int)n[0], (int)n[1], n[2], kb);
+  }
+  return cudaGetLastError();
+}
+
+// count floats from mapped pinned host memory to the device, 16 bytes a load
+// where both are aligned (the cells kernel reads each voxel from several
+// threads, so it takes its source from the device).
+__global__ void __launch_bounds__(256) fetch_kernel(const float* __restrict__ src, float* __restrict__ dst, int64_t count,
+                                                    int64_t vec) {
+  const int64_t step = (int64_t)gridDim.x * 256, t = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  for (int64_t q = t; q < vec; q += step)
+    reinterpret_cast<float4*>(dst)[q] = reinterpret_cast<const float4*>(src)[q];
+  for (int64_t q = 4 * vec + t; q < count; q += step) dst[q] = src[q];
+}
+
+cudaError_t launch_fetch(const float* src, float* dst, int64_t count, cudaStream_t s) {
+  const bool aligned = (((uintptr_t)src | (uintptr_t)dst) & 15) == 0;
+  const int64_t blocks = std::min<int64_t>((count / 4 + 255) / 256 + 1, 1 << 16);
+  fetch_kernel<<<(unsigned)blocks, 256, 0, s>>>(src, dst, count, aligned ? count / 4 : 0);
+  return cudaGetLastError();
+}
+
+// half(B * 2^27) of `count` values, ts floats apart in src.
+__global__ void quantize_half_kernel(const float* __restrict__ src, int ts, __half* __restrict__ dst, int64_t count) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < count) dst[i] = __float2half_rn(src[i * ts] * 134217728.0f);
+}
+
+cudaError_t launch_quantize_half(const float* src, int ts, __half* dst, int64_t count, cudaStream_t s) {
   const int64_t blocks = (count + 255) / 256;
-  quantize_half_kernel<<<(unsigned)blocks, 256, 0, s>>>(src, dst, count);
+  quantize_half_kernel<<<(unsigned)blocks, 256, 0, s>>>(src, ts, dst, count);
   return cudaGetLastError();
 }
 
@@ -131,7 +206,7 @@ cudaError_t launch_pair_build(const float* src, float2* dst, const int64_t pn[3]
 #endif
 
 template <int MODE>
-__global__ void __launch_bounds__(128, (MODE == kMIXED || MODE == kMIXED_PAIR) ? SRT_MIXED_MIN_BLOCKS : 1)
+__global__ void __launch_bounds__(128, (MODE == kMIXED || MODE >= kMIXED_PAIR) ? SRT_MIXED_MIN_BLOCKS : 1)
     trace_kernel(const TraceArgs A) {
   const int64_t tl = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (tl >= A.launch_rays) return;
@@ -147,9 +222,10 @@ __global__ void __launch_bounds__(128, (MODE == kMIXED || MODE == kMIXED_PAIR) ?
   if (o < 0 || o >= A.pix_count) return;
   const RayDir d = ray_dir_pix(A.nside, ring);
   float out[6];
-  if (MODE == kMIXED_PAIR || MODE == kMIXED) {
+  if (MODE >= kMIXED_PAIR || MODE == kMIXED) {
+    constexpr int kLayout = MODE == kMIXED_CELL ? kCells : (MODE == kMIXED_PAIR ? kPairs : kPlanes);
     __shared__ float guard_m[128][2];  // the ray's guard state, out of the register budget
-    const bool near = trace_ray_mixed<MODE == kMIXED_PAIR>(A.F, A.G, d, A.n_steps, out, guard_m[threadIdx.x]);
+    const bool near = trace_ray_mixed<kLayout>(A.F, A.G, d, A.n_steps, out, guard_m[threadIdx.x]);
     if (near && A.refine_list) {
       const unsigned long long k = atomicAdd(A.refine_count, 1ull);
       if (k < (unsigned long long)A.pix_count) A.refine_list[k] = o;
@@ -170,6 +246,7 @@ cudaError_t launch_trace(int mode, const TraceArgs& a, cudaStream_t s, int64_t* 
     case kFP64: trace_kernel<kFP64><<<(unsigned)blocks, threads, 0, s>>>(a); break;
     case kMIXED: trace_kernel<kMIXED><<<(unsigned)blocks, threads, 0, s>>>(a); break;
     case kREF16: trace_kernel<kREF16><<<(unsigned)blocks, threads, 0, s>>>(a); break;
+    case kMIXED_CELL: trace_kernel<kMIXED_CELL><<<(unsigned)blocks, threads, 0, s>>>(a); break;
     case kMIXED_PAIR: trace_kernel<kMIXED_PAIR><<<(unsigned)blocks, threads, 0, s>>>(a); break;
     default: return cudaErrorInvalidValue;
   }

@@ -137,7 +137,7 @@ extern "C" int srt_forward_noalloc(const srt_fields* fields, int64_t nside, int6
     a.refine_count = refine ? sc.count : nullptr;
     cudaError_t e = cudaSuccess;
     if (refine) e = cudaMemsetAsync(sc.count, 0, sizeof(unsigned long long), s);
-    const int kmode = (precision == SRT_PRECISION_MIXED && fields->pr[0]) ? kMIXED_PAIR : precision;
+    const int kmode = precision == SRT_PRECISION_MIXED ? fields->mixed_mode() : precision;
     if (e == cudaSuccess) e = launch_trace(kmode, a, s, nullptr);
     if (e == cudaSuccess && refine) e = launch_refine(a, s, nullptr);
     if (e == cudaSuccess && !(flags & SRT_ASYNC)) e = cudaStreamSynchronize(s);

@@ -38,13 +38,14 @@
 #pragma once
 #include <stdint.h>
 #include <math.h>
+#include <type_traits>
 #include <cuda_fp16.h>
 #include "srt_healpix.cuh"
 #include "srt_dd.cuh"
 
 namespace srt {
 
-enum { kFP64 = 0, kMIXED = 1, kREF16 = 2, kMIXED_PAIR = 3 };
+enum { kFP64 = 0, kMIXED = 1, kREF16 = 2, kMIXED_PAIR = 3, kMIXED_CELL = 4 };
 
 #if defined(__CUDA_ARCH__)
 template <typename T>
@@ -67,15 +68,25 @@ struct Geom {
   int64_t px, pxy;
   int64_t pxy2;  // slice stride of the row-pair arrays (float2 units): px * (py - 1)
   float invn[3];
+  int ts = 1;  // floats from one voxel's value to the next: 1 in planes, 4 in cells
 };
 
+// How a handle stores its fields (the MIXED kernels are compiled for each):
+// planes of values; planes beside row-pair copies; or cells, which hold the
+// values too, so nothing else is stored. kFourTaps: the four-tap passes on the
+// values of any layout (rays of the adjoint that come near a cell face).
+enum { kPlanes = 0, kPairs = 1, kCells = 2, kFourTaps = 3 };
+
 struct FieldPtrs {
-  const float* phi;     // padded FP32
-  const float* b[3];    // padded FP32 B components
+  const float* phi;     // padded FP32 values, Geom::ts floats apart
+  const float* b[3];    // the same for the B components
   const __half* bh[3];  // padded half(B * 2^27) (REF16 only)
-  // Row-pair arrays (MIXED fast path, optional): element (i, j, k), j < py - 1,
-  // holds (f(i, j, k), f(i, j + 1, k)) of the padded field; [0..2] B, [3] phi.
+  // Row-pair arrays (kPairs): element (i, j, k), j < py - 1, holds
+  // (f(i, j, k), f(i, j + 1, k)) of the padded field; [0..2] B, [3] phi.
   const float2* pr[4];
+  // Cells (kCells): element (i, j, k) of the padded grid holds the value and its
+  // second differences along y, along x and along both (cell_of); [0..2] B, [3] phi.
+  const float4* cell[4];
 };
 
 template <typename T>
@@ -107,9 +118,9 @@ SRT_HD void cr_weights(T t, CRW<T>& c) {
   c.h[3] = T(3) * t - T(1);
 }
 
-// The same weights in Horner form for the MIXED form's FP32 interpolation
-// (22 operations, two of them shared, against ~28 for the expanded
-// polynomials; the FP64 and REF16 forms keep cr_weights).
+// The same weights in Horner form for the MIXED form's z passes (22 operations,
+// two of them shared, against ~28 for the expanded polynomials; the REF16 form
+// keeps cr_weights).
 SRT_HD void cr_weights_mixed(float t, CRW<float>& c) {
   const float t2 = t * t;
   const float a2 = fmaf(-1.5f, t, 2.f);  // 2 - 3t/2, in w2 and g0
@@ -127,15 +138,41 @@ SRT_HD void cr_weights_mixed(float t, CRW<float>& c) {
   c.h[3] = fmaf(3.f, t, -1.f);
 }
 
+// The cubic from the values p1, p2 of the two inner taps and the second
+// differences e1 = p0 - 2 p1 + p2, e2 = p1 - 2 p2 + p3 there:
+//   value   p1 + t (p2 - p1) + w0 e1 + w3 e2
+//   d/dt    (p2 - p1) + g0 e1 + g3 e2
+//   d2/dt2  h0 e1 + h3 e2
+//   d3/dt3  3 (e2 - e1)
+// with w0, w3, g0, ... the outer taps' weights above (the weights sum to 1, 0
+// and 0 and are exact on linear data, so the inner taps' follow). Eight
+// operations for the first three against twelve on four taps, where the second
+// differences are stored (cells); as many as before where they are formed on
+// the spot; and half the weights to form. The second derivative comes from
+// second differences rather than from cancelling values.
+struct CWD {
+  float t, w0, w3, g0, g3, h0, h3;
+};
+SRT_HD void cr_weights_diff(float t, CWD& c) {
+  c.t = t;
+  c.w0 = fmaf(fmaf(-0.5f, t, 1.f), t, -0.5f) * t;
+  c.w3 = fmaf(0.5f, t, -0.5f) * (t * t);
+  c.g0 = fmaf(fmaf(-1.5f, t, 2.f), t, -0.5f);
+  c.g3 = fmaf(1.5f, t, -1.f) * t;
+  c.h0 = fmaf(-3.f, t, 2.f);
+  c.h3 = fmaf(3.f, t, -1.f);
+}
+
 template <typename T>
 SRT_HD T tapv(float x) { return (T)x; }
 template <typename T>
 SRT_HD T tapv(__half x) { return (T)__half2float(x); }
 
-// Tricubic value/gradient/Hessian from the 4x4x4 taps starting at padded
-// index `base` (= the voxel (cx-1, cy-1, cz-1) of cell (cx, cy, cz)).
+// Tricubic value/gradient/Hessian from the 4x4x4 taps (ts elements apart along
+// x) starting at padded index `base` (= the voxel (cx-1, cy-1, cz-1) of cell
+// (cx, cy, cz)).
 template <typename T, typename TapT>
-SRT_HD void tricubic(const TapT* __restrict__ f, int64_t base, int64_t px, int64_t pxy,
+SRT_HD void tricubic(const TapT* __restrict__ f, int64_t base, int64_t px, int64_t pxy, int ts,
                      const CRW<T>& X, const CRW<T>& Y, const CRW<T>& Z, Tri<T>& r) {
   T v = 0, g0 = 0, g1 = 0, g2 = 0, h00 = 0, h01 = 0, h02 = 0, h11 = 0, h12 = 0, h22 = 0;
 #pragma unroll
@@ -143,9 +180,9 @@ SRT_HD void tricubic(const TapT* __restrict__ f, int64_t base, int64_t px, int64
     T a = 0, ay = 0, ayy = 0, ax = 0, axy = 0, axx = 0;
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      const TapT* row = f + base + c * pxy + b * px;
-      const T p0 = tapv<T>(ldg(row + 0)), p1 = tapv<T>(ldg(row + 1));
-      const T p2 = tapv<T>(ldg(row + 2)), p3 = tapv<T>(ldg(row + 3));
+      const TapT* row = f + (base + c * pxy + b * px) * ts;
+      const T p0 = tapv<T>(ldg(row + 0)), p1 = tapv<T>(ldg(row + ts));
+      const T p2 = tapv<T>(ldg(row + 2 * ts)), p3 = tapv<T>(ldg(row + 3 * ts));
       const T rv = X.w[0] * p0 + X.w[1] * p1 + X.w[2] * p2 + X.w[3] * p3;
       const T rx = X.g[0] * p0 + X.g[1] * p1 + X.g[2] * p2 + X.g[3] * p3;
       const T rxx = X.h[0] * p0 + X.h[1] * p1 + X.h[2] * p2 + X.h[3] * p3;
@@ -201,43 +238,184 @@ SRT_HD float2 dup2(float v) { return make_float2(v, v); }
 // a - b, one rounding (there is no packed subtract: -1 * b + a)
 SRT_HD float2 fsub2(float2 a, float2 b) { return ffma2(dup2(-1.f), b, a); }
 
-// Where the packed passes get their taps: rows y and y+1 of a slice, tap i,
-// as one float2. Two sources:
-//   PairRows   the row-pair array (srt_fields.pr): one 64-bit load per tap
-//              pair; base is the pair index of voxel (cx-1, cy-1, cz-1);
-//   SingleRows the halo-padded single layout: two 32-bit loads (rows y and
-//              y+1, one row stride apart) placed in the two halves of the
-//              pair, so the packed arithmetic needs no second copy of the
-//              field; base is the voxel's padded index.
-// Both give the same float2 values, so the interpolations agree bit for bit.
-struct PairRows {
-  const float2* __restrict__ f;
-  int64_t base, px, pxy2;
-  SRT_HD float2 operator()(int c, int pr, int i) const { return ldg(f + base + c * pxy2 + 2 * pr * px + i); }
+// A voxel's cell from its 3 x 3 neighbourhood in the xy plane, v[j][i]: the
+// value, its second difference along y, along x, and along x of that along y.
+// Every source below forms these by the same operations, so the layouts'
+// interpolations agree bit for bit.
+SRT_HD float diff2(float a, float b, float c) { return fmaf(-2.f, b, a + c); }
+SRT_HD float4 cell_of(const float v[3][3]) {
+  const float y0 = diff2(v[0][0], v[1][0], v[2][0]), y1 = diff2(v[0][1], v[1][1], v[2][1]),
+              y2 = diff2(v[0][2], v[1][2], v[2][2]);
+  return make_float4(v[1][1], y1, diff2(v[1][0], v[1][1], v[1][2]), diff2(y0, y1, y2));
+}
+
+// x weights on both lanes of a packed pair.
+struct XDup {
+  float2 t, w0, w3, g0, g3, h0, h3;
+  SRT_HD explicit XDup(const CWD& c)
+      : t(dup2(c.t)), w0(dup2(c.w0)), w3(dup2(c.w3)), g0(dup2(c.g0)), g3(dup2(c.g3)), h0(dup2(c.h0)), h3(dup2(c.h3)) {}
 };
-struct SingleRows {
-  const float* __restrict__ f;
-  int64_t base, px, pxy;
-  SRT_HD float2 operator()(int c, int pr, int i) const {
-    const float* r = f + base + c * pxy + 2 * pr * px + i;
-    return make_float2(ldg(r), ldg(r + px));
+
+// x pass of one packed row: value, d, d2 and (K) a third of d3.
+struct XRow {
+  float2 v, g, h, k;
+};
+template <bool K>
+SRT_HD XRow x_row(const XDup& w, float2 p1, float2 e1, float2 p2, float2 e2) {
+  XRow r;
+  const float2 m = fsub2(p2, p1);
+  r.v = ffma2(w.w3, e2, ffma2(w.w0, e1, ffma2(w.t, m, p1)));
+  r.g = ffma2(w.g3, e2, ffma2(w.g0, e1, m));
+  r.h = ffma2(w.h3, e2, fmul2(w.h0, e1));
+  r.k = K ? fsub2(e2, e1) : make_float2(0.f, 0.f);
+  return r;
+}
+
+// One order in x of a slice's x pass as the y pass takes it: values (v) and
+// second differences along y (e) at the two inner rows.
+struct YIn {
+  float v1, v2, e1, e2;
+};
+
+// Where the packed passes get a slice (fixed z) of a tricubic footprint. load()
+// fetches it; x_pass() gives the x pass of its rows as two packed rows, and
+// at() picks one order's y inputs from them. Two kinds:
+//   CellSource  four 16-byte cells (rows 1 and 2, taps 1 and 2): each packed
+//               row is (value, second difference along y) of one grid row;
+//   TapSource   the sixteen values, the second differences formed on the spot:
+//               one packed row holds the two grid rows' values, the other
+//               their second differences along y (four 32-bit loads per tap
+//               column from planes, two 64-bit ones from row pairs).
+struct SliceData {
+  float4 q[4];
+};
+
+struct CellSource {
+  const float4* __restrict__ f;  // the cell of voxel (cx, cy, cz - 1)
+  int64_t px, pxy;
+  SRT_HD SliceData load(int c) const {
+    const float4* p = f + c * pxy;
+    return SliceData{{ldg(p), ldg(p + 1), ldg(p + px), ldg(p + px + 1)}};
+  }
+  template <bool K>
+  SRT_HD static void x_pass(const SliceData& d, const XDup& w, XRow* r) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float4 a = d.q[2 * j], b = d.q[2 * j + 1];
+      r[j] = x_row<K>(w, make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y), make_float2(b.z, b.w));
+    }
+  }
+  SRT_HD static YIn at(const float2& a, const float2& b) { return YIn{a.x, b.x, a.y, b.y}; }
+};
+
+// Tap column i of a slice: the values of its four rows.
+struct PairTaps {
+  const float2* __restrict__ f;  // pair index of voxel (cx - 1, cy - 1, cz - 1)
+  int64_t px, pxy2;
+  SRT_HD float4 operator()(int c, int i) const {
+    const float2 a = ldg(f + c * pxy2 + i), b = ldg(f + c * pxy2 + 2 * px + i);
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+};
+struct PlaneTaps {
+  const float* __restrict__ f;  // voxel (cx - 1, cy - 1, cz - 1)
+  int64_t px, pxy;
+  SRT_HD float4 operator()(int c, int i) const {
+    const float* p = f + c * pxy + i;
+    return make_float4(ldg(p), ldg(p + px), ldg(p + 2 * px), ldg(p + 3 * px));
   }
 };
 
-// The same interpolation as `tricubic` on packed pairs (two FP32 FMAs per
-// instruction): the x pass on rows y and y+1 at once with duplicated x
-// weights, the y pass with the weights of rows (0, 1) and (2, 3) (even / odd
-// partial sums). Per slice the six y sums are then completed (one add each)
-// and the z pass forms the ten outputs as five pairs with no idle lane:
+template <typename Taps>
+struct TapSource {
+  Taps taps;
+  SRT_HD SliceData load(int c) const { return SliceData{{taps(c, 0), taps(c, 1), taps(c, 2), taps(c, 3)}}; }
+  template <bool K>
+  SRT_HD static void x_pass(const SliceData& d, const XDup& w, XRow* r) {
+    const float2 n2 = dup2(-2.f);
+    float2 q[2][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      q[0][i] = make_float2(d.q[i].y, d.q[i].z);
+      q[1][i] = ffma2(n2, q[0][i], make_float2(d.q[i].x + d.q[i].z, d.q[i].y + d.q[i].w));
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      r[j] = x_row<K>(w, q[j][1], ffma2(n2, q[j][1], fadd2(q[j][0], q[j][2])), q[j][2],
+                      ffma2(n2, q[j][2], fadd2(q[j][1], q[j][3])));
+  }
+  SRT_HD static YIn at(const float2& a, const float2& b) { return YIn{a.x, a.y, b.x, b.y}; }
+};
+
+// The y pass of one order in x: value, d, d2 (m = v2 - v1).
+SRT_HD float y_value(const CWD& w, const YIn& q, float m) {
+  return fmaf(w.w3, q.e2, fmaf(w.w0, q.e1, fmaf(w.t, m, q.v1)));
+}
+SRT_HD float y_first(const CWD& w, const YIn& q, float m) { return fmaf(w.g3, q.e2, fmaf(w.g0, q.e1, m)); }
+SRT_HD float y_second(const CWD& w, const YIn& q) { return fmaf(w.h3, q.e2, w.h0 * q.e1); }
+
+// Tricubic value, gradient and Hessian of the MIXED form: per slice the x pass
+// on packed pairs (two FP32 FMAs per instruction, 16 of them from cells), the y
+// pass on scalars (18), and the z pass as five pairs with no idle lane:
 // (v, gx), (gy, hyy) and (hxx, hxy) from the value weight on both lanes,
 // (gz, hxz) from the derivative weight on both, and (hyz, hzz) from the
-// (derivative, second-derivative) weight pair on (ay, a). Three weight pairs
-// and four operand pairs per slice: each output is still its own chain of
-// FMAs over the slices, so the results do not depend on the pairing, and this
-// one needs the fewest register copies to build the pairs.
-template <typename Rows>
-SRT_HD void tricubic_pair(const Rows& rows, const CRW<float>& X, const CRW<float>& Y, const CRW<float>& Z,
-                          Tri<float>& r) {
+// (derivative, second-derivative) weight pair on (ay, a).
+// Bound by the FMA pipe and by issue: 240 FP32 lane operations in 156
+// instructions and 16 loads per interpolation from cells, against 352 in 188
+// and 32 for the four-tap passes on row pairs this replaces (1024^3 base pixel,
+// 1,048,576 rays x 512 steps: 149.8 -> 128.0 ms; FMA pipe 66 % of cycles, issue
+// 62 %, L1 data 50 %). Second differences along x alone (the y pass on four
+// packed taps) took 136.0 ms; stored along z too they would double the
+// memory for 8 operations more. Where they are formed on the spot (planes) the
+// trace is 0.6-3 % slower than the four-tap passes on planes were.
+template <typename Src>
+SRT_HD void tricubic_mixed(const Src& src, const CWD& X, const CWD& Y, const CRW<float>& Z, Tri<float>& r) {
+  const XDup xd(X);
+  const float2 z0 = make_float2(0.f, 0.f);
+  // z-pass accumulators: (v, gx), (gz, hxz), (gy, hyy), (hyz, hzz), (hxx, hxy)
+  float2 VG0 = z0, G2H02 = z0, G1H11 = z0, H12H22 = z0, H00H01 = z0;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    XRow x[2];
+    Src::template x_pass<false>(src.load(c), xd, x);
+    const YIn v = Src::at(x[0].v, x[1].v), g = Src::at(x[0].g, x[1].g), h = Src::at(x[0].h, x[1].h);
+    const float mv = v.v2 - v.v1, mg = g.v2 - g.v1, mh = h.v2 - h.v1;
+    const float a = y_value(Y, v, mv), ay = y_first(Y, v, mv), ayy = y_second(Y, v);
+    const float ax = y_value(Y, g, mg), axy = y_first(Y, g, mg), axx = y_value(Y, h, mh);
+    const float zw = Z.w[c], zg = Z.g[c], zh = Z.h[c];
+    VG0 = ffma2(dup2(zw), make_float2(a, ax), VG0);
+    G2H02 = ffma2(dup2(zg), make_float2(a, ax), G2H02);
+    G1H11 = ffma2(dup2(zw), make_float2(ay, ayy), G1H11);
+    H12H22 = ffma2(make_float2(zg, zh), make_float2(ay, a), H12H22);
+    H00H01 = ffma2(dup2(zw), make_float2(axx, axy), H00H01);
+  }
+  r.v = VG0.x;
+  r.g[0] = VG0.y;
+  r.g[1] = G1H11.x;
+  r.g[2] = G2H02.x;
+  r.h[0] = H00H01.x;
+  r.h[1] = H00H01.y;
+  r.h[2] = G2H02.y;
+  r.h[3] = G1H11.y;
+  r.h[4] = H12H22.x;
+  r.h[5] = H12H22.y;
+}
+
+// The same on the four taps' values: the x pass on rows y and y+1 at once with
+// duplicated x weights, the y pass with the weights of rows (0, 1) and (2, 3)
+// (even / odd partial sums), the z pass as above. Taken by the few rays of the
+// adjoint whose trajectory passes a cell face within FP32 rounding (kFourTaps).
+struct ValueRows {
+  const float* __restrict__ f;  // voxel (cx - 1, cy - 1, cz - 1)
+  int64_t px, pxy;
+  int ts;
+  SRT_HD float2 operator()(int c, int pr, int i) const {
+    const float* r = f + (c * pxy + 2 * pr * px + i) * ts;
+    return make_float2(ldg(r), ldg(r + px * ts));
+  }
+};
+SRT_HD void tricubic_mixed(const ValueRows& rows, const CRW<float>& X, const CRW<float>& Y, const CRW<float>& Z,
+                           Tri<float>& r) {
   float2 xw[4], xg[4], xh[4];
   for (int i = 0; i < 4; ++i) {
     xw[i] = dup2(X.w[i]);
@@ -294,6 +472,19 @@ SRT_HD void tricubic_pair(const Rows& rows, const CRW<float>& X, const CRW<float
   r.h[5] = H12H22.y;
 }
 
+// Padded coordinates of coordinate c on an axis of extent n: padded coordinate
+// q holds voxel (q - 1) mod n for q in [0, n + 3), so c appears at c + 1 and,
+// near the ends, in the halo (n - 1 -> 0, 0 -> n + 1, 1 -> n + 2). Returns how
+// many of out[0..3] it filled.
+SRT_HD int padded_coords(int64_t c, int64_t n, int64_t out[4]) {
+  int m = 0;
+  out[m++] = c + 1;
+  if (c == n - 1) out[m++] = 0;
+  if (c == 0) out[m++] = n + 1;
+  if (c == 1 % n) out[m++] = n + 2;
+  return m;
+}
+
 // ------------------------------------------------------------ cell lookup
 
 SRT_HD int wrap64(int64_t c, int n) {
@@ -325,6 +516,30 @@ SRT_HD int64_t cell_base_pair(const Geom& G, int cx, int cy, int cz) {
   return (int64_t)cx + G.px * (int64_t)cy + G.pxy2 * (int64_t)cz;
 }
 
+// Source of field f (0-2 B, 3 phi) at cell (cx, cy, cz) in a handle's layout.
+template <int LAYOUT>
+SRT_HD auto cell_source(const FieldPtrs& F, const Geom& G, int f, int64_t base, int64_t basep) {
+  if constexpr (LAYOUT == kCells)
+    return CellSource{F.cell[f] + base + G.px + 1, G.px, G.pxy};
+  else if constexpr (LAYOUT == kPairs)
+    return TapSource<PairTaps>{{F.pr[f] + basep, G.px, G.pxy2}};
+  else if constexpr (LAYOUT == kFourTaps)
+    return ValueRows{(f == 3 ? F.phi : F.b[f]) + base * G.ts, G.px, G.pxy, G.ts};
+  else
+    return TapSource<PlaneTaps>{{(f == 3 ? F.phi : F.b[f]) + base, G.px, G.pxy}};
+}
+template <int LAYOUT>
+SRT_HD auto cell_source(const FieldPtrs& F, const Geom& G, int f, int cx, int cy, int cz) {
+  return cell_source<LAYOUT>(F, G, f, LAYOUT == kPairs ? 0 : cell_base(G, cx, cy, cz),
+                             LAYOUT == kPairs ? cell_base_pair(G, cx, cy, cz) : 0);
+}
+
+// x and y weights of a layout's passes.
+template <int LAYOUT>
+using AxisWeights = typename std::conditional<LAYOUT == kFourTaps, CRW<float>, CWD>::type;
+SRT_HD void axis_weights(float t, CRW<float>& c) { cr_weights_mixed(t, c); }
+SRT_HD void axis_weights(float t, CWD& c) { cr_weights_diff(t, c); }
+
 // REF16 interpolation of one field at a double-precision position: FP32, the
 // cell offset taken as float(x) - float(floor(x)) (snapshot-raytracer.cu:223-230).
 template <typename TapT>
@@ -335,7 +550,8 @@ SRT_HD void interp_ref16(const TapT* f, const Geom& G, double x, double y, doubl
   cr_weights((float)y - (float)iy, Y);
   cr_weights((float)z - (float)iz, Z);
   const int64_t base = cell_base(G, wrap64(ix, G.n[0]), wrap64(iy, G.n[1]), wrap64(iz, G.n[2]));
-  tricubic<float, TapT>(f, base, G.px, G.pxy, X, Y, Z, r);
+  // the FP16 planes are never cells
+  tricubic<float, TapT>(f, base, G.px, G.pxy, sizeof(TapT) == sizeof(float) ? G.ts : 1, X, Y, Z, r);
 }
 
 // --------------------------------------------------- fused chains (FP64, dd)
@@ -431,11 +647,11 @@ SRT_HD void interp_fp64(const float* __restrict__ f, const Geom& G, double x, do
     double a = 0, ay = 0, ayy = 0, ax = 0, axy = 0, axx = 0;
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      const float* row = f + base + c * G.pxy + b * G.px;
+      const float* row = f + (base + c * G.pxy + b * G.px) * G.ts;
       Chain<double> rv, rx, rxx;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const double p = (double)ldg(row + i);
+        const double p = (double)ldg(row + i * G.ts);
         rv.add(X.w[i], p);
         rx.add(X.g[i], p);
         rxx.add(X.h[i], p);
@@ -882,20 +1098,22 @@ struct BAcc {
 // B component C interpolated at the position staggered by -1/2 along axis C,
 // folded into the accumulators. C is a compile-time constant so n[C], a[C]
 // and b[C] stay in registers.
-template <int C, bool PAIR>
+template <int C, int LAYOUT>
 SRT_HD void add_b_component(const FieldPtrs& F, const Geom& G, const int* cc, const int* cs,
-                            const float* ts, const CRW<float>& Cx, const CRW<float>& Cy, const CRW<float>& Cz,
+                            const float* ts, const AxisWeights<LAYOUT>& Cx, const AxisWeights<LAYOUT>& Cy,
+                            const CRW<float>& Cz,
                             const float* n, const float* a, const float* b, BAcc& A) {
-  CRW<float> S;
-  cr_weights_mixed(ts[C], S);
-  const int cx = C == 0 ? cs[0] : cc[0], cy = C == 1 ? cs[1] : cc[1], cz = C == 2 ? cs[2] : cc[2];
+  const auto src = cell_source<LAYOUT>(F, G, C, C == 0 ? cs[0] : cc[0], C == 1 ? cs[1] : cc[1], C == 2 ? cs[2] : cc[2]);
   Tri<float> r;
-  if (PAIR)
-    tricubic_pair(PairRows{F.pr[C], cell_base_pair(G, cx, cy, cz), G.px, G.pxy2}, C == 0 ? S : Cx, C == 1 ? S : Cy,
-                  C == 2 ? S : Cz, r);
-  else
-    tricubic_pair(SingleRows{F.b[C], cell_base(G, cx, cy, cz), G.px, G.pxy}, C == 0 ? S : Cx, C == 1 ? S : Cy,
-                  C == 2 ? S : Cz, r);
+  if constexpr (C == 2) {
+    CRW<float> S;
+    cr_weights_mixed(ts[2], S);
+    tricubic_mixed(src, Cx, Cy, S, r);
+  } else {
+    AxisWeights<LAYOUT> S;
+    axis_weights(ts[C], S);
+    tricubic_mixed(src, C == 0 ? S : Cx, C == 1 ? S : Cy, Cz, r);
+  }
   A.val[C] = r.v;
   for (int i = 0; i < 3; ++i) A.ngB[i] += r.g[i] * n[C];
   A.Gn[C] = r.g[0] * n[0] + r.g[1] * n[1] + r.g[2] * n[2];
@@ -957,7 +1175,7 @@ struct Guard {
   SRT_HD void end_step(int step) { near |= m[1] < kFaceGuardRel * ((float)(step + 1) * m[0] + kFaceGuardFloor); }
 };
 
-template <bool PAIR>
+template <int LAYOUT>
 SRT_HD void rhs_mixed(const float* d, float s, const MixedRay& R, const FieldPtrs& F, const Geom& G,
                       const float* x0, float* g, Guard& gd) {
   float Dn[3], Da[3], Db[3];
@@ -984,25 +1202,22 @@ SRT_HD void rhs_mixed(const float* d, float s, const MixedRay& R, const FieldPtr
   // at s = 0 the ray sits exactly on the observer (a grid node, offsets
   // exactly 0) in both precisions, so no cell choice can differ there
   gd.face(s > 0.f ? fminf(fminf(df[0], df[1]), df[2]) : 1.f);
-  CRW<float> Cx, Cy, Cz;  // centred weights, shared by phi and two axes of each B component
-  cr_weights_mixed(tc[0], Cx);
-  cr_weights_mixed(tc[1], Cy);
+  AxisWeights<LAYOUT> Cx, Cy;  // centred weights, shared by phi and two axes of each B component
+  CRW<float> Cz;
+  axis_weights(tc[0], Cx);
+  axis_weights(tc[1], Cy);
   cr_weights_mixed(tc[2], Cz);
   BAcc A;
   A.ngB[0] = A.ngB[1] = A.ngB[2] = 0.f;
   A.nlap = 0.f;
   for (int i = 0; i < 6; ++i) A.T[i] = 0.f;
-  add_b_component<0, PAIR>(F, G, cc, cs, ts, Cx, Cy, Cz, n, a, b, A);
-  add_b_component<1, PAIR>(F, G, cc, cs, ts, Cx, Cy, Cz, n, a, b, A);
+  add_b_component<0, LAYOUT>(F, G, cc, cs, ts, Cx, Cy, Cz, n, a, b, A);
+  add_b_component<1, LAYOUT>(F, G, cc, cs, ts, Cx, Cy, Cz, n, a, b, A);
   // phi between the second and third B components: the same values in any
-  // order (the B sums keep theirs), and this one schedules best (1.0 % over
-  // phi last, 3 % over phi first, on the 1024^3 trace)
+  // order (the B sums keep theirs), and this one schedules best
   Tri<float> p;
-  if (PAIR)
-    tricubic_pair(PairRows{F.pr[3], cell_base_pair(G, cc[0], cc[1], cc[2]), G.px, G.pxy2}, Cx, Cy, Cz, p);
-  else
-    tricubic_pair(SingleRows{F.phi, cell_base(G, cc[0], cc[1], cc[2]), G.px, G.pxy}, Cx, Cy, Cz, p);
-  add_b_component<2, PAIR>(F, G, cc, cs, ts, Cx, Cy, Cz, n, a, b, A);
+  tricubic_mixed(cell_source<LAYOUT>(F, G, 3, cc[0], cc[1], cc[2]), Cx, Cy, Cz, p);
+  add_b_component<2, LAYOUT>(F, G, cc, cs, ts, Cx, Cy, Cz, n, a, b, A);
 
   const float dA = s + d[12];
   const float dAp = d[13] - 1.f;
@@ -1115,7 +1330,7 @@ SRT_HD void mixed_stage(const float* y, const float* k, float c, float* ys) {
 // the compensations folded in) are stored there: component j of stage st at
 // us[(19 st + j) * stride]. gd.near is set when a stage of the step came
 // within the guards above.
-template <bool PAIR = false>
+template <int LAYOUT = kPlanes>
 SRT_HD void step_mixed(const MixedRay& R, const FieldPtrs& F, const Geom& G, const float* x0, int step, float* y,
                        float* us, int64_t stride, Guard& gd) {
   float k[19], acc[19], ys[19];
@@ -1127,7 +1342,7 @@ SRT_HD void step_mixed(const MixedRay& R, const FieldPtrs& F, const Geom& G, con
     mixed_stage(y, k, c, ys);
     if (us)
       for (int j = 0; j < 19; ++j) st_stream(us + (19 * st + j) * stride, ys[j]);
-    rhs_mixed<PAIR>(ys, s0 + c, R, F, G, x0, k, gd);
+    rhs_mixed<LAYOUT>(ys, s0 + c, R, F, G, x0, k, gd);
     {  // acc = k1 + 2 k2 + 2 k3 with weights 1, 2, 2, 0 on a zeroed accumulator
        // (stage 4's k is added at the update): the same FMAs where a stage
        // adds, exact no-ops where it does not, and no branch
@@ -1188,7 +1403,7 @@ SRT_HD void extract_mixed(const MixedRay& R, int n_steps, const float* y, float 
 
 // Returns true when the ray came within the guards (its FP64 trace may
 // differ by a cell choice; the caller re-traces it in FP64).
-template <bool PAIR = false>
+template <int LAYOUT = kPlanes>
 SRT_HD bool trace_ray_mixed(const FieldPtrs& F, const Geom& G, const RayDir& d, int n_steps, float out[6],
                             float* guard_m) {
   MixedRay R;
@@ -1201,7 +1416,7 @@ SRT_HD bool trace_ray_mixed(const FieldPtrs& F, const Geom& G, const RayDir& d, 
 #pragma unroll 1
   for (int step = 0; step < n_steps; ++step) {
     gd.begin_step(y);
-    step_mixed<PAIR>(R, F, G, x0, step, y, nullptr, 0, gd);
+    step_mixed<LAYOUT>(R, F, G, x0, step, y, nullptr, 0, gd);
     gd.end_step(step);
   }
   extract_mixed(R, n_steps, y, out);

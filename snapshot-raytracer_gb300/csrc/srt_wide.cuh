@@ -238,12 +238,12 @@ struct WideLane {
   SRT_HD void load_taps(const int* cell, const FieldPtrs& F, const Geom& G) {
     const int f = lane >> 3, sub = lane & 7;
     const float* src = f == 3 ? F.phi : (f == 0 ? F.b[0] : (f == 1 ? F.b[1] : F.b[2]));
-    const float* p = src + cell_base(G, cell[f == 0 ? 3 : 0], cell[f == 1 ? 4 : 1], cell[f == 2 ? 5 : 2]) +
-                     (sub >> 1) * G.pxy + 2 * (sub & 1) * G.px;
+    const float* p = src + (cell_base(G, cell[f == 0 ? 3 : 0], cell[f == 1 ? 4 : 1], cell[f == 2 ? 5 : 2]) +
+                            (sub >> 1) * G.pxy + 2 * (sub & 1) * G.px) * G.ts;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) tap[i] = ldg(p + i);
+    for (int i = 0; i < 4; ++i) tap[i] = ldg(p + i * G.ts);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) tap[4 + i] = ldg(p + G.px + i);
+    for (int i = 0; i < 4; ++i) tap[4 + i] = ldg(p + (G.px + i) * G.ts);
   }
 
   SRT_HD void weights(R* S) const {
