@@ -23,7 +23,6 @@
 #include <chrono>
 #include <cstring>
 #include <type_traits>
-#include <vector>
 #include "srt_adjoint.cuh"
 #include "srt_internal.h"
 
@@ -53,6 +52,32 @@ __global__ void ray_count_kernel(const RangeArgs a, int* counts) {
   const int in = ring_of_slot(a, t) >= 0;
   const int c = __syncthreads_count(in);
   if (threadIdx.x == 0) counts[blockIdx.x] = c;
+}
+
+// Exclusive sums of n block counts, by one block.
+__global__ void __launch_bounds__(1024) ray_scan_kernel(const int* counts, int64_t n, int64_t* offsets) {
+  __shared__ int warp_sum[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int64_t run = 0;
+  for (int64_t q0 = 0; q0 < n; q0 += 1024) {
+    const int64_t q = q0 + threadIdx.x;
+    const int c = q < n ? counts[q] : 0;
+    int sum = c;  // inclusive within the warp
+    for (int d = 1; d < 32; d *= 2) {
+      const int v = __shfl_up_sync(0xffffffffu, sum, d);
+      if (lane >= d) sum += v;
+    }
+    if (lane == 31) warp_sum[warp] = sum;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int w = 0; w < 32; ++w) {
+      before += w < warp ? warp_sum[w] : 0;
+      all += warp_sum[w];
+    }
+    if (q < n) offsets[q] = run + before + sum - c;
+    run += all;
+    __syncthreads();
+  }
 }
 
 __global__ void ray_write_kernel(const RangeArgs a, const int64_t* offsets, int64_t* rays) {
@@ -611,12 +636,14 @@ using namespace srt;
 
 namespace {
 
-struct DevBuf {
+struct DevBuf {  // scratch, given back on the stream it was taken on
   void* p = nullptr;
-  ~DevBuf() {
-    if (p) cudaFree(p);
+  cudaStream_t s = nullptr;
+  ~DevBuf() { pool_free(p, s); }
+  cudaError_t alloc(size_t bytes, cudaStream_t stream) {
+    s = stream;
+    return scratch_alloc(&p, bytes, stream);
   }
-  cudaError_t alloc(size_t bytes) { return dev_alloc(&p, bytes); }
 };
 
 template <typename Acc, typename E>
@@ -640,7 +667,7 @@ namespace {
 // Morton-ordered list of the RING pixels in [pix_begin, pix_begin + pix_count)
 // (the forward's launch order) -> rays.
 int build_ray_list(int64_t nside, int64_t pix_begin, int64_t pix_count, cudaStream_t s, DevBuf& counts,
-                   DevBuf& offsets, DevBuf& rays, int64_t* kernels, const char* who) {
+                   DevBuf& offsets, DevBuf& rays, int64_t* kernels) {
   int rc = SRT_OK;
   RangeArgs ra;
   ra.nside = nside;
@@ -651,30 +678,14 @@ int build_ray_list(int64_t nside, int64_t pix_begin, int64_t pix_count, cudaStre
   ra.pix_begin = pix_begin;
   ra.pix_count = pix_count;
   const int64_t nblk = (ra.launch_rays + kListBlock - 1) / kListBlock;
-  std::vector<int> hc(nblk);
-  std::vector<int64_t> ho(nblk);
-  int64_t run = 0;
-  VJP_TRY(counts.alloc(nblk * sizeof(int)), "cudaMalloc(ray counts)");
-  VJP_TRY(offsets.alloc(nblk * sizeof(int64_t)), "cudaMalloc(ray offsets)");
-  VJP_TRY(rays.alloc(pix_count * sizeof(int64_t)), "cudaMalloc(ray list)");
+  VJP_TRY(counts.alloc(nblk * sizeof(int), s), "allocate ray counts");
+  VJP_TRY(offsets.alloc(nblk * sizeof(int64_t), s), "allocate ray offsets");
+  VJP_TRY(rays.alloc(pix_count * sizeof(int64_t), s), "allocate ray list");
   ray_count_kernel<<<(unsigned)nblk, kListBlock, 0, s>>>(ra, (int*)counts.p);
-  ++*kernels;
-  VJP_TRY(cudaGetLastError(), "ray_count_kernel");
-  VJP_TRY(cudaMemcpyAsync(hc.data(), counts.p, nblk * sizeof(int), cudaMemcpyDeviceToHost, s), "copy counts");
-  VJP_TRY(cudaStreamSynchronize(s), "ray count");
-  for (int64_t b = 0; b < nblk; ++b) {
-    ho[b] = run;
-    run += hc[b];
-  }
-  if (run != pix_count)
-    return set_error(SRT_ERR_CUDA, "%s: ray list has %lld rays, expected %lld", who, (long long)run,
-                     (long long)pix_count);
-  VJP_TRY(cudaMemcpyAsync(offsets.p, ho.data(), nblk * sizeof(int64_t), cudaMemcpyHostToDevice, s), "copy offsets");
+  ray_scan_kernel<<<1, 1024, 0, s>>>((const int*)counts.p, nblk, (int64_t*)offsets.p);
   ray_write_kernel<<<(unsigned)nblk, kListBlock, 0, s>>>(ra, (const int64_t*)offsets.p, (int64_t*)rays.p);
-  ++*kernels;
-  VJP_TRY(cudaGetLastError(), "ray_write_kernel");
-  // the host vectors must outlive the asynchronous copy of the offsets
-  VJP_TRY(cudaStreamSynchronize(s), "ray list");
+  *kernels += 3;
+  VJP_TRY(cudaGetLastError(), "ray list kernels");
 done:
   return rc;
 }
@@ -751,14 +762,14 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
     if (!dev_io) {
       // host gradients: start from zero (or from the caller's values when accumulating)
       if (dphi) {
-        VJP_TRY(gout_phi.alloc(vox * sizeof(float)), "cudaMalloc(dphi)");
+        VJP_TRY(gout_phi.alloc(vox * sizeof(float), s), "allocate dphi");
         if (accumulate) {
           VJP_TRY(cudaMemcpyAsync(gout_phi.p, dphi, vox * sizeof(float), cudaMemcpyHostToDevice, s), "copy dphi");
           h2d += vox * sizeof(float);
         }
       }
       if (db_xyz) {
-        VJP_TRY(gout_b.alloc(3 * vox * sizeof(float)), "cudaMalloc(db)");
+        VJP_TRY(gout_b.alloc(3 * vox * sizeof(float), s), "allocate db");
         if (accumulate) {
           VJP_TRY(cudaMemcpyAsync(gout_b.p, db_xyz, 3 * vox * sizeof(float), cudaMemcpyHostToDevice, s), "copy db");
           h2d += 3 * vox * sizeof(float);
@@ -771,7 +782,7 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
       // ---- ray list (a tape brings its own)
       int64_t* ray_list = tape ? tape->rays : nullptr;
       if (!tape) {
-        rc = build_ray_list(nside, pix_begin, pix_count, s, counts, offsets, rays, &kernels, "srt_vjp");
+        rc = build_ray_list(nside, pix_begin, pix_count, s, counts, offsets, rays, &kernels);
         if (rc != SRT_OK) goto done;
         ray_list = (int64_t*)rays.p;
       }
@@ -781,7 +792,7 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
       if (dev_io) {
         for (int m = 0; m < 6; ++m) wd[m] = weights[m];
       } else {
-        VJP_TRY(wdev.alloc(6 * pix_count * sizeof(float)), "cudaMalloc(weights)");
+        VJP_TRY(wdev.alloc(6 * pix_count * sizeof(float), s), "allocate weights");
         for (int m = 0; m < 6; ++m) {
           VJP_TRY(cudaMemcpyAsync((float*)wdev.p + m * pix_count, weights[m], pix_count * sizeof(float),
                                   cudaMemcpyHostToDevice, s),
@@ -794,27 +805,27 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
       // ---- scratch: checkpoints, segment records, padded accumulators
       const int state = fp64 ? 19 : kMixedState;
       const size_t esz = fp64 ? sizeof(double) : sizeof(float);
-      if (!tape) VJP_TRY(ckpt.alloc((size_t)(nseg + 1) * state * pix_count * esz), "cudaMalloc(checkpoints)");
+      if (!tape) VJP_TRY(ckpt.alloc((size_t)(nseg + 1) * state * pix_count * esz, s), "allocate checkpoints");
       if (!tape && !fp64) {
-        VJP_TRY(near.alloc((pix_count + 1) * sizeof(int64_t)), "cudaMalloc(near rays)");
+        VJP_TRY(near.alloc((pix_count + 1) * sizeof(int64_t), s), "allocate near rays");
         VJP_TRY(cudaMemsetAsync(near.p, 0, sizeof(int64_t), s), "clear near rays");
-        VJP_TRY(bases.alloc((size_t)12 * pix_count * sizeof(float)), "cudaMalloc(ray bases)");
+        VJP_TRY(bases.alloc((size_t)12 * pix_count * sizeof(float), s), "allocate ray bases");
       }
       // copies of the region around the observer (FP32 accumulation), where the
       // grid holds the region
       const bool hot = !fp64 && !determ && std::min(f->n[0], std::min(f->n[1], f->n[2])) >= kHotSide;
       const int64_t acc_entries = pvox + (hot ? (int64_t)kHotCopies * kHotSide * kHotSide * kHotSide : 0);
       // per-step records of one segment: FP64 y, k1, k2, k3; MIXED the four stage inputs
-      VJP_TRY(seg.alloc((size_t)C * (fp64 ? state + 57 : kTapeStep) * pix_count * esz), "cudaMalloc(segment records)");
-      if (!fp64) VJP_TRY(lam.alloc((size_t)19 * pix_count * sizeof(float)), "cudaMalloc(state cotangents)");
+      VJP_TRY(seg.alloc((size_t)C * (fp64 ? state + 57 : kTapeStep) * pix_count * esz, s), "allocate segment records");
+      if (!fp64) VJP_TRY(lam.alloc((size_t)19 * pix_count * sizeof(float), s), "allocate state cotangents");
       for (int fld = 0; fld < 4; ++fld) {
         const bool want = (fld == 3) ? (dphi != nullptr) : (db_xyz != nullptr);
         if (!want) continue;
-        VJP_TRY(gacc[fld].alloc(acc_entries * accsz), "cudaMalloc(gradient accumulators)");
+        VJP_TRY(gacc[fld].alloc(acc_entries * accsz, s), "allocate gradient accumulators");
         VJP_TRY(cudaMemsetAsync(gacc[fld].p, 0, acc_entries * accsz, s), "clear accumulators");
       }
       if (determ) {  // fixed-point range flag
-        VJP_TRY(ovf.alloc(sizeof(unsigned)), "cudaMalloc(overflow flag)");
+        VJP_TRY(ovf.alloc(sizeof(unsigned), s), "allocate overflow flag");
         VJP_TRY(cudaMemsetAsync(ovf.p, 0, sizeof(unsigned), s), "clear overflow flag");
       }
 
@@ -924,10 +935,11 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
         d2h += 3 * vox * sizeof(float);
       }
     }
+    unsigned flag = 0;
+    if (ovf.p)
+      VJP_TRY(cudaMemcpyAsync(&flag, ovf.p, sizeof(flag), cudaMemcpyDeviceToHost, s), "read overflow flag");
     VJP_TRY(cudaStreamSynchronize(s), "srt_vjp");
     if (ovf.p) {
-      unsigned flag = 0;
-      VJP_TRY(cudaMemcpy(&flag, ovf.p, sizeof(flag), cudaMemcpyDeviceToHost), "read overflow flag");
       if (flag) {
         rc = set_error(SRT_ERR_OVERFLOW,
                        "srt_vjp: SRT_DETERMINISTIC gradient beyond the fixed-point range (|gradient| >= 2^30 per "
@@ -947,6 +959,7 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
     }
   }
 done:
+  if (rc != SRT_OK) cudaStreamSynchronize(s);  // copies from or to the caller's buffers may be under way
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   if (prev != f->device) cudaSetDevice(prev);
@@ -996,20 +1009,20 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
     goto done;
   }
   {
-    rc = build_ray_list(nside, pix_begin, pix_count, s, counts, offsets, rays, &kernels, "srt_forward_tape");
+    rc = build_ray_list(nside, pix_begin, pix_count, s, counts, offsets, rays, &kernels);
     if (rc != SRT_OK) goto done;
-    VJP_TRY(ckpt.alloc((size_t)(nseg + 1) * kMixedState * pix_count * sizeof(float)), "cudaMalloc(checkpoints)");
-    VJP_TRY(near.alloc((pix_count + 1) * sizeof(int64_t)), "cudaMalloc(near rays)");
+    VJP_TRY(ckpt.alloc((size_t)(nseg + 1) * kMixedState * pix_count * sizeof(float), s), "allocate checkpoints");
+    VJP_TRY(near.alloc((pix_count + 1) * sizeof(int64_t), s), "allocate near rays");
     VJP_TRY(cudaMemsetAsync(near.p, 0, sizeof(int64_t), s), "clear near rays");
-    VJP_TRY(bases.alloc((size_t)12 * pix_count * sizeof(float)), "cudaMalloc(ray bases)");
-    VJP_TRY(rlist.alloc(pix_count * sizeof(int64_t)), "cudaMalloc(refine list)");
-    VJP_TRY(rcount.alloc(sizeof(unsigned long long)), "cudaMalloc(refine count)");
+    VJP_TRY(bases.alloc((size_t)12 * pix_count * sizeof(float), s), "allocate ray bases");
+    VJP_TRY(rlist.alloc(pix_count * sizeof(int64_t), s), "allocate refine list");
+    VJP_TRY(rcount.alloc(sizeof(unsigned long long), s), "allocate refine count");
     VJP_TRY(cudaMemsetAsync(rcount.p, 0, sizeof(unsigned long long), s), "clear refine count");
     float* dm[6];
     if (dev_out) {
       for (int m = 0; m < 6; ++m) dm[m] = maps[m];
     } else {
-      VJP_TRY(dmaps.alloc(6 * pix_count * sizeof(float)), "cudaMalloc(maps)");
+      VJP_TRY(dmaps.alloc(6 * pix_count * sizeof(float), s), "allocate maps");
       for (int m = 0; m < 6; ++m) dm[m] = (float*)dmaps.p + m * pix_count;
     }
     AdjArgs A;
@@ -1053,6 +1066,8 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
       for (int m = 0; m < 6; ++m)
         VJP_TRY(cudaMemcpyAsync(maps[m], dm[m], pix_count * sizeof(float), cudaMemcpyDeviceToHost, s),
                 "copy maps to host");
+    unsigned long long refined = 0;
+    VJP_TRY(cudaMemcpyAsync(&refined, rcount.p, sizeof(refined), cudaMemcpyDeviceToHost, s), "read refine count");
     VJP_TRY(cudaStreamSynchronize(s), "srt_forward_tape");
     if (stats) {
       float ms = -1.f;
@@ -1062,9 +1077,7 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
       stats->ray_steps = pix_count * (int64_t)n_steps;
       stats->kernels = kernels;
       stats->d2h_bytes = dev_out ? 0 : 6 * pix_count * (int64_t)sizeof(float);
-      unsigned long long cnt = 0;
-      if (cudaMemcpy(&cnt, rcount.p, sizeof(cnt), cudaMemcpyDeviceToHost) == cudaSuccess)
-        stats->refined_rays = (int64_t)cnt;
+      stats->refined_rays = (int64_t)refined;
     }
     t->fields = f;
     t->device = f->device;
@@ -1087,6 +1100,7 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
     t = nullptr;
   }
 done:
+  if (rc != SRT_OK) cudaStreamSynchronize(s);
   delete t;
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
@@ -1111,10 +1125,8 @@ extern "C" int srt_tape_destroy(srt_tape* tape) {
   int prev = 0;
   cudaGetDevice(&prev);
   if (prev != tape->device) cudaSetDevice(tape->device);
-  if (tape->rays) cudaFree(tape->rays);
-  if (tape->near) cudaFree(tape->near);
-  if (tape->bases) cudaFree(tape->bases);
-  if (tape->ckpt) cudaFree(tape->ckpt);
+  // the calls that used the tape have returned, and they are synchronous
+  for (void* p : {(void*)tape->rays, (void*)tape->near, (void*)tape->bases, (void*)tape->ckpt}) pool_free(p, nullptr);
   if (prev != tape->device) cudaSetDevice(prev);
   delete tape;
   return SRT_OK;

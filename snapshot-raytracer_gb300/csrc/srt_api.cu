@@ -21,14 +21,22 @@ thread_local std::string g_last_error;
 // mapped memory instead of paying the driver's mapping cost (~0.3 s for the
 // 52 GB of a 1024^3 handle). A failed allocation trims the pool and retries
 // once; srt_release_cached_memory() trims it on request.
+//
+// Scratch (a call's lists, checkpoints, tapes and accumulators) comes from a
+// second pool that keeps at most kScratchKeep of what is handed back: a cudaMalloc
+// / cudaFree pair per buffer cost a 60x52x68 gradient 0.7 of its 2.5 ms, and the
+// default pool's mapping after each synchronisation a small forward ~20 us.
 constexpr int kMaxPoolDevices = 64;
+constexpr uint64_t kScratchKeep = 8ull << 30;
+enum { kFieldPool = 0, kScratchPool = 1 };
 std::mutex g_pool_mutex;
-cudaMemPool_t g_pool[kMaxPoolDevices] = {};
+cudaMemPool_t g_pool[2][kMaxPoolDevices] = {};
 
-cudaError_t device_pool(int dev, cudaMemPool_t* out) {
+cudaError_t device_pool(int which, int dev, cudaMemPool_t* out) {
   if (dev < 0 || dev >= kMaxPoolDevices) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lock(g_pool_mutex);
-  if (!g_pool[dev]) {
+  cudaMemPool_t& slot = g_pool[which][dev];
+  if (!slot) {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -36,16 +44,43 @@ cudaError_t device_pool(int dev, cudaMemPool_t* out) {
     cudaMemPool_t pool = nullptr;
     cudaError_t e = cudaMemPoolCreate(&pool, &props);
     if (e != cudaSuccess) return e;
-    uint64_t keep = ~0ull;
+    uint64_t keep = which == kFieldPool ? ~0ull : kScratchKeep;
     e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     if (e != cudaSuccess) {
       cudaMemPoolDestroy(pool);
       return e;
     }
-    g_pool[dev] = pool;
+    slot = pool;
   }
-  *out = g_pool[dev];
+  *out = slot;
   return cudaSuccess;
+}
+
+void trim_pools(int dev) {
+  for (int which : {kFieldPool, kScratchPool}) {
+    cudaMemPool_t pool = nullptr;
+    {
+      std::lock_guard<std::mutex> lock(g_pool_mutex);
+      pool = g_pool[which][dev];
+    }
+    if (pool) cudaMemPoolTrimTo(pool, 0);
+  }
+}
+
+cudaError_t alloc_from(int which, void** p, size_t bytes, cudaStream_t s) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  cudaMemPool_t pool = nullptr;
+  if (e == cudaSuccess) e = device_pool(which, dev, &pool);
+  if (e != cudaSuccess) return e;
+  e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, s);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    cudaStreamSynchronize(s);
+    trim_pools(dev);
+    e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, s);
+  }
+  return e;
 }
 }  // namespace
 
@@ -63,46 +98,32 @@ bool alloc_fault() {
   return false;
 }
 
-cudaError_t dev_alloc(void** p, size_t bytes) {
-  if (alloc_fault()) return cudaErrorMemoryAllocation;
-  return cudaMalloc(p, bytes ? bytes : 1);
-}
-
-cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s) {
-  if (alloc_fault()) return cudaErrorMemoryAllocation;
-  return cudaMallocAsync(p, bytes ? bytes : 1, s);
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+  return alloc_fault() ? cudaErrorMemoryAllocation : alloc_from(kScratchPool, p, bytes, s);
 }
 
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
-  if (alloc_fault()) return cudaErrorMemoryAllocation;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  cudaMemPool_t pool = nullptr;
-  if (e == cudaSuccess) e = device_pool(dev, &pool);
-  if (e != cudaSuccess) return e;
-  e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, s);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    cudaStreamSynchronize(s);
-    cudaMemPoolTrimTo(pool, 0);
-    e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, s);
-  }
-  return e;
+  return alloc_fault() ? cudaErrorMemoryAllocation : alloc_from(kFieldPool, p, bytes, s);
 }
 
 void pool_free(void* p, cudaStream_t s) {
   if (p) cudaFreeAsync(p, s);
 }
 
-// Bytes the device's pool holds but does not use (reusable by pool_alloc).
+// Bytes the device's pools hold but do not use (reusable by pool_alloc, which
+// trims both before it gives up).
 int64_t pool_reusable_bytes(int dev) {
-  cudaMemPool_t pool = nullptr;
-  if (device_pool(dev, &pool) != cudaSuccess) return 0;
-  uint64_t reserved = 0, used = 0;
-  if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
-      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
-    return 0;
-  return reserved > used ? (int64_t)(reserved - used) : 0;
+  int64_t sum = 0;
+  for (int which : {kFieldPool, kScratchPool}) {
+    cudaMemPool_t pool = nullptr;
+    uint64_t reserved = 0, used = 0;
+    if (device_pool(which, dev, &pool) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+      continue;
+    sum += reserved > used ? (int64_t)(reserved - used) : 0;
+  }
+  return sum;
 }
 
 }  // namespace srt
@@ -423,15 +444,13 @@ int srt_release_cached_memory(void) {
   int prev = 0;
   cudaGetDevice(&prev);
   for (int d = 0; d < n && d < kMaxPoolDevices; ++d) {
-    cudaMemPool_t pool = nullptr;
     {
       std::lock_guard<std::mutex> lock(g_pool_mutex);
-      pool = g_pool[d];
+      if (!g_pool[kFieldPool][d] && !g_pool[kScratchPool][d]) continue;
     }
-    if (!pool) continue;
     cudaSetDevice(d);
     cudaDeviceSynchronize();
-    cudaMemPoolTrimTo(pool, 0);
+    trim_pools(d);
   }
   cudaSetDevice(prev);
   return SRT_OK;
@@ -512,8 +531,8 @@ int srt_forward(const srt_fields* fields, int64_t nside, int64_t pix_begin, int6
     a.refine_count = nullptr;
     const bool refine = precision == SRT_PRECISION_MIXED && !(flags & SRT_MIXED_NO_REFINE);
     if (refine) {
-      SRT_CUDA_TRY(dev_alloc_async((void**)&refine_list, pix_count * sizeof(int64_t), s), "cudaMallocAsync(refine list)");
-      SRT_CUDA_TRY(dev_alloc_async((void**)&refine_count, sizeof(unsigned long long), s), "cudaMallocAsync(refine count)");
+      SRT_CUDA_TRY(scratch_alloc((void**)&refine_list, pix_count * sizeof(int64_t), s), "allocate refine list");
+      SRT_CUDA_TRY(scratch_alloc((void**)&refine_count, sizeof(unsigned long long), s), "allocate refine count");
       SRT_CUDA_TRY(cudaMemsetAsync(refine_count, 0, sizeof(unsigned long long), s), "clear refine count");
       a.refine_list = refine_list;
       a.refine_count = refine_count;
@@ -523,7 +542,7 @@ int srt_forward(const srt_fields* fields, int64_t nside, int64_t pix_begin, int6
     } else {
       // stream-ordered: a plain device allocation issued here would keep this
       // trace from running beside work already queued on other streams
-      SRT_CUDA_TRY(dev_alloc_async((void**)&dmaps, 6 * pix_count * sizeof(float), s), "cudaMallocAsync(maps)");
+      SRT_CUDA_TRY(scratch_alloc((void**)&dmaps, 6 * pix_count * sizeof(float), s), "allocate maps");
       for (int m = 0; m < 6; ++m) a.maps[m] = dmaps + m * pix_count;
     }
     const bool timed = !(flags & SRT_ASYNC);
@@ -543,6 +562,9 @@ int srt_forward(const srt_fields* fields, int64_t nside, int64_t pix_begin, int6
         SRT_CUDA_TRY(cudaMemcpyAsync(maps[m], a.maps[m], pix_count * sizeof(float), cudaMemcpyDeviceToHost, s),
                      "copy maps to host");
     }
+    unsigned long long refined = 0;
+    if (refine && timed && stats)
+      SRT_CUDA_TRY(cudaMemcpyAsync(&refined, refine_count, sizeof(refined), cudaMemcpyDeviceToHost, s), "read refine count");
     if (timed || !dev_out) SRT_CUDA_TRY(cudaStreamSynchronize(s), "trace");
     if (stats) {
       float ms = -1.f, rms = 0.f;
@@ -556,18 +578,14 @@ int srt_forward(const srt_fields* fields, int64_t nside, int64_t pix_begin, int6
       stats->ray_steps = pix_count * (int64_t)n_steps;
       stats->kernels = kernels;
       stats->d2h_bytes = dev_out ? 0 : 6 * pix_count * (int64_t)sizeof(float);
-      if (refine && timed) {
-        unsigned long long cnt = 0;
-        if (cudaMemcpy(&cnt, refine_count, sizeof(cnt), cudaMemcpyDeviceToHost) == cudaSuccess)
-          stats->refined_rays = (int64_t)cnt;
-      }
+      stats->refined_rays = (int64_t)refined;
     }
   }
 fail:
-  if (dmaps) cudaFreeAsync(dmaps, s);
+  pool_free(dmaps, s);
   // stream-ordered release: the refine kernel may still be queued (SRT_ASYNC)
-  if (refine_list) cudaFreeAsync(refine_list, s);
-  if (refine_count) cudaFreeAsync(refine_count, s);
+  pool_free(refine_list, s);
+  pool_free(refine_count, s);
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   if (em) cudaEventDestroy(em);

@@ -36,10 +36,10 @@ namespace srt {
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s);
 void pool_free(void* p, cudaStream_t s);
 int64_t pool_reusable_bytes(int dev);
-// cudaMalloc / cudaMallocAsync behind the failure-injection hook
-// (srt_debug_fail_alloc); pool_alloc checks the hook too.
-cudaError_t dev_alloc(void** p, size_t bytes);
-cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s);
+// A call's scratch, from a second pool that keeps a bounded amount; given back by
+// pool_free on the stream of its last use. Both allocations go through the
+// failure-injection hook (srt_debug_fail_alloc).
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
 
 // NVTX range over a scope (the public entry points and their phases), for
 // profilers' timelines and range filters; header-only, inert unless a tool
