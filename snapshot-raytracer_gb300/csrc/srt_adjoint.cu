@@ -203,7 +203,7 @@ __device__ __forceinline__ void ckpt_ray(const AdjArgs& A, int64_t slot, const R
   for (int st = 0; st < A.n_steps; ++st) {
     if (LAYOUT == kFourTaps) prefetch_step(A, R, x0, y, st);
     if (gd.m) gd.begin_step(y);
-    step_mixed<LAYOUT>(R, A.F, A.G, x0, st, y, nullptr, 0, gd);
+    step_mixed(OneLane<LAYOUT>(), R, A.F, A.G, x0, st, y, nullptr, 0, gd);
     if (gd.m) gd.end_step(st);
     const int done = st + 1;
     if (done % A.C == 0 || done == A.n_steps) {
@@ -309,7 +309,7 @@ __device__ __forceinline__ void segment_ray(const AdjArgs& A, int sgi, int64_t s
   for (int st = s0; st < s1; ++st) {
     Guard gd;  // disabled
     if (LAYOUT == kFourTaps) prefetch_step(A, R, x0, y, st);
-    step_mixed<LAYOUT>(R, A.F, A.G, x0, st, y, tape + (int64_t)(st - s0) * kTapeStep * A.count + slot, A.count, gd);
+    step_mixed(OneLane<LAYOUT>(), R, A.F, A.G, x0, st, y, tape + (int64_t)(st - s0) * kTapeStep * A.count + slot, A.count, gd);
   }
 }
 

@@ -20,7 +20,10 @@ struct srt_fields {
   float* phi = nullptr;
   float* b[3] = {nullptr, nullptr, nullptr};
   float2* pr[4] = {nullptr, nullptr, nullptr, nullptr};
-  __half* bh[3] = {nullptr, nullptr, nullptr};  // padded half(B * 2^27), made on first REF16 use
+  // made on first REF16 use: padded half(B * 2^27), and phi as a plane where the
+  // fields are cells
+  __half* bh[3] = {nullptr, nullptr, nullptr};
+  float* ref_phi = nullptr;
   int64_t bytes = 0;
   int layout() const { return cell[0] ? srt::kCells : (pr[0] ? srt::kPairs : srt::kPlanes); }
   // the MIXED trace kernel of this layout
@@ -85,6 +88,8 @@ cudaError_t launch_cells(const float* src, int comps, float4* const dst[3], cons
 // count floats from mapped pinned host memory to device memory.
 cudaError_t launch_fetch(const float* src, float* dst, int64_t count, cudaStream_t s);
 cudaError_t launch_quantize_half(const float* src, int ts, __half* dst, int64_t count, cudaStream_t s);
+// The same values as a plane.
+cudaError_t launch_extract(const float* src, int ts, float* dst, int64_t count, cudaStream_t s);
 cudaError_t launch_pair_build(const float* src, float2* dst, const int64_t pn[3], cudaStream_t s);
 
 // Trace kernel launch (mode = kFP64 / kREF16 / a handle's mixed_mode()).
@@ -110,6 +115,9 @@ void h5_field_close(H5Field* h);
 
 // Forgets srt_forward_noalloc's cached scratch addresses (srt_noalloc.cu).
 void noalloc_forget_scratch();
+
+// Number of SMs of the current device.
+cudaError_t sm_count(int* sms);
 
 // Peak issue-rate probes (FMA loop kernels); returns achieved FLOP/s.
 cudaError_t probe_fma(int kind, double* flops_per_s);

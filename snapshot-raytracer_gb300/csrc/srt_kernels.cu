@@ -179,6 +179,16 @@ cudaError_t launch_quantize_half(const float* src, int ts, __half* dst, int64_t 
   return cudaGetLastError();
 }
 
+__global__ void extract_kernel(const float* __restrict__ src, int ts, float* __restrict__ dst, int64_t count) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < count) dst[i] = src[i * ts];
+}
+
+cudaError_t launch_extract(const float* src, int ts, float* dst, int64_t count, cudaStream_t s) {
+  extract_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(src, ts, dst, count);
+  return cudaGetLastError();
+}
+
 // Row-pair array of a padded field: element (i, j, k), j < py - 1, holds
 // (f(i, j, k), f(i, j + 1, k)).
 __global__ void pair_build_kernel(const float* __restrict__ src, float2* __restrict__ dst, int64_t px, int64_t py,
@@ -205,21 +215,26 @@ cudaError_t launch_pair_build(const float* src, float2* dst, const int64_t pn[3]
 #define SRT_MIXED_MIN_BLOCKS 2
 #endif
 
-template <int MODE>
-__global__ void __launch_bounds__(128, (MODE == kMIXED || MODE >= kMIXED_PAIR) ? SRT_MIXED_MIN_BLOCKS : 1)
-    trace_kernel(const TraceArgs A) {
-  const int64_t tl = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (tl >= A.launch_rays) return;
-  // launch order: face-major, Morton (NESTED for power-of-two nside) in-face;
-  // a NESTED range launches its own slots
+// Output slot and RING pixel of launch slot tl; false where it has no ray.
+// Launch order: face-major, Morton (NESTED for power-of-two nside) in-face; a
+// NESTED range launches its own slots.
+__device__ __forceinline__ bool ray_of_slot(const TraceArgs& A, int64_t tl, int64_t* o, int64_t* ring) {
+  if (tl >= A.launch_rays) return false;
   const int64_t t = A.nested ? A.pix_begin + tl : tl;
   const int64_t face = t >> (2 * A.log2p);
   int64_t ix, iy;
   hp_deinterleave(t & ((int64_t(1) << (2 * A.log2p)) - 1), &ix, &iy);
-  if (ix >= A.nside || iy >= A.nside) return;
-  const int64_t ring = hp_xyf2ring(A.nside, ix, iy, (int)face);
-  const int64_t o = A.nested ? tl : ring - A.pix_begin;
-  if (o < 0 || o >= A.pix_count) return;
+  if (ix >= A.nside || iy >= A.nside) return false;
+  *ring = hp_xyf2ring(A.nside, ix, iy, (int)face);
+  *o = A.nested ? tl : *ring - A.pix_begin;
+  return *o >= 0 && *o < A.pix_count;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(128, (MODE == kMIXED || MODE >= kMIXED_PAIR) ? SRT_MIXED_MIN_BLOCKS : 1)
+    trace_kernel(const TraceArgs A) {
+  int64_t o, ring;
+  if (!ray_of_slot(A, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, &o, &ring)) return;
   const RayDir d = ray_dir_pix(A.nside, ring);
   float out[6];
   if (MODE >= kMIXED_PAIR || MODE == kMIXED) {
@@ -237,9 +252,98 @@ __global__ void __launch_bounds__(128, (MODE == kMIXED || MODE >= kMIXED_PAIR) ?
   for (int m = 0; m < 6; ++m) A.maps[m][o] = out[m];
 }
 
+// The stage's interpolations by a group of four lanes that hold the same ray,
+// one field each (B_x, B_y, B_z, phi), exchanged by shuffles; every lane then
+// folds them in OneLane's order, so the values are the same bits.
+template <int LAYOUT>
+struct FourLanes {
+  int field, first;  // this lane's field; the group's first lane
+  __device__ void operator()(const FieldPtrs& F, const Geom& G, const int* cc, const int* cs, const float* tc,
+                             const float* ts, const float* n, BAcc& A, Tri<float>& p) const {
+    Tri<float> own;
+    {
+      AxisWeights<LAYOUT> X, Y;
+      CRW<float> Z;
+      axis_weights(field == 0 ? ts[0] : tc[0], X);
+      axis_weights(field == 1 ? ts[1] : tc[1], Y);
+      cr_weights_mixed(field == 2 ? ts[2] : tc[2], Z);
+      const int cx = field == 0 ? cs[0] : cc[0], cy = field == 1 ? cs[1] : cc[1], cz = field == 2 ? cs[2] : cc[2];
+      tricubic_mixed(cell_source<LAYOUT>(F, G, field, cx, cy, cz), X, Y, Z, own);
+    }
+    Tri<float> r;
+    fetch(own, 0, r);
+    add_b_component<0>(r, n, A);
+    fetch(own, 1, r);
+    add_b_component<1>(r, n, A);
+    fetch(own, 2, r);
+    add_b_component<2>(r, n, A);
+    fetch(own, 3, p);
+  }
+  __device__ void fetch(const Tri<float>& own, int f, Tri<float>& r) const {
+    const unsigned mask = 0xfu << first;
+    r.v = __shfl_sync(mask, own.v, first + f);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) r.g[i] = __shfl_sync(mask, own.g[i], first + f);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) r.h[i] = __shfl_sync(mask, own.h[i], first + f);
+  }
+};
+
+// The MIXED trace of a small range, four lanes per ray in one-warp blocks: a warp
+// alone on its scheduler is bound by the latency of a stage's chains, and with
+// rays far apart by L1's lookups (a load of 32 rays' taps is 32 lines), so the
+// four interpolations run side by side (128^3, 48 steps: 768 rays 0.495 -> 0.287
+// ms, 3,072 rays 0.426 -> 0.303; from planes 1.06 -> 0.28 and 0.93 -> 0.30).
+// Prefetching the next step's lines made it 0.03 ms slower.
+template <int LAYOUT>
+__global__ void __launch_bounds__(32, 12) trace_small_kernel(const TraceArgs A) {
+  const int lane = threadIdx.x;
+  int64_t o, ring;
+  if (!ray_of_slot(A, (int64_t)blockIdx.x * 8 + (lane >> 2), &o, &ring)) return;
+  __shared__ float guard_m[32][2];
+  float out[6];
+  const bool near = trace_ray_mixed(FourLanes<LAYOUT>{lane & 3, lane & ~3}, A.F, A.G, ray_dir_pix(A.nside, ring),
+                                    A.n_steps, out, guard_m[lane]);
+  if ((lane & 3) != 0) return;
+  if (near && A.refine_list) {
+    const unsigned long long k = atomicAdd(A.refine_count, 1ull);
+    if (k < (unsigned long long)A.pix_count) A.refine_list[k] = o;
+  }
+#pragma unroll
+  for (int m = 0; m < 6; ++m) A.maps[m][o] = out[m];
+}
+
+// Ranges that trace_small_kernel takes: up to one of its warps per scheduler from
+// cells or row pairs (5,292 rays: 0.443 against 0.378 ms on one lane), up to four
+// from planes, whose loads are four times as many (19,200 rays: 1.02 against 1.08
+// ms, 27,648: 1.20 against 0.99). Not where most launch slots hold no ray of the
+// range.
+bool is_small(int mode, const TraceArgs& a, int sms) {
+  const int64_t rays = (int64_t)sms * 4 * 8 * (mode == kMIXED ? 4 : 1);
+  return a.pix_count <= rays && a.launch_rays <= 16 * rays;
+}
+
 cudaError_t launch_trace(int mode, const TraceArgs& a, cudaStream_t s, int64_t* kernels) {
   if (mode == kFP64 && a.pix_count <= kWideFp64Rays) return launch_wide_fp64(a, s, kernels);
-  const int threads = 128;
+  int sms = 0;
+  const cudaError_t e = sm_count(&sms);
+  if (e != cudaSuccess) return e;
+  if (mode != kFP64 && mode != kREF16 && is_small(mode, a, sms)) {
+    const unsigned small = (unsigned)((a.launch_rays + 7) / 8);
+    if (mode == kMIXED_CELL)
+      trace_small_kernel<kCells><<<small, 32, 0, s>>>(a);
+    else if (mode == kMIXED_PAIR)
+      trace_small_kernel<kPairs><<<small, 32, 0, s>>>(a);
+    else
+      trace_small_kernel<kPlanes><<<small, 32, 0, s>>>(a);
+    if (kernels) ++*kernels;
+    return cudaGetLastError();
+  }
+  // Ranges that would not give every SM a block of four warps go in one-warp
+  // blocks, so that all SMs' L1s and schedulers share them (128^3, 64 steps:
+  // 6,912 rays 0.555 -> 0.475 ms, 19,200 0.839 -> 0.775; 27,648 rays 0.754
+  // against 0.778, and four neighbouring warps to an SM share more lines).
+  const int threads = a.pix_count <= 128 * (int64_t)sms ? 32 : 128;
   const int64_t blocks = (a.launch_rays + threads - 1) / threads;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
   switch (mode) {

@@ -9,10 +9,65 @@ namespace srt {
 
 __device__ const WideTables kWideTables = make_wide_tables();
 
-// One-warp blocks; each traces rays blockIdx.x, + gridDim.x, ... of its list.
-// LIST: the rays a MIXED trace listed, count read on the device (no host round
-// trip); the kernel whose range [min_count, max_count] holds the count runs,
-// the other leaves at once. Otherwise every ray of the requested range.
+// The rays of a launch: those a MIXED trace listed (LIST; the count read on the
+// device, no host round trip, and nothing to do unless it lies in [min_count,
+// max_count]: one kernel per range of counts is queued), else the whole range.
+template <bool LIST>
+__device__ __forceinline__ int64_t ray_count(const TraceArgs& A, int64_t min_count, int64_t max_count) {
+  if (!LIST) return A.pix_count;
+  const int64_t n = min((int64_t)*A.refine_count, A.pix_count);
+  return n < min_count || n > max_count ? 0 : n;
+}
+template <bool LIST>
+__device__ __forceinline__ int64_t output_slot(const TraceArgs& A, int64_t i) { return LIST ? A.refine_list[i] : i; }
+__device__ __forceinline__ RayDir slot_direction(const TraceArgs& A, int64_t o) {
+  return ray_dir_pix(A.nside, A.nested ? hp_nest2ring(A.nside, A.pix_begin + o) : A.pix_begin + o);
+}
+
+// Lane j < 19 of a warp takes component j of the initial state.
+template <typename R>
+__device__ __forceinline__ void init_lane(WideLane<R>& L, const RayDir& d, const Geom& G) {
+  double y[19];
+  init_std(d, G, y);
+#pragma unroll
+  for (int j = 0; j < 19; ++j)
+    if (L.lane == j) L.y = R(y[j]);
+}
+
+// The maps from the state the warp's lanes hold.
+template <typename R>
+__device__ __forceinline__ void write_maps(const WideLane<R>& L, R* S, const TraceArgs& A, const RayDir& d, int64_t o) {
+  if (L.lane < 19) S[kWsY + L.lane] = L.y;
+  __syncwarp();
+  if (L.lane == 0) {
+    double y[19];
+    for (int j = 0; j < 19; ++j) y[j] = (double)S[kWsY + j];
+    float out[6];
+    extract_std(d, A.G, y, out);
+#pragma unroll
+    for (int m = 0; m < 6; ++m) A.maps[m][o] = out[m];
+  }
+  __syncwarp();
+}
+
+// The right-hand side from the interpolations and the frame in the scratch.
+template <typename R>
+__device__ __forceinline__ void run_rounds(WideLane<R>& L, R* S, int st) {
+  L.round1(S);
+  __syncwarp();
+  L.round2(S);
+  __syncwarp();
+  L.round3(S);
+  __syncwarp();
+  L.round4(S);
+  __syncwarp();
+  L.round5(S);
+  __syncwarp();
+  L.round6(S, st);
+  __syncwarp();
+}
+
+// One warp per ray, one-warp blocks; each traces rays blockIdx.x, + gridDim.x, ...
 template <typename R, bool LIST>
 __global__ void __launch_bounds__(32, 16) wide_kernel(const TraceArgs A, int64_t min_count, int64_t max_count) {
   // raw storage viewed as R: dd has a constructor, which a shared array of it
@@ -20,27 +75,17 @@ __global__ void __launch_bounds__(32, 16) wide_kernel(const TraceArgs A, int64_t
   __shared__ float2 scratch[kWsSize];
   __shared__ int cell[6];
   R* S = reinterpret_cast<R*>(scratch);
-  int64_t n = A.pix_count;
-  if (LIST) {
-    n = min((int64_t)*A.refine_count, n);
-    if (n < min_count || n > max_count) return;
-  }
+  const int64_t n = ray_count<LIST>(A, min_count, max_count);
+  if (blockIdx.x >= n) return;
   WideLane<R> L;
   L.start((int)threadIdx.x, kWideTables);
   L.constants(S);
 #pragma unroll 1
   for (int64_t i = blockIdx.x; i < n; i += gridDim.x) {
-    const int64_t o = LIST ? A.refine_list[i] : i;  // output slot
-    const int64_t ring = A.nested ? hp_nest2ring(A.nside, A.pix_begin + o) : A.pix_begin + o;
-    const RayDir d = ray_dir_pix(A.nside, ring);
-    {
-      double y[19];
-      init_std(d, A.G, y);
-      __syncwarp();
-#pragma unroll
-      for (int j = 0; j < 19; ++j)
-        if (L.lane == j) L.y = R(y[j]);
-    }
+    const int64_t o = output_slot<LIST>(A, i);
+    const RayDir d = slot_direction(A, o);
+    init_lane(L, d, A.G);
+    __syncwarp();
 #pragma unroll 1
     for (int step = 0; step < A.n_steps; ++step) {
 #pragma unroll 1
@@ -59,62 +104,94 @@ __global__ void __launch_bounds__(32, 16) wide_kernel(const TraceArgs A, int64_t
         __syncwarp();
         L.z_pass(S);
         __syncwarp();
-        L.round1(S);
-        __syncwarp();
-        L.round2(S);
-        __syncwarp();
-        L.round3(S);
-        __syncwarp();
-        L.round4(S);
-        __syncwarp();
-        L.round5(S);
-        __syncwarp();
-        L.round6(S, st);
-        __syncwarp();
+        run_rounds(L, S, st);
       }
     }
-    if (L.lane < 19) S[kWsY + L.lane] = L.y;
-    __syncwarp();
-    if (L.lane == 0) {
-      double y[19];
-      for (int j = 0; j < 19; ++j) y[j] = (double)S[kWsY + j];
-      float out[6];
-      extract_std(d, A.G, y, out);
-#pragma unroll
-      for (int m = 0; m < 6; ++m) A.maps[m][o] = out[m];
+    write_maps(L, S, A, d, o);
+  }
+}
+
+// Five warps per ray in FP64 (FieldLane): the shortest way through a stage, for
+// lists and ranges of at most kBlockRaysPerSM rays per SM.
+constexpr int kBlockThreads = 160, kBlockRaysPerSM = 4;
+
+template <bool LIST>
+__global__ void __launch_bounds__(kBlockThreads, kBlockRaysPerSM)
+    block_kernel(const TraceArgs A, int64_t min_count, int64_t max_count) {
+  __shared__ double S[kWsBlockSize];
+  __shared__ int cell[12];
+  const int64_t n = ray_count<LIST>(A, min_count, max_count);
+  if (blockIdx.x >= n) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  WideLane<double> L;  // warp 0: the state and the rounds; warp 4: the frame
+  FieldLane<double> I;
+  L.start(lane, kWideTables);
+  I.start(lane, warp < 4 ? warp : 0);
+  if (warp == 0) L.constants(S);
+#pragma unroll 1
+  for (int64_t i = blockIdx.x; i < n; i += gridDim.x) {
+    const int64_t o = output_slot<LIST>(A, i);
+    RayDir d = {};
+    if (warp == 0) {
+      d = slot_direction(A, o);
+      init_lane(L, d, A.G);
     }
-    __syncwarp();
+#pragma unroll 1
+    for (int step = 0; step < A.n_steps; ++step) {
+#pragma unroll 1
+      for (int st = 0; st < 4; ++st) {
+        if (warp == 0) L.stage(S, st);
+        __syncthreads();
+        if (warp < 4) {
+          I.position(S, cell, A.G);
+          __syncwarp();
+          I.load_taps(cell, A.F, A.G);
+          I.weights(S);
+          __syncwarp();
+          I.x_pass(S);
+          __syncwarp();
+          I.y_pass(S);
+          __syncwarp();
+          I.z_pass(S);
+        } else {
+          L.frame(S);
+        }
+        __syncthreads();
+        if (warp == 0) run_rounds(L, S, st);
+      }
+    }
+    if (warp == 0) write_maps(L, S, A, d, o);
   }
 }
 
 constexpr int kWideBlocksPerSM = 16;
 
-namespace {
 cudaError_t sm_count(int* sms) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   return e == cudaSuccess ? cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) : e;
 }
-}  // namespace
 
-// Lists up to dd_min rays (two warps per SM sub-partition) are re-traced in
-// FP64 with the one-lane FP64 form's operations (bit-identical maps), longer
-// ones in double-float arithmetic on the FP32 pipes (maps within one float
-// ulp). The environment variable SRT_REFINE_DD_MIN overrides dd_min (tests use
-// it to reach both on small skies).
-constexpr int64_t kRefineWarpsPerSubpartition = 1;
-
+// Lists of up to dd_min rays (four per SM) are re-traced in FP64 with the one-lane
+// FP64 form's operations (bit-identical maps), longer ones in double-float
+// arithmetic on the FP32 pipes (maps within one float ulp; 2.4e3 rays x 256 steps
+// 3.9 ms against 15.6 in FP64). The environment variable SRT_REFINE_DD_MIN
+// overrides dd_min (tests use it to reach both on small skies).
 cudaError_t launch_refine(const TraceArgs& a, cudaStream_t s, int64_t* kernels) {
   int sms = 0;
   cudaError_t e = sm_count(&sms);
   if (e != cudaSuccess) return e;
-  int64_t dd_min = kRefineWarpsPerSubpartition * 4 * (int64_t)sms;
+  int64_t dd_min = kBlockRaysPerSM * (int64_t)sms;
   if (const char* v = getenv("SRT_REFINE_DD_MIN")) dd_min = strtoll(v, nullptr, 10);
-  const int64_t blocks = std::min(a.pix_count, kWideBlocksPerSM * (int64_t)sms);
-  if (blocks < 1) return cudaSuccess;
-  wide_kernel<double, true><<<(unsigned)blocks, 32, 0, s>>>(a, 1, dd_min);
-  wide_kernel<dd, true><<<(unsigned)blocks, 32, 0, s>>>(a, std::max<int64_t>(dd_min, 0) + 1, a.pix_count);
-  if (kernels) *kernels += 2;
+  if (a.pix_count < 1) return cudaSuccess;
+  const int64_t blocks = std::min(a.pix_count, kBlockRaysPerSM * (int64_t)sms);
+  const int64_t warps = std::min(a.pix_count, kWideBlocksPerSM * (int64_t)sms);
+  block_kernel<true><<<(unsigned)blocks, kBlockThreads, 0, s>>>(a, 1, dd_min);
+  if (kernels) ++*kernels;
+  if (a.pix_count > dd_min) {
+    wide_kernel<dd, true><<<(unsigned)warps, 32, 0, s>>>(a, std::max<int64_t>(dd_min, 0) + 1, a.pix_count);
+    if (kernels) ++*kernels;
+  }
   return cudaGetLastError();
 }
 
@@ -122,8 +199,11 @@ cudaError_t launch_wide_fp64(const TraceArgs& a, cudaStream_t s, int64_t* kernel
   int sms = 0;
   cudaError_t e = sm_count(&sms);
   if (e != cudaSuccess) return e;
-  const int64_t blocks = std::min(a.pix_count, kWideBlocksPerSM * (int64_t)sms);
-  wide_kernel<double, false><<<(unsigned)blocks, 32, 0, s>>>(a, 0, 0);
+  if (a.pix_count <= kBlockRaysPerSM * (int64_t)sms)
+    block_kernel<false><<<(unsigned)a.pix_count, kBlockThreads, 0, s>>>(a, 0, 0);
+  else
+    wide_kernel<double, false>
+        <<<(unsigned)std::min(a.pix_count, kWideBlocksPerSM * (int64_t)sms), 32, 0, s>>>(a, 0, 0);
   if (kernels) ++*kernels;
   return cudaGetLastError();
 }

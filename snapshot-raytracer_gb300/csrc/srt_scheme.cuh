@@ -1095,25 +1095,10 @@ struct BAcc {
   float val[3], ngB[3], Gn[3], nlap, T[6];
 };
 
-// B component C interpolated at the position staggered by -1/2 along axis C,
-// folded into the accumulators. C is a compile-time constant so n[C], a[C]
-// and b[C] stay in registers.
-template <int C, int LAYOUT>
-SRT_HD void add_b_component(const FieldPtrs& F, const Geom& G, const int* cc, const int* cs,
-                            const float* ts, const AxisWeights<LAYOUT>& Cx, const AxisWeights<LAYOUT>& Cy,
-                            const CRW<float>& Cz,
-                            const float* n, const float* a, const float* b, BAcc& A) {
-  const auto src = cell_source<LAYOUT>(F, G, C, C == 0 ? cs[0] : cc[0], C == 1 ? cs[1] : cc[1], C == 2 ? cs[2] : cc[2]);
-  Tri<float> r;
-  if constexpr (C == 2) {
-    CRW<float> S;
-    cr_weights_mixed(ts[2], S);
-    tricubic_mixed(src, Cx, Cy, S, r);
-  } else {
-    AxisWeights<LAYOUT> S;
-    axis_weights(ts[C], S);
-    tricubic_mixed(src, C == 0 ? S : Cx, C == 1 ? S : Cy, Cz, r);
-  }
+// B component C's interpolation r folded into the accumulators. C is a
+// compile-time constant so n[C] stays in a register.
+template <int C>
+SRT_HD void add_b_component(const Tri<float>& r, const float* n, BAcc& A) {
   A.val[C] = r.v;
   for (int i = 0; i < 3; ++i) A.ngB[i] += r.g[i] * n[C];
   A.Gn[C] = r.g[0] * n[0] + r.g[1] * n[1] + r.g[2] * n[2];
@@ -1128,6 +1113,44 @@ SRT_HD void add_b_component(const FieldPtrs& F, const Geom& G, const int* cc, co
   A.T[5] += r.h[5] * n[C] - (C == 2 ? Hn[2] : 0.f);
   A.nlap += (r.h[0] + r.h[3] + r.h[5]) * n[C];
 }
+
+// A stage's four interpolations and the B sums, by one lane: B component C at
+// the position staggered by -1/2 along axis C (cells cs, offsets ts on that
+// axis), phi at the centred one.
+template <int LAYOUT>
+struct OneLane {
+  template <int C>
+  SRT_HD static void b_component(const FieldPtrs& F, const Geom& G, const int* cc, const int* cs, const float* ts,
+                                 const AxisWeights<LAYOUT>& Cx, const AxisWeights<LAYOUT>& Cy, const CRW<float>& Cz,
+                                 const float* n, BAcc& A) {
+    const auto src = cell_source<LAYOUT>(F, G, C, C == 0 ? cs[0] : cc[0], C == 1 ? cs[1] : cc[1], C == 2 ? cs[2] : cc[2]);
+    Tri<float> r;
+    if constexpr (C == 2) {
+      CRW<float> S;
+      cr_weights_mixed(ts[2], S);
+      tricubic_mixed(src, Cx, Cy, S, r);
+    } else {
+      AxisWeights<LAYOUT> S;
+      axis_weights(ts[C], S);
+      tricubic_mixed(src, C == 0 ? S : Cx, C == 1 ? S : Cy, Cz, r);
+    }
+    add_b_component<C>(r, n, A);
+  }
+  SRT_HD void operator()(const FieldPtrs& F, const Geom& G, const int* cc, const int* cs, const float* tc,
+                         const float* ts, const float* n, BAcc& A, Tri<float>& p) const {
+    AxisWeights<LAYOUT> Cx, Cy;  // centred weights, shared by phi and two axes of each B component
+    CRW<float> Cz;
+    axis_weights(tc[0], Cx);
+    axis_weights(tc[1], Cy);
+    cr_weights_mixed(tc[2], Cz);
+    b_component<0>(F, G, cc, cs, ts, Cx, Cy, Cz, n, A);
+    b_component<1>(F, G, cc, cs, ts, Cx, Cy, Cz, n, A);
+    // phi between the second and third B components: the same values in any
+    // order (the B sums keep theirs), and this one schedules best
+    tricubic_mixed(cell_source<LAYOUT>(F, G, 3, cc[0], cc[1], cc[2]), Cx, Cy, Cz, p);
+    b_component<2>(F, G, cc, cs, ts, Cx, Cy, Cz, n, A);
+  }
+};
 
 // Perturbation right-hand side g = f(y0(s) + d) - f(y0(s)) (FP32). `s` is the
 // affine parameter of the stage (step + 0, 1/2 or 1), d the stage state
@@ -1175,9 +1198,9 @@ struct Guard {
   SRT_HD void end_step(int step) { near |= m[1] < kFaceGuardRel * ((float)(step + 1) * m[0] + kFaceGuardFloor); }
 };
 
-template <int LAYOUT>
-SRT_HD void rhs_mixed(const float* d, float s, const MixedRay& R, const FieldPtrs& F, const Geom& G,
-                      const float* x0, float* g, Guard& gd) {
+template <typename Interp>
+SRT_HD void rhs_mixed(const Interp& interp, const float* d, float s, const MixedRay& R, const FieldPtrs& F,
+                      const Geom& G, const float* x0, float* g, Guard& gd) {
   float Dn[3], Da[3], Db[3];
   unit_pert(R.n0, d + 3, R.eta[0], Dn);
   unit_pert(R.a0, d + 6, R.eta[1], Da);
@@ -1202,22 +1225,12 @@ SRT_HD void rhs_mixed(const float* d, float s, const MixedRay& R, const FieldPtr
   // at s = 0 the ray sits exactly on the observer (a grid node, offsets
   // exactly 0) in both precisions, so no cell choice can differ there
   gd.face(s > 0.f ? fminf(fminf(df[0], df[1]), df[2]) : 1.f);
-  AxisWeights<LAYOUT> Cx, Cy;  // centred weights, shared by phi and two axes of each B component
-  CRW<float> Cz;
-  axis_weights(tc[0], Cx);
-  axis_weights(tc[1], Cy);
-  cr_weights_mixed(tc[2], Cz);
   BAcc A;
   A.ngB[0] = A.ngB[1] = A.ngB[2] = 0.f;
   A.nlap = 0.f;
   for (int i = 0; i < 6; ++i) A.T[i] = 0.f;
-  add_b_component<0, LAYOUT>(F, G, cc, cs, ts, Cx, Cy, Cz, n, a, b, A);
-  add_b_component<1, LAYOUT>(F, G, cc, cs, ts, Cx, Cy, Cz, n, a, b, A);
-  // phi between the second and third B components: the same values in any
-  // order (the B sums keep theirs), and this one schedules best
   Tri<float> p;
-  tricubic_mixed(cell_source<LAYOUT>(F, G, 3, cc[0], cc[1], cc[2]), Cx, Cy, Cz, p);
-  add_b_component<2, LAYOUT>(F, G, cc, cs, ts, Cx, Cy, Cz, n, a, b, A);
+  interp(F, G, cc, cs, tc, ts, n, A, p);
 
   const float dA = s + d[12];
   const float dAp = d[13] - 1.f;
@@ -1330,8 +1343,8 @@ SRT_HD void mixed_stage(const float* y, const float* k, float c, float* ys) {
 // the compensations folded in) are stored there: component j of stage st at
 // us[(19 st + j) * stride]. gd.near is set when a stage of the step came
 // within the guards above.
-template <int LAYOUT = kPlanes>
-SRT_HD void step_mixed(const MixedRay& R, const FieldPtrs& F, const Geom& G, const float* x0, int step, float* y,
+template <typename Interp>
+SRT_HD void step_mixed(const Interp& interp, const MixedRay& R, const FieldPtrs& F, const Geom& G, const float* x0, int step, float* y,
                        float* us, int64_t stride, Guard& gd) {
   float k[19], acc[19], ys[19];
   for (int j = 0; j < 19; ++j) k[j] = acc[j] = 0.f;
@@ -1342,7 +1355,7 @@ SRT_HD void step_mixed(const MixedRay& R, const FieldPtrs& F, const Geom& G, con
     mixed_stage(y, k, c, ys);
     if (us)
       for (int j = 0; j < 19; ++j) st_stream(us + (19 * st + j) * stride, ys[j]);
-    rhs_mixed<LAYOUT>(ys, s0 + c, R, F, G, x0, k, gd);
+    rhs_mixed(interp, ys, s0 + c, R, F, G, x0, k, gd);
     {  // acc = k1 + 2 k2 + 2 k3 with weights 1, 2, 2, 0 on a zeroed accumulator
        // (stage 4's k is added at the update): the same FMAs where a stage
        // adds, exact no-ops where it does not, and no branch
@@ -1403,8 +1416,8 @@ SRT_HD void extract_mixed(const MixedRay& R, int n_steps, const float* y, float 
 
 // Returns true when the ray came within the guards (its FP64 trace may
 // differ by a cell choice; the caller re-traces it in FP64).
-template <int LAYOUT = kPlanes>
-SRT_HD bool trace_ray_mixed(const FieldPtrs& F, const Geom& G, const RayDir& d, int n_steps, float out[6],
+template <typename Interp>
+SRT_HD bool trace_ray_mixed(const Interp& interp, const FieldPtrs& F, const Geom& G, const RayDir& d, int n_steps, float out[6],
                             float* guard_m) {
   MixedRay R;
   float y[kMixedState], x0[3];
@@ -1416,11 +1429,16 @@ SRT_HD bool trace_ray_mixed(const FieldPtrs& F, const Geom& G, const RayDir& d, 
 #pragma unroll 1
   for (int step = 0; step < n_steps; ++step) {
     gd.begin_step(y);
-    step_mixed<LAYOUT>(R, F, G, x0, step, y, nullptr, 0, gd);
+    step_mixed(interp, R, F, G, x0, step, y, nullptr, 0, gd);
     gd.end_step(step);
   }
   extract_mixed(R, n_steps, y, out);
   return gd.near;
+}
+template <int LAYOUT = kPlanes>
+SRT_HD bool trace_ray_mixed(const FieldPtrs& F, const Geom& G, const RayDir& d, int n_steps, float out[6],
+                            float* guard_m) {
+  return trace_ray_mixed(OneLane<LAYOUT>(), F, G, d, n_steps, out, guard_m);
 }
 
 // Ray direction of a RING pixel centre (FP64: cos/sin of the colatitude from

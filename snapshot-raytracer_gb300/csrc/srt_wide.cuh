@@ -60,7 +60,11 @@ enum {
   kWsW = 164,      // weights: 6 axis sets x (w, g, h) x 4 taps
   kWsX = 236,      // x pass: 4 fields x 16 rows x (value, d, d2)
   kWsYp = 428,     // y pass: 4 fields x 4 slices x (a, ay, ayy, ax, axy, axx)
-  kWsSize = 524
+  kWsSize = 524,
+  // five warps per ray (FieldLane): each field's own weights and offsets
+  kWsWf = 524,  // 4 fields x 3 axes x (w, g, h) x 4 taps
+  kWsTf = 668,  // 4 fields x 3 axes
+  kWsBlockSize = 680
 };
 
 // Operands of the rounds, one 32-bit word per lane and round.
@@ -185,6 +189,28 @@ SRT_HD dd floor_r(const dd& x) { return dd_floor(x); }
 SRT_HD bool above_half(double x) { return x > 0.5; }
 SRT_HD bool above_half(const dd& x) { return x > dd(0.5f); }
 
+// A tap's three weights at w[0], w[4], w[8].
+template <typename R>
+SRT_HD void wide_weights(const WideCoef& cf, const R& t, R* w) {
+  R v = fma_r(R(cf.v[3]), t, R(cf.v[2]));
+  v = fma_r(v, t, R(cf.v[1]));
+  w[0] = fma_r(v, t, R(cf.v[0]));
+  const R g = fma_r(R(cf.g[2]), t, R(cf.g[1]));
+  w[4] = fma_r(g, t, R(cf.g[0]));
+  w[8] = fma_r(R(cf.h[1]), t, R(cf.h[0]));
+}
+
+// Output o of a slice's y pass (a, ay, ayy, ax, axy, axx) from the y weights and
+// the slice's four rows of x pass results.
+template <typename R>
+SRT_HD void wide_y_output(const R* w, const R* x, R* out, int o) {
+  const int wo = o == 1 || o == 4 ? 4 : (o == 2 ? 8 : 0), xo = o < 3 ? 0 : (o == 5 ? 2 : 1);
+  Chain<R> s;
+#pragma unroll
+  for (int b = 0; b < 4; ++b) s.add(w[wo + b], x[3 * b + xo]);
+  out[o] = s.value();
+}
+
 // ------------------------------------------------------------- lane phases
 
 // What one lane keeps in registers through a ray: its operand words, its
@@ -249,14 +275,7 @@ struct WideLane {
   SRT_HD void weights(R* S) const {
     if (lane >= 24) return;
     const int set = lane >> 2, i = lane & 3;
-    const R t = S[kWsT + set];
-    R* w = S + kWsW + 12 * set + i;
-    R v = fma_r(R(cf.v[3]), t, R(cf.v[2]));
-    v = fma_r(v, t, R(cf.v[1]));
-    w[0] = fma_r(v, t, R(cf.v[0]));
-    R g = fma_r(R(cf.g[2]), t, R(cf.g[1]));
-    w[4] = fma_r(g, t, R(cf.g[0]));
-    w[8] = fma_r(R(cf.h[1]), t, R(cf.h[0]));
+    wide_weights(cf, S[kWsT + set], S + kWsW + 12 * set + i);
   }
 
   // Lanes 0-8: component i of unit vector v. Lanes 9-12: the branch's
@@ -314,12 +333,7 @@ struct WideLane {
     const R* x = S + kWsX + 48 * f + 12 * c;
 #pragma unroll
     for (int o = 0; o < 3; ++o) {
-      const int wo = odd ? (o == 1 ? 4 : 0) : 4 * o;  // axx takes the value weights
-      const int xo = odd ? (o == 2 ? 2 : 1) : 0;
-      Chain<R> s;
-#pragma unroll
-      for (int b = 0; b < 4; ++b) s.add(w[wo + b], x[3 * b + xo]);
-      S[kWsYp + 24 * f + 6 * c + 3 * odd + o] = s.value();
+      wide_y_output(w, x, S + kWsYp + 24 * f + 6 * c, 3 * odd + o);
     }
   }
 
@@ -396,6 +410,80 @@ struct WideLane {
       acc = fma_r(R(2.f), k, acc);
     else
       y = fma_r(acc + k, R(1.0 / 6.0), y);
+  }
+};
+
+// --------------------------------------------------- five warps per ray
+//
+// The same stage cut over warps: warps 0-3 interpolate one field each (FieldLane:
+// positions, weights, passes; only warp barriers between them), warp 4 forms the
+// frame (WideLane::frame) beside them, then warp 0 runs the rounds. ~24 FP64
+// instructions on a field warp's path, ~26 on the frame's and 18 in the rounds
+// against ~104 for one warp, and ~140 in all, so an SM's FP64 rate (19 cycles an
+// instruction) still carries four rays at a time as fast as one warp each would.
+
+template <typename R>
+struct FieldLane {
+  int lane, f;
+  WideCoef cf;
+  float tap[4];
+
+  SRT_HD void start(int l, int field) {
+    lane = l;
+    f = field;
+    cf = wide_coef(l & 3);
+  }
+
+  // offset and cell on one axis (lanes 0-2)
+  SRT_HD void position(R* S, int* cell, const Geom& G) const {
+    if (lane >= 3) return;
+    R x = S[kWsY + lane];
+    if (lane == f) x = x - R(0.5f);
+    const R fl = floor_r(x);
+    S[kWsTf + 3 * f + lane] = x - fl;
+    const int64_t c = int_r(fl);
+    cell[3 * f + lane] = (uint64_t)c < (uint64_t)G.n[lane] ? (int)c : wrap64(c, G.n[lane]);
+  }
+
+  // taps of row lane % 16 (4 slice + row in slice)
+  SRT_HD void load_taps(const int* cell, const FieldPtrs& F, const Geom& G) {
+    const int* c = cell + 3 * f;
+    const int row = lane & 15;
+    const float* src = f == 3 ? F.phi : (f == 0 ? F.b[0] : (f == 1 ? F.b[1] : F.b[2]));
+    const float* p = src + (cell_base(G, c[0], c[1], c[2]) + (row >> 2) * G.pxy + (row & 3) * G.px) * G.ts;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) tap[i] = ldg(p + i * G.ts);
+  }
+
+  SRT_HD void weights(R* S) const {
+    if (lane >= 12) return;
+    const R t = S[kWsTf + 3 * f + (lane >> 2)];
+    wide_weights(cf, t, S + kWsWf + 36 * f + 12 * (lane >> 2) + (lane & 3));
+  }
+
+  // value (lanes 0-15) and first derivative (16-31), then the second (0-15)
+  SRT_HD void x_pass(R* S) const {
+    x_chain(S, lane >> 4);
+    if (lane < 16) x_chain(S, 2);
+  }
+  SRT_HD void x_chain(R* S, int o) const {
+    const R* w = S + kWsWf + 36 * f + 4 * o;
+    Chain<R> c;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c.add(w[i], tap[i]);
+    S[kWsX + 48 * f + 3 * (lane & 15) + o] = c.value();
+  }
+
+  // lane 6 slice + output
+  SRT_HD void y_pass(R* S) const {
+    if (lane >= 24) return;
+    const int c = lane / 6, o = lane - 6 * c;
+    wide_y_output(S + kWsWf + 36 * f + 12, S + kWsX + 48 * f + 12 * c, S + kWsYp + 24 * f + 6 * c, o);
+  }
+
+  SRT_HD void z_pass(R* S) const {
+    if (lane >= 10) return;
+    WideLane<R>::z_output(S + kWsWf + 36 * f + 24, S + kWsYp + 24 * f, S + kWsTri + kWsTriStride * f, lane);
   }
 };
 

@@ -1,6 +1,7 @@
-"""The warp-per-ray trace (srt_wide.cuh: the re-trace of flagged rays and the
-FP64 form of small ranges), its lanes emulated on the host: in FP64 it must
-give the one-lane FP64 form's state bit for bit (the two write the same fused
+"""The warp-per-ray and block-per-ray traces (srt_wide.cuh: the re-trace of
+flagged rays and the FP64 form of small ranges), their lanes emulated on the
+host: in FP64 they must
+give the one-lane FP64 form's state bit for bit (all write the same fused
 chains), in double-float the same state to ~1e-12. Odd, non-cubic and very
 small grids, rays that wrap around the box, and the dA > 1/2 branch (off in
 the first step, on after it)."""
@@ -30,7 +31,7 @@ def host(tmp_path_factory):
     assert r.returncode == 0, r.stderr[-2000:]
     L = ctypes.CDLL(out)
     P, I, Q = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
-    L.trace_states.argtypes = [P, P, P, P, I, I, I, Q, Q, Q, I, P, P, P]
+    L.trace_states.argtypes = [P, P, P, P, I, I, I, Q, Q, Q, I, P, P, P, P]
     return L
 
 
@@ -41,10 +42,10 @@ def test_wide_equals_one_lane(host, n, nside, steps):
     pad = lambda f: np.ascontiguousarray(np.pad(f, ((1, 2), (1, 2), (1, 2)), mode="wrap"), np.float32)
     F = [pad(phi)] + [pad(b[..., c]) for c in range(3)]
     count = 12 * nside * nside
-    y = [np.zeros((count, 19)) for _ in range(3)]
+    y = [np.zeros((count, 19)) for _ in range(4)]
     host.trace_states(*[f.ctypes.data for f in F], *n, nside, 0, count, steps, *[v.ctypes.data for v in y])
-    one, wide, ddf = y
-    assert np.array_equal(one, wide)
+    one, wide, ddf, block = y
+    assert np.array_equal(one, wide) and np.array_equal(one, block)
     assert np.all(np.isfinite(one)) and (steps == 1 or np.abs(one[:, 16:18]).max() > 1e-6)
     # double-float: 2^-45 or so per operation, a few hundred operations deep, on O(1)..O(n) values; a ray
     # whose stage position lies within that of a cell face may take the other cell
