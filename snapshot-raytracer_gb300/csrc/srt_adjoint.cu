@@ -336,11 +336,11 @@ __global__ void __launch_bounds__(128, 2) segment_kernel_mixed(const AdjArgs A, 
 // running sum of the a's live in shared memory (one column per thread) to keep
 // registers for the field passes.
 template <typename AccB, typename AccP, int LAYOUT>
-__device__ __forceinline__ void sweep_segment(const AdjArgs& A, int sgi, int64_t slot, const MixedRay& R,
+__device__ __forceinline__ void sweep_segment(const AdjArgs& A, int sgi, int64_t slot, bool live, const MixedRay& R,
                                               const float* x0, float* lam, const AccB* accb, const AccP& accp,
                                               float (*s_lam)[128], float (*s_tot)[128]) {
   const int t = threadIdx.x;
-  for (int j = 0; j < 19; ++j) s_lam[j][t] = lam[(int64_t)j * A.count + slot];
+  for (int j = 0; j < 19; ++j) s_lam[j][t] = live ? lam[(int64_t)j * A.count + slot] : 0.f;
   const float* tape = (const float*)A.seg + slot;
   const int s0 = sgi * A.C, s1 = min(s0 + A.C, A.n_steps);
   // flattened (step, stage) index, descending; u holds the stage inputs of q
@@ -370,7 +370,8 @@ __device__ __forceinline__ void sweep_segment(const AdjArgs& A, int sgi, int64_t
     if (stage == 0)
       for (int j = 0; j < 19; ++j) s_lam[j][t] += s_tot[j][t];
   }
-  for (int j = 0; j < 19; ++j) lam[(int64_t)j * A.count + slot] = s_lam[j][t];
+  if (live)
+    for (int j = 0; j < 19; ++j) lam[(int64_t)j * A.count + slot] = s_lam[j][t];
 }
 
 // Resident blocks of 128 threads per SM the sweep is compiled for (register
@@ -386,13 +387,20 @@ __global__ void __launch_bounds__(128, SRT_SWEEP_MIN_BLOCKS)
     sweep_kernel_mixed(const AdjArgs A, int sgi, float* lam, Acc a0, Acc a1, Acc a2, Acc a3) {
   __shared__ float s_lam[19][128];
   __shared__ float s_tot[19][128];
-  const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (slot >= A.count) return;
-  if constexpr (TakesCells<Acc>::value) {  // this warp's copy of the region around the observer
+  int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  // the warp's lanes stay together for the paired atomics: one past the last ray
+  // follows it with a zero cotangent and stores nothing
+  const bool live = slot < A.count;
+  if (!__any_sync(0xffffffffu, live)) return;
+  if constexpr (TakesCells<Acc>::value) {
+    // this warp's copy of the region around the observer
     const int64_t copy = ((slot >> 5) % kHotCopies) * (kHotSide * kHotSide * kHotSide);
     for (Acc* a : {&a0, &a1, &a2, &a3})
       if (a->hot) a->hot += copy;
+  } else if (!live) {
+    return;
   }
+  if (!live) slot = A.count - 1;
   typedef typename std::conditional<BGRAD, Acc, AccNone>::type AccB;
   AccB accb[3];
   if constexpr (BGRAD) {
@@ -404,7 +412,7 @@ __global__ void __launch_bounds__(128, SRT_SWEEP_MIN_BLOCKS)
   float x0[3];
   load_bases(A, slot, R);
   mixed_observer(A.G, x0);
-  sweep_segment<AccB, Acc, LAYOUT>(A, sgi, slot, R, x0, lam, accb, a3, s_lam, s_tot);
+  sweep_segment<AccB, Acc, LAYOUT>(A, sgi, slot, live, R, x0, lam, accb, a3, s_lam, s_tot);
 }
 
 // f(std::integral_constant<int, LAYOUT>()) for a handle's layout.

@@ -58,11 +58,6 @@ SRT_HD void cr_weights4(T t, CRW4<T>& c) {
 //             so repeated runs give identical bits), by rows too.
 // A null grid (gradient not requested) ignores the contributions, and the
 // passes skip forming them (active() is false).
-// base: accumulator index of voxel (cx-1, cy-1, cz-1); px, pxy: its strides.
-struct Scatter {
-  int64_t base, px, pxy;
-};
-
 // Near the observer every ray adds to the same few voxels, and atomics on one
 // address run one after another: there each warp adds to one of kHotCopies
 // copies of a kHotSide^3 region around the observer (behind the grid, merged
@@ -79,28 +74,72 @@ SRT_HD int hot_base(const Geom& G, const int* c) {
   return in ? (int)(x + kHotSide * (y + kHotSide * z)) : -1;
 }
 
+// A sweep's atomics go to 32 lines an instruction and held its loads up behind
+// them (64 a stage; long-scoreboard stalls 3.2 of 5.9 cycles an instruction), so
+// the lanes work in pairs: the two cells of a grid row that a ray adds to are
+// neighbours in memory, and each atomic instruction takes both cells of one of
+// the pair's rays, half the lines (long-scoreboard stalls 0.7; a 512^3 / nside
+// 256 / 256 steps gradient 389 -> 373 ms). All lanes of a warp call these
+// together; a lane without a ray follows one with a zero cotangent.
 struct AccF32 {
   float4* g;
   int64_t hot = 0;  // index of this warp's copy; 0: no copies
   SRT_HD bool active() const { return g != nullptr; }
-  // where the footprint at padded base index `base` goes
-  SRT_HD Scatter place(int64_t base, int hbase, const Geom& G) const {
-    if (hot && hbase >= 0) return Scatter{hot + hbase, kHotSide, kHotSide * kHotSide};
-    return Scatter{base, G.px, G.pxy};
-  }
-  SRT_HD void add_cell(int64_t q, float4 v) const {
+  SRT_HD static int lane() {
 #if defined(__CUDA_ARCH__)
-    atomicAdd(g + q, v);
+    return threadIdx.x & 1;
 #else
-    g[q].x += v.x;
-    g[q].y += v.y;
-    g[q].z += v.z;
-    g[q].w += v.w;
+    return 0;
+#endif
+  }
+  // Where a field's footprint goes: entries of the pair's even and odd ray for
+  // this lane's cell of the first slice's first inner row, and the strides.
+  struct Place {
+    float4 *even, *odd;
+    int64_t px, pxy;
+  };
+  SRT_HD Place place(int64_t base, int hbase, const Geom& G) const {
+    Place p{nullptr, nullptr, G.px, G.pxy};
+#if defined(__CUDA_ARCH__)
+    if (hot && __all_sync(0xffffffffu, hbase >= 0)) {
+#else
+    if (hot && hbase >= 0) {
+#endif
+      base = hot + hbase;
+      p.px = kHotSide;
+      p.pxy = kHotSide * kHotSide;
+    }
+    int64_t other = base;
+#if defined(__CUDA_ARCH__)
+    other = __shfl_xor_sync(0xffffffffu, base, 1);
+#endif
+    const int me = lane();
+    p.even = g + (me ? other : base) + p.px + 1 + me;
+    p.odd = g + (me ? base : other) + p.px + 1 + me;
+    return p;
+  }
+  // A row's two cells: this lane's (me = lane(): tap 1 or 2) and the other.
+  SRT_HD static void add_row2(float4* even, float4* odd, float4 own, float4 other) {
+#if defined(__CUDA_ARCH__)
+    const int me = lane();
+    const float4 in = make_float4(__shfl_xor_sync(0xffffffffu, other.x, 1), __shfl_xor_sync(0xffffffffu, other.y, 1),
+                                  __shfl_xor_sync(0xffffffffu, other.z, 1), __shfl_xor_sync(0xffffffffu, other.w, 1));
+    atomicAdd(even, me ? in : own);
+    atomicAdd(odd, me ? own : in);
+#else
+    (void)odd;
+    for (int e = 0; e < 2; ++e) {
+      const float4 v = e ? other : own;
+      even[e].x += v.x;
+      even[e].y += v.y;
+      even[e].z += v.z;
+      even[e].w += v.w;
+    }
 #endif
   }
 };
 
-// Accumulators that take a tap's cell (add_cell) rather than rows of taps.
+// Accumulators that take cells (add_row2) rather than rows of taps.
 template <typename Acc>
 struct TakesCells : std::false_type {};
 template <>
@@ -277,28 +316,32 @@ SRT_HD void tricubic_vjp(const float* __restrict__ f, int64_t base, int64_t px, 
 // vector atomic per inner tap, and fold_kernel applies the (symmetric) second
 // differences once per voxel; the other accumulators get them expanded to taps.
 // 332 lane operations without the scatter against 536 on four taps.
-template <typename Acc, typename Src>
-SRT_HD void tricubic_vjp_mixed(const Src& src, const Scatter& sc, float tx, float ty, float tz, const float* qb,
+template <int UNROLL, typename Acc, typename Src>
+SRT_HD void tricubic_vjp_mixed(const Src& src, int64_t base, int hbase, const Geom& G, const float* t, const float* qb,
                                Tri<float>& Q, float* xb, const Acc& acc) {
   CWD X, Y;
   CRW<float> Z;
-  cr_weights_diff(tx, X);
-  cr_weights_diff(ty, Y);
-  cr_weights_mixed(tz, Z);
+  cr_weights_diff(t[0], X);
+  cr_weights_diff(t[1], Y);
+  cr_weights_mixed(t[2], Z);
   const XDup xd(X);
   const bool scatter = acc.active();  // this field's gradient was requested
+  AccF32::Place at = {};
+  int me = 0;
+  float2 ow, og, oh, nw, ng, nh;  // difference weights of this lane's cell of a pair and the other
+  if constexpr (TakesCells<Acc>::value) {
+    if (scatter) at = acc.place(base, hbase, G);
+    me = AccF32::lane();
+    ow = me ? xd.w3 : xd.w0, og = me ? xd.g3 : xd.g0, oh = me ? xd.h3 : xd.h0;
+    nw = me ? xd.w0 : xd.w3, ng = me ? xd.g0 : xd.g3, nh = me ? xd.h0 : xd.h3;
+  }
   // outputs oXYZ by derivative order, as pairs (two orders of the same z weight);
   // x and y third derivatives are summed as thirds
   const float2 z0 = make_float2(0.f, 0.f);
   float2 W0 = z0, W1 = z0, W2 = z0, W3 = z0, W4 = z0, G0 = z0, G1 = z0, G2 = z0, H0 = z0;
   float o102 = 0.f, o003 = 0.f;
   SliceData nt = src.load(0);
-  // whole where no scatter follows each slice (the phi-only sweep at 512^3 /
-  // nside 256 / 256 steps: 217 -> 200 ms), by two with it (fully unrolled it
-  // costs more in instruction fetch than it saves: 58.7 against 60.6 ms for a
-  // 256^3 / nside 128 / 128 steps vjp, 59.3 in a loop)
-  constexpr int kUnroll = std::is_same<Acc, AccNone>::value ? 4 : 2;
-#pragma unroll kUnroll
+#pragma unroll UNROLL
   for (int c = 0; c < 4; ++c) {
     // this slice's z weights by selection (an indexed read of Z would put
     // it in local memory)
@@ -341,20 +384,28 @@ SRT_HD void tricubic_vjp_mixed(const Src& src, const Scatter& sc, float tx, floa
       const float2 Cg[2] = {make_float2(b0 - g2, fmaf(Y.w0, b0, Y.g0 * b1)),
                             make_float2(g2, fmaf(Y.w3, b0, Y.g3 * b1))};
       const float2 Ch[2] = {make_float2(c0 - h2, Y.w0 * c0), make_float2(h2, Y.w3 * c0)};
-      const int64_t row = sc.base + c * sc.pxy, px = sc.px;
-      float2 p1[2], p2[2], e1[2], e2[2];
+      if constexpr (TakesCells<Acc>::value) {
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        p2[j] = ffma2(xd.t, Cw[j], Cg[j]);
-        p1[j] = fsub2(Cw[j], p2[j]);
-        e1[j] = ffma2(xd.w0, Cw[j], ffma2(xd.g0, Cg[j], fmul2(xd.h0, Ch[j])));
-        e2[j] = ffma2(xd.w3, Cw[j], ffma2(xd.g3, Cg[j], fmul2(xd.h3, Ch[j])));
-        if constexpr (TakesCells<Acc>::value) {
-          acc.add_cell(row + (j + 1) * px + 1, make_float4(p1[j].x, p1[j].y, e1[j].x, e1[j].y));
-          acc.add_cell(row + (j + 1) * px + 2, make_float4(p2[j].x, p2[j].y, e2[j].x, e2[j].y));
+        for (int j = 0; j < 2; ++j) {
+          const float2 p2 = ffma2(xd.t, Cw[j], Cg[j]), p1 = fsub2(Cw[j], p2);
+          const float2 po = me ? p2 : p1, pn = me ? p1 : p2;
+          const float2 eo = ffma2(ow, Cw[j], ffma2(og, Cg[j], fmul2(oh, Ch[j])));
+          const float2 en = ffma2(nw, Cw[j], ffma2(ng, Cg[j], fmul2(nh, Ch[j])));
+          AccF32::add_row2(at.even + j * at.px, at.odd + j * at.px, make_float4(po.x, po.y, eo.x, eo.y),
+                           make_float4(pn.x, pn.y, en.x, en.y));
         }
-      }
-      if constexpr (!TakesCells<Acc>::value) {
+        at.even += at.pxy;
+        at.odd += at.pxy;
+      } else {
+        const int64_t row = base + c * G.pxy, px = G.px;
+        float2 p1[2], p2[2], e1[2], e2[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          p2[j] = ffma2(xd.t, Cw[j], Cg[j]);
+          p1[j] = fsub2(Cw[j], p2[j]);
+          e1[j] = ffma2(xd.w0, Cw[j], ffma2(xd.g0, Cg[j], fmul2(xd.h0, Ch[j])));
+          e2[j] = ffma2(xd.w3, Cw[j], ffma2(xd.g3, Cg[j], fmul2(xd.h3, Ch[j])));
+        }
         const float2 n2 = dup2(-2.f);
         float2 t[2][4];  // taps along x of (value, difference along y) at rows 1 and 2
 #pragma unroll
@@ -421,16 +472,14 @@ SRT_HD int sym_idx(int i, int j) {
 }
 
 // One field's pass: FP32 (MIXED) from the handle's layout; FP64 in the plain form.
-template <int LAYOUT, typename T, typename Acc>
+template <int LAYOUT, int UNROLL, typename T, typename Acc>
 SRT_HD void field_pass(const FieldPtrs& F, int f, const StageView<T>& V, const Geom& G, const T* qb, Tri<T>& Q, T* xb,
                        const Acc& acc) {
   const int64_t base = V.base[f], basep = V.basep[f];
   const T* t = V.t[f];
-  if constexpr (sizeof(T) == sizeof(float)) {
-    Scatter sc{base, G.px, G.pxy};
-    if constexpr (TakesCells<Acc>::value) sc = acc.place(base, V.hbase[f], G);
-    tricubic_vjp_mixed<Acc>(cell_source<LAYOUT>(F, G, f, base, basep), sc, t[0], t[1], t[2], qb, Q, xb, acc);
-  } else
+  if constexpr (sizeof(T) == sizeof(float))
+    tricubic_vjp_mixed<UNROLL, Acc>(cell_source<LAYOUT>(F, G, f, base, basep), base, V.hbase[f], G, t, qb, Q, xb, acc);
+  else
     tricubic_vjp<T, Acc>(f == 3 ? F.phi : F.b[f], base, G.px, G.pxy, G.ts, t[0], t[1], t[2], qb, Q, xb, acc);
 }
 
@@ -458,7 +507,7 @@ struct BVjp {
 // One B component's share of rhs_vjp: its cotangents (value, gradient,
 // Hessian), the fused pass, the forward sums and its terms of nb, the cotangent
 // of n (those of e1 and e2 follow from the sums).
-template <int C, int LAYOUT, typename T, typename Acc>
+template <int C, int LAYOUT, int UNROLL, typename T, typename Acc>
 SRT_HD void vjp_b_component(const StageView<T>& V, const FieldPtrs& F, const Geom& G, const T* fb, BVjp<T>& B,
                             const Acc& acc, T* xb, T* nb) {
   const T* n = V.n;
@@ -475,7 +524,7 @@ SRT_HD void vjp_b_component(const StageView<T>& V, const FieldPtrs& F, const Geo
       qb[4 + sym_idx(i, j)] = fm(n2, B.Tb[sym_idx(i, j)], -fm(Tc[i], n[j], Tc[j] * n[i]));
   }
   Tri<T> Q;
-  field_pass<LAYOUT, T, Acc>(F, C, V, G, qb, Q, xb, acc);
+  field_pass<LAYOUT, UNROLL, T, Acc>(F, C, V, G, qb, Q, xb, acc);
   for (int i = 0; i < 3; ++i) B.ngB[i] = fm(Q.g[i], nc, C == 0 ? T(0) : B.ngB[i]);
   B.Gn[C] = vdot(Q.g, n);
   B.nlap = fm(nc, Q.h[0] + Q.h[3] + Q.h[5], C == 0 ? T(0) : B.nlap);
@@ -500,6 +549,11 @@ SRT_HD void rhs_vjp(const StageView<T>& V, const FieldPtrs& F, const Geom& G, co
   const T* n = V.n;
   const T* a = V.a;
   const T* b = V.b;
+  // The passes' slice loops: unrolled where only phi's scatter follows them
+  // (512^3 / nside 256 / 256 steps, backward half: 183 ms in loops, 181 unrolled),
+  // in loops with four scatters, where the code outgrows the instruction cache
+  // (256^3 / nside 128 / 128 steps: 49.6 ms against 50.8).
+  constexpr int kUnroll = std::is_same<AccB, AccNone>::value ? 4 : 1;
   // ---- intermediate cotangents (state only)
   const T nfx = vdot(n, fb), nfn = vdot(n, fb + 3);
   const T e1b = -vdot(n, fb + 6), e2b = -vdot(n, fb + 9);
@@ -549,9 +603,9 @@ SRT_HD void rhs_vjp(const StageView<T>& V, const FieldPtrs& F, const Geom& G, co
   T nb[3] = {0, 0, 0}, xb[3] = {0, 0, 0};
 
   // ---- B components (compile-time component index: no local-memory arrays)
-  vjp_b_component<0, LAYOUT, T, AccB>(V, F, G, fb, B, accb[0], xb, nb);
-  vjp_b_component<1, LAYOUT, T, AccB>(V, F, G, fb, B, accb[1], xb, nb);
-  vjp_b_component<2, LAYOUT, T, AccB>(V, F, G, fb, B, accb[2], xb, nb);
+  vjp_b_component<0, LAYOUT, kUnroll, T, AccB>(V, F, G, fb, B, accb[0], xb, nb);
+  vjp_b_component<1, LAYOUT, kUnroll, T, AccB>(V, F, G, fb, B, accb[1], xb, nb);
+  vjp_b_component<2, LAYOUT, kUnroll, T, AccB>(V, F, G, fb, B, accb[2], xb, nb);
 
   // ---- phi
   Tri<T> P;
@@ -565,7 +619,7 @@ SRT_HD void rhs_vjp(const StageView<T>& V, const FieldPtrs& F, const Geom& G, co
       qb[4 + sym_idx(i, i)] = fm(n[i], t, Heb[sym_idx(i, i)] - PHb);
       for (int j = i + 1; j < 3; ++j) qb[4 + sym_idx(i, j)] = T(2) * fm(t, n[j], Heb[sym_idx(i, j)]);
     }
-    field_pass<LAYOUT, T, AccP>(F, 3, V, G, qb, P, xb, accp);
+    field_pass<LAYOUT, kUnroll, T, AccP>(F, 3, V, G, qb, P, xb, accp);
   }
   const T* g = P.g;
   // ---- the rest of n's cotangent, and those of e1, e2 and the scalars
