@@ -24,6 +24,7 @@
 #include <cstring>
 #include <type_traits>
 #include "srt_adjoint.cuh"
+#include "srt_four_lanes.cuh"
 #include "srt_internal.h"
 
 namespace srt {
@@ -190,20 +191,21 @@ __device__ __forceinline__ void prefetch_step(const AdjArgs& A, const MixedRay& 
 
 // Forward trace of one ray storing the state every C steps (and the final
 // state); y holds the final state.
-template <int LAYOUT>
-__device__ __forceinline__ void ckpt_ray(const AdjArgs& A, int64_t slot, const RayDir& d, MixedRay& R, float* y,
-                                         Guard& gd) {
+template <typename Interp>
+__device__ __forceinline__ void ckpt_ray(const Interp& interp, const AdjArgs& A, int64_t slot, const RayDir& d,
+                                         MixedRay& R, float* y, Guard& gd) {
+  constexpr bool kNear = std::is_same<Interp, OneLane<kFourTaps>>::value;
   float x0[3];
   mixed_observer(A.G, x0);
   init_mixed(d, R, y);
-  if (LAYOUT != kFourTaps) store_bases(A, slot, R);
+  if (!kNear) store_bases(A, slot, R);
   float* ck = (float*)A.ckpt;
   store_vec(ck, A.count, slot, y, kMixedState);
 #pragma unroll 1
   for (int st = 0; st < A.n_steps; ++st) {
-    if (LAYOUT == kFourTaps) prefetch_step(A, R, x0, y, st);
+    if (kNear) prefetch_step(A, R, x0, y, st);
     if (gd.m) gd.begin_step(y);
-    step_mixed(OneLane<LAYOUT>(), R, A.F, A.G, x0, st, y, nullptr, 0, gd);
+    step_mixed(interp, R, A.F, A.G, x0, st, y, nullptr, 0, gd);
     if (gd.m) gd.end_step(st);
     const int done = st + 1;
     if (done % A.C == 0 || done == A.n_steps) {
@@ -213,22 +215,21 @@ __device__ __forceinline__ void ckpt_ray(const AdjArgs& A, int64_t slot, const R
   }
 }
 
-// The checkpoints of every ray, with the cell-face guard of the trace kernel;
-// marks the rays it catches. MAPS (srt_forward_tape): also the maps and the
-// list of rays to re-trace; the arithmetic is the trace kernel's, so the maps
-// are srt_forward's.
-template <int LAYOUT, bool MAPS>
-__global__ void __launch_bounds__(128, 2) ckpt_kernel_mixed(const AdjArgs A) {
-  const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (slot >= A.count) return;
+// The checkpoints of one ray, with the cell-face guard of the trace kernel; marks
+// and lists it where the guard catches it. MAPS (srt_forward_tape): also its maps
+// and the list of rays to re-trace; the arithmetic is the trace kernels', so the
+// maps are srt_forward's. first: this lane writes what a ray has once.
+template <bool MAPS, typename Interp>
+__device__ __forceinline__ void ckpt_one(const Interp& interp, const AdjArgs& A, int64_t slot, bool first,
+                                         float* guard_m) {
   const int64_t ring = ring_of(A, slot);
   MixedRay R;
   float y[kMixedState];
-  __shared__ float guard_m[128][2];
   Guard gd;
-  gd.m = guard_m[threadIdx.x];
+  gd.m = guard_m;
   gd.m[0] = 0.f;
-  ckpt_ray<LAYOUT>(A, slot, ray_dir_pix(A.nside, ring), R, y, gd);
+  ckpt_ray(interp, A, slot, ray_dir_pix(A.nside, ring), R, y, gd);
+  if (!first) return;
   if (gd.near) {
     A.rays[slot] = ring | kNearBit;
     A.near[1 + atomicAdd((unsigned long long*)A.near, 1ull)] = slot;
@@ -246,6 +247,24 @@ __global__ void __launch_bounds__(128, 2) ckpt_kernel_mixed(const AdjArgs A) {
   }
 }
 
+template <int LAYOUT, bool MAPS>
+__global__ void __launch_bounds__(128, 2) ckpt_kernel_mixed(const AdjArgs A) {
+  const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (slot >= A.count) return;
+  __shared__ float guard_m[128][2];
+  ckpt_one<MAPS>(OneLane<LAYOUT>(), A, slot, true, guard_m[threadIdx.x]);
+}
+
+// Small ranges, forward and adjoint: four lanes per ray, one-warp blocks.
+template <int LAYOUT, bool MAPS>
+__global__ void __launch_bounds__(32, 12) ckpt_small_kernel(const AdjArgs A) {
+  const int lane = threadIdx.x;
+  const int64_t slot = (int64_t)blockIdx.x * 8 + (lane >> 2);
+  if (slot >= A.count) return;
+  __shared__ float guard_m[32][2];
+  ckpt_one<MAPS>(FourLanes<LAYOUT>{lane & 3, lane & ~3}, A, slot, (lane & 3) == 0, guard_m[lane]);
+}
+
 // The marked rays' checkpoints by the four-tap passes, one warp per ray. Few
 // rays: the launch is about one ray's latency.
 __global__ void __launch_bounds__(128, 2) near_ckpt_kernel(const AdjArgs A) {
@@ -253,7 +272,7 @@ __global__ void __launch_bounds__(128, 2) near_ckpt_kernel(const AdjArgs A) {
     MixedRay R;
     float y[kMixedState];
     Guard gd;  // disabled
-    ckpt_ray<kFourTaps>(A, slot, ray_dir_pix(A.nside, ring_of(A, slot)), R, y, gd);
+    ckpt_ray(OneLane<kFourTaps>(), A, slot, ray_dir_pix(A.nside, ring_of(A, slot)), R, y, gd);
   });
 }
 
@@ -296,8 +315,9 @@ __global__ void __launch_bounds__(128) final_cotangent_kernel_mixed(const AdjArg
 
 // Recompute segment sgi of one ray from its checkpoint, storing the four stage
 // inputs of every step: tape [C][4 x 19][count].
-template <int LAYOUT>
-__device__ __forceinline__ void segment_ray(const AdjArgs& A, int sgi, int64_t slot) {
+template <typename Interp>
+__device__ __forceinline__ void segment_ray(const Interp& interp, const AdjArgs& A, int sgi, int64_t slot,
+                                            bool first = true) {
   MixedRay R;
   float y[kMixedState], x0[3];
   mixed_observer(A.G, x0);
@@ -308,8 +328,9 @@ __device__ __forceinline__ void segment_ray(const AdjArgs& A, int sgi, int64_t s
 #pragma unroll 1
   for (int st = s0; st < s1; ++st) {
     Guard gd;  // disabled
-    if (LAYOUT == kFourTaps) prefetch_step(A, R, x0, y, st);
-    step_mixed(OneLane<LAYOUT>(), R, A.F, A.G, x0, st, y, tape + (int64_t)(st - s0) * kTapeStep * A.count + slot, A.count, gd);
+    if (std::is_same<Interp, OneLane<kFourTaps>>::value) prefetch_step(A, R, x0, y, st);
+    step_mixed(interp, R, A.F, A.G, x0, st, y,
+               first ? tape + (int64_t)(st - s0) * kTapeStep * A.count + slot : nullptr, A.count, gd);
   }
 }
 
@@ -321,11 +342,24 @@ constexpr int kNearCkptBlocks = 304;
 template <int LAYOUT>
 __global__ void __launch_bounds__(128, 2) segment_kernel_mixed(const AdjArgs A, int sgi) {
   if (blockIdx.x < kNearBlocks) {
-    for_near_rays(A, kNearBlocks * 4, [&](int64_t slot) { segment_ray<kFourTaps>(A, sgi, slot); });
+    for_near_rays(A, kNearBlocks * 4, [&](int64_t slot) { segment_ray(OneLane<kFourTaps>(), A, sgi, slot); });
     return;
   }
   const int64_t slot = (int64_t)(blockIdx.x - kNearBlocks) * 128 + threadIdx.x;
-  if (slot < A.count && !is_near(A, slot)) segment_ray<LAYOUT>(A, sgi, slot);
+  if (slot < A.count && !is_near(A, slot)) segment_ray(OneLane<LAYOUT>(), A, sgi, slot);
+}
+
+template <int LAYOUT>
+__global__ void __launch_bounds__(32, 12) segment_small_kernel(const AdjArgs A, int sgi) {
+  const int lane = threadIdx.x;
+  const int64_t slot = (int64_t)blockIdx.x * 8 + (lane >> 2);
+  if (slot < A.count && !is_near(A, slot))
+    segment_ray(FourLanes<LAYOUT>{lane & 3, lane & ~3}, A, sgi, slot, (lane & 3) == 0);
+}
+
+// The marked rays of a segment, beside segment_small_kernel.
+__global__ void __launch_bounds__(128, 2) near_segment_kernel(const AdjArgs A, int sgi) {
+  for_near_rays(A, (int64_t)gridDim.x * 4, [&](int64_t slot) { segment_ray(OneLane<kFourTaps>(), A, sgi, slot); });
 }
 
 // Backward sweep over segment sgi: per step, backwards, the RK4 adjoint
@@ -335,10 +369,11 @@ __global__ void __launch_bounds__(128, 2) segment_kernel_mixed(const AdjArgs A, 
 // while the current stage runs); l carried in lam between segments. l and the
 // running sum of the a's live in shared memory (one column per thread) to keep
 // registers for the field passes.
-template <typename AccB, typename AccP, int LAYOUT>
-__device__ __forceinline__ void sweep_segment(const AdjArgs& A, int sgi, int64_t slot, bool live, const MixedRay& R,
-                                              const float* x0, float* lam, const AccB* accb, const AccP& accp,
-                                              float (*s_lam)[128], float (*s_tot)[128]) {
+// live: this lane's ray counts; store: it writes the cotangent back.
+template <int THREADS, typename Passes>
+__device__ __forceinline__ void sweep_segment(const AdjArgs& A, int sgi, int64_t slot, bool live, bool store,
+                                              const MixedRay& R, const float* x0, float* lam, const Passes& passes,
+                                              float (*s_lam)[THREADS], float (*s_tot)[THREADS]) {
   const int t = threadIdx.x;
   for (int j = 0; j < 19; ++j) s_lam[j][t] = live ? lam[(int64_t)j * A.count + slot] : 0.f;
   const float* tape = (const float*)A.seg + slot;
@@ -364,13 +399,13 @@ __device__ __forceinline__ void sweep_segment(const AdjArgs& A, int sgi, int64_t
       for (int j = 0; j < 19; ++j) u[j] = ld_stream(tape + ((int64_t)(qn >> 2) * kTapeStep + 19 * (qn & 3) + j) * A.count);
     }
     for (int j = 0; j < 19; ++j) an[j] = 0.f;
-    rhs_vjp<float, AccB, AccP, LAYOUT>(V, A.F, A.G, fb, an, accb, accp);
+    rhs_vjp_with(V, fb, an, passes);
     // the step's running sum of the a's restarts at its last stage
     for (int j = 0; j < 19; ++j) s_tot[j][t] = (stage == 3 ? 0.f : s_tot[j][t]) + an[j];
     if (stage == 0)
       for (int j = 0; j < 19; ++j) s_lam[j][t] += s_tot[j][t];
   }
-  if (live)
+  if (store)
     for (int j = 0; j < 19; ++j) lam[(int64_t)j * A.count + slot] = s_lam[j][t];
 }
 
@@ -412,7 +447,76 @@ __global__ void __launch_bounds__(128, SRT_SWEEP_MIN_BLOCKS)
   float x0[3];
   load_bases(A, slot, R);
   mixed_observer(A.G, x0);
-  sweep_segment<AccB, Acc, LAYOUT>(A, sgi, slot, live, R, x0, lam, accb, a3, s_lam, s_tot);
+  sweep_segment<128>(A, sgi, slot, live, live, R, x0, lam, OneLanePasses<LAYOUT, float, AccB, Acc>{A.F, A.G, accb, a3},
+                     s_lam, s_tot);
+}
+
+// The four passes of a stage by four lanes that hold the same ray, one field
+// each; every lane then folds them.
+template <int LAYOUT, typename Acc>
+struct FourLanePasses {
+  const FieldPtrs& F;
+  const Geom& G;
+  const Acc& acc;  // this lane's field's
+  int field, first;
+  __device__ void operator()(const StageView<float>& V, const float* fb, const PhiVjp<float>& p, BVjp<float>& B,
+                             float* nb, float* xb, Tri<float>& P) const {
+    float qb[10], q[10];
+    phi_cotangent(V, p, qb);
+    b_cotangent<0>(V, fb, B, q);
+    for (int i = 0; i < 10; ++i) qb[i] = field == 0 ? q[i] : qb[i];
+    b_cotangent<1>(V, fb, B, q);
+    for (int i = 0; i < 10; ++i) qb[i] = field == 1 ? q[i] : qb[i];
+    b_cotangent<2>(V, fb, B, q);
+    for (int i = 0; i < 10; ++i) qb[i] = field == 2 ? q[i] : qb[i];
+    StageView<float> W;  // this lane's field's cell in the place of all (selects, no indexed arrays)
+    W.base[0] = field == 0 ? V.base[0] : (field == 1 ? V.base[1] : (field == 2 ? V.base[2] : V.base[3]));
+    W.basep[0] = field == 0 ? V.basep[0] : (field == 1 ? V.basep[1] : (field == 2 ? V.basep[2] : V.basep[3]));
+    W.hbase[0] = field == 0 ? V.hbase[0] : (field == 1 ? V.hbase[1] : (field == 2 ? V.hbase[2] : V.hbase[3]));
+    for (int i = 0; i < 3; ++i)
+      W.t[0][i] = field == 0 ? V.t[0][i] : (field == 1 ? V.t[1][i] : (field == 2 ? V.t[2][i] : V.t[3][i]));
+    Tri<float> own;
+    float x[3] = {0.f, 0.f, 0.f};
+    tricubic_vjp_mixed<1, Acc>(cell_source<LAYOUT>(F, G, field, W.base[0], W.basep[0]), W.base[0], W.hbase[0], G, W.t[0],
+                               qb, own, x, acc);
+    const unsigned mask = 0xfu << first;
+    for (int i = 0; i < 3; ++i) {
+      float v = __shfl_sync(mask, x[i], first);
+      for (int f = 1; f < 4; ++f) v += __shfl_sync(mask, x[i], first + f);
+      xb[i] += v;
+    }
+    Tri<float> Q;
+    fetch_tri(own, 0, first, Q);
+    b_fold<0>(V, Q, B, nb);
+    fetch_tri(own, 1, first, Q);
+    b_fold<1>(V, Q, B, nb);
+    fetch_tri(own, 2, first, Q);
+    b_fold<2>(V, Q, B, nb);
+    fetch_tri(own, 3, first, P);
+  }
+};
+
+// The sweep of a small range: four lanes per ray, one-warp blocks.
+template <typename Acc, int LAYOUT>
+__global__ void __launch_bounds__(32, 8)
+    sweep_small_kernel(const AdjArgs A, int sgi, float* lam, Acc a0, Acc a1, Acc a2, Acc a3) {
+  __shared__ float s_lam[19][32];
+  __shared__ float s_tot[19][32];
+  const int lane = threadIdx.x, field = lane & 3;
+  int64_t slot = (int64_t)blockIdx.x * 8 + (lane >> 2);
+  const bool live = slot < A.count;  // lanes past the last ray follow it with a zero cotangent
+  if (!live) slot = A.count - 1;
+  Acc acc = field == 0 ? a0 : (field == 1 ? a1 : (field == 2 ? a2 : a3));
+  if constexpr (TakesCells<Acc>::value) {
+    if (acc.hot) acc.hot += (blockIdx.x % kHotCopies) * (kHotSide * kHotSide * kHotSide);
+    acc.mask = __ballot_sync(0xffffffffu, acc.active());
+  }
+  MixedRay R;
+  float x0[3];
+  load_bases(A, slot, R);
+  mixed_observer(A.G, x0);
+  sweep_segment<32>(A, sgi, slot, live, live && field == 0, R, x0, lam,
+                    FourLanePasses<LAYOUT, Acc>{A.F, A.G, acc, field, lane & ~3}, s_lam, s_tot);
 }
 
 // f(std::integral_constant<int, LAYOUT>()) for a handle's layout.
@@ -426,11 +530,24 @@ void with_layout(int layout, const Fn& f) {
     f(std::integral_constant<int, kPlanes>());
 }
 
+inline void copy_extra(AccPaired<4>& to, const AccF32& from) { to.hot = from.hot; }
+inline void copy_extra(AccFixed& to, const AccFixed& from) { to.ovf = from.ovf; }
+
 template <typename Acc>
-void launch_sweep(const AdjArgs& A, int sgi, float* lam, const Acc* a, int layout, bool bgrad, unsigned blocks,
-                  cudaStream_t s) {
+void launch_sweep(const AdjArgs& A, int sgi, float* lam, const Acc* a, int layout, bool bgrad, bool small,
+                  unsigned blocks, cudaStream_t s) {
   with_layout(layout, [&](auto l) {
     constexpr int L = decltype(l)::value;
+    if (small) {
+      typedef typename std::conditional<TakesCells<Acc>::value, AccPaired<4>, Acc>::type AccS;
+      AccS b[4];
+      for (int f = 0; f < 4; ++f) {
+        b[f].g = a[f].g;
+        copy_extra(b[f], a[f]);
+      }
+      sweep_small_kernel<AccS, L><<<(unsigned)((A.count + 7) / 8), 32, 0, s>>>(A, sgi, lam, b[0], b[1], b[2], b[3]);
+      return;
+    }
     if (bgrad)
       sweep_kernel_mixed<Acc, L, true><<<blocks, 128, 0, s>>>(A, sgi, lam, a[0], a[1], a[2], a[3]);
     else
@@ -700,6 +817,11 @@ done:
 
 }  // namespace
 
+// Ranges the small kernels take: up to one of their warps per scheduler (128^3, 48
+// steps, both gradients: 768 rays 3.22 -> 1.57 ms, 4,800 rays 2.82 -> 1.64, 12,288
+// rays 3.41 against 4.18).
+static bool small_adjoint(int64_t rays, int sms) { return rays <= (int64_t)sms * 4 * 8; }
+
 // A forward trace's checkpoints (srt_forward_tape) for srt_vjp_tape.
 struct srt_tape {
   const srt_fields* fields = nullptr;
@@ -857,6 +979,8 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
       A.refine_list = nullptr;
       A.refine_count = nullptr;
 
+      int sms = 0;
+      VJP_TRY(sm_count(&sms), "device attributes");
       VJP_TRY(cudaEventCreate(&e0), "cudaEventCreate");
       VJP_TRY(cudaEventCreate(&e1), "cudaEventCreate");
       VJP_TRY(cudaEventRecord(e0, s), "cudaEventRecord");
@@ -877,8 +1001,14 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
         // forward with checkpoints; then per segment, backwards: recompute
         // the segment's tape, sweep it
         const int layout = f->layout();
+        const bool small = small_adjoint(pix_count, sms);
         if (!tape) {  // else the checkpoints come from srt_forward_tape
-          with_layout(layout, [&](auto l) { ckpt_kernel_mixed<decltype(l)::value, false><<<blocks, 128, 0, s>>>(A); });
+          with_layout(layout, [&](auto l) {
+            if (small)
+              ckpt_small_kernel<decltype(l)::value, false><<<(unsigned)((pix_count + 7) / 8), 32, 0, s>>>(A);
+            else
+              ckpt_kernel_mixed<decltype(l)::value, false><<<blocks, 128, 0, s>>>(A);
+          });
           near_ckpt_kernel<<<std::min<unsigned>(blocks * 32, kNearCkptBlocks), 128, 0, s>>>(A);
         }
         final_cotangent_kernel_mixed<<<blocks, 128, 0, s>>>(A, (float*)lam.p);
@@ -891,11 +1021,18 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
         for (int fld = 0; fld < 4; ++fld) ax[fld].ovf = (unsigned*)ovf.p;
         const bool bgrad = db_xyz != nullptr;
         for (int sgi = nseg - 1; sgi >= 0; --sgi) {
-          with_layout(layout, [&](auto l) { segment_kernel_mixed<decltype(l)::value><<<blocks + kNearBlocks, 128, 0, s>>>(A, sgi); });
+          with_layout(layout, [&](auto l) {
+            if (small) {
+              segment_small_kernel<decltype(l)::value><<<(unsigned)((pix_count + 7) / 8), 32, 0, s>>>(A, sgi);
+              near_segment_kernel<<<kNearBlocks, 128, 0, s>>>(A, sgi);
+            } else {
+              segment_kernel_mixed<decltype(l)::value><<<blocks + kNearBlocks, 128, 0, s>>>(A, sgi);
+            }
+          });
           if (determ)
-            launch_sweep<AccFixed>(A, sgi, (float*)lam.p, ax, layout, bgrad, blocks, s);
+            launch_sweep<AccFixed>(A, sgi, (float*)lam.p, ax, layout, bgrad, small, blocks, s);
           else
-            launch_sweep<AccF32>(A, sgi, (float*)lam.p, af, layout, bgrad, blocks, s);
+            launch_sweep<AccF32>(A, sgi, (float*)lam.p, af, layout, bgrad, small, blocks, s);
           kernels += 2;
         }
       }
@@ -1054,7 +1191,15 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
     VJP_TRY(cudaEventCreate(&e1), "cudaEventCreate");
     VJP_TRY(cudaEventRecord(e0, s), "cudaEventRecord");
     const unsigned blocks = (unsigned)((pix_count + 127) / 128);
-    with_layout(f->layout(), [&](auto l) { ckpt_kernel_mixed<decltype(l)::value, true><<<blocks, 128, 0, s>>>(A); });
+    int sms = 0;
+    VJP_TRY(sm_count(&sms), "device attributes");
+    const bool small = small_adjoint(pix_count, sms);
+    with_layout(f->layout(), [&](auto l) {
+      if (small)
+        ckpt_small_kernel<decltype(l)::value, true><<<(unsigned)((pix_count + 7) / 8), 32, 0, s>>>(A);
+      else
+        ckpt_kernel_mixed<decltype(l)::value, true><<<blocks, 128, 0, s>>>(A);
+    });
     near_ckpt_kernel<<<std::min<unsigned>(blocks * 32, kNearCkptBlocks), 128, 0, s>>>(A);
     kernels += 2;
     VJP_TRY(cudaGetLastError(), "checkpointing forward");

@@ -81,13 +81,17 @@ SRT_HD int hot_base(const Geom& G, const int* c) {
 // the pair's rays, half the lines (long-scoreboard stalls 0.7; a 512^3 / nside
 // 256 / 256 steps gradient 389 -> 373 ms). All lanes of a warp call these
 // together; a lane without a ray follows one with a zero cotangent.
-struct AccF32 {
+// DISTANCE: lanes from one ray of a pair to the other (1, or 4 where four lanes
+// share a ray and `mask` holds the lanes whose field takes part).
+template <int DISTANCE>
+struct AccPaired {
   float4* g;
   int64_t hot = 0;  // index of this warp's copy; 0: no copies
+  unsigned mask = 0xffffffffu;
   SRT_HD bool active() const { return g != nullptr; }
   SRT_HD static int lane() {
 #if defined(__CUDA_ARCH__)
-    return threadIdx.x & 1;
+    return (threadIdx.x / DISTANCE) & 1;
 #else
     return 0;
 #endif
@@ -101,7 +105,7 @@ struct AccF32 {
   SRT_HD Place place(int64_t base, int hbase, const Geom& G) const {
     Place p{nullptr, nullptr, G.px, G.pxy};
 #if defined(__CUDA_ARCH__)
-    if (hot && __all_sync(0xffffffffu, hbase >= 0)) {
+    if (hot && __all_sync(mask, hbase >= 0)) {
 #else
     if (hot && hbase >= 0) {
 #endif
@@ -111,7 +115,7 @@ struct AccF32 {
     }
     int64_t other = base;
 #if defined(__CUDA_ARCH__)
-    other = __shfl_xor_sync(0xffffffffu, base, 1);
+    other = __shfl_xor_sync(mask, base, DISTANCE);
 #endif
     const int me = lane();
     p.even = g + (me ? other : base) + p.px + 1 + me;
@@ -119,11 +123,12 @@ struct AccF32 {
     return p;
   }
   // A row's two cells: this lane's (me = lane(): tap 1 or 2) and the other.
-  SRT_HD static void add_row2(float4* even, float4* odd, float4 own, float4 other) {
+  SRT_HD void add_row2(float4* even, float4* odd, float4 own, float4 other) const {
 #if defined(__CUDA_ARCH__)
     const int me = lane();
-    const float4 in = make_float4(__shfl_xor_sync(0xffffffffu, other.x, 1), __shfl_xor_sync(0xffffffffu, other.y, 1),
-                                  __shfl_xor_sync(0xffffffffu, other.z, 1), __shfl_xor_sync(0xffffffffu, other.w, 1));
+    const float4 in =
+        make_float4(__shfl_xor_sync(mask, other.x, DISTANCE), __shfl_xor_sync(mask, other.y, DISTANCE),
+                    __shfl_xor_sync(mask, other.z, DISTANCE), __shfl_xor_sync(mask, other.w, DISTANCE));
     atomicAdd(even, me ? in : own);
     atomicAdd(odd, me ? own : in);
 #else
@@ -142,8 +147,9 @@ struct AccF32 {
 // Accumulators that take cells (add_row2) rather than rows of taps.
 template <typename Acc>
 struct TakesCells : std::false_type {};
-template <>
-struct TakesCells<AccF32> : std::true_type {};
+typedef AccPaired<1> AccF32;
+template <int D>
+struct TakesCells<AccPaired<D>> : std::true_type {};
 
 struct AccF64 {
   double* g;
@@ -330,8 +336,11 @@ SRT_HD void tricubic_vjp_mixed(const Src& src, int64_t base, int hbase, const Ge
   int me = 0;
   float2 ow, og, oh, nw, ng, nh;  // difference weights of this lane's cell of a pair and the other
   if constexpr (TakesCells<Acc>::value) {
-    if (scatter) at = acc.place(base, hbase, G);
-    me = AccF32::lane();
+    if (scatter) {
+      const auto p = acc.place(base, hbase, G);
+      at = {p.even, p.odd, p.px, p.pxy};
+    }
+    me = Acc::lane();
     ow = me ? xd.w3 : xd.w0, og = me ? xd.g3 : xd.g0, oh = me ? xd.h3 : xd.h0;
     nw = me ? xd.w0 : xd.w3, ng = me ? xd.g0 : xd.g3, nh = me ? xd.h0 : xd.h3;
   }
@@ -391,7 +400,7 @@ SRT_HD void tricubic_vjp_mixed(const Src& src, int64_t base, int hbase, const Ge
           const float2 po = me ? p2 : p1, pn = me ? p1 : p2;
           const float2 eo = ffma2(ow, Cw[j], ffma2(og, Cg[j], fmul2(oh, Ch[j])));
           const float2 en = ffma2(nw, Cw[j], ffma2(ng, Cg[j], fmul2(nh, Ch[j])));
-          AccF32::add_row2(at.even + j * at.px, at.odd + j * at.px, make_float4(po.x, po.y, eo.x, eo.y),
+          acc.add_row2(at.even + j * at.px, at.odd + j * at.px, make_float4(po.x, po.y, eo.x, eo.y),
                            make_float4(pn.x, pn.y, en.x, en.y));
         }
         at.even += at.pxy;
@@ -504,16 +513,12 @@ struct BVjp {
   T Gn[3], ngB[3], S[6], K[6], nlap;
 };
 
-// One B component's share of rhs_vjp: its cotangents (value, gradient,
-// Hessian), the fused pass, the forward sums and its terms of nb, the cotangent
-// of n (those of e1 and e2 follow from the sums).
-template <int C, int LAYOUT, int UNROLL, typename T, typename Acc>
-SRT_HD void vjp_b_component(const StageView<T>& V, const FieldPtrs& F, const Geom& G, const T* fb, BVjp<T>& B,
-                            const Acc& acc, T* xb, T* nb) {
+// B component C's cotangents (value, gradient, Hessian).
+template <int C, typename T>
+SRT_HD void b_cotangent(const StageView<T>& V, const T* fb, const BVjp<T>& B, T* qb) {
   const T* n = V.n;
   const T nc = n[C], n2 = T(2) * nc, kap = fm(B.h1, V.a[C], B.h2 * V.b[C]);
   const T Tc[3] = {B.Tb[sym_idx(C, 0)], B.Tb[sym_idx(C, 1)], B.Tb[sym_idx(C, 2)]};
-  T qb[10];
   qb[0] = -fb[C];
   for (int i = 0; i < 3; ++i) qb[1 + i] = fm(nc, B.u[i], kap * n[i]);
   // Hessian cotangent n_c (Tb + nlapb I) - sym(Tb_c. (x) n), off-diagonals
@@ -523,8 +528,15 @@ SRT_HD void vjp_b_component(const StageView<T>& V, const FieldPtrs& F, const Geo
     for (int j = i + 1; j < 3; ++j)
       qb[4 + sym_idx(i, j)] = fm(n2, B.Tb[sym_idx(i, j)], -fm(Tc[i], n[j], Tc[j] * n[i]));
   }
-  Tri<T> Q;
-  field_pass<LAYOUT, UNROLL, T, Acc>(F, C, V, G, qb, Q, xb, acc);
+}
+
+// Its interpolation Q folded into the sums and into nb, the cotangent of n
+// (those of e1 and e2 follow from the sums).
+template <int C, typename T>
+SRT_HD void b_fold(const StageView<T>& V, const Tri<T>& Q, BVjp<T>& B, T* nb) {
+  const T* n = V.n;
+  const T nc = n[C], kap = fm(B.h1, V.a[C], B.h2 * V.b[C]);
+  const T Tc[3] = {B.Tb[sym_idx(C, 0)], B.Tb[sym_idx(C, 1)], B.Tb[sym_idx(C, 2)]};
   for (int i = 0; i < 3; ++i) B.ngB[i] = fm(Q.g[i], nc, C == 0 ? T(0) : B.ngB[i]);
   B.Gn[C] = vdot(Q.g, n);
   B.nlap = fm(nc, Q.h[0] + Q.h[3] + Q.h[5], C == 0 ? T(0) : B.nlap);
@@ -541,19 +553,61 @@ SRT_HD void vjp_b_component(const StageView<T>& V, const FieldPtrs& F, const Geo
   for (int k = 0; k < 3; ++k) nb[k] += fm(kap, Q.g[k], -sym_row(Q.h, k, Tc));
 }
 
-// yb += J(u)^T fb for the stage described by V; tap cotangents go to accb[0..2]
-// (B_x, B_y, B_z) and accp (phi).
-template <typename T, typename AccB, typename AccP, int LAYOUT = kPlanes>
-SRT_HD void rhs_vjp(const StageView<T>& V, const FieldPtrs& F, const Geom& G, const T* fb, T* yb, const AccB* accb,
-                    const AccP& accp) {
+// What phi's cotangents take from the state.
+template <typename T>
+struct PhiVjp {
+  T nfx, e1b, e2b, Lb, PHb, vb[3], Heb[6];
+};
+template <typename T>
+SRT_HD void phi_cotangent(const StageView<T>& V, const PhiVjp<T>& p, T* qb) {
+  qb[0] = T(-2) * p.nfx;
+  for (int i = 0; i < 3; ++i)
+    qb[1 + i] = fm(T(2), fm(p.e1b, V.a[i], fm(p.e2b, V.b[i], p.vb[i])), V.n[i] * p.Lb);
+  for (int i = 0; i < 3; ++i) {
+    const T t = V.n[i] * p.PHb;
+    qb[4 + sym_idx(i, i)] = fm(V.n[i], t, p.Heb[sym_idx(i, i)] - p.PHb);
+    for (int j = i + 1; j < 3; ++j) qb[4 + sym_idx(i, j)] = T(2) * fm(t, V.n[j], p.Heb[sym_idx(i, j)]);
+  }
+}
+
+// The four fused passes of a stage by one lane: the B sums and nb, the position
+// cotangent xb and phi's interpolation P. The slice loops are unrolled where only
+// phi's scatter follows them (512^3 / nside 256 / 256 steps, backward half: 183
+// ms in loops, 181 unrolled), loops with four scatters, where the code outgrows
+// the instruction cache (256^3 / nside 128 / 128 steps: 49.6 ms against 50.8).
+template <int LAYOUT, typename T, typename AccB, typename AccP>
+struct OneLanePasses {
+  const FieldPtrs& F;
+  const Geom& G;
+  const AccB* accb;
+  const AccP& accp;
+  static constexpr int kUnroll = std::is_same<AccB, AccNone>::value ? 4 : 1;
+  template <int C>
+  SRT_HD void component(const StageView<T>& V, const T* fb, BVjp<T>& B, T* nb, T* xb) const {
+    T qb[10];
+    b_cotangent<C>(V, fb, B, qb);
+    Tri<T> Q;
+    field_pass<LAYOUT, kUnroll, T, AccB>(F, C, V, G, qb, Q, xb, accb[C]);
+    b_fold<C>(V, Q, B, nb);
+  }
+  SRT_HD void operator()(const StageView<T>& V, const T* fb, const PhiVjp<T>& p, BVjp<T>& B, T* nb, T* xb,
+                         Tri<T>& P) const {
+    // compile-time component index: no local-memory arrays
+    component<0>(V, fb, B, nb, xb);
+    component<1>(V, fb, B, nb, xb);
+    component<2>(V, fb, B, nb, xb);
+    T qb[10];
+    phi_cotangent(V, p, qb);
+    field_pass<LAYOUT, kUnroll, T, AccP>(F, 3, V, G, qb, P, xb, accp);
+  }
+};
+
+// yb += J(u)^T fb for the stage described by V, its four passes by `passes`.
+template <typename T, typename Passes>
+SRT_HD void rhs_vjp_with(const StageView<T>& V, const T* fb, T* yb, const Passes& passes) {
   const T* n = V.n;
   const T* a = V.a;
   const T* b = V.b;
-  // The passes' slice loops: unrolled where only phi's scatter follows them
-  // (512^3 / nside 256 / 256 steps, backward half: 183 ms in loops, 181 unrolled),
-  // in loops with four scatters, where the code outgrows the instruction cache
-  // (256^3 / nside 128 / 128 steps: 49.6 ms against 50.8).
-  constexpr int kUnroll = std::is_same<AccB, AccNone>::value ? 4 : 1;
   // ---- intermediate cotangents (state only)
   const T nfx = vdot(n, fb), nfn = vdot(n, fb + 3);
   const T e1b = -vdot(n, fb + 6), e2b = -vdot(n, fb + 9);
@@ -600,27 +654,13 @@ SRT_HD void rhs_vjp(const StageView<T>& V, const FieldPtrs& F, const Geom& G, co
     const T ngBb = fm(T(0.25) * n[i], Lb, vb[i]);
     B.u[i] = fm(B.h1, a[i], fm(B.h2, b[i], ngBb));
   }
+  PhiVjp<T> ph;
+  ph.nfx = nfx, ph.e1b = e1b, ph.e2b = e2b, ph.Lb = Lb, ph.PHb = PHb;
+  for (int i = 0; i < 3; ++i) ph.vb[i] = vb[i];
+  for (int k = 0; k < 6; ++k) ph.Heb[k] = Heb[k];
   T nb[3] = {0, 0, 0}, xb[3] = {0, 0, 0};
-
-  // ---- B components (compile-time component index: no local-memory arrays)
-  vjp_b_component<0, LAYOUT, kUnroll, T, AccB>(V, F, G, fb, B, accb[0], xb, nb);
-  vjp_b_component<1, LAYOUT, kUnroll, T, AccB>(V, F, G, fb, B, accb[1], xb, nb);
-  vjp_b_component<2, LAYOUT, kUnroll, T, AccB>(V, F, G, fb, B, accb[2], xb, nb);
-
-  // ---- phi
   Tri<T> P;
-  {
-    T qb[10];
-    qb[0] = T(-2) * nfx;
-    for (int i = 0; i < 3; ++i)
-      qb[1 + i] = fm(T(2), fm(e1b, a[i], fm(e2b, b[i], vb[i])), n[i] * Lb);
-    for (int i = 0; i < 3; ++i) {
-      const T t = n[i] * PHb;
-      qb[4 + sym_idx(i, i)] = fm(n[i], t, Heb[sym_idx(i, i)] - PHb);
-      for (int j = i + 1; j < 3; ++j) qb[4 + sym_idx(i, j)] = T(2) * fm(t, n[j], Heb[sym_idx(i, j)]);
-    }
-    field_pass<LAYOUT, kUnroll, T, AccP>(F, 3, V, G, qb, P, xb, accp);
-  }
+  passes(V, fb, ph, B, nb, xb, P);
   const T* g = P.g;
   // ---- the rest of n's cotangent, and those of e1, e2 and the scalars
   T v[3], w[3], Hn[3];
@@ -673,6 +713,14 @@ SRT_HD void rhs_vjp(const StageView<T>& V, const FieldPtrs& F, const Geom& G, co
   yb[15] += s2b;
   yb[16] += el1b;
   yb[17] += el2b;
+}
+
+// The same by one lane; tap cotangents go to accb[0..2] (B_x, B_y, B_z) and accp
+// (phi).
+template <typename T, typename AccB, typename AccP, int LAYOUT = kPlanes>
+SRT_HD void rhs_vjp(const StageView<T>& V, const FieldPtrs& F, const Geom& G, const T* fb, T* yb, const AccB* accb,
+                    const AccP& accp) {
+  rhs_vjp_with(V, fb, yb, OneLanePasses<LAYOUT, T, AccB, AccP>{F, G, accb, accp});
 }
 
 // ------------------------------------------------------- stage views

@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include "srt_internal.h"
+#include "srt_four_lanes.cuh"
 
 namespace srt {
 
@@ -251,43 +252,6 @@ __global__ void __launch_bounds__(128, (MODE == kMIXED || MODE >= kMIXED_PAIR) ?
 #pragma unroll
   for (int m = 0; m < 6; ++m) A.maps[m][o] = out[m];
 }
-
-// The stage's interpolations by a group of four lanes that hold the same ray,
-// one field each (B_x, B_y, B_z, phi), exchanged by shuffles; every lane then
-// folds them in OneLane's order, so the values are the same bits.
-template <int LAYOUT>
-struct FourLanes {
-  int field, first;  // this lane's field; the group's first lane
-  __device__ void operator()(const FieldPtrs& F, const Geom& G, const int* cc, const int* cs, const float* tc,
-                             const float* ts, const float* n, BAcc& A, Tri<float>& p) const {
-    Tri<float> own;
-    {
-      AxisWeights<LAYOUT> X, Y;
-      CRW<float> Z;
-      axis_weights(field == 0 ? ts[0] : tc[0], X);
-      axis_weights(field == 1 ? ts[1] : tc[1], Y);
-      cr_weights_mixed(field == 2 ? ts[2] : tc[2], Z);
-      const int cx = field == 0 ? cs[0] : cc[0], cy = field == 1 ? cs[1] : cc[1], cz = field == 2 ? cs[2] : cc[2];
-      tricubic_mixed(cell_source<LAYOUT>(F, G, field, cx, cy, cz), X, Y, Z, own);
-    }
-    Tri<float> r;
-    fetch(own, 0, r);
-    add_b_component<0>(r, n, A);
-    fetch(own, 1, r);
-    add_b_component<1>(r, n, A);
-    fetch(own, 2, r);
-    add_b_component<2>(r, n, A);
-    fetch(own, 3, p);
-  }
-  __device__ void fetch(const Tri<float>& own, int f, Tri<float>& r) const {
-    const unsigned mask = 0xfu << first;
-    r.v = __shfl_sync(mask, own.v, first + f);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) r.g[i] = __shfl_sync(mask, own.g[i], first + f);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) r.h[i] = __shfl_sync(mask, own.h[i], first + f);
-  }
-};
 
 // The MIXED trace of a small range, four lanes per ray in one-warp blocks: a warp
 // alone on its scheduler is bound by the latency of a stage's chains, and with
