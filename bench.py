@@ -51,20 +51,23 @@ import numpy as np  # noqa: E402
 # each with 4 tricubic interpolations of value, gradient and Hessian), counted
 # operation by operation from the scheme (snapshot-raytracer.cu:195-550) as
 # this build forms it, one FMA = 2 FLOP:
-#   tricubic, separable: x pass 16 rows x 3 outputs x 4 taps, y pass 4 x 6 x 4,
-#     z pass 10 x 4 multiply-adds = 328 FMA                     ->  656 FLOP
-#   Catmull-Rom weights of value, d/dt, d2/dt2 (Horner form, 38 FLOP a set):
-#     6 sets per right-hand side (3 centred axes shared by phi and by the two
-#     unstaggered axes of each B component, 3 staggered)        ->  228 FLOP
+#   tricubic, separable, from two inner taps and their second differences:
+#     x pass 16 rows x 14, y pass 4 slices x 32, z pass 10 x 4 multiply-adds
+#                                                               ->  432 FLOP
+#   Catmull-Rom weights (Horner form): per right-hand side 3 centred axes shared
+#     by phi and by the two unstaggered axes of each B component, 3 staggered;
+#     x and y in the second-difference form (20 FLOP a set), z on four taps (38)
+#                                                               ->  156 FLOP
 #   right-hand side outside the interpolations: unit n, e1, e2 (27), the B
 #     sums n.grad B, e.n.grad B, tidal matrix, n.lap B (3 x 72), the geodesic,
 #     transport and Sachs terms with the dA > 1/2 branch (203)  ->  446 FLOP
 #   RK4 stage states (3 x 38), accumulation (76), update (57)   ->  247 FLOP
-# The packed z pass's idle half-lanes, the perturbation form's compensated
-# sums and the exact position split are implementation overhead, not counted.
-FLOP_PER_RAY_STEP = 4 * (4 * 656 + 228 + 446) + 247    # = 13,439
-# Bytes gathered per ray-step: 4 stages x 4 fields x 64 taps x 4 B (FP32 fields).
-GATHER_BYTES_PER_RAY_STEP = 4 * 4 * 64 * 4               # = 4,096
+# The perturbation form's compensated sums and the exact position split are
+# implementation overhead, not counted. (On four taps the interpolation takes
+# 656 FLOP and the weights 228: 13,439 a ray-step.)
+FLOP_PER_RAY_STEP = 4 * (4 * 432 + 156 + 446) + 247    # = 9,567
+# Bytes gathered per ray-step: 4 stages x 4 fields x 16 cells x 16 B.
+GATHER_BYTES_PER_RAY_STEP = 4 * 4 * 16 * 16              # = 4,096
 MAP_NAMES = ("dA", "ellipticity1", "ellipticity2", "rotation", "deflection1", "deflection2")
 
 
@@ -82,8 +85,8 @@ def parse():
     ap.add_argument("--precision", default="mixed", choices=("mixed", "fp64", "ref16"))
     ap.add_argument("--seed", type=int, default=2024)
     ap.add_argument("--no-pairs", dest="pairs", action="store_false",
-                    help="lay the fields out without their row-pair copies (SRT_FIELDS_NO_PAIRS): the packed MIXED "
-                         "passes then form their tap pairs from the single layout")
+                    help="keep the fields as planes (SRT_FIELDS_NO_PAIRS): the MIXED passes then form their second "
+                         "differences on the spot")
     ap.add_argument("--e2e-steps", type=int, default=7,
                     help="timed snapshots of the pipelined end-to-end leg, less one (the serial leg times "
                          "min(this, 3)); 0 skips both")
@@ -484,10 +487,11 @@ def run_ours(args):
     torch.cuda.synchronize()
     stream = torch.cuda.current_stream(dev)
     fields = srt.Fields(phi_d, b_d, stream=stream, pairs=args.pairs)
-    # the row-pair copies are built only when they fit (not at 2048^3)
-    with_pairs = fields.nbytes > 16 * (n + 3) ** 3
-    cfg["field_layout"] = "halo-padded planes" + (" + row-pair copies" if with_pairs else
-                                                  " (packed passes form their pairs from the single layout)")
+    # cells, or planes and row pairs, where they fit (not at 2048^3)
+    per_voxel = fields.nbytes / (n + 3) ** 3
+    cfg["field_layout"] = ("cells (value and second differences)" if per_voxel == 64 else
+                           "halo-padded planes + row-pair copies" if per_voxel > 16 else
+                           "halo-padded planes (second differences formed on the spot)")
     if args.e2e_steps <= 0:  # the laid-out copy is all the trace needs (2048^3: 137 GB freed)
         torch.cuda.synchronize()
         del phi_d, b_d

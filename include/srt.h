@@ -74,9 +74,9 @@ extern "C" {
                                 overwriting them */
 #define SRT_DETERMINISTIC 16u /* srt_vjp: order-independent (bitwise
                                  reproducible) FP64 gradient accumulation */
-#define SRT_FIELDS_NO_PAIRS 32u /* srt_fields_create: do not build the row-pair
-                                   copies of the fields (2x the field memory)
-                                   that the MIXED forward reads when present */
+#define SRT_FIELDS_NO_PAIRS 32u /* srt_fields_create: keep the fields as planes (16
+                                   bytes per voxel) instead of the larger layouts
+                                   the MIXED kernels read faster */
 #define SRT_FIELDS_STAGED 256u /* srt_fields_create: copy host inputs through a
                                   device slab even when they are mapped pinned
                                   memory the layout kernel could read directly */
@@ -123,17 +123,19 @@ int srt_device_count(void);
 
 /* Upload (or adopt from device memory) the Weyl potential phi and the shift
  * vector field B and lay them out for tracing: a periodic halo of one voxel
- * before and two after on every axis, one FP32 plane per B component.
+ * before and two after on every axis, each component apart.
  * phi: n0*n1*n2 floats; b_xyz: 3*n0*n1*n2 floats interleaved per voxel
  * (B_x, B_y, B_z of voxel v at b_xyz[3v+0..2]), the layout of the reference's
  * HDF5 vector read (snapshot-raytracer.cu:89-186). Host inputs in mapped
  * pinned memory (cudaHostAlloc, or cudaHostRegister with mapping) are read by
- * the layout kernel directly over the host link; other host inputs (or all,
- * with SRT_FIELDS_STAGED) are streamed through a device slab, so peak device
- * memory is the laid-out fields plus one slab.
- * Unless SRT_FIELDS_NO_PAIRS, and when device memory allows, each field is
- * also stored as row pairs (f(i,j,k), f(i,j+1,k)) for the packed-FMA MIXED
- * forward; without them MIXED reads the single copy.
+ * a kernel over the host link; other host inputs (or all, with
+ * SRT_FIELDS_STAGED) by the copy engines; either way through a device slab, so
+ * peak device memory is the laid-out fields plus one slab.
+ * Where they take at most two fifths of the free device memory, and unless
+ * SRT_FIELDS_NO_PAIRS, the fields are stored as cells: per voxel and component
+ * the value and its second differences along y, x and both (16 bytes; nothing
+ * else is kept). Else as FP32 planes (4 bytes), beside them, when they fit,
+ * row-pair copies (8 bytes). MIXED gives the same bits on each.
  * Replaces snapshot-raytracer.cu:752-855 (cudaMalloc of the fields, the three
  * staged vector3_to_half passes and the phi copy). */
 int srt_fields_create(const float* phi, const float* b_xyz, int64_t n0, int64_t n1,
@@ -189,8 +191,8 @@ int64_t srt_fields_bytes(const srt_fields* fields);
 
 /* Field memory comes from a per-device pool that keeps what srt_fields_destroy
  * hands back, so that the next srt_fields_create of the same size is not slowed
- * down by the driver mapping tens of GB again. This returns the pool's unused
- * memory to the device (a failed allocation also does, before retrying), and
+ * down by the driver mapping tens of GB again; the calls' scratch from another
+ * that keeps up to 8 GiB. This returns the pools' unused memory to the device (a failed allocation also does, before retrying), and
  * forgets the device addresses srt_forward_noalloc looked up (call it after a
  * cudaDeviceReset, before the next srt_forward_noalloc). No counterpart in the
  * reference. */
@@ -219,7 +221,8 @@ int srt_debug_fail_alloc(int64_t after);
  * the FP32 trajectory's error bound, 4e-7 (s max|dn| + 1e-3) grid units at
  * affine distance s, where the FP32 and FP64 trajectories could pick different cells (the
  * Catmull-Rom Hessian jumps across faces); those rays then equal the FP64
- * result bit for bit (SRT_MIXED_NO_REFINE skips this). The CLI's batch b is
+ * result bit for bit, or, in calls with more than four of them per SM, to a
+ * float ulp (SRT_MIXED_NO_REFINE skips this). The CLI's batch b is
  * pix_begin = b*nside^2, pix_count = nside^2 (snapshot-raytracer.cu:708-717);
  * all pixels is pix_begin = 0, pix_count = 12*nside^2. With SRT_NESTED_RANGE
  * the range counts NESTED pixels instead (HEALPix base pixel b, the batch the
@@ -280,8 +283,8 @@ typedef struct srt_tape srt_tape;
  * every ckpt_every steps (<= 0 picks ~sqrt(n_steps)), so that srt_vjp_tape can
  * form the gradient without tracing the rays forward again: the forward half
  * of a forward/vjp pair. The maps are srt_forward's (flagged rays re-traced
- * in FP64). The tape holds (n_steps/ckpt_every + 1) x 38 floats and one
- * index per ray; the fields must outlive it. pix_count >= 1; flags:
+ * in FP64). The tape holds (n_steps/ckpt_every + 1) x 38 + 12 floats and two
+ * indices per ray; the fields must outlive it. pix_count >= 1; flags:
  * SRT_OUTPUT_DEVICE. No counterpart in the reference (it has no
  * derivatives). */
 int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t pix_begin, int64_t pix_count,

@@ -676,7 +676,8 @@ struct PadRead<unsigned long long> {  // fixed point: exact integer sums
 // Value of padded position (i, j, k) of an accumulator grid; for cells, the
 // transpose of cell_of: the second differences gather their neighbours'
 // cotangents (symmetric stencils; only positions 1 .. n + 1 hold any).
-template <typename G>
+// INSIDE: the neighbours are known to lie in the grid.
+template <bool INSIDE, typename G>
 __device__ __forceinline__ typename PadRead<G>::T pad_value(const PadRead<G>& rd, int64_t i, int64_t j, int64_t k,
                                                             int64_t p0, int64_t p1) {
   return rd(i + p0 * (j + p1 * k));
@@ -687,15 +688,17 @@ struct PadRead<float4> {
   const float4* g;
   __device__ static double value(T s) { return (double)s; }
 };
+template <bool INSIDE>
 __device__ __forceinline__ float pad_value(const PadRead<float4>& rd, int64_t i, int64_t j, int64_t k, int64_t p0,
                                            int64_t p1) {
   float s = 0.f;
+  const float4* at = rd.g + i + p0 * (j + p1 * k);
 #pragma unroll
   for (int b = -1; b <= 1; ++b)
 #pragma unroll
     for (int a = -1; a <= 1; ++a) {
-      if (i + a < 0 || i + a >= p0 || j + b < 0 || j + b >= p1) continue;
-      const float4 c = __ldg(rd.g + (i + a) + p0 * ((j + b) + p1 * k));
+      if (!INSIDE && (i + a < 0 || i + a >= p0 || j + b < 0 || j + b >= p1)) continue;
+      const float4 c = __ldg(at + a + p0 * b);
       const float wx = a == 0 ? -2.f : 1.f, wy = b == 0 ? -2.f : 1.f;
       float v = wx * wy * c.w;
       if (a == 0) v += wy * c.y;
@@ -736,16 +739,18 @@ __global__ void __launch_bounds__(256) fold_kernel(const G* __restrict__ padded,
   if (i >= n0) return;
   const PadRead<G> rd{padded};
   const int64_t p0 = n0 + 3, p1 = n1 + 3;
-  int64_t pi[4], pj[4], pk[4];
-  const int ni = padded_coords(i, n0, pi);
   for (int64_t k = blockIdx.z; k < n2; k += gridDim.z) {
-    const int nk = padded_coords(k, n2, pk);
     for (int64_t j = (int64_t)blockIdx.y * 8 + threadIdx.y; j < n1; j += (int64_t)gridDim.y * 8) {
-      const int nj = padded_coords(j, n1, pj);
       typename PadRead<G>::T sum = 0;
-      for (int a = 0; a < nk; ++a)
-        for (int b = 0; b < nj; ++b)
-          for (int c = 0; c < ni; ++c) sum += pad_value(rd, pi[c], pj[b], pk[a], p0, p1);
+      if (i > 1 && i < n0 - 1 && j > 1 && j < n1 - 1 && k > 1 && k < n2 - 1) {  // no halo copies
+        sum = pad_value<true>(rd, i + 1, j + 1, k + 1, p0, p1);
+      } else {
+        int64_t pi[4], pj[4], pk[4];
+        const int ni = padded_coords(i, n0, pi), nj = padded_coords(j, n1, pj), nk = padded_coords(k, n2, pk);
+        for (int a = 0; a < nk; ++a)
+          for (int b = 0; b < nj; ++b)
+            for (int c = 0; c < ni; ++c) sum += pad_value<false>(rd, pi[c], pj[b], pk[a], p0, p1);
+      }
       const double dval = PadRead<G>::value(sum);
       if (ovf && !(fabs(dval) < kFixedLimit)) atomicOr(ovf, 1u);  // fixed point near or past its range
       const float val = (float)dval;

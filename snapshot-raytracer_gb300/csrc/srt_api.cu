@@ -257,9 +257,11 @@ int64_t field_budget(const srt_fields* f) {
 }
 
 // Device arrays of the laid-out fields of an n0 x n1 x n2 grid (no contents):
-// cells where they fit (64 bytes per padded voxel for the four fields) unless
-// SRT_FIELDS_NO_PAIRS, else planes (16 bytes), which finish_fields may add row
-// pairs to (another 32).
+// cells (64 bytes per padded voxel for the four fields) unless
+// SRT_FIELDS_NO_PAIRS, where they take at most two fifths of the budget (so that
+// a gradient's accumulators, another 64 bytes, and its scratch fit beside them as
+// they do beside planes and row pairs), else planes (16 bytes), which
+// finish_fields may add row pairs to (another 32).
 int alloc_fields(srt_fields* f, int64_t n0, int64_t n1, int64_t n2, unsigned flags, cudaStream_t s) {
   cudaGetDevice(&f->device);
   for (int i = 0; i < 3; ++i) {
@@ -267,7 +269,7 @@ int alloc_fields(srt_fields* f, int64_t n0, int64_t n1, int64_t n2, unsigned fla
     f->pn[i] = f->n[i] + 3;
   }
   const int64_t pvox = f->pn[0] * f->pn[1] * f->pn[2];
-  if (!(flags & SRT_FIELDS_NO_PAIRS) && 64 * pvox < field_budget(f)) {
+  if (!(flags & SRT_FIELDS_NO_PAIRS) && 64 * pvox <= field_budget(f) / 5 * 2) {
     for (int c = 3; c >= 0; --c) {
       cudaError_t e = pool_alloc((void**)&f->cell[c], pvox * sizeof(float4), s);
       if (e != cudaSuccess) return cuda_error(e, c == 3 ? "allocate phi" : "allocate B");
