@@ -106,7 +106,8 @@ struct AdjArgs {
   int n_steps, C, nseg;
   const float* w[6];  // map weights, indexed by ring - pix_begin
   void* ckpt;         // [nseg + 1][state][count]
-  void* seg;          // [C][state + 57][count]
+  void* seg;          // [C][state + 57][count] (FP64); MIXED: the tape (kTapeStep)
+  int tape_from;      // MIXED forward: steps from here on go to the tape at once
   void* acc[4];       // padded gradient accumulators B_x, B_y, B_z, phi (NULL: not wanted)
   // forward with a tape (srt_forward_tape): the maps, indexed by ring - pix_begin,
   // and the output slots of rays that came within the cell-face guard
@@ -191,9 +192,11 @@ __device__ __forceinline__ void prefetch_step(const AdjArgs& A, const MixedRay& 
 
 // Forward trace of one ray storing the state every C steps (and the final
 // state); y holds the final state.
-template <typename Interp>
+// TAPE: the stage inputs of steps tape_from on go to the tape (by lanes with
+// `tape`), so that those segments are not recomputed.
+template <bool TAPE, typename Interp>
 __device__ __forceinline__ void ckpt_ray(const Interp& interp, const AdjArgs& A, int64_t slot, const RayDir& d,
-                                         MixedRay& R, float* y, Guard& gd) {
+                                         MixedRay& R, float* y, Guard& gd, bool tape = true) {
   constexpr bool kNear = std::is_same<Interp, OneLane<kFourTaps>>::value;
   float x0[3];
   mixed_observer(A.G, x0);
@@ -205,7 +208,10 @@ __device__ __forceinline__ void ckpt_ray(const Interp& interp, const AdjArgs& A,
   for (int st = 0; st < A.n_steps; ++st) {
     if (kNear) prefetch_step(A, R, x0, y, st);
     if (gd.m) gd.begin_step(y);
-    step_mixed(interp, R, A.F, A.G, x0, st, y, nullptr, 0, gd);
+    float* us = TAPE && tape && st >= A.tape_from
+                    ? (float*)A.seg + (int64_t)(st - A.tape_from) * kTapeStep * A.count + slot
+                    : nullptr;
+    step_mixed(interp, R, A.F, A.G, x0, st, y, us, A.count, gd);
     if (gd.m) gd.end_step(st);
     const int done = st + 1;
     if (done % A.C == 0 || done == A.n_steps) {
@@ -228,7 +234,7 @@ __device__ __forceinline__ void ckpt_one(const Interp& interp, const AdjArgs& A,
   Guard gd;
   gd.m = guard_m;
   gd.m[0] = 0.f;
-  ckpt_ray(interp, A, slot, ray_dir_pix(A.nside, ring), R, y, gd);
+  ckpt_ray<!MAPS>(interp, A, slot, ray_dir_pix(A.nside, ring), R, y, gd, first);
   if (!first) return;
   if (gd.near) {
     A.rays[slot] = ring | kNearBit;
@@ -267,12 +273,13 @@ __global__ void __launch_bounds__(32, 12) ckpt_small_kernel(const AdjArgs A) {
 
 // The marked rays' checkpoints by the four-tap passes, one warp per ray. Few
 // rays: the launch is about one ray's latency.
+template <bool TAPE>
 __global__ void __launch_bounds__(128, 2) near_ckpt_kernel(const AdjArgs A) {
   for_near_rays(A, (int64_t)gridDim.x * 4, [&](int64_t slot) {
     MixedRay R;
     float y[kMixedState];
     Guard gd;  // disabled
-    ckpt_ray(OneLane<kFourTaps>(), A, slot, ray_dir_pix(A.nside, ring_of(A, slot)), R, y, gd);
+    ckpt_ray<TAPE>(OneLane<kFourTaps>(), A, slot, ray_dir_pix(A.nside, ring_of(A, slot)), R, y, gd);
   });
 }
 
@@ -827,6 +834,22 @@ done:
 // rays 3.41 against 4.18).
 static bool small_adjoint(int64_t rays, int sms) { return rays <= (int64_t)sms * 4 * 8; }
 
+// Segments whose tape srt_vjp's forward writes at once, the last ones, instead of
+// a recompute (256^3 / nside 128 / 128 steps, C = 12: 5 of 11, 49.8 -> 46.9 ms): as many as
+// 4 GiB hold; none where device memory is short (an eighth of what is free beside the
+// outputs' staging).
+static int kept_segments(int nseg, int64_t seg_bytes, int64_t out_bytes, int device) {
+  const int64_t most = int64_t(4) << 30, few = int64_t(256) << 20;
+  const int kept = (int)std::min<int64_t>(nseg, most / std::max<int64_t>(seg_bytes, 1));
+  if (kept * seg_bytes > few) {
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess ||
+        (int64_t)free_b + pool_reusable_bytes(device) < out_bytes + 8 * kept * seg_bytes)
+      return 0;
+  }
+  return kept;
+}
+
 // A forward trace's checkpoints (srt_forward_tape) for srt_vjp_tape.
 struct srt_tape {
   const srt_fields* fields = nullptr;
@@ -950,8 +973,6 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
       // grid holds the region
       const bool hot = !fp64 && !determ && std::min(f->n[0], std::min(f->n[1], f->n[2])) >= kHotSide;
       const int64_t acc_entries = pvox + (hot ? (int64_t)kHotCopies * kHotSide * kHotSide * kHotSide : 0);
-      // per-step records of one segment: FP64 y, k1, k2, k3; MIXED the four stage inputs
-      VJP_TRY(seg.alloc((size_t)C * (fp64 ? state + 57 : kTapeStep) * pix_count * esz, s), "allocate segment records");
       if (!fp64) VJP_TRY(lam.alloc((size_t)19 * pix_count * sizeof(float), s), "allocate state cotangents");
       for (int fld = 0; fld < 4; ++fld) {
         const bool want = (fld == 3) ? (dphi != nullptr) : (db_xyz != nullptr);
@@ -959,6 +980,10 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
         VJP_TRY(gacc[fld].alloc(acc_entries * accsz, s), "allocate gradient accumulators");
         VJP_TRY(cudaMemsetAsync(gacc[fld].p, 0, acc_entries * accsz, s), "clear accumulators");
       }
+      // per-step records of one segment: FP64 y, k1, k2, k3; MIXED the four stage inputs
+      const int64_t seg_bytes = (int64_t)C * (fp64 ? state + 57 : kTapeStep) * pix_count * (int64_t)esz;
+      const int kept = fp64 || tape ? 0 : kept_segments(nseg, seg_bytes, 32 * pvox, f->device);
+      VJP_TRY(seg.alloc(std::max(kept, 1) * seg_bytes, s), "allocate segment records");
       if (determ) {  // fixed-point range flag
         VJP_TRY(ovf.alloc(sizeof(unsigned), s), "allocate overflow flag");
         VJP_TRY(cudaMemsetAsync(ovf.p, 0, sizeof(unsigned), s), "clear overflow flag");
@@ -979,6 +1004,7 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
       for (int m = 0; m < 6; ++m) A.w[m] = wd[m];
       A.ckpt = tape ? (void*)tape->ckpt : ckpt.p;
       A.seg = seg.p;
+      A.tape_from = (nseg - kept) * C;
       for (int fld = 0; fld < 4; ++fld) A.acc[fld] = gacc[fld].p;
       for (int m = 0; m < 6; ++m) A.maps[m] = nullptr;
       A.refine_list = nullptr;
@@ -1014,7 +1040,7 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
             else
               ckpt_kernel_mixed<decltype(l)::value, false><<<blocks, 128, 0, s>>>(A);
           });
-          near_ckpt_kernel<<<std::min<unsigned>(blocks * 32, kNearCkptBlocks), 128, 0, s>>>(A);
+          near_ckpt_kernel<true><<<std::min<unsigned>(blocks * 32, kNearCkptBlocks), 128, 0, s>>>(A);
         }
         final_cotangent_kernel_mixed<<<blocks, 128, 0, s>>>(A, (float*)lam.p);
         kernels += tape ? 1 : 3;
@@ -1025,8 +1051,11 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
         make_acc<AccFixed, unsigned long long>(ax, A.acc);
         for (int fld = 0; fld < 4; ++fld) ax[fld].ovf = (unsigned*)ovf.p;
         const bool bgrad = db_xyz != nullptr;
+        const int kept_from = nseg - kept;  // segments from here on are on the tape already
         for (int sgi = nseg - 1; sgi >= 0; --sgi) {
-          with_layout(layout, [&](auto l) {
+          A.seg = seg.p;
+          if (sgi >= kept_from) A.seg = (float*)seg.p + (int64_t)(sgi - kept_from) * C * kTapeStep * pix_count;
+          if (sgi < kept_from) with_layout(layout, [&](auto l) {
             if (small) {
               segment_small_kernel<decltype(l)::value><<<(unsigned)((pix_count + 7) / 8), 32, 0, s>>>(A, sgi);
               near_segment_kernel<<<kNearBlocks, 128, 0, s>>>(A, sgi);
@@ -1038,7 +1067,7 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
             launch_sweep<AccFixed>(A, sgi, (float*)lam.p, ax, layout, bgrad, small, blocks, s);
           else
             launch_sweep<AccF32>(A, sgi, (float*)lam.p, af, layout, bgrad, small, blocks, s);
-          kernels += 2;
+          kernels += sgi < kept_from ? 2 : 1;
         }
       }
       if (fp64) kernels += 2;
@@ -1205,7 +1234,7 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
       else
         ckpt_kernel_mixed<decltype(l)::value, true><<<blocks, 128, 0, s>>>(A);
     });
-    near_ckpt_kernel<<<std::min<unsigned>(blocks * 32, kNearCkptBlocks), 128, 0, s>>>(A);
+    near_ckpt_kernel<false><<<std::min<unsigned>(blocks * 32, kNearCkptBlocks), 128, 0, s>>>(A);
     kernels += 2;
     VJP_TRY(cudaGetLastError(), "checkpointing forward");
     TraceArgs ta;
