@@ -85,8 +85,7 @@ def parse():
     ap.add_argument("--precision", default="mixed", choices=("mixed", "fp64", "ref16"))
     ap.add_argument("--seed", type=int, default=2024)
     ap.add_argument("--no-pairs", dest="pairs", action="store_false",
-                    help="keep the fields as planes (SRT_FIELDS_NO_PAIRS): the MIXED passes then form their second "
-                         "differences on the spot")
+                    help="keep the fields as planes (SRT_FIELDS_NO_PAIRS): a quarter of the memory, a slower trace")
     ap.add_argument("--e2e-steps", type=int, default=7,
                     help="timed snapshots of the pipelined end-to-end leg, less one (the serial leg times "
                          "min(this, 3)); 0 skips both")
@@ -491,7 +490,7 @@ def run_ours(args):
     per_voxel = fields.nbytes / (n + 3) ** 3
     cfg["field_layout"] = ("cells (value and second differences)" if per_voxel == 64 else
                            "halo-padded planes + row-pair copies" if per_voxel > 16 else
-                           "halo-padded planes (second differences formed on the spot)")
+                           "halo-padded planes")
     if args.e2e_steps <= 0:  # the laid-out copy is all the trace needs (2048^3: 137 GB freed)
         torch.cuda.synchronize()
         del phi_d, b_d

@@ -537,6 +537,35 @@ void with_layout(int layout, const Fn& f) {
     f(std::integral_constant<int, kPlanes>());
 }
 
+// The same for the forward's passes (the sweep interpolates at positions it is
+// given, so it takes the second differences in every layout).
+template <typename Fn>
+void with_forward_layout(const srt_fields* f, const Fn& fn) {
+  if (!f->four_taps)
+    with_layout(f->layout(), fn);
+  else if (f->layout() == kPairs)
+    fn(std::integral_constant<int, kFourPairs>());
+  else
+    fn(std::integral_constant<int, kFourPlanes>());
+}
+
+template <int LAYOUT, bool MAPS>
+void launch_ckpt(const AdjArgs& A, bool small, unsigned blocks, cudaStream_t s) {
+  if (small)
+    ckpt_small_kernel<LAYOUT, MAPS><<<(unsigned)((A.count + 7) / 8), 32, 0, s>>>(A);
+  else
+    ckpt_kernel_mixed<LAYOUT, MAPS><<<blocks, 128, 0, s>>>(A);
+}
+template <int LAYOUT>
+void launch_segment(const AdjArgs& A, int sgi, bool small, unsigned blocks, cudaStream_t s) {
+  if (small) {
+    segment_small_kernel<LAYOUT><<<(unsigned)((A.count + 7) / 8), 32, 0, s>>>(A, sgi);
+    near_segment_kernel<<<kNearBlocks, 128, 0, s>>>(A, sgi);
+  } else {
+    segment_kernel_mixed<LAYOUT><<<blocks + kNearBlocks, 128, 0, s>>>(A, sgi);
+  }
+}
+
 inline void copy_extra(AccPaired<4>& to, const AccF32& from) { to.hot = from.hot; }
 inline void copy_extra(AccFixed& to, const AccFixed& from) { to.ovf = from.ovf; }
 
@@ -1034,12 +1063,7 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
         const int layout = f->layout();
         const bool small = small_adjoint(pix_count, sms);
         if (!tape) {  // else the checkpoints come from srt_forward_tape
-          with_layout(layout, [&](auto l) {
-            if (small)
-              ckpt_small_kernel<decltype(l)::value, false><<<(unsigned)((pix_count + 7) / 8), 32, 0, s>>>(A);
-            else
-              ckpt_kernel_mixed<decltype(l)::value, false><<<blocks, 128, 0, s>>>(A);
-          });
+          with_forward_layout(f, [&](auto l) { launch_ckpt<decltype(l)::value, false>(A, small, blocks, s); });
           near_ckpt_kernel<true><<<std::min<unsigned>(blocks * 32, kNearCkptBlocks), 128, 0, s>>>(A);
         }
         final_cotangent_kernel_mixed<<<blocks, 128, 0, s>>>(A, (float*)lam.p);
@@ -1055,14 +1079,8 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
         for (int sgi = nseg - 1; sgi >= 0; --sgi) {
           A.seg = seg.p;
           if (sgi >= kept_from) A.seg = (float*)seg.p + (int64_t)(sgi - kept_from) * C * kTapeStep * pix_count;
-          if (sgi < kept_from) with_layout(layout, [&](auto l) {
-            if (small) {
-              segment_small_kernel<decltype(l)::value><<<(unsigned)((pix_count + 7) / 8), 32, 0, s>>>(A, sgi);
-              near_segment_kernel<<<kNearBlocks, 128, 0, s>>>(A, sgi);
-            } else {
-              segment_kernel_mixed<decltype(l)::value><<<blocks + kNearBlocks, 128, 0, s>>>(A, sgi);
-            }
-          });
+          if (sgi < kept_from)
+            with_forward_layout(f, [&](auto l) { launch_segment<decltype(l)::value>(A, sgi, small, blocks, s); });
           if (determ)
             launch_sweep<AccFixed>(A, sgi, (float*)lam.p, ax, layout, bgrad, small, blocks, s);
           else
@@ -1228,12 +1246,7 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
     int sms = 0;
     VJP_TRY(sm_count(&sms), "device attributes");
     const bool small = small_adjoint(pix_count, sms);
-    with_layout(f->layout(), [&](auto l) {
-      if (small)
-        ckpt_small_kernel<decltype(l)::value, true><<<(unsigned)((pix_count + 7) / 8), 32, 0, s>>>(A);
-      else
-        ckpt_kernel_mixed<decltype(l)::value, true><<<blocks, 128, 0, s>>>(A);
-    });
+    with_forward_layout(f, [&](auto l) { launch_ckpt<decltype(l)::value, true>(A, small, blocks, s); });
     near_ckpt_kernel<false><<<std::min<unsigned>(blocks * 32, kNearCkptBlocks), 128, 0, s>>>(A);
     kernels += 2;
     VJP_TRY(cudaGetLastError(), "checkpointing forward");

@@ -256,6 +256,8 @@ int64_t field_budget(const srt_fields* f) {
   return (int64_t)free_b + pool_reusable_bytes(f->device) - (int64_t(4) << 30);
 }
 
+constexpr int64_t kFourTapVoxels = int64_t(1) << 27;
+
 // Device arrays of the laid-out fields of an n0 x n1 x n2 grid (no contents):
 // cells (64 bytes per padded voxel for the four fields) unless
 // SRT_FIELDS_NO_PAIRS, where they take at most two fifths of the budget (so that
@@ -269,15 +271,28 @@ int alloc_fields(srt_fields* f, int64_t n0, int64_t n1, int64_t n2, unsigned fla
     f->pn[i] = f->n[i] + 3;
   }
   const int64_t pvox = f->pn[0] * f->pn[1] * f->pn[2];
-  if (!(flags & SRT_FIELDS_NO_PAIRS) && 64 * pvox <= field_budget(f) / 5 * 2) {
+  size_t free_b = 0, total_b = 0;
+  cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+  if (e != cudaSuccess) return cuda_error(e, "device memory");
+  // From planes and row pairs the four-tap passes are faster than the second
+  // differences formed on the spot (trace kernel from planes: 512^3 / nside 256 / 256
+  // steps 83.6 against 90.3 ms, 1024^3 / nside 512 / 512 steps 655 against 709, 2048^3
+  // / nside 2048 / 1024 steps 15.9 against 18.1 s; from row pairs, 1024^3 base pixel,
+  // 149.8 against 164.3 ms). They are taken by grids whose cells no handle would
+  // hold (some 1,230^3 on 288 GB) and by SRT_FIELDS_NO_PAIRS from 512^3 on, where
+  // full skies are bound by throughput; smaller grids, and those whose cells did not
+  // find room, keep the bits of a default handle.
+  f->four_taps =
+      64 * pvox > (int64_t)total_b / 5 * 2 || ((flags & SRT_FIELDS_NO_PAIRS) && n0 * n1 * n2 >= kFourTapVoxels);
+  if (!(flags & SRT_FIELDS_NO_PAIRS) && !f->four_taps && 64 * pvox <= field_budget(f) / 5 * 2) {
     for (int c = 3; c >= 0; --c) {
-      cudaError_t e = pool_alloc((void**)&f->cell[c], pvox * sizeof(float4), s);
+      e = pool_alloc((void**)&f->cell[c], pvox * sizeof(float4), s);
       if (e != cudaSuccess) return cuda_error(e, c == 3 ? "allocate phi" : "allocate B");
     }
     f->bytes = 64 * pvox;
     return SRT_OK;
   }
-  cudaError_t e = pool_alloc((void**)&f->phi, pvox * sizeof(float), s);
+  e = pool_alloc((void**)&f->phi, pvox * sizeof(float), s);
   if (e != cudaSuccess) return cuda_error(e, "allocate phi");
   for (int c = 0; c < 3; ++c) {
     e = pool_alloc((void**)&f->b[c], pvox * sizeof(float), s);

@@ -25,9 +25,16 @@ struct srt_fields {
   __half* bh[3] = {nullptr, nullptr, nullptr};
   float* ref_phi = nullptr;
   int64_t bytes = 0;
+  // The MIXED forward takes the four-tap passes (alloc_fields), else the second
+  // differences, in every layout: MIXED's bits depend on the grid, the flags and the
+  // device, not on what memory was free.
+  bool four_taps = false;
   int layout() const { return cell[0] ? srt::kCells : (pr[0] ? srt::kPairs : srt::kPlanes); }
   // the MIXED trace kernel of this layout
-  int mixed_mode() const { return cell[0] ? srt::kMIXED_CELL : (pr[0] ? srt::kMIXED_PAIR : srt::kMIXED); }
+  int mixed_mode() const {
+    if (four_taps) return pr[0] ? srt::kMIXED_FOUR_PAIR : srt::kMIXED_FOUR;
+    return cell[0] ? srt::kMIXED_CELL : (pr[0] ? srt::kMIXED_PAIR : srt::kMIXED);
+  }
   // the values of B component c (0-2) or phi (3), make_geom's ts floats apart
   const float* values(int c) const { return cell[c] ? &cell[c]->x : (c == 3 ? phi : b[c]); }
 };

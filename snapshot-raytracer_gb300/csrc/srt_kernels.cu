@@ -231,6 +231,15 @@ __device__ __forceinline__ bool ray_of_slot(const TraceArgs& A, int64_t tl, int6
   return *o >= 0 && *o < A.pix_count;
 }
 
+// The layout that a MIXED mode's passes read.
+constexpr __host__ __device__ int layout_of(int mode) {
+  return mode == kMIXED_CELL ? kCells
+         : mode == kMIXED_PAIR ? kPairs
+         : mode == kMIXED_FOUR ? kFourPlanes
+         : mode == kMIXED_FOUR_PAIR ? kFourPairs
+                               : kPlanes;
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(128, (MODE == kMIXED || MODE >= kMIXED_PAIR) ? SRT_MIXED_MIN_BLOCKS : 1)
     trace_kernel(const TraceArgs A) {
@@ -239,7 +248,7 @@ __global__ void __launch_bounds__(128, (MODE == kMIXED || MODE >= kMIXED_PAIR) ?
   const RayDir d = ray_dir_pix(A.nside, ring);
   float out[6];
   if (MODE >= kMIXED_PAIR || MODE == kMIXED) {
-    constexpr int kLayout = MODE == kMIXED_CELL ? kCells : (MODE == kMIXED_PAIR ? kPairs : kPlanes);
+    constexpr int kLayout = layout_of(MODE);
     __shared__ float guard_m[128][2];  // the ray's guard state, out of the register budget
     const bool near = trace_ray_mixed<kLayout>(A.F, A.G, d, A.n_steps, out, guard_m[threadIdx.x]);
     if (near && A.refine_list) {
@@ -283,7 +292,8 @@ __global__ void __launch_bounds__(32, 12) trace_small_kernel(const TraceArgs A) 
 // ms, 27,648: 1.20 against 0.99). Not where most launch slots hold no ray of the
 // range.
 bool is_small(int mode, const TraceArgs& a, int sms) {
-  const int64_t rays = (int64_t)sms * 4 * 8 * (mode == kMIXED ? 4 : 1);
+  const bool planes = mode == kMIXED || mode == kMIXED_FOUR;
+  const int64_t rays = (int64_t)sms * 4 * 8 * (planes ? 4 : 1);
   return a.pix_count <= rays && a.launch_rays <= 16 * rays;
 }
 
@@ -294,12 +304,13 @@ cudaError_t launch_trace(int mode, const TraceArgs& a, cudaStream_t s, int64_t* 
   if (e != cudaSuccess) return e;
   if (mode != kFP64 && mode != kREF16 && is_small(mode, a, sms)) {
     const unsigned small = (unsigned)((a.launch_rays + 7) / 8);
-    if (mode == kMIXED_CELL)
-      trace_small_kernel<kCells><<<small, 32, 0, s>>>(a);
-    else if (mode == kMIXED_PAIR)
-      trace_small_kernel<kPairs><<<small, 32, 0, s>>>(a);
-    else
-      trace_small_kernel<kPlanes><<<small, 32, 0, s>>>(a);
+    switch (mode) {
+      case kMIXED_CELL: trace_small_kernel<kCells><<<small, 32, 0, s>>>(a); break;
+      case kMIXED_PAIR: trace_small_kernel<kPairs><<<small, 32, 0, s>>>(a); break;
+      case kMIXED_FOUR: trace_small_kernel<kFourPlanes><<<small, 32, 0, s>>>(a); break;
+      case kMIXED_FOUR_PAIR: trace_small_kernel<kFourPairs><<<small, 32, 0, s>>>(a); break;
+      default: trace_small_kernel<kPlanes><<<small, 32, 0, s>>>(a);
+    }
     if (kernels) ++*kernels;
     return cudaGetLastError();
   }
@@ -316,6 +327,8 @@ cudaError_t launch_trace(int mode, const TraceArgs& a, cudaStream_t s, int64_t* 
     case kREF16: trace_kernel<kREF16><<<(unsigned)blocks, threads, 0, s>>>(a); break;
     case kMIXED_CELL: trace_kernel<kMIXED_CELL><<<(unsigned)blocks, threads, 0, s>>>(a); break;
     case kMIXED_PAIR: trace_kernel<kMIXED_PAIR><<<(unsigned)blocks, threads, 0, s>>>(a); break;
+    case kMIXED_FOUR: trace_kernel<kMIXED_FOUR><<<(unsigned)blocks, threads, 0, s>>>(a); break;
+    case kMIXED_FOUR_PAIR: trace_kernel<kMIXED_FOUR_PAIR><<<(unsigned)blocks, threads, 0, s>>>(a); break;
     default: return cudaErrorInvalidValue;
   }
   if (kernels) ++*kernels;

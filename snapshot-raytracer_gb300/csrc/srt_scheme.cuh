@@ -45,7 +45,7 @@
 
 namespace srt {
 
-enum { kFP64 = 0, kMIXED = 1, kREF16 = 2, kMIXED_PAIR = 3, kMIXED_CELL = 4 };
+enum { kFP64 = 0, kMIXED = 1, kREF16 = 2, kMIXED_PAIR = 3, kMIXED_CELL = 4, kMIXED_FOUR = 5, kMIXED_FOUR_PAIR = 6 };
 
 #if defined(__CUDA_ARCH__)
 template <typename T>
@@ -74,8 +74,10 @@ struct Geom {
 // How a handle stores its fields (the MIXED kernels are compiled for each):
 // planes of values; planes beside row-pair copies; or cells, which hold the
 // values too, so nothing else is stored. kFourTaps: the four-tap passes on the
-// values of any layout (rays of the adjoint that come near a cell face).
-enum { kPlanes = 0, kPairs = 1, kCells = 2, kFourTaps = 3 };
+// values of any layout (rays of the adjoint that come near a cell face);
+// kFourPlanes, kFourPairs: the same on planes and on row pairs (grids too large for
+// cells, srt_fields::four_taps).
+enum { kPlanes = 0, kPairs = 1, kCells = 2, kFourTaps = 3, kFourPlanes = 4, kFourPairs = 5 };
 
 struct FieldPtrs {
   const float* phi;     // padded FP32 values, Geom::ts floats apart
@@ -366,8 +368,8 @@ SRT_HD float y_second(const CWD& w, const YIn& q) { return fmaf(w.h3, q.e2, w.h0
 // 1,048,576 rays x 512 steps: 149.8 -> 128.0 ms; FMA pipe 66 % of cycles, issue
 // 62 %, L1 data 50 %). Second differences along x alone (the y pass on four
 // packed taps) took 136.0 ms; stored along z too they would double the
-// memory for 8 operations more. Where they are formed on the spot (planes) the
-// trace is 0.6-3 % slower than the four-tap passes on planes were.
+
+
 template <typename Src>
 SRT_HD void tricubic_mixed(const Src& src, const CWD& X, const CWD& Y, const CRW<float>& Z, Tri<float>& r) {
   const XDup xd(X);
@@ -404,17 +406,27 @@ SRT_HD void tricubic_mixed(const Src& src, const CWD& X, const CWD& Y, const CRW
 // The same on the four taps' values: the x pass on rows y and y+1 at once with
 // duplicated x weights, the y pass with the weights of rows (0, 1) and (2, 3)
 // (even / odd partial sums), the z pass as above. Taken by the few rays of the
-// adjoint whose trajectory passes a cell face within FP32 rounding (kFourTaps).
+// adjoint whose trajectory passes a cell face within FP32 rounding (kFourTaps), and
+// on grids too large for cells: 352 lane operations in 188 instructions, against 368
+// in 236 with the second differences formed on the spot (kFourPlanes, kFourPairs).
+template <bool PLANES>
 struct ValueRows {
   const float* __restrict__ f;  // voxel (cx - 1, cy - 1, cz - 1)
   int64_t px, pxy;
-  int ts;
+  int stride;
   SRT_HD float2 operator()(int c, int pr, int i) const {
+    const int ts = PLANES ? 1 : stride;
     const float* r = f + (c * pxy + 2 * pr * px + i) * ts;
     return make_float2(ldg(r), ldg(r + px * ts));
   }
 };
-SRT_HD void tricubic_mixed(const ValueRows& rows, const CRW<float>& X, const CRW<float>& Y, const CRW<float>& Z,
+struct PairRows {
+  const float2* __restrict__ f;  // pair index of voxel (cx - 1, cy - 1, cz - 1)
+  int64_t px, pxy2;
+  SRT_HD float2 operator()(int c, int pr, int i) const { return ldg(f + c * pxy2 + 2 * pr * px + i); }
+};
+template <typename Rows>
+SRT_HD void tricubic_mixed(const Rows& rows, const CRW<float>& X, const CRW<float>& Y, const CRW<float>& Z,
                            Tri<float>& r) {
   float2 xw[4], xg[4], xh[4];
   for (int i = 0; i < 4; ++i) {
@@ -524,19 +536,24 @@ SRT_HD auto cell_source(const FieldPtrs& F, const Geom& G, int f, int64_t base, 
   else if constexpr (LAYOUT == kPairs)
     return TapSource<PairTaps>{{F.pr[f] + basep, G.px, G.pxy2}};
   else if constexpr (LAYOUT == kFourTaps)
-    return ValueRows{(f == 3 ? F.phi : F.b[f]) + base * G.ts, G.px, G.pxy, G.ts};
+    return ValueRows<false>{(f == 3 ? F.phi : F.b[f]) + base * G.ts, G.px, G.pxy, G.ts};
+  else if constexpr (LAYOUT == kFourPlanes)
+    return ValueRows<true>{(f == 3 ? F.phi : F.b[f]) + base, G.px, G.pxy, 1};
+  else if constexpr (LAYOUT == kFourPairs)
+    return PairRows{F.pr[f] + basep, G.px, G.pxy2};
   else
     return TapSource<PlaneTaps>{{(f == 3 ? F.phi : F.b[f]) + base, G.px, G.pxy}};
 }
 template <int LAYOUT>
 SRT_HD auto cell_source(const FieldPtrs& F, const Geom& G, int f, int cx, int cy, int cz) {
-  return cell_source<LAYOUT>(F, G, f, LAYOUT == kPairs ? 0 : cell_base(G, cx, cy, cz),
-                             LAYOUT == kPairs ? cell_base_pair(G, cx, cy, cz) : 0);
+  constexpr bool kFromPairs = LAYOUT == kPairs || LAYOUT == kFourPairs;
+  return cell_source<LAYOUT>(F, G, f, kFromPairs ? 0 : cell_base(G, cx, cy, cz),
+                             kFromPairs ? cell_base_pair(G, cx, cy, cz) : 0);
 }
 
 // x and y weights of a layout's passes.
 template <int LAYOUT>
-using AxisWeights = typename std::conditional<LAYOUT == kFourTaps, CRW<float>, CWD>::type;
+using AxisWeights = typename std::conditional<(LAYOUT >= kFourTaps), CRW<float>, CWD>::type;
 SRT_HD void axis_weights(float t, CRW<float>& c) { cr_weights_mixed(t, c); }
 SRT_HD void axis_weights(float t, CWD& c) { cr_weights_diff(t, c); }
 

@@ -1,4 +1,4 @@
-// Host build of the MIXED form on each field layout (planes, row pairs, cells;
+// Host build of the MIXED form on each field layout (planes, row pairs, cells, four taps;
 // snapshot-raytracer_gb300/csrc/srt_scheme.cuh, srt_adjoint.cuh) for
 // tests/test_layouts_host.py. Fields are halo-padded float arrays (extents
 // n + 3, voxel (i, j, k) at (i+1) + px ((j+1) + py (k+1))), in the order B_x,
@@ -10,7 +10,7 @@ namespace {
 
 struct Layouts {
   srt::Geom G;
-  srt::FieldPtrs F[3];  // by layout
+  srt::FieldPtrs F[6];  // by layout
   std::vector<float2> pair[4];
   std::vector<float4> cell[4];
   Layouts(const float* const* f, int n0, int n1, int n2) {
@@ -47,6 +47,8 @@ struct Layouts {
     }
     F[srt::kPlanes].phi = f[3];
     for (int c = 0; c < 3; ++c) F[srt::kPlanes].b[c] = f[c];
+    F[srt::kFourTaps] = F[srt::kFourPlanes] = F[srt::kPlanes];
+    F[srt::kFourPairs] = F[srt::kPairs];
   }
 };
 
@@ -81,6 +83,9 @@ void layout_maps(const float* const* f, int n0, int n1, int n2, long long nside,
   maps_of<srt::kPlanes>(Y, nside, count, n_steps, maps, flagged);
   maps_of<srt::kPairs>(Y, nside, count, n_steps, maps + 6 * count, flagged + count);
   maps_of<srt::kCells>(Y, nside, count, n_steps, maps + 12 * count, flagged + 2 * count);
+  maps_of<srt::kFourTaps>(Y, nside, count, n_steps, maps + 18 * count, flagged + 3 * count);
+  maps_of<srt::kFourPlanes>(Y, nside, count, n_steps, maps + 24 * count, flagged + 4 * count);
+  maps_of<srt::kFourPairs>(Y, nside, count, n_steps, maps + 30 * count, flagged + 5 * count);
 }
 
 // Cotangents of `count` rays' right-hand side at affine parameter s[r] and

@@ -1,6 +1,7 @@
 """The MIXED form on the three field layouts (planes, row pairs, cells), built
 for the host: the second differences a layout stores are the ones the others
-form on the spot, so maps, guard flags and state cotangents agree bit for bit;
+form on the spot, so maps, guard flags and state cotangents agree bit for bit,
+as do the four-tap passes from any of them with each other;
 and the tap cotangents scattered by cells (with the copies of the region around
 the observer) and gathered through the second differences' transpose equal the
 ones scattered tap by tap. Odd, non-cubic and very small grids, rays that wrap
@@ -48,13 +49,13 @@ def padded_fields(n, seed):
 def test_layouts_trace_alike(host, n, nside, steps):
     F, ptrs = padded_fields(n, 7)
     count = 12 * nside * nside
-    maps = np.zeros((3, count, 6), np.float32)
-    flags = np.zeros((3, count), np.int32)
+    maps = np.zeros((6, count, 6), np.float32)
+    flags = np.zeros((6, count), np.int32)
     host.layout_maps(ptrs, *n, nside, count, steps, maps.ctypes.data, flags.ctypes.data)
     assert np.all(np.isfinite(maps))
-    for k in (1, 2):
-        assert np.array_equal(maps[k].view(np.uint32), maps[0].view(np.uint32))
-        assert np.array_equal(flags[k], flags[0])
+    for k in (1, 2, 4, 5):  # 0-2 second differences, 3-5 four taps
+        assert np.array_equal(maps[k].view(np.uint32), maps[k // 3 * 3].view(np.uint32))
+        assert np.array_equal(flags[k], flags[k // 3 * 3])
 
 
 def diff2(a, ax):
