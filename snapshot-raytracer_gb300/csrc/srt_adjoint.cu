@@ -3,22 +3,25 @@
 // differentiated is its forward scheme, snapshot-raytracer.cu:315-583, as
 // restated in srt_scheme.cuh.
 //
-// Kernels (one thread per ray, rays in the forward's launch order):
-//   ray_count_kernel / ray_write_kernel  Morton-ordered list of the RING pixels
-//                                        of the requested range
-//   ckpt_kernel<MODE>      forward trace storing the state every C steps
-//                          (and the final state) in device memory
-//   reverse_kernel<MODE>   per segment, backwards: recompute the segment from
-//                          its checkpoint storing y_i, k1, k2, k3 per step;
-//                          then per step, backwards, the RK4 adjoint
-//                            a4 = J(u4)^T l/6, a3 = J(u3)^T (l/3 + a4),
-//                            a2 = J(u2)^T (l/3 + a3/2), a1 = J(u1)^T (l/6 + a2/2),
-//                            l <- l + a1 + a2 + a3 + a4,
-//                          scattering the tap cotangents into halo-padded
-//                          gradient grids (FP32 atomics, FP64 atomics, or
-//                          64-bit fixed point for SRT_DETERMINISTIC)
-//   fold_kernel            sums the halo copies of each voxel back onto the
-//                          periodic grid and writes the caller's layout
+// Kernels (rays in the forward's launch order):
+//   ray_count_, ray_scan_,  Morton-ordered list of the RING pixels of the
+//   ray_write_kernel        requested range
+//   ckpt_kernel             forward trace storing the state every C steps (and
+//                           the final state); of the last segments the tape too
+//   near_ckpt_kernel        the same for the rays that came near a cell face, by
+//                           the four-tap passes
+//   final_cotangent_kernel  cotangent of the final state from the map weights
+//   segment_kernel          per segment, backwards: recompute it from its
+//                           checkpoint, writing every stage's input (the tape)
+//   sweep_kernel            then its steps, backwards, by the RK4 adjoint,
+//                           scattering the tap cotangents into halo-padded
+//                           gradient grids (FP32 atomics on cells, or 64-bit
+//                           fixed point for SRT_DETERMINISTIC)
+//   reverse_kernel_fp64     both in one, FP64 (atomics, or fixed point)
+//   *_small_kernel          ranges of few rays, four lanes per ray
+//   merge_hot_kernel        adds the copies of the region around the observer
+//   fold_kernel             sums the halo copies of each voxel back onto the
+//                           periodic grid and writes the caller's layout
 #include <algorithm>
 #include <chrono>
 #include <cstring>
@@ -369,6 +372,127 @@ __global__ void __launch_bounds__(128, 2) near_segment_kernel(const AdjArgs A, i
   for_near_rays(A, (int64_t)gridDim.x * 4, [&](int64_t slot) { segment_ray(OneLane<kFourTaps>(), A, sgi, slot); });
 }
 
+// The four passes of a stage by one lane, FP32 accumulation: the interpolations,
+// and every second stage one scatter for two. In the backward order the stages come
+// in pairs (the midpoint stages of a step; a step's first stage and the last one of
+// the step before) whose positions differ by ~1e-4 cells or less, so their 16 cells
+// per field are the same unless a face lies between them, and adding their tap
+// cotangents before they go to memory halves the atomics, whose way to L2 the sweep
+// waited for with both gradients (61 % of its cycles). 256^3 / nside 128 / 128 steps:
+// 46.9 -> 41.6 ms; 512^3 / nside 256 / 256 steps: 359.7 -> 317 ms, phi only (the
+// backward half) 181 -> 171. The interpolations, with no scatter in them, are best
+// unrolled (rolled: 47.7 and 361 ms), the scatter in a loop over its slices
+// (unrolled: 43.4 and 329 ms, the code outgrows the instruction cache).
+template <int LAYOUT, bool BGRAD>
+struct DeferredPasses {
+  // a pending stage per thread: 10 cotangents per field, the offsets on the centred
+  // (and staggered) axes, the fields' cells (base, hot_base)
+  static constexpr int kFields = BGRAD ? 4 : 1, kQ = 0, kT = 10 * kFields, kBase = kT + (BGRAD ? 6 : 3),
+                       kHot = kBase + 2 * kFields, kWords = kHot + kFields;
+  const FieldPtrs& F;
+  const Geom& G;
+  AccF32 acc[4];
+  float (*pend)[128];
+  bool second = false, pending = false;
+
+  __device__ float& word(int w) const { return pend[w][threadIdx.x]; }
+  template <int f>
+  __device__ void load_pending(float* t, float* q, int64_t* base, int* hbase) const {
+    constexpr int k = BGRAD ? f : 0;
+    for (int i = 0; i < 10; ++i) q[i] = word(kQ + 10 * k + i);
+    for (int i = 0; i < 3; ++i) t[i] = word(kT + i + (i == f ? 3 : 0));
+    *base = (int64_t)(((unsigned long long)__float_as_uint(word(kBase + 2 * k + 1)) << 32) |
+                      __float_as_uint(word(kBase + 2 * k)));
+    *hbase = __float_as_int(word(kHot + k));
+  }
+  template <int f>
+  __device__ void deposit(const StageView<float>& V, const float* qb) const {
+    constexpr int k = BGRAD ? f : 0;
+    if (BGRAD && f == 3 && !second)  // phi's axes serve the B components too
+      for (int i = 0; i < 3; ++i) word(kT + i) = V.t[3][i];
+    if (!acc[f].active()) return;
+    if (!second) {
+      for (int i = 0; i < 10; ++i) word(kQ + 10 * k + i) = qb[i];
+      if (f != 3)
+        word(kT + 3 + f) = V.t[f][f];
+      else if (!BGRAD)
+        for (int i = 0; i < 3; ++i) word(kT + i) = V.t[3][i];
+      word(kBase + 2 * k) = __uint_as_float((unsigned)V.base[f]);
+      word(kBase + 2 * k + 1) = __uint_as_float((unsigned)((unsigned long long)V.base[f] >> 32));
+      word(kHot + k) = __int_as_float(V.hbase[f]);
+      return;
+    }
+    float ta[3], tb[3], qa[10], q[10];
+    int64_t base = V.base[f], base_a = base;
+    int hbase = V.hbase[f], hbase_a = hbase;
+    for (int i = 0; i < 10; ++i) q[i] = qb[i];
+    for (int i = 0; i < 3; ++i) tb[i] = ta[i] = V.t[f][i];
+    if (pending)
+      load_pending<f>(ta, qa, &base_a, &hbase_a);
+    else
+      for (int i = 0; i < 10; ++i) qa[i] = 0.f;
+    // the pending stage with this one where their cells agree, else (rarely) in a
+    // round of its own
+    bool same = base_a == base;
+    float qs[10];
+    for (int i = 0; i < 10; ++i) qs[i] = same ? qa[i] : 0.f;
+#pragma unroll 1
+    for (;;) {
+      scatter_two(acc[f], base, hbase, G, ta, qs, tb, q);
+      if (!__any_sync(0xffffffffu, !same)) break;
+      for (int i = 0; i < 10; ++i) {
+        q[i] = 0.f;
+        qs[i] = same ? 0.f : qa[i];
+      }
+      base = base_a;
+      hbase = hbase_a;
+      same = true;
+    }
+  }
+  // The last pending stage of a segment.
+  template <int f>
+  __device__ void flush_field() const {
+    if (!acc[f].active()) return;
+    float t[3], q[10], none[10];
+    int64_t base;
+    int hbase;
+    load_pending<f>(t, q, &base, &hbase);
+    for (int i = 0; i < 10; ++i) none[i] = 0.f;
+    scatter_two(acc[f], base, hbase, G, t, q, t, none);
+  }
+  __device__ void flush() const {
+    if constexpr (BGRAD) {
+      flush_field<0>();
+      flush_field<1>();
+      flush_field<2>();
+    }
+    flush_field<3>();
+  }
+  template <int C>
+  __device__ void component(const StageView<float>& V, const float* fb, BVjp<float>& B, float* nb, float* xb) const {
+    float qb[10];
+    b_cotangent<C>(V, fb, B, qb);
+    Tri<float> Q;
+    field_pass<LAYOUT, 4, float, AccNone>(F, C, V, G, qb, Q, xb, AccNone());
+    if constexpr (BGRAD) deposit<C>(V, qb);
+    b_fold<C>(V, Q, B, nb);
+  }
+  __device__ void operator()(const StageView<float>& V, const float* fb, const PhiVjp<float>& p, BVjp<float>& B,
+                             float* nb, float* xb, Tri<float>& P) const {
+    component<0>(V, fb, B, nb, xb);
+    component<1>(V, fb, B, nb, xb);
+    component<2>(V, fb, B, nb, xb);
+    float qb[10];
+    phi_cotangent(V, p, qb);
+    field_pass<LAYOUT, 4, float, AccNone>(F, 3, V, G, qb, P, xb, AccNone());
+    deposit<3>(V, qb);
+  }
+};
+template <typename P>
+struct IsDeferred : std::false_type {};
+template <int LAYOUT, bool BGRAD>
+struct IsDeferred<DeferredPasses<LAYOUT, BGRAD>> : std::true_type {};
+
 // Backward sweep over segment sgi: per step, backwards, the RK4 adjoint
 //   a4 = J(u4)^T l/6, a3 = J(u3)^T (l/3 + a4), a2 = J(u2)^T (l/3 + a3/2),
 //   a1 = J(u1)^T (l/6 + a2/2), l <- l + a1 + a2 + a3 + a4,
@@ -379,7 +503,7 @@ __global__ void __launch_bounds__(128, 2) near_segment_kernel(const AdjArgs A, i
 // live: this lane's ray counts; store: it writes the cotangent back.
 template <int THREADS, typename Passes>
 __device__ __forceinline__ void sweep_segment(const AdjArgs& A, int sgi, int64_t slot, bool live, bool store,
-                                              const MixedRay& R, const float* x0, float* lam, const Passes& passes,
+                                              const MixedRay& R, const float* x0, float* lam, Passes passes,
                                               float (*s_lam)[THREADS], float (*s_tot)[THREADS]) {
   const int t = threadIdx.x;
   for (int j = 0; j < 19; ++j) s_lam[j][t] = live ? lam[(int64_t)j * A.count + slot] : 0.f;
@@ -406,12 +530,15 @@ __device__ __forceinline__ void sweep_segment(const AdjArgs& A, int sgi, int64_t
       for (int j = 0; j < 19; ++j) u[j] = ld_stream(tape + ((int64_t)(qn >> 2) * kTapeStep + 19 * (qn & 3) + j) * A.count);
     }
     for (int j = 0; j < 19; ++j) an[j] = 0.f;
+    if constexpr (IsDeferred<Passes>::value) passes.second = (q & 1) != 0;
     rhs_vjp_with(V, fb, an, passes);
+    if constexpr (IsDeferred<Passes>::value) passes.pending = (q & 1) == 0;
     // the step's running sum of the a's restarts at its last stage
     for (int j = 0; j < 19; ++j) s_tot[j][t] = (stage == 3 ? 0.f : s_tot[j][t]) + an[j];
     if (stage == 0)
       for (int j = 0; j < 19; ++j) s_lam[j][t] += s_tot[j][t];
   }
+  if constexpr (IsDeferred<Passes>::value) passes.flush();
   if (store)
     for (int j = 0; j < 19; ++j) lam[(int64_t)j * A.count + slot] = s_lam[j][t];
 }
@@ -454,6 +581,12 @@ __global__ void __launch_bounds__(128, SRT_SWEEP_MIN_BLOCKS)
   float x0[3];
   load_bases(A, slot, R);
   mixed_observer(A.G, x0);
+  if constexpr (TakesCells<Acc>::value) {
+    typedef DeferredPasses<LAYOUT, BGRAD> Passes;
+    __shared__ float pend[Passes::kWords][128];
+    sweep_segment<128>(A, sgi, slot, live, live, R, x0, lam, Passes{A.F, A.G, {a0, a1, a2, a3}, pend}, s_lam, s_tot);
+    return;
+  }
   sweep_segment<128>(A, sgi, slot, live, live, R, x0, lam, OneLanePasses<LAYOUT, float, AccB, Acc>{A.F, A.G, accb, a3},
                      s_lam, s_tot);
 }

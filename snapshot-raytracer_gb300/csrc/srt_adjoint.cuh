@@ -310,6 +310,22 @@ SRT_HD void tricubic_vjp(const float* __restrict__ f, int64_t base, int64_t px, 
            qb[6] * o102 + qb[7] * o021 + qb[8] * o012 + qb[9] * o003;
 }
 
+// Per order in x (w: value, g: first, h: second), the cotangents of a slice's row
+// values and of their second differences along y at rows 1 and 2: (value,
+// difference) pairs per row, for the slice's z weights.
+struct SliceCotangents {
+  float2 w[2], g[2], h[2];
+};
+SRT_HD SliceCotangents slice_cotangents(const float* qb, const CWD& Y, float zw, float zg, float zh) {
+  const float a0 = fmaf(qb[0], zw, fmaf(qb[3], zg, qb[9] * zh)), a1 = fmaf(qb[2], zw, qb[8] * zg), a2 = qb[7] * zw;
+  const float b0 = fmaf(qb[1], zw, qb[6] * zg), b1 = qb[5] * zw, c0 = qb[4] * zw;
+  const float w2 = fmaf(Y.t, a0, a1), g2 = fmaf(Y.t, b0, b1), h2 = Y.t * c0;
+  return SliceCotangents{{make_float2(a0 - w2, fmaf(Y.w0, a0, fmaf(Y.g0, a1, Y.h0 * a2))),
+                          make_float2(w2, fmaf(Y.w3, a0, fmaf(Y.g3, a1, Y.h3 * a2)))},
+                         {make_float2(b0 - g2, fmaf(Y.w0, b0, Y.g0 * b1)), make_float2(g2, fmaf(Y.w3, b0, Y.g3 * b1))},
+                         {make_float2(c0 - h2, Y.w0 * c0), make_float2(h2, Y.w3 * c0)}};
+}
+
 // The same pass for the MIXED form, in FP32 on the second-difference form of
 // the cubic (CWD): the x pass on packed pairs as in tricubic_mixed, with its
 // third derivative (one packed subtraction a row), the y pass on scalars, the
@@ -383,16 +399,8 @@ SRT_HD void tricubic_vjp_mixed(const Src& src, int64_t base, int hbase, const Ge
     o102 = fmaf(zh, s10, o102);
     o003 = fmaf(zk, s00, o003);
     if (scatter) {
-      // per order in x, the cotangents of the row's value and second difference
-      // along y at rows 1 and 2: (value, difference) pairs per row
-      const float a0 = fmaf(qb[0], zw, fmaf(qb[3], zg, qb[9] * zh)), a1 = fmaf(qb[2], zw, qb[8] * zg), a2 = qb[7] * zw;
-      const float b0 = fmaf(qb[1], zw, qb[6] * zg), b1 = qb[5] * zw, c0 = qb[4] * zw;
-      const float w2 = fmaf(Y.t, a0, a1), g2 = fmaf(Y.t, b0, b1), h2 = Y.t * c0;
-      const float2 Cw[2] = {make_float2(a0 - w2, fmaf(Y.w0, a0, fmaf(Y.g0, a1, Y.h0 * a2))),
-                            make_float2(w2, fmaf(Y.w3, a0, fmaf(Y.g3, a1, Y.h3 * a2)))};
-      const float2 Cg[2] = {make_float2(b0 - g2, fmaf(Y.w0, b0, Y.g0 * b1)),
-                            make_float2(g2, fmaf(Y.w3, b0, Y.g3 * b1))};
-      const float2 Ch[2] = {make_float2(c0 - h2, Y.w0 * c0), make_float2(h2, Y.w3 * c0)};
+      const SliceCotangents sc = slice_cotangents(qb, Y, zw, zg, zh);
+      const float2 *Cw = sc.w, *Cg = sc.g, *Ch = sc.h;
       if constexpr (TakesCells<Acc>::value) {
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
@@ -457,6 +465,53 @@ SRT_HD void tricubic_vjp_mixed(const Src& src, int64_t base, int hbase, const Ge
            qb[7] * o030 + qb[8] * G2.x + qb[9] * H0.y;
   xb[2] += qb[0] * G0.x + qb[1] * G1.x + qb[2] * G0.y + qb[3] * H0.x + qb[4] * G2.y + qb[5] * G1.y + qb[6] * o102 +
            qb[7] * G2.x + qb[8] * H0.y + qb[9] * o003;
+}
+
+// The scatter of two stages whose footprints are the same cell (AccF32): the tap
+// cotangents of (ta, qa) and (tb, qb) are added before they go to memory.
+struct ScatterWeights {
+  float2 t, ow, og, oh, nw, ng, nh;  // x: difference weights of this lane's cell of a pair and the other
+  CWD y;
+  CRW<float> z;
+  SRT_HD ScatterWeights(const float* tt, int me) {
+    CWD X;
+    cr_weights_diff(tt[0], X);
+    cr_weights_diff(tt[1], y);
+    cr_weights_mixed(tt[2], z);
+    t = dup2(X.t);
+    ow = dup2(me ? X.w3 : X.w0), og = dup2(me ? X.g3 : X.g0), oh = dup2(me ? X.h3 : X.h0);
+    nw = dup2(me ? X.w0 : X.w3), ng = dup2(me ? X.g0 : X.g3), nh = dup2(me ? X.h0 : X.h3);
+  }
+};
+SRT_HD float of_slice(const float* w, int c) { return c == 0 ? w[0] : (c == 1 ? w[1] : (c == 2 ? w[2] : w[3])); }
+SRT_HD void scatter_two(const AccF32& acc, int64_t base, int hbase, const Geom& G, const float* ta, const float* qa,
+                        const float* tb, const float* qb) {
+  AccF32::Place at = acc.place(base, hbase, G);
+  const int me = AccF32::lane();
+  const ScatterWeights a(ta, me), b(tb, me);
+#pragma unroll 1
+  for (int c = 0; c < 4; ++c) {
+    const SliceCotangents ca =
+        slice_cotangents(qa, a.y, of_slice(a.z.w, c), of_slice(a.z.g, c), of_slice(a.z.h, c));
+    const SliceCotangents cb =
+        slice_cotangents(qb, b.y, of_slice(b.z.w, c), of_slice(b.z.g, c), of_slice(b.z.h, c));
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float2 p2 = ffma2(a.t, ca.w[j], fadd2(ca.g[j], ffma2(b.t, cb.w[j], cb.g[j])));
+      const float2 p1 = fsub2(fadd2(ca.w[j], cb.w[j]), p2);
+      const float2 po = me ? p2 : p1, pn = me ? p1 : p2;
+      const float2 eo =
+          ffma2(a.ow, ca.w[j], ffma2(a.og, ca.g[j], ffma2(a.oh, ca.h[j],
+          ffma2(b.ow, cb.w[j], ffma2(b.og, cb.g[j], fmul2(b.oh, cb.h[j]))))));
+      const float2 en =
+          ffma2(a.nw, ca.w[j], ffma2(a.ng, ca.g[j], ffma2(a.nh, ca.h[j],
+          ffma2(b.nw, cb.w[j], ffma2(b.ng, cb.g[j], fmul2(b.nh, cb.h[j]))))));
+      acc.add_row2(at.even + j * at.px, at.odd + j * at.px, make_float4(po.x, po.y, eo.x, eo.y),
+                   make_float4(pn.x, pn.y, en.x, en.y));
+    }
+    at.even += at.pxy;
+    at.odd += at.pxy;
+  }
 }
 
 // -------------------------------------------------------- stage and core
@@ -572,9 +627,9 @@ SRT_HD void phi_cotangent(const StageView<T>& V, const PhiVjp<T>& p, T* qb) {
 
 // The four fused passes of a stage by one lane: the B sums and nb, the position
 // cotangent xb and phi's interpolation P. The slice loops are unrolled where only
-// phi's scatter follows them (512^3 / nside 256 / 256 steps, backward half: 183
-// ms in loops, 181 unrolled), loops with four scatters, where the code outgrows
-// the instruction cache (256^3 / nside 128 / 128 steps: 49.6 ms against 50.8).
+// phi's scatter follows them, loops with four scatters, where the code outgrows
+// the instruction cache (SRT_DETERMINISTIC's sweep; the FP32 one scatters apart
+// from the interpolations).
 template <int LAYOUT, typename T, typename AccB, typename AccP>
 struct OneLanePasses {
   const FieldPtrs& F;

@@ -130,5 +130,22 @@ void layout_vjp(const float* const* f, int n0, int n1, int n2, int count, const 
     }
 }
 
+// The scatter of two stages in one cell (padded index base) at offsets ta, tb with
+// cotangents qa, qb, into cells[padded x 4]; and the same by the two stages' own
+// passes over field f, into apart[padded x 4].
+void scatter_pair(const float* f, int n0, int n1, int n2, long long base, const float* ta, const float* qa,
+                  const float* tb, const float* qb, float* cells, float* apart) {
+  const float* const four[4] = {f, f, f, f};
+  const Layouts Y(four, n0, n1, n2);
+  srt::AccF32 two{(float4*)cells}, one{(float4*)apart};
+  srt::scatter_two(two, base, -1, Y.G, ta, qa, tb, qb);
+  for (int k = 0; k < 2; ++k) {
+    srt::Tri<float> Q;
+    float xb[3] = {0, 0, 0};
+    srt::tricubic_vjp_mixed<1, srt::AccF32>(srt::cell_source<srt::kPlanes>(Y.F[srt::kPlanes], Y.G, 0, base, 0), base, -1,
+                                            Y.G, k ? tb : ta, k ? qb : qa, Q, xb, one);
+  }
+}
+
 int hot_side() { return srt::kHotSide; }
 }

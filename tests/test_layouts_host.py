@@ -33,6 +33,7 @@ def host(tmp_path_factory):
     L = ctypes.CDLL(out)
     P, I, Q = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
     L.layout_maps.argtypes = [P, I, I, I, Q, Q, I, P, P]
+    L.scatter_pair.argtypes = [P, I, I, I, Q] + [P] * 6
     L.layout_vjp.argtypes = [P, I, I, I, I] + [P] * 9 + [I]
     return L
 
@@ -93,3 +94,22 @@ def test_cell_scatter_equals_tap_scatter(host, n, hot):
     for c in range(4):
         scale = np.abs(rows[c]).max()
         assert scale > 0 and np.abs(got[c] - rows[c]).max() <= 1e-5 * scale, c
+
+
+@pytest.mark.parametrize("t", [(0.0, 0.0, 0.0), (0.25, 0.5, 0.875), (0.999999, 0.0, 0.5)])
+def test_two_stages_scatter_as_one(host, t):
+    """Two stages' cotangents added before they go to the cells: FP32 roundings of
+    the same products, a few ulps of the largest (16 terms: 1e-6)."""
+    n = (7, 6, 5)
+    F, _ = padded_fields(n, 11)
+    rng = np.random.default_rng(8)
+    shape = (n[2] + 3, n[1] + 3, n[0] + 3, 4)
+    for cell in ((0, 0, 0), (6, 5, 4), (3, 2, 1)):
+        base = cell[0] + (n[0] + 3) * (cell[1] + (n[1] + 3) * cell[2])
+        ta = np.array(t, np.float32)
+        tb = np.clip(ta + np.float32(1e-5), 0, np.float32(1 - 2.0 ** -24)).astype(np.float32)
+        qa, qb = rng.standard_normal((2, 10)).astype(np.float32)
+        two, one = np.zeros(shape, np.float32), np.zeros(shape, np.float32)
+        host.scatter_pair(F[0].ctypes.data, *n, base, *(a.ctypes.data for a in (ta, qa, tb, qb, two, one)))
+        assert np.count_nonzero(one) > 0
+        assert np.abs(two - one).max() <= 1e-6 * np.abs(one).max()
