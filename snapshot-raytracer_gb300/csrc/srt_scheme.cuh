@@ -629,6 +629,12 @@ SRT_HD R fma_r(const R& a, const R& b, const R& c) {
   return s.value();
 }
 
+// y + c k of the RK4 state: one fused operation in FP64, the double-word sum of
+// the rounded product in dd (a chain's compensation would carry the product's and
+// the sum's errors at the size of y's low word).
+SRT_HD double axpy_r(double c, double k, double y) { return fma(c, k, y); }
+SRT_HD dd axpy_r(const dd& c, const dd& k, const dd& y) { return y + c * k; }
+
 SRT_HD double sqrt_r(double x) { return sqrt(x); }
 SRT_HD dd sqrt_r(const dd& x) { return dd_sqrt(x); }
 

@@ -245,7 +245,7 @@ struct WideLane {
 
   // stage input y + c k
   SRT_HD void stage(R* S, int st) {
-    if (lane < 19) S[kWsY + lane] = st == 0 ? y : fma_r(R(st == 3 ? 1.f : 0.5f), k, y);
+    if (lane < 19) S[kWsY + lane] = st == 0 ? y : axpy_r(R(st == 3 ? 1.f : 0.5f), k, y);
   }
 
   // one axis of the centred (lanes 0-2) or staggered grid (3-5)
@@ -407,9 +407,9 @@ struct WideLane {
     if (st == 0)
       acc = k;
     else if (st < 3)
-      acc = fma_r(R(2.f), k, acc);
+      acc = axpy_r(R(2.f), k, acc);
     else
-      y = fma_r(acc + k, R(1.0 / 6.0), y);
+      y = axpy_r(acc + k, R(1.0 / 6.0), y);
   }
 };
 
