@@ -225,8 +225,9 @@ int srt_debug_fail_alloc(int64_t after);
  * the FP32 trajectory's error bound, 4e-7 (s max|dn| + 1e-3) grid units at
  * affine distance s, where the FP32 and FP64 trajectories could pick different cells (the
  * Catmull-Rom Hessian jumps across faces); those rays then equal the FP64
- * result bit for bit, or, in calls with more than four of them per SM, to a
- * float ulp (SRT_MIXED_NO_REFINE skips this). The CLI's batch b is
+ * result bit for bit, or, in calls with more than 64 of them per SM, to four
+ * float ulps (a ray within ~1e-12 grid units of a face may still take the other
+ * cell there; SRT_MIXED_NO_REFINE skips the re-trace). The CLI's batch b is
  * pix_begin = b*nside^2, pix_count = nside^2 (snapshot-raytracer.cu:708-717);
  * all pixels is pix_begin = 0, pix_count = 12*nside^2. With SRT_NESTED_RANGE
  * the range counts NESTED pixels instead (HEALPix base pixel b, the batch the

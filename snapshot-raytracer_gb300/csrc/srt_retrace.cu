@@ -172,24 +172,37 @@ cudaError_t sm_count(int* sms) {
   return e == cudaSuccess ? cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) : e;
 }
 
-// Lists of up to dd_min rays (four per SM) are re-traced in FP64 with the one-lane
-// FP64 form's operations (bit-identical maps), longer ones in double-float
-// arithmetic on the FP32 pipes (maps within one float ulp; 2.4e3 rays x 256 steps
-// 3.9 ms against 15.6 in FP64). The environment variable SRT_REFINE_DD_MIN
-// overrides dd_min (tests use it to reach both on small skies).
+// Lists of up to 64 rays per SM are re-traced in FP64 with the one-lane FP64 form's
+// operations (bit-identical maps): by five warps per ray up to kBlockRaysPerSM rays
+// per SM, where a stage's latency counts, by one warp per ray above, where the FP64
+// unit's rate does. Longer lists run in double-float arithmetic on the FP32 pipes:
+// maps within four float ulps of FP64 (tested), but for a ray within ~1e-12 cells of
+// a face, which may take the other cell. Double-float is the faster from four rays
+// per SM on already (256^3, 1024 steps: 2,813 rays 85 ms in FP64, 24.5 in
+// double-float; 7,850 rays 212 and 56.6), so the line costs time: up to it a sky and
+// the same sky in batches, whose lists are shorter, have the same bits. The
+// environment variable SRT_REFINE_DD_MIN overrides dd_min (tests use it to reach
+// both on small skies).
+constexpr int kFp64ListRaysPerSM = 64;
+
 cudaError_t launch_refine(const TraceArgs& a, cudaStream_t s, int64_t* kernels) {
   int sms = 0;
   cudaError_t e = sm_count(&sms);
   if (e != cudaSuccess) return e;
-  int64_t dd_min = kBlockRaysPerSM * (int64_t)sms;
-  if (const char* v = getenv("SRT_REFINE_DD_MIN")) dd_min = strtoll(v, nullptr, 10);
+  int64_t dd_min = kFp64ListRaysPerSM * (int64_t)sms;
+  if (const char* v = getenv("SRT_REFINE_DD_MIN")) dd_min = std::max(0LL, strtoll(v, nullptr, 10));
   if (a.pix_count < 1) return cudaSuccess;
+  const int64_t block_max = std::min(dd_min, kBlockRaysPerSM * (int64_t)sms);
   const int64_t blocks = std::min(a.pix_count, kBlockRaysPerSM * (int64_t)sms);
   const int64_t warps = std::min(a.pix_count, kWideBlocksPerSM * (int64_t)sms);
-  block_kernel<true><<<(unsigned)blocks, kBlockThreads, 0, s>>>(a, 1, dd_min);
+  block_kernel<true><<<(unsigned)blocks, kBlockThreads, 0, s>>>(a, 1, block_max);
   if (kernels) ++*kernels;
+  if (a.pix_count > block_max && dd_min > block_max) {
+    wide_kernel<double, true><<<(unsigned)warps, 32, 0, s>>>(a, block_max + 1, dd_min);
+    if (kernels) ++*kernels;
+  }
   if (a.pix_count > dd_min) {
-    wide_kernel<dd, true><<<(unsigned)warps, 32, 0, s>>>(a, std::max<int64_t>(dd_min, 0) + 1, a.pix_count);
+    wide_kernel<dd, true><<<(unsigned)warps, 32, 0, s>>>(a, dd_min + 1, a.pix_count);
     if (kernels) ++*kernels;
   }
   return cudaGetLastError();
