@@ -1182,15 +1182,19 @@ struct OneLane {
 // (delta components in the layout of rhs_std), x0 the observer.
 // Cell-face guard. Catmull-Rom's Hessian jumps across cell faces, so where
 // the FP32 and FP64 trajectories pass a face on different sides the maps of
-// that ray differ by up to ~1% of their rms. The FP32 trajectory's distance
-// from the FP64 one was measured on the GPU, stage by stage (a lockstep
-// FP64 / MIXED kernel: 256^3 / 256 steps / 49k rays, 512^3 / 512 steps / 49k
-// rays, 1024^3 / 1024 steps / 12k rays) against candidate bounds; the one that
-// holds with the smallest margin is s Mn, the affine distance times the
-// running maximum Mn = max |dn| of the direction perturbation:
-// |x32 - x64| <= k (s Mn + 1e-3) with k below 1.6e-7 for 99% of the rays and
-// below 3.3e-7 for all, at every length (a bound that also carries
-// Mx = max |dx| needed k up to 5.5e-7 at 1024 steps and flags 2-3x more rays).
+// that ray differ by up to ~1% of their rms. The FP32 trajectory's distance from
+// the FP64 one was measured on the GPU, stage by stage (a lockstep FP64 / MIXED
+// kernel, each of the MIXED passes: 256^3 / 256 steps and 512^3 / 512 steps, eight
+// skies of 49k rays, 1024^3 / 1024 steps, 12k rays, and 512 steps, 49k), against
+// candidate bounds; the one that holds with the smallest margin is s Mn, the affine
+// distance times the running maximum Mn = max |dn| of the direction perturbation:
+// |x32 - x64| <= k (s Mn + 1e-3). By second differences k is below 2.1e-7 for 99% of
+// the rays and 2.9e-7 for 99.9% of every sky, by the four taps below 2.2e-7 and
+// 3.0e-7 (medians 0.7 to 0.9e-7, the former the lower throughout); 12 and 6 of 450k
+// rays have a stage above 4e-7 (at most 5.0e-7 and 4.7e-7). Such a stage goes
+// unflagged where a face lies in the ~1e-8 grid units between: ~1e-10 per ray.
+// Fields ten times stronger: 99.9% below 3.9e-7 by either. (A bound that also carries
+// Mx = max |dx| flags 2-3x more rays.)
 // A stage whose position lies within g = kFaceGuardRel (s Mn + kFaceGuardFloor)
 // of a cell face (either face, centred or staggered grid) marks the ray for
 // an FP64 re-trace.
