@@ -935,10 +935,16 @@ using namespace srt;
 
 namespace {
 
-struct DevBuf {  // scratch, given back on the stream it was taken on
+// Scratch, given back on the stream it was taken on: by release() before a call's
+// last wait, with the handle's device current (a NULL stream is that device's).
+struct DevBuf {
   void* p = nullptr;
   cudaStream_t s = nullptr;
-  ~DevBuf() { pool_free(p, s); }
+  ~DevBuf() { release(); }
+  void release() {
+    pool_free(p, s);
+    p = nullptr;
+  }
   cudaError_t alloc(size_t bytes, cudaStream_t stream) {
     s = stream;
     return scratch_alloc(&p, bytes, stream);
@@ -1074,6 +1080,11 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
   cudaGetDevice(&prev);
   if (prev != f->device) cudaSetDevice(f->device);
   DevBuf counts, offsets, rays, near, bases, wdev, ckpt, seg, lam, gacc[4], gout_phi, gout_b, ovf;
+  const auto release = [&] {
+    for (DevBuf* b : {&counts, &offsets, &rays, &near, &bases, &wdev, &ckpt, &seg, &lam, &gacc[0], &gacc[1], &gacc[2],
+                      &gacc[3], &gout_phi, &gout_b, &ovf})
+      b->release();
+  };
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   int64_t kernels = 0, h2d = 0, d2h = 0;
   {
@@ -1268,14 +1279,13 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
     unsigned flag = 0;
     if (ovf.p)
       VJP_TRY(cudaMemcpyAsync(&flag, ovf.p, sizeof(flag), cudaMemcpyDeviceToHost, s), "read overflow flag");
+    release();
     VJP_TRY(cudaStreamSynchronize(s), "srt_vjp");
-    if (ovf.p) {
-      if (flag) {
-        rc = set_error(SRT_ERR_OVERFLOW,
-                       "srt_vjp: SRT_DETERMINISTIC gradient beyond the fixed-point range (|gradient| >= 2^30 per "
-                       "voxel, or not finite); the gradients are not valid (use the FP32/FP64 accumulation)");
-        goto done;
-      }
+    if (flag) {
+      rc = set_error(SRT_ERR_OVERFLOW,
+                     "srt_vjp: SRT_DETERMINISTIC gradient beyond the fixed-point range (|gradient| >= 2^30 per "
+                     "voxel, or not finite); the gradients are not valid (use the FP32/FP64 accumulation)");
+      goto done;
     }
     if (stats) {
       float ms = -1.f;
@@ -1289,7 +1299,9 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
     }
   }
 done:
+  release();
   if (rc != SRT_OK) cudaStreamSynchronize(s);  // copies from or to the caller's buffers may be under way
+  scratch_settle(f->device, s);
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   if (prev != f->device) cudaSetDevice(prev);
@@ -1332,6 +1344,9 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
   if (prev != f->device) cudaSetDevice(f->device);
   srt_tape* t = new (std::nothrow) srt_tape();
   DevBuf counts, offsets, rays, near, bases, ckpt, dmaps, rlist, rcount;
+  const auto release = [&] {  // all but what the tape takes over
+    for (DevBuf* b : {&counts, &offsets, &dmaps, &rlist, &rcount}) b->release();
+  };
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   int64_t kernels = 0;
   if (!t) {
@@ -1401,6 +1416,7 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
                 "copy maps to host");
     unsigned long long refined = 0;
     VJP_TRY(cudaMemcpyAsync(&refined, rcount.p, sizeof(refined), cudaMemcpyDeviceToHost, s), "read refine count");
+    release();
     VJP_TRY(cudaStreamSynchronize(s), "srt_forward_tape");
     if (stats) {
       float ms = -1.f;
@@ -1433,7 +1449,10 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
     t = nullptr;
   }
 done:
+  release();
+  for (DevBuf* b : {&rays, &near, &bases, &ckpt}) b->release();  // of a failed call
   if (rc != SRT_OK) cudaStreamSynchronize(s);
+  scratch_settle(f->device, s);
   delete t;
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
@@ -1460,6 +1479,7 @@ extern "C" int srt_tape_destroy(srt_tape* tape) {
   if (prev != tape->device) cudaSetDevice(tape->device);
   // the calls that used the tape have returned, and they are synchronous
   for (void* p : {(void*)tape->rays, (void*)tape->near, (void*)tape->bases, (void*)tape->ckpt}) pool_free(p, nullptr);
+  scratch_settle(tape->device, nullptr);
   if (prev != tape->device) cudaSetDevice(prev);
   delete tape;
   return SRT_OK;

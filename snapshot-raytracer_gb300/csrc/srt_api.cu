@@ -25,7 +25,10 @@ thread_local std::string g_last_error;
 // Scratch (a call's lists, checkpoints, tapes and accumulators) comes from a
 // second pool that keeps at most kScratchKeep of what is handed back: a cudaMalloc
 // / cudaFree pair per buffer cost a 60x52x68 gradient 0.7 of its 2.5 ms, and the
-// default pool's mapping after each synchronisation a small forward ~20 us.
+// default pool's mapping after each synchronisation a small forward ~20 us. A pool
+// gives memory back at a synchronisation that finds it unused, so the calls hand
+// their scratch back before their last one, and scratch_settle after it returns
+// what is left above the bound.
 constexpr int kMaxPoolDevices = 64;
 constexpr uint64_t kScratchKeep = 8ull << 30;
 enum { kFieldPool = 0, kScratchPool = 1 };
@@ -108,6 +111,20 @@ cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
 
 void pool_free(void* p, cudaStream_t s) {
   if (p) cudaFreeAsync(p, s);
+}
+
+void scratch_settle(int dev, cudaStream_t s) {
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (dev >= 0 && dev < kMaxPoolDevices) pool = g_pool[kScratchPool][dev];
+  }
+  uint64_t reserved = 0;
+  if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+      reserved <= kScratchKeep)
+    return;
+  cudaStreamSynchronize(s);
+  cudaMemPoolTrimTo(pool, kScratchKeep);
 }
 
 // Bytes the device's pools hold but do not use (reusable by pool_alloc, which
@@ -597,7 +614,15 @@ int srt_forward(const srt_fields* fields, int64_t nside, int64_t pix_begin, int6
     unsigned long long refined = 0;
     if (refine && timed && stats)
       SRT_CUDA_TRY(cudaMemcpyAsync(&refined, refine_count, sizeof(refined), cudaMemcpyDeviceToHost, s), "read refine count");
-    if (timed || !dev_out) SRT_CUDA_TRY(cudaStreamSynchronize(s), "trace");
+    // stream-ordered: after the last kernel and copy that use them (SRT_ASYNC)
+    for (void* p : {(void*)dmaps, (void*)refine_list, (void*)refine_count}) pool_free(p, s);
+    dmaps = nullptr;
+    refine_list = nullptr;
+    refine_count = nullptr;
+    if (timed || !dev_out) {
+      SRT_CUDA_TRY(cudaStreamSynchronize(s), "trace");
+      scratch_settle(f->device, s);
+    }
     if (stats) {
       float ms = -1.f, rms = 0.f;
       if (timed) {
@@ -615,7 +640,6 @@ int srt_forward(const srt_fields* fields, int64_t nside, int64_t pix_begin, int6
   }
 fail:
   pool_free(dmaps, s);
-  // stream-ordered release: the refine kernel may still be queued (SRT_ASYNC)
   pool_free(refine_list, s);
   pool_free(refine_count, s);
   if (e0) cudaEventDestroy(e0);

@@ -50,6 +50,9 @@ int64_t pool_reusable_bytes(int dev);
 // pool_free on the stream of its last use. Both allocations go through the
 // failure-injection hook (srt_debug_fail_alloc).
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+// Returns to the device what the scratch pool of `dev` holds unused above its bound
+// (waits for s, where the scratch was given back, only if it holds more).
+void scratch_settle(int dev, cudaStream_t s);
 
 // NVTX range over a scope (the public entry points and their phases), for
 // profilers' timelines and range filters; header-only, inert unless a tool
