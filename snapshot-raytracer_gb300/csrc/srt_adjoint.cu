@@ -162,12 +162,26 @@ constexpr int64_t kNearBit = int64_t(1) << 62;
 __device__ __forceinline__ int64_t ring_of(const AdjArgs& A, int64_t slot) { return A.rays[slot] & ~kNearBit; }
 __device__ __forceinline__ bool is_near(const AdjArgs& A, int64_t slot) { return (A.rays[slot] & kNearBit) != 0; }
 
-// f(slot) for each marked ray of `warps` warps' list, all 32 lanes of a warp
-// together.
+// f(slot, together) for each marked ray, by blocks 0 .. blocks - 1 of four warps: up
+// to kNearPerWarp rays per warp of the first warp_blocks by a warp each (together: all
+// 32 lanes hold the ray; 12 us a step), longer lists by a lane each in all blocks (~40
+// us a step, 32 rays at a time). A warp per ray whatever the list made the gradient of
+// strong fields slower than one without this pass: 256^3 / nside 128 / 128 steps, C =
+// 12, 669 / 1,881 / 6,024 rays marked of 196,608: 46.6 / 59.6 / 99.2 ms, now 43.9 /
+// 49.6 / 57.4, and 41.4 with 8.
+constexpr int kNearPerWarp = 2;
+
 template <typename Fn>
-__device__ __forceinline__ void for_near_rays(const AdjArgs& A, int64_t warps, const Fn& f) {
-  const int64_t n = A.near[0];
-  for (int64_t i = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5); i < n; i += warps) f(A.near[1 + i]);
+__device__ __forceinline__ void for_near_rays(const AdjArgs& A, int64_t blocks, int64_t warp_blocks, const Fn& f) {
+  const int64_t n = A.near[0], warp = threadIdx.x >> 5;
+  const bool together = n <= kNearPerWarp * warp_blocks * 4;
+  if (together && blockIdx.x >= warp_blocks) return;
+  // consecutive warps of rays in consecutive blocks
+  const int64_t step = together ? warp_blocks * 4 : blocks * 128;
+  const int64_t first = together ? warp * warp_blocks + blockIdx.x
+                                 : (warp * blocks + blockIdx.x) * 32 + (threadIdx.x & 31);
+#pragma unroll 1
+  for (int64_t i = first; i < n; i += step) f(A.near[1 + i], together);
 }
 
 // Touches the footprints of the step after `step` along the straight ray, two
@@ -196,10 +210,11 @@ __device__ __forceinline__ void prefetch_step(const AdjArgs& A, const MixedRay& 
 // Forward trace of one ray storing the state every C steps (and the final
 // state); y holds the final state.
 // TAPE: the stage inputs of steps tape_from on go to the tape (by lanes with
-// `tape`), so that those segments are not recomputed.
+// `tape`), so that those segments are not recomputed. together: a marked ray that all
+// lanes of the warp hold.
 template <bool TAPE, typename Interp>
 __device__ __forceinline__ void ckpt_ray(const Interp& interp, const AdjArgs& A, int64_t slot, const RayDir& d,
-                                         MixedRay& R, float* y, Guard& gd, bool tape = true) {
+                                         MixedRay& R, float* y, Guard& gd, bool tape = true, bool together = false) {
   constexpr bool kNear = std::is_same<Interp, OneLane<kFourTaps>>::value;
   float x0[3];
   mixed_observer(A.G, x0);
@@ -209,7 +224,7 @@ __device__ __forceinline__ void ckpt_ray(const Interp& interp, const AdjArgs& A,
   store_vec(ck, A.count, slot, y, kMixedState);
 #pragma unroll 1
   for (int st = 0; st < A.n_steps; ++st) {
-    if (kNear) prefetch_step(A, R, x0, y, st);
+    if (kNear && together) prefetch_step(A, R, x0, y, st);
     if (gd.m) gd.begin_step(y);
     float* us = TAPE && tape && st >= A.tape_from
                     ? (float*)A.seg + (int64_t)(st - A.tape_from) * kTapeStep * A.count + slot
@@ -274,15 +289,15 @@ __global__ void __launch_bounds__(32, 12) ckpt_small_kernel(const AdjArgs A) {
   ckpt_one<MAPS>(FourLanes<LAYOUT>{lane & 3, lane & ~3}, A, slot, (lane & 3) == 0, guard_m[lane]);
 }
 
-// The marked rays' checkpoints by the four-tap passes, one warp per ray. Few
-// rays: the launch is about one ray's latency.
+// The marked rays' checkpoints by the four-tap passes. Few rays: the launch is about
+// one ray's latency.
 template <bool TAPE>
 __global__ void __launch_bounds__(128, 2) near_ckpt_kernel(const AdjArgs A) {
-  for_near_rays(A, (int64_t)gridDim.x * 4, [&](int64_t slot) {
+  for_near_rays(A, gridDim.x, gridDim.x, [&](int64_t slot, bool together) {
     MixedRay R;
     float y[kMixedState];
     Guard gd;  // disabled
-    ckpt_ray<TAPE>(OneLane<kFourTaps>(), A, slot, ray_dir_pix(A.nside, ring_of(A, slot)), R, y, gd);
+    ckpt_ray<TAPE>(OneLane<kFourTaps>(), A, slot, ray_dir_pix(A.nside, ring_of(A, slot)), R, y, gd, true, together);
   });
 }
 
@@ -327,7 +342,7 @@ __global__ void __launch_bounds__(128) final_cotangent_kernel_mixed(const AdjArg
 // inputs of every step: tape [C][4 x 19][count].
 template <typename Interp>
 __device__ __forceinline__ void segment_ray(const Interp& interp, const AdjArgs& A, int sgi, int64_t slot,
-                                            bool first = true) {
+                                            bool first = true, bool together = false) {
   MixedRay R;
   float y[kMixedState], x0[3];
   mixed_observer(A.G, x0);
@@ -338,24 +353,24 @@ __device__ __forceinline__ void segment_ray(const Interp& interp, const AdjArgs&
 #pragma unroll 1
   for (int st = s0; st < s1; ++st) {
     Guard gd;  // disabled
-    if (std::is_same<Interp, OneLane<kFourTaps>>::value) prefetch_step(A, R, x0, y, st);
+    if (std::is_same<Interp, OneLane<kFourTaps>>::value && together) prefetch_step(A, R, x0, y, st);
     step_mixed(interp, R, A.F, A.G, x0, st, y,
                first ? tape + (int64_t)(st - s0) * kTapeStep * A.count + slot : nullptr, A.count, gd);
   }
 }
 
-// The first kNearBlocks blocks take the marked rays by the four-tap passes
-// (first, so that their latency hides behind the other rays').
-constexpr int kNearBlocks = 38;
-constexpr int kNearCkptBlocks = 304;
-
+// The first near_blocks blocks (one per SM) take the marked rays by the four-tap
+// passes: first, so that their latency hides behind the other rays', and a short list
+// in a quarter of them (with its warps in all of them the segment is 1-2 % longer).
 template <int LAYOUT>
-__global__ void __launch_bounds__(128, 2) segment_kernel_mixed(const AdjArgs A, int sgi) {
-  if (blockIdx.x < kNearBlocks) {
-    for_near_rays(A, kNearBlocks * 4, [&](int64_t slot) { segment_ray(OneLane<kFourTaps>(), A, sgi, slot); });
+__global__ void __launch_bounds__(128, 2) segment_kernel_mixed(const AdjArgs A, int sgi, unsigned near_blocks) {
+  if (blockIdx.x < near_blocks) {
+    for_near_rays(A, near_blocks, (near_blocks + 3) / 4, [&](int64_t slot, bool together) {
+      segment_ray(OneLane<kFourTaps>(), A, sgi, slot, true, together);
+    });
     return;
   }
-  const int64_t slot = (int64_t)(blockIdx.x - kNearBlocks) * 128 + threadIdx.x;
+  const int64_t slot = (int64_t)(blockIdx.x - near_blocks) * 128 + threadIdx.x;
   if (slot < A.count && !is_near(A, slot)) segment_ray(OneLane<LAYOUT>(), A, sgi, slot);
 }
 
@@ -369,7 +384,9 @@ __global__ void __launch_bounds__(32, 12) segment_small_kernel(const AdjArgs A, 
 
 // The marked rays of a segment, beside segment_small_kernel.
 __global__ void __launch_bounds__(128, 2) near_segment_kernel(const AdjArgs A, int sgi) {
-  for_near_rays(A, (int64_t)gridDim.x * 4, [&](int64_t slot) { segment_ray(OneLane<kFourTaps>(), A, sgi, slot); });
+  for_near_rays(A, gridDim.x, gridDim.x, [&](int64_t slot, bool together) {
+    segment_ray(OneLane<kFourTaps>(), A, sgi, slot, true, together);
+  });
 }
 
 // The four passes of a stage by one lane, FP32 accumulation: the interpolations,
@@ -682,6 +699,10 @@ void with_forward_layout(const srt_fields* f, const Fn& fn) {
     fn(std::integral_constant<int, kFourPlanes>());
 }
 
+// Blocks of the launches for the marked rays alone: all that are resident at once, and
+// no more than give each ray a warp.
+inline unsigned near_ckpt_blocks(unsigned blocks, int sms) { return std::min<unsigned>(blocks * 32, 2 * sms); }
+
 template <int LAYOUT, bool MAPS>
 void launch_ckpt(const AdjArgs& A, bool small, unsigned blocks, cudaStream_t s) {
   if (small)
@@ -690,12 +711,12 @@ void launch_ckpt(const AdjArgs& A, bool small, unsigned blocks, cudaStream_t s) 
     ckpt_kernel_mixed<LAYOUT, MAPS><<<blocks, 128, 0, s>>>(A);
 }
 template <int LAYOUT>
-void launch_segment(const AdjArgs& A, int sgi, bool small, unsigned blocks, cudaStream_t s) {
+void launch_segment(const AdjArgs& A, int sgi, bool small, unsigned blocks, unsigned near, cudaStream_t s) {
   if (small) {
     segment_small_kernel<LAYOUT><<<(unsigned)((A.count + 7) / 8), 32, 0, s>>>(A, sgi);
-    near_segment_kernel<<<kNearBlocks, 128, 0, s>>>(A, sgi);
+    near_segment_kernel<<<near, 128, 0, s>>>(A, sgi);
   } else {
-    segment_kernel_mixed<LAYOUT><<<blocks + kNearBlocks, 128, 0, s>>>(A, sgi);
+    segment_kernel_mixed<LAYOUT><<<blocks + near, 128, 0, s>>>(A, sgi, near);
   }
 }
 
@@ -1208,7 +1229,7 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
         const bool small = small_adjoint(pix_count, sms);
         if (!tape) {  // else the checkpoints come from srt_forward_tape
           with_forward_layout(f, [&](auto l) { launch_ckpt<decltype(l)::value, false>(A, small, blocks, s); });
-          near_ckpt_kernel<true><<<std::min<unsigned>(blocks * 32, kNearCkptBlocks), 128, 0, s>>>(A);
+          near_ckpt_kernel<true><<<near_ckpt_blocks(blocks, sms), 128, 0, s>>>(A);
         }
         final_cotangent_kernel_mixed<<<blocks, 128, 0, s>>>(A, (float*)lam.p);
         kernels += tape ? 1 : 3;
@@ -1224,7 +1245,7 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
           A.seg = seg.p;
           if (sgi >= kept_from) A.seg = (float*)seg.p + (int64_t)(sgi - kept_from) * C * kTapeStep * pix_count;
           if (sgi < kept_from)
-            with_forward_layout(f, [&](auto l) { launch_segment<decltype(l)::value>(A, sgi, small, blocks, s); });
+            with_forward_layout(f, [&](auto l) { launch_segment<decltype(l)::value>(A, sgi, small, blocks, sms, s); });
           if (determ)
             launch_sweep<AccFixed>(A, sgi, (float*)lam.p, ax, layout, bgrad, small, blocks, s);
           else
@@ -1395,7 +1416,7 @@ extern "C" int srt_forward_tape(const srt_fields* fields, int64_t nside, int64_t
     VJP_TRY(sm_count(&sms), "device attributes");
     const bool small = small_adjoint(pix_count, sms);
     with_forward_layout(f, [&](auto l) { launch_ckpt<decltype(l)::value, true>(A, small, blocks, s); });
-    near_ckpt_kernel<false><<<std::min<unsigned>(blocks * 32, kNearCkptBlocks), 128, 0, s>>>(A);
+    near_ckpt_kernel<false><<<near_ckpt_blocks(blocks, sms), 128, 0, s>>>(A);
     kernels += 2;
     VJP_TRY(cudaGetLastError(), "checkpointing forward");
     TraceArgs ta;
