@@ -101,7 +101,7 @@ typedef struct srt_stats {
   int64_t kernels;     /* kernels this call launched */
   int64_t h2d_bytes;   /* bytes copied host -> device by this call */
   int64_t d2h_bytes;   /* bytes copied device -> host by this call */
-  int64_t refined_rays; /* MIXED: rays re-traced in FP64 (synchronous calls) */
+  int64_t refined_rays; /* MIXED: rays re-traced (synchronous calls) */
   double retrace_ms;    /* srt_forward, MIXED: the re-trace launches' share of trace_ms
                            (synchronous calls; 0 elsewhere). Added in ABI version 4. */
 } srt_stats;

@@ -710,14 +710,16 @@ void launch_ckpt(const AdjArgs& A, bool small, unsigned blocks, cudaStream_t s) 
   else
     ckpt_kernel_mixed<LAYOUT, MAPS><<<blocks, 128, 0, s>>>(A);
 }
+// Returns the number of kernels launched.
 template <int LAYOUT>
-void launch_segment(const AdjArgs& A, int sgi, bool small, unsigned blocks, unsigned near, cudaStream_t s) {
+int launch_segment(const AdjArgs& A, int sgi, bool small, unsigned blocks, unsigned near, cudaStream_t s) {
   if (small) {
     segment_small_kernel<LAYOUT><<<(unsigned)((A.count + 7) / 8), 32, 0, s>>>(A, sgi);
     near_segment_kernel<<<near, 128, 0, s>>>(A, sgi);
-  } else {
-    segment_kernel_mixed<LAYOUT><<<blocks + near, 128, 0, s>>>(A, sgi, near);
+    return 2;
   }
+  segment_kernel_mixed<LAYOUT><<<blocks + near, 128, 0, s>>>(A, sgi, near);
+  return 1;
 }
 
 inline void copy_extra(AccPaired<4>& to, const AccF32& from) { to.hot = from.hot; }
@@ -1109,7 +1111,7 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   int64_t kernels = 0, h2d = 0, d2h = 0;
   {
-    // padded accumulator entry: 8 B (FP64 / fixed point), 16 B (FP32 rows)
+    // padded accumulator entry: 8 B (FP64 / fixed point), 16 B (FP32: a cell's four cotangents)
     const size_t accsz = (determ || fp64) ? 8 : 16;
     if (!dev_io) {
       // host gradients: start from zero (or from the caller's values when accumulating)
@@ -1245,12 +1247,13 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
           A.seg = seg.p;
           if (sgi >= kept_from) A.seg = (float*)seg.p + (int64_t)(sgi - kept_from) * C * kTapeStep * pix_count;
           if (sgi < kept_from)
-            with_forward_layout(f, [&](auto l) { launch_segment<decltype(l)::value>(A, sgi, small, blocks, sms, s); });
+            with_forward_layout(
+                f, [&](auto l) { kernels += launch_segment<decltype(l)::value>(A, sgi, small, blocks, sms, s); });
           if (determ)
             launch_sweep<AccFixed>(A, sgi, (float*)lam.p, ax, layout, bgrad, small, blocks, s);
           else
             launch_sweep<AccF32>(A, sgi, (float*)lam.p, af, layout, bgrad, small, blocks, s);
-          kernels += sgi < kept_from ? 2 : 1;
+          ++kernels;
         }
       }
       if (fp64) kernels += 2;

@@ -79,7 +79,7 @@ struct TraceArgs {
   int n_steps = 0;
   float* maps[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   // MIXED: the output slots of rays that came within the cell-face guard are
-  // appended here (NULL: no fallback) and re-traced in FP64 by launch_refine.
+  // appended here (NULL: no fallback) and re-traced by launch_refine.
   int64_t* refine_list = nullptr;
   unsigned long long* refine_count = nullptr;
 };
@@ -104,7 +104,8 @@ cudaError_t launch_pair_build(const float* src, float2* dst, const int64_t pn[3]
 
 // Trace kernel launch (mode = kFP64 / kREF16 / a handle's mixed_mode()).
 cudaError_t launch_trace(int mode, const TraceArgs& a, cudaStream_t s, int64_t* kernels);
-// FP64 re-trace of the rays listed by a MIXED trace (count read on the device).
+// Re-trace of the rays listed by a MIXED trace (count read on the device), in FP64 or,
+// long lists, in double-float.
 cudaError_t launch_refine(const TraceArgs& a, cudaStream_t s, int64_t* kernels);
 // The FP64 form of a small range, one warp per ray (srt_retrace.cu): launch_trace
 // takes it up to kWideFp64Rays rays.

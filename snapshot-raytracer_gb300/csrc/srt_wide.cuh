@@ -22,7 +22,7 @@
 //   x, y, z passes        32 lanes 6, 3 and 1-2 four-term chains per lane
 //   right-hand side       six rounds of dot products and linear combinations
 //   RK4                   lane j holds component j of the state
-// ~96 FP64 instructions per stage against ~730 for the four-lane groups this
+// ~104 FP64 instructions per stage against ~730 for the four-lane groups this
 // replaces (one field per lane, the rest of the right-hand side repeated on
 // each).
 //
@@ -162,7 +162,7 @@ constexpr WideTables make_wide_tables() {
 }
 
 // Catmull-Rom coefficients per tap: value c0..c3, derivative c0..c2, second
-// derivative c0, c1 (cr_weights_fma's, with the powers a tap lacks as zeros).
+// derivative c0, c1 (cr_weights_fp64's, with the powers a tap lacks as zeros).
 struct WideCoef {
   float v[4], g[3], h[2];
 };
