@@ -107,9 +107,11 @@ cudaError_t launch_trace(int mode, const TraceArgs& a, cudaStream_t s, int64_t* 
 // Re-trace of the rays listed by a MIXED trace (count read on the device), in FP64 or,
 // long lists, in double-float.
 cudaError_t launch_refine(const TraceArgs& a, cudaStream_t s, int64_t* kernels);
-// The FP64 form of a small range, one warp per ray (srt_retrace.cu): launch_trace
-// takes it up to kWideFp64Rays rays.
-constexpr int64_t kWideFp64Rays = 14000;
+// The FP64 form of a small range, five warps or one per ray (srt_retrace.cu):
+// launch_trace takes it up to kWideFp64RaysPerSM rays per SM, where a lane per ray
+// leaves the FP64 unit waiting (256^3, 16 steps, 152 SMs: 2,000 rays 0.89 against 4.88
+// ms, 14,000 5.9 against 8.2, 20,000 8.4 against 9.3, 24,000 10.0 against 9.3).
+constexpr int64_t kWideFp64RaysPerSM = 140;
 cudaError_t launch_wide_fp64(const TraceArgs& a, cudaStream_t s, int64_t* kernels);
 
 // Progressive reads of an HDF5 field (srt_io.cpp), for srt_fields_load_h5.

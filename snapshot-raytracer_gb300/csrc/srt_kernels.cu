@@ -298,10 +298,10 @@ bool is_small(int mode, const TraceArgs& a, int sms) {
 }
 
 cudaError_t launch_trace(int mode, const TraceArgs& a, cudaStream_t s, int64_t* kernels) {
-  if (mode == kFP64 && a.pix_count <= kWideFp64Rays) return launch_wide_fp64(a, s, kernels);
   int sms = 0;
   const cudaError_t e = sm_count(&sms);
   if (e != cudaSuccess) return e;
+  if (mode == kFP64 && a.pix_count <= kWideFp64RaysPerSM * sms) return launch_wide_fp64(a, s, kernels);
   if (mode != kFP64 && mode != kREF16 && is_small(mode, a, sms)) {
     const unsigned small = (unsigned)((a.launch_rays + 7) / 8);
     switch (mode) {
