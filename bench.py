@@ -486,10 +486,10 @@ def run_ours(args):
     torch.cuda.synchronize()
     stream = torch.cuda.current_stream(dev)
     fields = srt.Fields(phi_d, b_d, stream=stream, pairs=args.pairs)
-    # cells, or planes and row pairs, where they fit (not at 2048^3)
+    # cells, or planes and half cells, where they fit (not at 2048^3)
     per_voxel = fields.nbytes / (n + 3) ** 3
     cfg["field_layout"] = ("cells (value and second differences)" if per_voxel == 64 else
-                           "halo-padded planes + row-pair copies" if per_voxel > 16 else
+                           "halo-padded planes + half cells or row pairs" if per_voxel > 16 else
                            "halo-padded planes")
     if args.e2e_steps <= 0:  # the laid-out copy is all the trace needs (2048^3: 137 GB freed)
         torch.cuda.synchronize()

@@ -135,7 +135,8 @@ int srt_device_count(void);
  * SRT_FIELDS_NO_PAIRS, the fields are stored as cells: per voxel and component
  * the value and its second differences along y, x and both (16 bytes; nothing
  * else is kept). Else as FP32 planes (4 bytes), beside them, when they fit,
- * row-pair copies (8 bytes). MIXED's bits depend on the grid, the flags and the
+ * half cells (the value and its second difference along y, 8 bytes; row pairs where
+ * the four-tap form below is taken). MIXED's bits depend on the grid, the flags and the
  * device, not on the free memory: the second differences on every layout, or, on
  * grids whose cells would take more than two fifths of the whole device and with
  * SRT_FIELDS_NO_PAIRS from 512^3 voxels on, the four-tap form of the same

@@ -676,27 +676,36 @@ __global__ void __launch_bounds__(32, 8)
                     FourLanePasses<LAYOUT, Acc>{A.F, A.G, acc, field, lane & ~3}, s_lam, s_tot);
 }
 
-// f(std::integral_constant<int, LAYOUT>()) for a handle's layout.
-template <typename Fn>
-void with_layout(int layout, const Fn& f) {
-  if (layout == kCells)
-    f(std::integral_constant<int, kCells>());
-  else if (layout == kPairs)
-    f(std::integral_constant<int, kPairs>());
-  else
-    f(std::integral_constant<int, kPlanes>());
-}
-
-// The same for the forward's passes (the sweep interpolates at positions it is
-// given, so it takes the second differences in every layout).
+// fn(std::integral_constant<int, LAYOUT>()) for the passes of a handle's forward:
+// second differences or four taps.
 template <typename Fn>
 void with_forward_layout(const srt_fields* f, const Fn& fn) {
-  if (!f->four_taps)
-    with_layout(f->layout(), fn);
-  else if (f->layout() == kPairs)
+  const int layout = f->layout();
+  if (layout == kCells)
+    fn(std::integral_constant<int, kCells>());
+  else if (layout == kHalf)
+    fn(std::integral_constant<int, kHalf>());
+  else if (layout == kPairs)
     fn(std::integral_constant<int, kFourPairs>());
-  else
+  else if (f->four_taps)
     fn(std::integral_constant<int, kFourPlanes>());
+  else
+    fn(std::integral_constant<int, kPlanes>());
+}
+
+// The same for the sweep, which interpolates at positions it is given and takes the
+// second differences in every layout.
+template <typename Fn>
+void with_sweep_layout(const srt_fields* f, const Fn& fn) {
+  const int layout = f->layout();
+  if (layout == kCells)
+    fn(std::integral_constant<int, kCells>());
+  else if (layout == kHalf)
+    fn(std::integral_constant<int, kHalf>());
+  else if (layout == kPairs)
+    fn(std::integral_constant<int, kPairs>());
+  else
+    fn(std::integral_constant<int, kPlanes>());
 }
 
 // Blocks of the launches for the marked rays alone: all that are resident at once, and
@@ -726,9 +735,9 @@ inline void copy_extra(AccPaired<4>& to, const AccF32& from) { to.hot = from.hot
 inline void copy_extra(AccFixed& to, const AccFixed& from) { to.ovf = from.ovf; }
 
 template <typename Acc>
-void launch_sweep(const AdjArgs& A, int sgi, float* lam, const Acc* a, int layout, bool bgrad, bool small,
+void launch_sweep(const AdjArgs& A, int sgi, float* lam, const Acc* a, const srt_fields* f, bool bgrad, bool small,
                   unsigned blocks, cudaStream_t s) {
-  with_layout(layout, [&](auto l) {
+  with_sweep_layout(f, [&](auto l) {
     constexpr int L = decltype(l)::value;
     if (small) {
       typedef typename std::conditional<TakesCells<Acc>::value, AccPaired<4>, Acc>::type AccS;
@@ -1227,7 +1236,6 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
       } else {
         // forward with checkpoints; then per segment, backwards: recompute
         // the segment's tape, sweep it
-        const int layout = f->layout();
         const bool small = small_adjoint(pix_count, sms);
         if (!tape) {  // else the checkpoints come from srt_forward_tape
           with_forward_layout(f, [&](auto l) { launch_ckpt<decltype(l)::value, false>(A, small, blocks, s); });
@@ -1250,9 +1258,9 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
             with_forward_layout(
                 f, [&](auto l) { kernels += launch_segment<decltype(l)::value>(A, sgi, small, blocks, sms, s); });
           if (determ)
-            launch_sweep<AccFixed>(A, sgi, (float*)lam.p, ax, layout, bgrad, small, blocks, s);
+            launch_sweep<AccFixed>(A, sgi, (float*)lam.p, ax, f, bgrad, small, blocks, s);
           else
-            launch_sweep<AccF32>(A, sgi, (float*)lam.p, af, layout, bgrad, small, blocks, s);
+            launch_sweep<AccF32>(A, sgi, (float*)lam.p, af, f, bgrad, small, blocks, s);
           ++kernels;
         }
       }

@@ -525,7 +525,7 @@ struct StageView {
   T A, Ap, s1, s2, e1, e2;
   bool branch;         // dA > 1/2
   int64_t base[4];     // padded base index per field: B_x, B_y, B_z, phi
-  int64_t basep[4];    // the same cells in the row-pair layout (kPairs)
+  int64_t basep[4];    // the same cells in the row-pair and half-cell layouts
   int hbase[4];        // the same cells near the observer (hot_base; MIXED)
   T t[4][3];           // cell offsets per field and axis
 };

@@ -279,8 +279,15 @@ constexpr int64_t kFourTapVoxels = int64_t(1) << 27;
 // cells (64 bytes per padded voxel for the four fields) unless
 // SRT_FIELDS_NO_PAIRS, where they take at most two fifths of the budget (so that
 // a gradient's accumulators, another 64 bytes, and its scratch fit beside them as
-// they do beside planes and row pairs), else planes (16 bytes), which
-// finish_fields may add row pairs to (another 32).
+// they do beside planes and half cells), else planes (16 bytes), which
+// finish_fields may add half cells or row pairs to (another 32). The environment
+// variable SRT_FIELDS_LAYOUT makes a handle find no room for cells ("half") or for
+// anything but planes ("planes"), for tests.
+bool room_for(const char* layout) {
+  const char* v = getenv("SRT_FIELDS_LAYOUT");
+  return !v || strcmp(v, "cells") == 0 || (strcmp(v, "half") == 0 && strcmp(layout, "half") == 0);
+}
+
 int alloc_fields(srt_fields* f, int64_t n0, int64_t n1, int64_t n2, unsigned flags, cudaStream_t s) {
   cudaGetDevice(&f->device);
   for (int i = 0; i < 3; ++i) {
@@ -298,10 +305,13 @@ int alloc_fields(srt_fields* f, int64_t n0, int64_t n1, int64_t n2, unsigned fla
   // 149.8 against 164.3 ms). They are taken by grids whose cells no handle would
   // hold (some 1,230^3 on 288 GB) and by SRT_FIELDS_NO_PAIRS from 512^3 on, where
   // full skies are bound by throughput; smaller grids, and those whose cells did not
-  // find room, keep the bits of a default handle.
+  // find room, keep the bits of a default handle. The latter read half cells, which
+  // hold the second differences along y (the base pixel 141.2 ms against 149.8 on four
+  // taps and 124.7 from cells; 256^3 / nside 128 / 128 steps 7.9, 8.3 and 6.9), and
+  // planes only where those find no room either.
   f->four_taps =
       64 * pvox > (int64_t)total_b / 5 * 2 || ((flags & SRT_FIELDS_NO_PAIRS) && n0 * n1 * n2 >= kFourTapVoxels);
-  if (!(flags & SRT_FIELDS_NO_PAIRS) && !f->four_taps && 64 * pvox <= field_budget(f) / 5 * 2) {
+  if (!(flags & SRT_FIELDS_NO_PAIRS) && !f->four_taps && room_for("cells") && 64 * pvox <= field_budget(f) / 5 * 2) {
     for (int c = 3; c >= 0; --c) {
       e = pool_alloc((void**)&f->cell[c], pvox * sizeof(float4), s);
       if (e != cudaSuccess) return cuda_error(e, c == 3 ? "allocate phi" : "allocate B");
@@ -330,20 +340,20 @@ cudaError_t lay_out(srt_fields* f, const float* src, int comps, int64_t k0, int6
   return launch_pad_fields(src, comps, dst, f->n, f->pn, k0, k1, s);
 }
 
-// The last step of a layout: row-pair copies of planes, when they fit
-// (unless SRT_FIELDS_NO_PAIRS).
+// The last step of a layout: half cells of planes, or row pairs for the four taps,
+// when they fit (unless SRT_FIELDS_NO_PAIRS).
 int finish_fields(srt_fields* f, unsigned flags, cudaStream_t s) {
   if ((flags & SRT_FIELDS_NO_PAIRS) || f->cell[0]) return SRT_OK;
   const int64_t pair_bytes = 4 * f->pn[0] * (f->pn[1] - 1) * f->pn[2] * (int64_t)sizeof(float2);
-  if (pair_bytes >= field_budget(f)) return SRT_OK;
+  if (!room_for("half") || pair_bytes >= field_budget(f)) return SRT_OK;
   const float* srcs[4] = {f->b[0], f->b[1], f->b[2], f->phi};
   cudaError_t e = cudaSuccess;
   for (int c = 0; c < 4 && e == cudaSuccess; ++c) {
     e = pool_alloc((void**)&f->pr[c], pair_bytes / 4, s);
-    if (e != cudaSuccess) return cuda_error(e, "allocate row pairs");
-    e = launch_pair_build(srcs[c], f->pr[c], f->pn, s);
+    if (e != cudaSuccess) return cuda_error(e, "allocate half cells");
+    e = launch_pair_build(srcs[c], f->pr[c], f->pn, !f->four_taps, s);
   }
-  if (e != cudaSuccess) return cuda_error(e, "row pairs");
+  if (e != cudaSuccess) return cuda_error(e, "half cells");
   f->bytes += pair_bytes;
   return SRT_OK;
 }

@@ -15,7 +15,7 @@ struct srt_fields {
   int64_t n[3] = {0, 0, 0};
   int64_t pn[3] = {0, 0, 0};  // padded extents n + 3
   // either cells (B_x, B_y, B_z, phi; 16 bytes per padded voxel), or padded FP32
-  // planes and, where they fit, row-pair copies in the same order
+  // planes and, where they fit, half cells or (four_taps) row pairs in the same order
   float4* cell[4] = {nullptr, nullptr, nullptr, nullptr};
   float* phi = nullptr;
   float* b[3] = {nullptr, nullptr, nullptr};
@@ -29,11 +29,13 @@ struct srt_fields {
   // differences, in every layout: MIXED's bits depend on the grid, the flags and the
   // device, not on what memory was free.
   bool four_taps = false;
-  int layout() const { return cell[0] ? srt::kCells : (pr[0] ? srt::kPairs : srt::kPlanes); }
+  int layout() const {
+    return cell[0] ? srt::kCells : (pr[0] ? (four_taps ? srt::kPairs : srt::kHalf) : srt::kPlanes);
+  }
   // the MIXED trace kernel of this layout
   int mixed_mode() const {
     if (four_taps) return pr[0] ? srt::kMIXED_FOUR_PAIR : srt::kMIXED_FOUR;
-    return cell[0] ? srt::kMIXED_CELL : (pr[0] ? srt::kMIXED_PAIR : srt::kMIXED);
+    return cell[0] ? srt::kMIXED_CELL : (pr[0] ? srt::kMIXED_HALF : srt::kMIXED);
   }
   // the values of B component c (0-2) or phi (3), make_geom's ts floats apart
   const float* values(int c) const { return cell[c] ? &cell[c]->x : (c == 3 ? phi : b[c]); }
@@ -100,7 +102,8 @@ cudaError_t launch_fetch(const float* src, float* dst, int64_t count, cudaStream
 cudaError_t launch_quantize_half(const float* src, int ts, __half* dst, int64_t count, cudaStream_t s);
 // The same values as a plane.
 cudaError_t launch_extract(const float* src, int ts, float* dst, int64_t count, cudaStream_t s);
-cudaError_t launch_pair_build(const float* src, float2* dst, const int64_t pn[3], cudaStream_t s);
+// Row pairs or half cells of a padded plane array.
+cudaError_t launch_pair_build(const float* src, float2* dst, const int64_t pn[3], bool half, cudaStream_t s);
 
 // Trace kernel launch (mode = kFP64 / kREF16 / a handle's mixed_mode()).
 cudaError_t launch_trace(int mode, const TraceArgs& a, cudaStream_t s, int64_t* kernels);

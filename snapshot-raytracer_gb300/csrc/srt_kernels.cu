@@ -191,7 +191,9 @@ cudaError_t launch_extract(const float* src, int ts, float* dst, int64_t count, 
 }
 
 // Row-pair array of a padded field: element (i, j, k), j < py - 1, holds
-// (f(i, j, k), f(i, j + 1, k)).
+// (f(i, j, k), f(i, j + 1, k)); or half cells (HALF): f(i, j, k) and its second
+// difference along y (0 in row 0, which no footprint's inner rows reach).
+template <bool HALF>
 __global__ void pair_build_kernel(const float* __restrict__ src, float2* __restrict__ dst, int64_t px, int64_t py,
                                   int64_t pz) {
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -199,12 +201,17 @@ __global__ void pair_build_kernel(const float* __restrict__ src, float2* __restr
   if (q >= px * rows * pz) return;
   const int64_t i = q % px, j = (q / px) % rows, k = q / (px * rows);
   const int64_t s0 = i + px * (j + py * k);
-  dst[q] = make_float2(src[s0], src[s0 + px]);
+  const float v = src[s0], up = src[s0 + px];
+  dst[q] = make_float2(v, HALF ? (j > 0 ? diff2(src[s0 - px], v, up) : 0.f) : up);
 }
 
-cudaError_t launch_pair_build(const float* src, float2* dst, const int64_t pn[3], cudaStream_t s) {
+cudaError_t launch_pair_build(const float* src, float2* dst, const int64_t pn[3], bool half, cudaStream_t s) {
   const int64_t count = pn[0] * (pn[1] - 1) * pn[2];
-  pair_build_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(src, dst, pn[0], pn[1], pn[2]);
+  const unsigned blocks = (unsigned)((count + 255) / 256);
+  if (half)
+    pair_build_kernel<true><<<blocks, 256, 0, s>>>(src, dst, pn[0], pn[1], pn[2]);
+  else
+    pair_build_kernel<false><<<blocks, 256, 0, s>>>(src, dst, pn[0], pn[1], pn[2]);
   return cudaGetLastError();
 }
 
@@ -234,20 +241,20 @@ __device__ __forceinline__ bool ray_of_slot(const TraceArgs& A, int64_t tl, int6
 // The layout that a MIXED mode's passes read.
 constexpr __host__ __device__ int layout_of(int mode) {
   return mode == kMIXED_CELL ? kCells
-         : mode == kMIXED_PAIR ? kPairs
+         : mode == kMIXED_HALF ? kHalf
          : mode == kMIXED_FOUR ? kFourPlanes
          : mode == kMIXED_FOUR_PAIR ? kFourPairs
                                : kPlanes;
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(128, (MODE == kMIXED || MODE >= kMIXED_PAIR) ? SRT_MIXED_MIN_BLOCKS : 1)
+__global__ void __launch_bounds__(128, (MODE == kMIXED || MODE >= kMIXED_HALF) ? SRT_MIXED_MIN_BLOCKS : 1)
     trace_kernel(const TraceArgs A) {
   int64_t o, ring;
   if (!ray_of_slot(A, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, &o, &ring)) return;
   const RayDir d = ray_dir_pix(A.nside, ring);
   float out[6];
-  if (MODE >= kMIXED_PAIR || MODE == kMIXED) {
+  if (MODE >= kMIXED_HALF || MODE == kMIXED) {
     constexpr int kLayout = layout_of(MODE);
     __shared__ float guard_m[128][2];  // the ray's guard state, out of the register budget
     const bool near = trace_ray_mixed<kLayout>(A.F, A.G, d, A.n_steps, out, guard_m[threadIdx.x]);
@@ -287,7 +294,7 @@ __global__ void __launch_bounds__(32, 12) trace_small_kernel(const TraceArgs A) 
 }
 
 // Ranges that trace_small_kernel takes: up to one of its warps per scheduler from
-// cells or row pairs (5,292 rays: 0.443 against 0.378 ms on one lane), up to four
+// cells, half cells or row pairs (5,292 rays: 0.443 against 0.378 ms on one lane), up to four
 // from planes, whose loads are four times as many (19,200 rays: 1.02 against 1.08
 // ms, 27,648: 1.20 against 0.99). Not where most launch slots hold no ray of the
 // range.
@@ -306,7 +313,7 @@ cudaError_t launch_trace(int mode, const TraceArgs& a, cudaStream_t s, int64_t* 
     const unsigned small = (unsigned)((a.launch_rays + 7) / 8);
     switch (mode) {
       case kMIXED_CELL: trace_small_kernel<kCells><<<small, 32, 0, s>>>(a); break;
-      case kMIXED_PAIR: trace_small_kernel<kPairs><<<small, 32, 0, s>>>(a); break;
+      case kMIXED_HALF: trace_small_kernel<kHalf><<<small, 32, 0, s>>>(a); break;
       case kMIXED_FOUR: trace_small_kernel<kFourPlanes><<<small, 32, 0, s>>>(a); break;
       case kMIXED_FOUR_PAIR: trace_small_kernel<kFourPairs><<<small, 32, 0, s>>>(a); break;
       default: trace_small_kernel<kPlanes><<<small, 32, 0, s>>>(a);
@@ -326,7 +333,7 @@ cudaError_t launch_trace(int mode, const TraceArgs& a, cudaStream_t s, int64_t* 
     case kMIXED: trace_kernel<kMIXED><<<(unsigned)blocks, threads, 0, s>>>(a); break;
     case kREF16: trace_kernel<kREF16><<<(unsigned)blocks, threads, 0, s>>>(a); break;
     case kMIXED_CELL: trace_kernel<kMIXED_CELL><<<(unsigned)blocks, threads, 0, s>>>(a); break;
-    case kMIXED_PAIR: trace_kernel<kMIXED_PAIR><<<(unsigned)blocks, threads, 0, s>>>(a); break;
+    case kMIXED_HALF: trace_kernel<kMIXED_HALF><<<(unsigned)blocks, threads, 0, s>>>(a); break;
     case kMIXED_FOUR: trace_kernel<kMIXED_FOUR><<<(unsigned)blocks, threads, 0, s>>>(a); break;
     case kMIXED_FOUR_PAIR: trace_kernel<kMIXED_FOUR_PAIR><<<(unsigned)blocks, threads, 0, s>>>(a); break;
     default: return cudaErrorInvalidValue;

@@ -45,7 +45,7 @@
 
 namespace srt {
 
-enum { kFP64 = 0, kMIXED = 1, kREF16 = 2, kMIXED_PAIR = 3, kMIXED_CELL = 4, kMIXED_FOUR = 5, kMIXED_FOUR_PAIR = 6 };
+enum { kFP64 = 0, kMIXED = 1, kREF16 = 2, kMIXED_HALF = 3, kMIXED_CELL = 4, kMIXED_FOUR = 5, kMIXED_FOUR_PAIR = 6 };
 
 #if defined(__CUDA_ARCH__)
 template <typename T>
@@ -66,25 +66,26 @@ SRT_HD float ld_stream(const float* p) { return *p; }
 struct Geom {
   int n[3];
   int64_t px, pxy;
-  int64_t pxy2;  // slice stride of the row-pair arrays (float2 units): px * (py - 1)
+  int64_t pxy2;  // slice stride of the row-pair and half-cell arrays (float2 units): px * (py - 1)
   float invn[3];
   int ts = 1;  // floats from one voxel's value to the next: 1 in planes, 4 in cells
 };
 
 // How a handle stores its fields (the MIXED kernels are compiled for each):
-// planes of values; planes beside row-pair copies; or cells, which hold the
-// values too, so nothing else is stored. kFourTaps: the four-tap passes on the
-// values of any layout (rays of the adjoint that come near a cell face);
-// kFourPlanes, kFourPairs: the same on planes and on row pairs (grids too large for
-// cells, srt_fields::four_taps).
-enum { kPlanes = 0, kPairs = 1, kCells = 2, kFourTaps = 3, kFourPlanes = 4, kFourPairs = 5 };
+// cells, which hold the values too, so nothing else is stored; planes of values; or
+// planes beside half cells, or beside row pairs where the forward takes the four taps
+// (srt_fields::four_taps). kFourTaps: the four-tap passes on the values of any layout
+// (rays of the adjoint that come near a cell face); kFourPlanes, kFourPairs: the same
+// on planes and on row pairs.
+enum { kPlanes = 0, kPairs = 1, kCells = 2, kFourTaps = 3, kFourPlanes = 4, kFourPairs = 5, kHalf = 6 };
 
 struct FieldPtrs {
   const float* phi;     // padded FP32 values, Geom::ts floats apart
   const float* b[3];    // the same for the B components
   const __half* bh[3];  // padded half(B * 2^27) (REF16 only)
-  // Row-pair arrays (kPairs): element (i, j, k), j < py - 1, holds
-  // (f(i, j, k), f(i, j + 1, k)) of the padded field; [0..2] B, [3] phi.
+  // Row-pair arrays (kPairs) or half cells (kHalf): element (i, j, k), j < py - 1, of
+  // the first holds (f(i, j, k), f(i, j + 1, k)) of the padded field, of the second
+  // f(i, j, k) and its second difference along y; [0..2] B, [3] phi.
   const float2* pr[4];
   // Cells (kCells): element (i, j, k) of the padded grid holds the value and its
   // second differences along y, along x and along both (cell_of); [0..2] B, [3] phi.
@@ -281,9 +282,11 @@ struct YIn {
 
 // Where the packed passes get a slice (fixed z) of a tricubic footprint. load()
 // fetches it; x_pass() gives the x pass of its rows as two packed rows, and
-// at() picks one order's y inputs from them. Two kinds:
+// at() picks one order's y inputs from them. Three kinds:
 //   CellSource  four 16-byte cells (rows 1 and 2, taps 1 and 2): each packed
 //               row is (value, second difference along y) of one grid row;
+//   HalfSource  the same rows' (value, second difference along y) at the four tap
+//               columns (eight 64-bit loads), the ones along x formed on the spot;
 //   TapSource   the sixteen values, the second differences formed on the spot:
 //               one packed row holds the two grid rows' values, the other
 //               their second differences along y (four 32-bit loads per tap
@@ -305,6 +308,35 @@ struct CellSource {
     for (int j = 0; j < 2; ++j) {
       const float4 a = d.q[2 * j], b = d.q[2 * j + 1];
       r[j] = x_row<K>(w, make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y), make_float2(b.z, b.w));
+    }
+  }
+  SRT_HD static YIn at(const float2& a, const float2& b) { return YIn{a.x, b.x, a.y, b.y}; }
+};
+
+// 304 lane operations in 188 instructions and 32 loads an interpolation, where row
+// pairs take 368 in 236 (all second differences on the spot) or 352 in 188 (four
+// taps): 1024^3 base pixel, 141.2 ms against 164.4 and 149.8.
+struct HalfSource {
+  const float2* __restrict__ f;  // the half cell of voxel (cx - 1, cy, cz - 1)
+  int64_t px, pxy2;
+  SRT_HD SliceData load(int c) const {
+    SliceData d;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 a = ldg(f + c * pxy2 + i), b = ldg(f + c * pxy2 + px + i);
+      d.q[i] = make_float4(a.x, a.y, b.x, b.y);
+    }
+    return d;
+  }
+  template <bool K>
+  SRT_HD static void x_pass(const SliceData& d, const XDup& w, XRow* r) {
+    const float2 n2 = dup2(-2.f);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      float2 q[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = j ? make_float2(d.q[i].z, d.q[i].w) : make_float2(d.q[i].x, d.q[i].y);
+      r[j] = x_row<K>(w, q[1], ffma2(n2, q[1], fadd2(q[0], q[2])), q[2], ffma2(n2, q[2], fadd2(q[1], q[3])));
     }
   }
   SRT_HD static YIn at(const float2& a, const float2& b) { return YIn{a.x, b.x, a.y, b.y}; }
@@ -525,7 +557,7 @@ SRT_HD int64_t cell_base(const Geom& G, int cx, int cy, int cz) {
   return (int64_t)cx + G.px * (int64_t)cy + G.pxy * (int64_t)cz;
 }
 
-// The same voxel's index in a row-pair array.
+// The same voxel's index in a row-pair or half-cell array.
 SRT_HD int64_t cell_base_pair(const Geom& G, int cx, int cy, int cz) {
   return (int64_t)cx + G.px * (int64_t)cy + G.pxy2 * (int64_t)cz;
 }
@@ -537,6 +569,8 @@ SRT_HD auto cell_source(const FieldPtrs& F, const Geom& G, int f, int64_t base, 
     return CellSource{F.cell[f] + base + G.px + 1, G.px, G.pxy};
   else if constexpr (LAYOUT == kPairs)
     return TapSource<PairTaps>{{F.pr[f] + basep, G.px, G.pxy2}};
+  else if constexpr (LAYOUT == kHalf)
+    return HalfSource{F.pr[f] + basep + G.px, G.px, G.pxy2};
   else if constexpr (LAYOUT == kFourTaps)
     return ValueRows<false>{(f == 3 ? F.phi : F.b[f]) + base * G.ts, G.px, G.pxy, G.ts};
   else if constexpr (LAYOUT == kFourPlanes)
@@ -548,14 +582,14 @@ SRT_HD auto cell_source(const FieldPtrs& F, const Geom& G, int f, int64_t base, 
 }
 template <int LAYOUT>
 SRT_HD auto cell_source(const FieldPtrs& F, const Geom& G, int f, int cx, int cy, int cz) {
-  constexpr bool kFromPairs = LAYOUT == kPairs || LAYOUT == kFourPairs;
+  constexpr bool kFromPairs = LAYOUT == kPairs || LAYOUT == kFourPairs || LAYOUT == kHalf;
   return cell_source<LAYOUT>(F, G, f, kFromPairs ? 0 : cell_base(G, cx, cy, cz),
                              kFromPairs ? cell_base_pair(G, cx, cy, cz) : 0);
 }
 
 // x and y weights of a layout's passes.
 template <int LAYOUT>
-using AxisWeights = typename std::conditional<(LAYOUT >= kFourTaps), CRW<float>, CWD>::type;
+using AxisWeights = typename std::conditional<(LAYOUT >= kFourTaps && LAYOUT <= kFourPairs), CRW<float>, CWD>::type;
 SRT_HD void axis_weights(float t, CRW<float>& c) { cr_weights_mixed(t, c); }
 SRT_HD void axis_weights(float t, CWD& c) { cr_weights_diff(t, c); }
 
