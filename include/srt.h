@@ -139,7 +139,7 @@ int srt_device_count(void);
  * the four-tap form below is taken). MIXED's bits depend on the grid, the flags and the
  * device, not on the free memory: the second differences on every layout, or, on
  * grids whose cells would take more than two fifths of the whole device and with
- * SRT_FIELDS_NO_PAIRS from 512^3 voxels on, the four-tap form of the same
+ * SRT_FIELDS_NO_PAIRS from 2^19 voxels (80^3) on, the four-tap form of the same
  * interpolation (equal but for FP32 rounding, and faster there).
  * Replaces snapshot-raytracer.cu:752-855 (cudaMalloc of the fields, the three
  * staged vector3_to_half passes and the phi copy). */
