@@ -282,10 +282,10 @@ constexpr int64_t kFourTapVoxels = int64_t(1) << 19;
 // they do beside planes and half cells), else planes (16 bytes), which
 // finish_fields may add half cells or row pairs to (another 32). The environment
 // variable SRT_FIELDS_LAYOUT makes a handle find no room for cells ("half") or for
-// anything but planes ("planes"), for tests.
-bool room_for(const char* layout) {
+// anything but planes ("planes"), or be too large for cells ("pairs"), for tests.
+bool forced_layout(const char* layout) {
   const char* v = getenv("SRT_FIELDS_LAYOUT");
-  return !v || strcmp(v, "cells") == 0 || (strcmp(v, "half") == 0 && strcmp(layout, "half") == 0);
+  return v && strcmp(v, layout) == 0;
 }
 
 int alloc_fields(srt_fields* f, int64_t n0, int64_t n1, int64_t n2, unsigned flags, cudaStream_t s) {
@@ -313,9 +313,10 @@ int alloc_fields(srt_fields* f, int64_t n0, int64_t n1, int64_t n2, unsigned fla
   // hold the second differences along y (the base pixel 141.2 ms against 149.8 on four
   // taps and 124.7 from cells; 256^3 / nside 128 / 128 steps 7.9, 8.3 and 6.9), and
   // planes only where those find no room either.
-  f->four_taps =
-      64 * pvox > (int64_t)total_b / 5 * 2 || ((flags & SRT_FIELDS_NO_PAIRS) && n0 * n1 * n2 >= kFourTapVoxels);
-  if (!(flags & SRT_FIELDS_NO_PAIRS) && !f->four_taps && room_for("cells") && 64 * pvox <= field_budget(f) / 5 * 2) {
+  f->four_taps = 64 * pvox > (int64_t)total_b / 5 * 2 || forced_layout("pairs") ||
+                 ((flags & SRT_FIELDS_NO_PAIRS) && n0 * n1 * n2 >= kFourTapVoxels);
+  if (!(flags & SRT_FIELDS_NO_PAIRS) && !f->four_taps && !forced_layout("half") && !forced_layout("planes") &&
+      64 * pvox <= field_budget(f) / 5 * 2) {
     for (int c = 3; c >= 0; --c) {
       e = pool_alloc((void**)&f->cell[c], pvox * sizeof(float4), s);
       if (e != cudaSuccess) return cuda_error(e, c == 3 ? "allocate phi" : "allocate B");
@@ -349,7 +350,7 @@ cudaError_t lay_out(srt_fields* f, const float* src, int comps, int64_t k0, int6
 int finish_fields(srt_fields* f, unsigned flags, cudaStream_t s) {
   if ((flags & SRT_FIELDS_NO_PAIRS) || f->cell[0]) return SRT_OK;
   const int64_t pair_bytes = 4 * f->pn[0] * (f->pn[1] - 1) * f->pn[2] * (int64_t)sizeof(float2);
-  if (!room_for("half") || pair_bytes >= field_budget(f)) return SRT_OK;
+  if (forced_layout("planes") || pair_bytes >= field_budget(f)) return SRT_OK;
   const float* srcs[4] = {f->b[0], f->b[1], f->b[2], f->phi};
   cudaError_t e = cudaSuccess;
   for (int c = 0; c < 4 && e == cudaSuccess; ++c) {
