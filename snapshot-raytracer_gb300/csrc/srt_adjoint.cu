@@ -374,19 +374,18 @@ __global__ void __launch_bounds__(128, 2) segment_kernel_mixed(const AdjArgs A, 
   if (slot < A.count && !is_near(A, slot)) segment_ray(OneLane<LAYOUT>(), A, sgi, slot);
 }
 
+// Marked rays by their four lanes too: the other groups of the warp wait for them (a
+// launch of their own, 12 us a step after this one, was 3 us even with none marked).
 template <int LAYOUT>
 __global__ void __launch_bounds__(32, 12) segment_small_kernel(const AdjArgs A, int sgi) {
+  constexpr bool kFour = LAYOUT == kFourPlanes || LAYOUT == kFourPairs;  // all rays by the four taps
   const int lane = threadIdx.x;
   const int64_t slot = (int64_t)blockIdx.x * 8 + (lane >> 2);
-  if (slot < A.count && !is_near(A, slot))
+  if (slot >= A.count) return;
+  if (kFour || !is_near(A, slot))
     segment_ray(FourLanes<LAYOUT>{lane & 3, lane & ~3}, A, sgi, slot, (lane & 3) == 0);
-}
-
-// The marked rays of a segment, beside segment_small_kernel.
-__global__ void __launch_bounds__(128, 2) near_segment_kernel(const AdjArgs A, int sgi) {
-  for_near_rays(A, gridDim.x, gridDim.x, [&](int64_t slot, bool together) {
-    segment_ray(OneLane<kFourTaps>(), A, sgi, slot, true, together);
-  });
+  else
+    segment_ray(FourLanes<kFour ? LAYOUT : kFourTaps>{lane & 3, lane & ~3}, A, sgi, slot, (lane & 3) == 0);
 }
 
 // The four passes of a stage by one lane, FP32 accumulation: the interpolations,
@@ -719,16 +718,12 @@ void launch_ckpt(const AdjArgs& A, bool small, unsigned blocks, cudaStream_t s) 
   else
     ckpt_kernel_mixed<LAYOUT, MAPS><<<blocks, 128, 0, s>>>(A);
 }
-// Returns the number of kernels launched.
 template <int LAYOUT>
-int launch_segment(const AdjArgs& A, int sgi, bool small, unsigned blocks, unsigned near, cudaStream_t s) {
-  if (small) {
+void launch_segment(const AdjArgs& A, int sgi, bool small, unsigned blocks, unsigned near, cudaStream_t s) {
+  if (small)
     segment_small_kernel<LAYOUT><<<(unsigned)((A.count + 7) / 8), 32, 0, s>>>(A, sgi);
-    near_segment_kernel<<<near, 128, 0, s>>>(A, sgi);
-    return 2;
-  }
-  segment_kernel_mixed<LAYOUT><<<blocks + near, 128, 0, s>>>(A, sgi, near);
-  return 1;
+  else
+    segment_kernel_mixed<LAYOUT><<<blocks + near, 128, 0, s>>>(A, sgi, near);
 }
 
 inline void copy_extra(AccPaired<4>& to, const AccF32& from) { to.hot = from.hot; }
@@ -1255,13 +1250,12 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
           A.seg = seg.p;
           if (sgi >= kept_from) A.seg = (float*)seg.p + (int64_t)(sgi - kept_from) * C * kTapeStep * pix_count;
           if (sgi < kept_from)
-            with_forward_layout(
-                f, [&](auto l) { kernels += launch_segment<decltype(l)::value>(A, sgi, small, blocks, sms, s); });
+            with_forward_layout(f, [&](auto l) { launch_segment<decltype(l)::value>(A, sgi, small, blocks, sms, s); });
           if (determ)
             launch_sweep<AccFixed>(A, sgi, (float*)lam.p, ax, f, bgrad, small, blocks, s);
           else
             launch_sweep<AccF32>(A, sgi, (float*)lam.p, af, f, bgrad, small, blocks, s);
-          ++kernels;
+          kernels += sgi < kept_from ? 2 : 1;
         }
       }
       if (fp64) kernels += 2;
