@@ -974,7 +974,9 @@ struct DevBuf {
   }
   cudaError_t alloc(size_t bytes, cudaStream_t stream) {
     s = stream;
-    return scratch_alloc(&p, bytes, stream);
+    const cudaError_t e = scratch_alloc(&p, bytes, stream);
+    if (e != cudaSuccess) p = nullptr;
+    return e;
   }
 };
 
@@ -1032,7 +1034,8 @@ static bool small_adjoint(int64_t rays, int sms) { return rays <= (int64_t)sms *
 // Segments whose tape srt_vjp's forward writes at once, the last ones, instead of
 // a recompute (256^3 / nside 128 / 128 steps, C = 12: 5 of 11, 49.8 -> 46.9 ms): as many as
 // 4 GiB hold; none where device memory is short (an eighth of what is free beside the
-// outputs' staging).
+// outputs' staging), looked at above 256 MiB (where the query's microseconds no longer
+// count). The caller goes back to one segment where the allocation fails.
 static int kept_segments(int nseg, int64_t seg_bytes, int64_t out_bytes, int device) {
   const int64_t most = int64_t(4) << 30, few = int64_t(256) << 20;
   const int kept = (int)std::min<int64_t>(nseg, most / std::max<int64_t>(seg_bytes, 1));
@@ -1182,8 +1185,13 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
       }
       // per-step records of one segment: FP64 y, k1, k2, k3; MIXED the four stage inputs
       const int64_t seg_bytes = (int64_t)C * (fp64 ? state + 57 : kTapeStep) * pix_count * (int64_t)esz;
-      const int kept = fp64 || tape ? 0 : kept_segments(nseg, seg_bytes, 32 * pvox, f->device);
-      VJP_TRY(seg.alloc(std::max(kept, 1) * seg_bytes, s), "allocate segment records");
+      int kept = fp64 || tape ? 0 : kept_segments(nseg, seg_bytes, 32 * pvox, f->device);
+      cudaError_t seg_err = seg.alloc(std::max(kept, 1) * seg_bytes, s);
+      if (seg_err == cudaErrorMemoryAllocation && kept > 1) {  // one segment's records always do
+        kept = 1;
+        seg_err = seg.alloc(seg_bytes, s);
+      }
+      VJP_TRY(seg_err, "allocate segment records");
       if (determ) {  // fixed-point range flag
         VJP_TRY(ovf.alloc(sizeof(unsigned), s), "allocate overflow flag");
         VJP_TRY(cudaMemsetAsync(ovf.p, 0, sizeof(unsigned), s), "clear overflow flag");
