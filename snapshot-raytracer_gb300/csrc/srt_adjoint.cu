@@ -1048,6 +1048,9 @@ static int kept_segments(int nseg, int64_t seg_bytes, int64_t out_bytes, int dev
   return kept;
 }
 
+// Rays below which a gradient's scratch is not cut further.
+constexpr int64_t kLeastPart = 4096;
+
 // A forward trace's checkpoints (srt_forward_tape) for srt_vjp_tape.
 struct srt_tape {
   const srt_fields* fields = nullptr;
@@ -1163,38 +1166,54 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
         h2d += 6 * pix_count * (int64_t)sizeof(float);
       }
 
-      // ---- scratch: checkpoints, segment records, padded accumulators
-      const int state = fp64 ? 19 : kMixedState;
-      const size_t esz = fp64 ? sizeof(double) : sizeof(float);
-      if (!tape) VJP_TRY(ckpt.alloc((size_t)(nseg + 1) * state * pix_count * esz, s), "allocate checkpoints");
-      if (!tape && !fp64) {
-        VJP_TRY(near.alloc((pix_count + 1) * sizeof(int64_t), s), "allocate near rays");
-        VJP_TRY(cudaMemsetAsync(near.p, 0, sizeof(int64_t), s), "clear near rays");
-        VJP_TRY(bases.alloc((size_t)12 * pix_count * sizeof(float), s), "allocate ray bases");
-      }
+      // ---- padded accumulators
       // copies of the region around the observer (FP32 accumulation), where the
       // grid holds the region
       const bool hot = !fp64 && !determ && std::min(f->n[0], std::min(f->n[1], f->n[2])) >= kHotSide;
       const int64_t acc_entries = pvox + (hot ? (int64_t)kHotCopies * kHotSide * kHotSide * kHotSide : 0);
-      if (!fp64) VJP_TRY(lam.alloc((size_t)19 * pix_count * sizeof(float), s), "allocate state cotangents");
       for (int fld = 0; fld < 4; ++fld) {
         const bool want = (fld == 3) ? (dphi != nullptr) : (db_xyz != nullptr);
         if (!want) continue;
         VJP_TRY(gacc[fld].alloc(acc_entries * accsz, s), "allocate gradient accumulators");
         VJP_TRY(cudaMemsetAsync(gacc[fld].p, 0, acc_entries * accsz, s), "clear accumulators");
       }
-      // per-step records of one segment: FP64 y, k1, k2, k3; MIXED the four stage inputs
-      const int64_t seg_bytes = (int64_t)C * (fp64 ? state + 57 : kTapeStep) * pix_count * (int64_t)esz;
-      int kept = fp64 || tape ? 0 : kept_segments(nseg, seg_bytes, 32 * pvox, f->device);
-      cudaError_t seg_err = seg.alloc(std::max(kept, 1) * seg_bytes, s);
-      if (seg_err == cudaErrorMemoryAllocation && kept > 1) {  // one segment's records always do
-        kept = 1;
-        seg_err = seg.alloc(seg_bytes, s);
-      }
-      VJP_TRY(seg_err, "allocate segment records");
       if (determ) {  // fixed-point range flag
         VJP_TRY(ovf.alloc(sizeof(unsigned), s), "allocate overflow flag");
         VJP_TRY(cudaMemsetAsync(ovf.p, 0, sizeof(unsigned), s), "clear overflow flag");
+      }
+
+      // ---- the rays' scratch: checkpoints, the segments' records, cotangents; for
+      // half the rays at a time, or a quarter, ..., where it finds no room for all
+      const int state = fp64 ? 19 : kMixedState;
+      const size_t esz = fp64 ? sizeof(double) : sizeof(float);
+      int64_t part = pix_count, seg_bytes = 0;
+      int kept = 0;
+      for (;; part = (part + 1) / 2) {
+        // per-step records of one segment: FP64 y, k1, k2, k3; MIXED the four stage inputs
+        seg_bytes = (int64_t)C * (fp64 ? state + 57 : kTapeStep) * part * (int64_t)esz;
+        kept = fp64 || tape ? 0 : kept_segments(nseg, seg_bytes, 32 * pvox, f->device);
+        cudaError_t e = cudaSuccess;
+        const char* what = "";
+        const auto take = [&](DevBuf& b, size_t bytes, const char* name) {
+          if (e == cudaSuccess) e = b.alloc(bytes, s), what = name;
+        };
+        if (!tape) take(ckpt, (size_t)(nseg + 1) * state * part * esz, "allocate checkpoints");
+        if (!tape && !fp64) {
+          take(near, (part + 1) * sizeof(int64_t), "allocate near rays");
+          take(bases, (size_t)12 * part * sizeof(float), "allocate ray bases");
+        }
+        if (!fp64) take(lam, (size_t)19 * part * sizeof(float), "allocate state cotangents");
+        if (e == cudaSuccess) {
+          e = seg.alloc(std::max(kept, 1) * seg_bytes, s);
+          if (e == cudaErrorMemoryAllocation && kept > 1) {  // one segment's records always do
+            kept = 1;
+            e = seg.alloc(seg_bytes, s);
+          }
+          what = "allocate segment records";
+        }
+        if (e == cudaSuccess) break;
+        if (e != cudaErrorMemoryAllocation || tape || part <= kLeastPart) VJP_TRY(e, what);
+        for (DevBuf* b : {&ckpt, &near, &bases, &lam}) b->release();
       }
 
       AdjArgs A;
@@ -1202,8 +1221,6 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
       A.G = make_geom(f);
       A.nside = nside;
       A.pix_begin = pix_begin;
-      A.count = pix_count;
-      A.rays = ray_list;
       A.near = tape ? tape->near : (int64_t*)near.p;
       A.bases = tape ? tape->bases : (float*)bases.p;
       A.n_steps = n_steps;
@@ -1223,50 +1240,56 @@ static int vjp_impl(const srt_fields* fields, int64_t nside, int64_t pix_begin, 
       VJP_TRY(cudaEventCreate(&e0), "cudaEventCreate");
       VJP_TRY(cudaEventCreate(&e1), "cudaEventCreate");
       VJP_TRY(cudaEventRecord(e0, s), "cudaEventRecord");
-      const unsigned blocks = (unsigned)((pix_count + 127) / 128);
-      if (fp64) {
-        ckpt_kernel_fp64<<<blocks, 128, 0, s>>>(A);
-        if (determ) {
-          AccFixed ac[4];
-          make_acc<AccFixed, unsigned long long>(ac, A.acc);
-          for (int fld = 0; fld < 4; ++fld) ac[fld].ovf = (unsigned*)ovf.p;
-          reverse_kernel_fp64<AccFixed><<<blocks, 128, 0, s>>>(A, ac[0], ac[1], ac[2], ac[3]);
+      for (int64_t first = 0; first < pix_count; first += part) {
+        A.rays = ray_list + first;
+        A.count = std::min(part, pix_count - first);
+        A.seg = seg.p;
+        const unsigned blocks = (unsigned)((A.count + 127) / 128);
+        if (fp64) {
+          ckpt_kernel_fp64<<<blocks, 128, 0, s>>>(A);
+          if (determ) {
+            AccFixed ac[4];
+            make_acc<AccFixed, unsigned long long>(ac, A.acc);
+            for (int fld = 0; fld < 4; ++fld) ac[fld].ovf = (unsigned*)ovf.p;
+            reverse_kernel_fp64<AccFixed><<<blocks, 128, 0, s>>>(A, ac[0], ac[1], ac[2], ac[3]);
+          } else {
+            AccF64 ac[4];
+            make_acc<AccF64, double>(ac, A.acc);
+            reverse_kernel_fp64<AccF64><<<blocks, 128, 0, s>>>(A, ac[0], ac[1], ac[2], ac[3]);
+          }
+          kernels += 2;
         } else {
-          AccF64 ac[4];
-          make_acc<AccF64, double>(ac, A.acc);
-          reverse_kernel_fp64<AccF64><<<blocks, 128, 0, s>>>(A, ac[0], ac[1], ac[2], ac[3]);
-        }
-      } else {
-        // forward with checkpoints; then per segment, backwards: recompute
-        // the segment's tape, sweep it
-        const bool small = small_adjoint(pix_count, sms);
-        if (!tape) {  // else the checkpoints come from srt_forward_tape
-          with_forward_layout(f, [&](auto l) { launch_ckpt<decltype(l)::value, false>(A, small, blocks, s); });
-          near_ckpt_kernel<true><<<near_ckpt_blocks(blocks, sms), 128, 0, s>>>(A);
-        }
-        final_cotangent_kernel_mixed<<<blocks, 128, 0, s>>>(A, (float*)lam.p);
-        kernels += tape ? 1 : 3;
-        AccF32 af[4];
-        AccFixed ax[4];
-        make_acc<AccF32, float4>(af, A.acc);
-        for (int fld = 0; fld < 4; ++fld) af[fld].hot = hot ? pvox : 0;
-        make_acc<AccFixed, unsigned long long>(ax, A.acc);
-        for (int fld = 0; fld < 4; ++fld) ax[fld].ovf = (unsigned*)ovf.p;
-        const bool bgrad = db_xyz != nullptr;
-        const int kept_from = nseg - kept;  // segments from here on are on the tape already
-        for (int sgi = nseg - 1; sgi >= 0; --sgi) {
-          A.seg = seg.p;
-          if (sgi >= kept_from) A.seg = (float*)seg.p + (int64_t)(sgi - kept_from) * C * kTapeStep * pix_count;
-          if (sgi < kept_from)
-            with_forward_layout(f, [&](auto l) { launch_segment<decltype(l)::value>(A, sgi, small, blocks, sms, s); });
-          if (determ)
-            launch_sweep<AccFixed>(A, sgi, (float*)lam.p, ax, f, bgrad, small, blocks, s);
-          else
-            launch_sweep<AccF32>(A, sgi, (float*)lam.p, af, f, bgrad, small, blocks, s);
-          kernels += sgi < kept_from ? 2 : 1;
+          // forward with checkpoints; then per segment, backwards: recompute
+          // the segment's tape, sweep it
+          const bool small = small_adjoint(A.count, sms);
+          if (!tape) {  // else the checkpoints come from srt_forward_tape
+            VJP_TRY(cudaMemsetAsync(near.p, 0, sizeof(int64_t), s), "clear near rays");
+            with_forward_layout(f, [&](auto l) { launch_ckpt<decltype(l)::value, false>(A, small, blocks, s); });
+            near_ckpt_kernel<true><<<near_ckpt_blocks(blocks, sms), 128, 0, s>>>(A);
+          }
+          final_cotangent_kernel_mixed<<<blocks, 128, 0, s>>>(A, (float*)lam.p);
+          kernels += tape ? 1 : 3;
+          AccF32 af[4];
+          AccFixed ax[4];
+          make_acc<AccF32, float4>(af, A.acc);
+          for (int fld = 0; fld < 4; ++fld) af[fld].hot = hot ? pvox : 0;
+          make_acc<AccFixed, unsigned long long>(ax, A.acc);
+          for (int fld = 0; fld < 4; ++fld) ax[fld].ovf = (unsigned*)ovf.p;
+          const bool bgrad = db_xyz != nullptr;
+          const int kept_from = nseg - kept;  // segments from here on are on the tape already
+          for (int sgi = nseg - 1; sgi >= 0; --sgi) {
+            A.seg = seg.p;
+            if (sgi >= kept_from) A.seg = (float*)seg.p + (int64_t)(sgi - kept_from) * C * kTapeStep * A.count;
+            if (sgi < kept_from)
+              with_forward_layout(f, [&](auto l) { launch_segment<decltype(l)::value>(A, sgi, small, blocks, sms, s); });
+            if (determ)
+              launch_sweep<AccFixed>(A, sgi, (float*)lam.p, ax, f, bgrad, small, blocks, s);
+            else
+              launch_sweep<AccF32>(A, sgi, (float*)lam.p, af, f, bgrad, small, blocks, s);
+            kernels += sgi < kept_from ? 2 : 1;
+          }
         }
       }
-      if (fp64) kernels += 2;
       for (int fld = 0; fld < 4 && hot; ++fld) {
         if (!gacc[fld].p) continue;
         merge_hot_kernel<<<kHotSide * kHotSide * kHotSide / 256, 256, 0, s>>>((float4*)gacc[fld].p, pvox, A.G);

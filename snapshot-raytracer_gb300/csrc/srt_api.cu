@@ -82,6 +82,7 @@ cudaError_t alloc_from(int which, void** p, size_t bytes, cudaStream_t s) {
     cudaStreamSynchronize(s);
     trim_pools(dev);
     e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, s);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // returned; callers may go on with less
   }
   return e;
 }

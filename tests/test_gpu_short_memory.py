@@ -1,5 +1,5 @@
 """A gradient whose larger scratch finds no room takes less of it instead of failing:
-one segment's tape where several do not fit. The allocation is made to fail on the host
+one segment's tape where several do not fit, and half the rays at a time. The allocation is made to fail on the host
 (srt_debug_fail_alloc); the gradient keeps its bits (SRT_DETERMINISTIC)."""
 import numpy as np
 import pytest
@@ -26,17 +26,19 @@ def completes_without_failure_at(srt, call, allocations):
     return out
 
 
-@pytest.mark.parametrize("nside", [4, 32])
-def test_gradient_with_less_scratch(srt, nside):
+@pytest.mark.parametrize("nside,precision,less", [(4, "mixed", 1), (32, "mixed", 5), (20, "fp64", 2)])
+def test_gradient_with_less_scratch(srt, nside, precision, less):
     phi, b = srt_fields.gaussian_fields_np(24, seed=6)
     w = np.random.default_rng(7).standard_normal((6, 12 * nside * nside)).astype(np.float32)
     with srt.Fields(phi, b) as f:
-        call = lambda: f.vjp(nside, 20, w, ckpt_every=3, deterministic=True)[:2]  # 7 segments, all kept
+        # 7 segments, all kept
+        call = lambda: f.vjp(nside, 20, w, ckpt_every=3, deterministic=True, precision=precision)[:2]
         want = call()
-        # outputs 2, ray list 3, weights 1, checkpoints, marks, bases, cotangents,
-        # accumulators 4, segment records, range flag
+        # outputs 2, ray list 3, weights 1, accumulators 4, range flag; then what goes by
+        # rays: checkpoints, marks, bases, cotangents, segment records (FP64: the first
+        # and the last; 192 rays: only the records of several segments)
         done = completes_without_failure_at(srt, call, 16)
-        assert 14 in done
+        assert len([k for k in done if k >= 11]) >= less and all(k >= 11 for k in done), sorted(done)
         for g in done.values():
             for a, c in zip(g, want):
                 assert np.array_equal(a.view(np.uint32), c.view(np.uint32))
