@@ -131,7 +131,8 @@ int srt_device_count(void);
  * a kernel over the host link; other host inputs (or all, with
  * SRT_FIELDS_STAGED) by the copy engines; either way through a device slab, so
  * peak device memory is the laid-out fields plus one slab.
- * Where they take at most two fifths of the free device memory, and unless
+ * Where they take at most two fifths of the free and three tenths of the whole device
+ * memory, and unless
  * SRT_FIELDS_NO_PAIRS, the fields are stored as cells: per voxel and component
  * the value and its second differences along y, x and both (16 bytes; nothing
  * else is kept). Else as FP32 planes (4 bytes), beside them, when they fit,

@@ -1,5 +1,6 @@
 // srt_api.cu — the C ABI of libsrt (declared in include/srt.h): field upload
 // and layout, the forward trace, HEALPix helpers and error reporting.
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -278,9 +279,10 @@ constexpr int64_t kFourTapVoxels = int64_t(1) << 19;
 
 // Device arrays of the laid-out fields of an n0 x n1 x n2 grid (no contents):
 // cells (64 bytes per padded voxel for the four fields) unless
-// SRT_FIELDS_NO_PAIRS, where they take at most two fifths of the budget (so that
-// a gradient's accumulators, another 64 bytes, and its scratch fit beside them as
-// they do beside planes and half cells), else planes (16 bytes), which
+// SRT_FIELDS_NO_PAIRS, where they take at most two fifths of the budget and three
+// tenths of the device (some 1,115^3 on 288 GB: above, a gradient's accumulators,
+// another 64 bytes, the caller's fields and gradients, 32, and the checkpoints need the
+// 16 that cells take more), else planes (16 bytes), which
 // finish_fields may add half cells or row pairs to (another 32). The environment
 // variable SRT_FIELDS_LAYOUT makes a handle find no room for cells ("half") or for
 // anything but planes ("planes"), or be too large for cells ("pairs"), for tests.
@@ -317,7 +319,7 @@ int alloc_fields(srt_fields* f, int64_t n0, int64_t n1, int64_t n2, unsigned fla
   f->four_taps = 64 * pvox > (int64_t)total_b / 5 * 2 || forced_layout("pairs") ||
                  ((flags & SRT_FIELDS_NO_PAIRS) && n0 * n1 * n2 >= kFourTapVoxels);
   if (!(flags & SRT_FIELDS_NO_PAIRS) && !f->four_taps && !forced_layout("half") && !forced_layout("planes") &&
-      64 * pvox <= field_budget(f) / 5 * 2) {
+      64 * pvox <= std::min<int64_t>(field_budget(f) / 5 * 2, (int64_t)total_b / 10 * 3)) {
     for (int c = 3; c >= 0; --c) {
       e = pool_alloc((void**)&f->cell[c], pvox * sizeof(float4), s);
       if (e != cudaSuccess) return cuda_error(e, c == 3 ? "allocate phi" : "allocate B");
