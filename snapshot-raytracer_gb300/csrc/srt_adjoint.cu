@@ -279,9 +279,10 @@ __global__ void __launch_bounds__(128, 2) ckpt_kernel_mixed(const AdjArgs A) {
   ckpt_one<MAPS>(OneLane<LAYOUT>(), A, slot, true, guard_m[threadIdx.x]);
 }
 
-// Small ranges, forward and adjoint: four lanes per ray, one-warp blocks.
+// Small ranges, forward and adjoint: four lanes per ray, one-warp blocks (at most four
+// per SM, so the four taps get the registers that trace_small_kernel gives them).
 template <int LAYOUT, bool MAPS>
-__global__ void __launch_bounds__(32, 12) ckpt_small_kernel(const AdjArgs A) {
+__global__ void __launch_bounds__(32, by_four_taps(LAYOUT) ? 8 : 12) ckpt_small_kernel(const AdjArgs A) {
   const int lane = threadIdx.x;
   const int64_t slot = (int64_t)blockIdx.x * 8 + (lane >> 2);
   if (slot >= A.count) return;
@@ -377,8 +378,8 @@ __global__ void __launch_bounds__(128, 2) segment_kernel_mixed(const AdjArgs A, 
 // Marked rays by their four lanes too: the other groups of the warp wait for them (a
 // launch of their own, 12 us a step after this one, was 3 us even with none marked).
 template <int LAYOUT>
-__global__ void __launch_bounds__(32, 12) segment_small_kernel(const AdjArgs A, int sgi) {
-  constexpr bool kFour = LAYOUT == kFourPlanes || LAYOUT == kFourPairs;  // all rays by the four taps
+__global__ void __launch_bounds__(32, by_four_taps(LAYOUT) ? 8 : 12) segment_small_kernel(const AdjArgs A, int sgi) {
+  constexpr bool kFour = by_four_taps(LAYOUT);  // all rays are traced so
   const int lane = threadIdx.x;
   const int64_t slot = (int64_t)blockIdx.x * 8 + (lane >> 2);
   if (slot >= A.count) return;

@@ -307,12 +307,12 @@ int alloc_fields(srt_fields* f, int64_t n0, int64_t n1, int64_t n2, unsigned fla
   // 1.73 against 2.12, 256^3 / nside 128 / 128 steps 11.1 against 12.1, 512^3 / nside 256 /
   // 256 steps 83.6 against 90.3, 1024^3 / nside 512 / 512 steps 655 against 709, 2048^3 /
   // nside 2048 / 1024 steps 15.9 against 18.1 s; from row pairs, 1024^3 base pixel,
-  // 149.8 against 164.3 ms); a few thousand rays, four lanes each, take 8-10 % longer
-  // (96^3, 3,072 rays: 0.327 against 0.297 ms). They are taken by grids whose cells no
-  // handle would hold (some 1,230^3 on 288 GB) and by SRT_FIELDS_NO_PAIRS from 80^3
-  // voxels on, where a sky of nside n / 2 is as fast either way (80^3 / nside 40: 0.814
-  // and 0.816 ms); smaller grids, and those whose cells did not find room, keep the bits
-  // of a default handle. The latter read half cells, which
+  // 149.8 against 164.3 ms), and for a few thousand rays, four lanes each (128^3, 3,072
+  // rays: 0.260 against 0.300 ms). They are taken by grids whose cells no handle would
+  // hold (some 1,230^3 on 288 GB) and by SRT_FIELDS_NO_PAIRS from 80^3 voxels on, where
+  // a sky of nside n / 2 is as fast either way (80^3 / nside 40: 0.814 and 0.816 ms);
+  // smaller grids, and those whose cells did not find room, keep the bits of a default
+  // handle. The latter read half cells, which
   // hold the second differences along y (the base pixel 141.2 ms against 149.8 on four
   // taps and 124.7 from cells; 256^3 / nside 128 / 128 steps 7.9, 8.3 and 6.9), and
   // planes only where those find no room either.

@@ -274,9 +274,13 @@ __global__ void __launch_bounds__(128, (MODE == kMIXED || MODE >= kMIXED_HALF) ?
 // rays far apart by L1's lookups (a load of 32 rays' taps is 32 lines), so the
 // four interpolations run side by side (128^3, 48 steps: 768 rays 0.495 -> 0.287
 // ms, 3,072 rays 0.426 -> 0.303; from planes 1.06 -> 0.28 and 0.93 -> 0.30).
-// Prefetching the next step's lines made it 0.03 ms slower.
-template <int LAYOUT>
-__global__ void __launch_bounds__(32, 12) trace_small_kernel(const TraceArgs A) {
+// Prefetching the next step's lines made it 0.03 ms slower. BLOCKS: resident per SM;
+// the four taps hold 24 x weights where the second differences hold 14, and at 168
+// registers their loads wait for them (planes, 128^3, 48 steps: 768 rays 0.318 ms with
+// 12, 0.225 with 8; 6,912 rays 0.568 and 0.494; 12,288, which 8 do not hold at once,
+// 0.611 and 0.692; by second differences 0.281, 0.581 and 0.613).
+template <int LAYOUT, int BLOCKS>
+__global__ void __launch_bounds__(32, BLOCKS) trace_small_kernel(const TraceArgs A) {
   const int lane = threadIdx.x;
   int64_t o, ring;
   if (!ray_of_slot(A, (int64_t)blockIdx.x * 8 + (lane >> 2), &o, &ring)) return;
@@ -311,12 +315,18 @@ cudaError_t launch_trace(int mode, const TraceArgs& a, cudaStream_t s, int64_t* 
   if (mode == kFP64 && a.pix_count <= kWideFp64RaysPerSM * sms) return launch_wide_fp64(a, s, kernels);
   if (mode != kFP64 && mode != kREF16 && is_small(mode, a, sms)) {
     const unsigned small = (unsigned)((a.launch_rays + 7) / 8);
+    const bool few = a.pix_count <= 8 * 8 * (int64_t)sms;  // eight blocks of eight rays per SM
     switch (mode) {
-      case kMIXED_CELL: trace_small_kernel<kCells><<<small, 32, 0, s>>>(a); break;
-      case kMIXED_HALF: trace_small_kernel<kHalf><<<small, 32, 0, s>>>(a); break;
-      case kMIXED_FOUR: trace_small_kernel<kFourPlanes><<<small, 32, 0, s>>>(a); break;
-      case kMIXED_FOUR_PAIR: trace_small_kernel<kFourPairs><<<small, 32, 0, s>>>(a); break;
-      default: trace_small_kernel<kPlanes><<<small, 32, 0, s>>>(a);
+      case kMIXED_CELL: trace_small_kernel<kCells, 12><<<small, 32, 0, s>>>(a); break;
+      case kMIXED_HALF: trace_small_kernel<kHalf, 12><<<small, 32, 0, s>>>(a); break;
+      case kMIXED_FOUR:
+        if (few)
+          trace_small_kernel<kFourPlanes, 8><<<small, 32, 0, s>>>(a);
+        else
+          trace_small_kernel<kFourPlanes, 12><<<small, 32, 0, s>>>(a);
+        break;
+      case kMIXED_FOUR_PAIR: trace_small_kernel<kFourPairs, 8><<<small, 32, 0, s>>>(a); break;  // always few
+      default: trace_small_kernel<kPlanes, 12><<<small, 32, 0, s>>>(a);
     }
     if (kernels) ++*kernels;
     return cudaGetLastError();

@@ -588,8 +588,9 @@ SRT_HD auto cell_source(const FieldPtrs& F, const Geom& G, int f, int cx, int cy
 }
 
 // x and y weights of a layout's passes.
+constexpr SRT_HD bool by_four_taps(int layout) { return layout >= kFourTaps && layout <= kFourPairs; }
 template <int LAYOUT>
-using AxisWeights = typename std::conditional<(LAYOUT >= kFourTaps && LAYOUT <= kFourPairs), CRW<float>, CWD>::type;
+using AxisWeights = typename std::conditional<by_four_taps(LAYOUT), CRW<float>, CWD>::type;
 SRT_HD void axis_weights(float t, CRW<float>& c) { cr_weights_mixed(t, c); }
 SRT_HD void axis_weights(float t, CWD& c) { cr_weights_diff(t, c); }
 
