@@ -563,10 +563,16 @@ int srt_forward(const srt_fields* fields, int64_t nside, int64_t pix_begin, int6
         ++kernels;
       }
       float* phi = nullptr;
+      // where that finds no room, phi is read from the cells
       if (e == cudaSuccess && f->cell[0]) {
         e = pool_alloc((void**)&phi, pvox * sizeof(float), s);
-        if (e == cudaSuccess) e = launch_extract(f->values(3), 4, phi, pvox, s);
-        ++kernels;
+        if (e == cudaSuccess) {
+          e = launch_extract(f->values(3), 4, phi, pvox, s);
+          ++kernels;
+        } else if (e == cudaErrorMemoryAllocation) {
+          phi = nullptr;
+          e = cudaSuccess;
+        }
       }
       if (e != cudaSuccess) {
         for (int c = 0; c < 3; ++c) pool_free(h[c], s);

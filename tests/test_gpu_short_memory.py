@@ -42,3 +42,22 @@ def test_gradient_with_less_scratch(srt, nside, precision, less):
         for g in done.values():
             for a, c in zip(g, want):
                 assert np.array_equal(a.view(np.uint32), c.view(np.uint32))
+
+
+def test_ref16_without_its_phi_plane(srt):
+    """The phi plane that REF16 makes beside cells is only faster: without room for it the
+    maps are the same."""
+    phi, b = srt_fields.gaussian_fields_np((24, 21, 26), seed=6)
+    with srt.Fields(phi, b) as f:
+        assert f.nbytes == 64 * 27 * 24 * 29
+        want, _ = f.forward(4, 16, precision="ref16")
+    L = srt.lib()
+    with srt.Fields(phi, b) as f:
+        L.srt_debug_fail_alloc(3)  # after the three B planes
+        try:
+            got, _ = f.forward(4, 16, precision="ref16")
+        finally:
+            L.srt_debug_fail_alloc(-1)
+        again, _ = f.forward(4, 16, precision="ref16")
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    assert np.array_equal(again.view(np.uint32), want.view(np.uint32))
