@@ -11,7 +11,8 @@ __device__ const WideTables kWideTables = make_wide_tables();
 
 // The rays of a launch: those a MIXED trace listed (LIST; the count read on the
 // device, no host round trip, and nothing to do unless it lies in [min_count,
-// max_count]: one kernel per range of counts is queued), else the whole range.
+// max_count]: the kernels for short and for long lists are both queued), else the whole
+// range.
 template <bool LIST>
 __device__ __forceinline__ int64_t ray_count(const TraceArgs& A, int64_t min_count, int64_t max_count) {
   if (!LIST) return A.pix_count;
@@ -67,16 +68,9 @@ __device__ __forceinline__ void run_rounds(WideLane<R>& L, R* S, int st) {
   __syncwarp();
 }
 
-// One warp per ray, one-warp blocks; each traces rays blockIdx.x, + gridDim.x, ...
+// One warp per ray: rays blockIdx.x, + gridDim.x, ... of the n, by one-warp blocks.
 template <typename R, bool LIST>
-__global__ void __launch_bounds__(32, 16) wide_kernel(const TraceArgs A, int64_t min_count, int64_t max_count) {
-  // raw storage viewed as R: dd has a constructor, which a shared array of it
-  // would not run anyway
-  __shared__ float2 scratch[kWsSize];
-  __shared__ int cell[6];
-  R* S = reinterpret_cast<R*>(scratch);
-  const int64_t n = ray_count<LIST>(A, min_count, max_count);
-  if (blockIdx.x >= n) return;
+__device__ __forceinline__ void wide_trace(const TraceArgs& A, R* S, int* cell, int64_t n) {
   WideLane<R> L;
   L.start((int)threadIdx.x, kWideTables);
   L.constants(S);
@@ -109,6 +103,28 @@ __global__ void __launch_bounds__(32, 16) wide_kernel(const TraceArgs A, int64_t
     }
     write_maps(L, S, A, d, o);
   }
+}
+
+// A list of more than min_count - 1 rays: in FP64 up to fp64_max of them, else in
+// double-float (one launch for both: an empty one takes 4 us, 0.8 % of a 128^3 sky).
+__global__ void __launch_bounds__(32, 16) wide_list_kernel(const TraceArgs A, int64_t min_count, int64_t fp64_max) {
+  // raw storage viewed as double or dd: dd has a constructor, which a shared array
+  // of it would not run anyway
+  __shared__ float2 scratch[kWsSize];
+  __shared__ int cell[6];
+  const int64_t n = ray_count<true>(A, min_count, A.pix_count);
+  if (blockIdx.x >= n) return;
+  if (n <= fp64_max)
+    wide_trace<double, true>(A, reinterpret_cast<double*>(scratch), cell, n);
+  else
+    wide_trace<dd, true>(A, reinterpret_cast<dd*>(scratch), cell, n);
+}
+
+// The FP64 form of a range.
+__global__ void __launch_bounds__(32, 16) wide_range_kernel(const TraceArgs A) {
+  __shared__ double scratch[kWsSize];
+  __shared__ int cell[6];
+  wide_trace<double, false>(A, scratch, cell, A.pix_count);
 }
 
 // Five warps per ray in FP64 (FieldLane): the shortest way through a stage, for
@@ -197,12 +213,8 @@ cudaError_t launch_refine(const TraceArgs& a, cudaStream_t s, int64_t* kernels) 
   const int64_t warps = std::min(a.pix_count, kWideBlocksPerSM * (int64_t)sms);
   block_kernel<true><<<(unsigned)blocks, kBlockThreads, 0, s>>>(a, 1, block_max);
   if (kernels) ++*kernels;
-  if (a.pix_count > block_max && dd_min > block_max) {
-    wide_kernel<double, true><<<(unsigned)warps, 32, 0, s>>>(a, block_max + 1, dd_min);
-    if (kernels) ++*kernels;
-  }
-  if (a.pix_count > dd_min) {
-    wide_kernel<dd, true><<<(unsigned)warps, 32, 0, s>>>(a, dd_min + 1, a.pix_count);
+  if (a.pix_count > block_max) {
+    wide_list_kernel<<<(unsigned)warps, 32, 0, s>>>(a, block_max + 1, dd_min);
     if (kernels) ++*kernels;
   }
   return cudaGetLastError();
@@ -215,8 +227,7 @@ cudaError_t launch_wide_fp64(const TraceArgs& a, cudaStream_t s, int64_t* kernel
   if (a.pix_count <= kBlockRaysPerSM * (int64_t)sms)
     block_kernel<false><<<(unsigned)a.pix_count, kBlockThreads, 0, s>>>(a, 0, 0);
   else
-    wide_kernel<double, false>
-        <<<(unsigned)std::min(a.pix_count, kWideBlocksPerSM * (int64_t)sms), 32, 0, s>>>(a, 0, 0);
+    wide_range_kernel<<<(unsigned)std::min(a.pix_count, kWideBlocksPerSM * (int64_t)sms), 32, 0, s>>>(a);
   if (kernels) ++*kernels;
   return cudaGetLastError();
 }
